@@ -498,7 +498,7 @@ void enqueue_plain_step(stz_ctx* c, cudaEvent_t t0 = nullptr, cudaEvent_t t1 = n
   const int* gate = &f.ctl->solve_req;
   const double* ebar = f.ctl->eps_avg;
   if (t0) cudaEventRecord(t0, c->stream);
-  launch_rate_fp64(kp, f, c->stream);
+  launch_rate_fp64(kp, f, c->rx, c->stream);
   if (t1) cudaEventRecord(t1, c->stream);
   launch_athermal(kp, f, 0, c->stream);
   solve_plain(c, gate, ebar);
@@ -847,6 +847,18 @@ int stz::create_ctx(const stz_params* pin, stz_ctx** out, int units_per_block) {
   st = ref2d ? init_ref2d(c, &rng) : init_global3d(c, &rng);
   if (st) return fail(st);
   if (mixed) mixed_constants(c);
+  if (!mixed && !ref2d) {
+    std::vector<FxExp> tab(kFxExpCells);
+    fx_exp_table(tab.data());
+    if ((st = dalloc(&c->exptab, tab.size()))) return fail(st);
+    if ((st = upload(c->exptab, tab.data(), sizeof(FxExp) * tab.size(), c->stream))) return fail(st);
+    CK(cudaStreamSynchronize(c->stream));
+    rate_fx_constants(kp, &c->rx);
+    c->rx.tab = c->exptab;
+    int sms = 1;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device);
+    kp.rate_grid = std::min(kp.nblk, sms * rate_fx_blocks_per_sm(kp.bsites / kRateThreads));
+  }
 
   // control block
   Ctl& h = c->host_ctl;
@@ -896,7 +908,7 @@ extern "C" void stz_destroy(stz_ctx* c) {
   void* ptrs[] = {f.eps0, f.sig, f.sdev, f.dF, f.dF32, f.Q0, f.Q1, f.deps, f.dnorm, f.rtab64, f.mro, f.prev_deps, f.perm_soft, f.temp_soft,
                   f.tlast, f.amark, f.part, f.gsum, f.gticket, f.lsum, f.lbnd, f.psum, f.spec, f.ktab, f.log,
                   f.ctl, f.scratch, f.msum, c->err_dev, c->l2buf, c->qbuf, f.lam_site, f.mu_site,
-                  f.inh_tau0, f.inh_eeff, f.inh_last, f.inh_part};
+                  f.inh_tau0, f.inh_eeff, f.inh_last, f.inh_part, c->exptab};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->fft) {

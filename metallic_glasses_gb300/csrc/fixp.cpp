@@ -1,0 +1,87 @@
+// fixp.cpp -- host side of the fixed-point rates: the exponential's table and
+// the constants of a context.
+#include "fixp.cuh"
+
+#include <cmath>
+
+#include "stz_internal.h"
+
+namespace stz {
+namespace {
+
+typedef unsigned __int128 u128;
+
+// a b 2^-126 for a, b below 2^127
+u128 mul_q126(u128 a, u128 b) {
+  const uint64_t ah = (uint64_t)(a >> 64), al = (uint64_t)a, bh = (uint64_t)(b >> 64), bl = (uint64_t)b;
+  const u128 hh = (u128)ah * bh, hl = (u128)ah * bl, lh = (u128)al * bh, ll = (u128)al * bl;
+  const u128 mid = (ll >> 64) + (uint64_t)hl + (uint64_t)lh;
+  const u128 hi = hh + (hl >> 64) + (lh >> 64) + (mid >> 64);
+  return (hi << 2) | ((uint64_t)mid >> 62);
+}
+
+// 2^(2^-i) 2^126 for i = 1 .. 12 (repeated square roots of 2)
+const uint64_t kRoots[12][2] = {
+    {0x5a827999fcef3242, 0x2cbec4d9baa55f50}, {0x4c1bf828c6dc54b7, 0xa356918c17217b7b},
+    {0x45cae0f1f545eb73, 0x7df23143ac529e48}, {0x42d561b3e6243d8a, 0x62e4adc610aa60d9},
+    {0x4166c34c5615d0eb, 0x9f1523ada3290600}, {0x40b268f9de0183b9, 0xbdf2b293de8a6f7a},
+    {0x4058f6a7ecccd5b6, 0x1299ab8cdb737e90}, {0x402c6be96af2fb58, 0x4a6ac4fb04772551},
+    {0x4016321b687027a8, 0x7fc674a533cbd9e7}, {0x400b18178ba33b14, 0x1b486ff22688e804},
+    {0x40058bce410147e8, 0x4a2f2a71570c7978}, {0x4002c5d7bff71dae, 0x8e38c59c72a4e5ca}};
+// ln 2 2^126
+const uint64_t kLn2[2] = {0x2c5c85fdf473de6a, 0xf278ece600fcbdac};
+
+constexpr long double kLog2e = 1.44269504088896340735992468100189214L;
+
+int64_t fixed(long double v, int s) { return (int64_t)std::llrint(std::ldexp(v, s)); }
+
+}  // namespace
+
+void fx_exp_table(FxExp* t) {
+  const u128 ln2 = (u128)kLn2[0] << 64 | kLn2[1];
+  for (int j = 0; j < kFxExpCells; j++) {
+    u128 v = (u128)1 << 126;
+    const int h = 2 * j + 1;  // the 12 bits of (j + 1/2) / 2048
+    for (int i = 0; i < 12; i++)
+      if (h >> (11 - i) & 1) v = mul_q126(v, (u128)kRoots[i][0] << 64 | kRoots[i][1]);
+    t[j].t = (int64_t)((uint64_t)(v >> 64) + ((uint64_t)(v >> 63) & 1));
+    const Fx s = fx_split((int64_t)((mul_q126(v, ln2) + ((u128)1 << 64)) >> 65));
+    t[j].ph = s.h;
+    t[j].pl = s.l;
+  }
+}
+
+// The constants of a 3D FP64 context (see RateFx); on = 0 when they do not fit.
+void rate_fx_constants(const KParams& kp, RateFx* x) {
+  x->on = 0;
+  const long double kT = kp.kT, w = (long double)kp.V0 * 1e-18L * (long double)kJInEv / (2 * kT) * kLog2e;
+  const long double b = kLog2e / kT, c = std::log2((long double)kp.vt) + 1022;
+  long double M[STZ_MODES][5], smax = 0;
+  for (int m = 0; m < STZ_MODES; m++) {
+    const double* d = kp.modes[m];
+    M[m][0] = w * d[0];
+    M[m][1] = w * d[1];
+    for (int k = 2; k < 5; k++) M[m][k] = 2 * w * d[k + 1];
+    long double s = 0;
+    for (int k = 0; k < 5; k++) s += std::fabs(M[m][k]);
+    // the trace of a mode is rounding; a mode set with one is not represented
+    if (!(std::fabs((long double)d[0] + d[1] + d[2]) <= 1e-15L * (std::fabs(d[0]) + std::fabs(d[1]) + std::fabs(d[2]))))
+      return;
+    if (!(s <= 1e15L)) return;
+    smax = std::max(smax, s);
+  }
+  if (!(smax > 1e-15L) || !(b > 1e-15L && b < 1e15L) || !(c > 600 && c < 1440)) return;
+  const int L = (int)std::ceil(std::log2(smax)), LB = (int)std::ceil(std::log2(b));
+  x->sw = 51 + L;
+  x->sq = 51 + LB;
+  for (int m = 0; m < STZ_MODES; m++)
+    for (int k = 0; k < 5; k++) x->m[m][k] = fx_split(fixed(M[m][k], 61 - L));
+  x->nb = fx_split(fixed(-b, 61 - LB));
+  const uint64_t c53 = (uint64_t)fixed(c - 1024, 53) + ((uint64_t)1024 << 53);  // c 2^53 may exceed 2^63
+  x->c_hh = (int64_t)(c53 >> kFxRateShift);
+  x->c_mid = (int64_t)(c53 & ((1u << kFxRateShift) - 1)) << (32 - kFxRateShift);
+  x->neg = c53;
+  x->on = 1;
+}
+
+}  // namespace stz

@@ -493,6 +493,48 @@ __device__ __forceinline__ double g3_arg(const KParams& kp, const G3Arg& a, int 
   return x;
 }
 
+// A 3D site's stresses (with the uniform part ufx already in fixed point) and
+// barrier as the fixed-point operands of its 20 rate arguments; false when a
+// value does not fit (RateFx). Integer work only: no FP64 instruction per site.
+__device__ __forceinline__ bool g3_fx_site(const RateFx& rx, const Fields& f, long long N, const int64_t* ufx,
+                                           long long s, Fx* W, FxAcc* a0) {
+  bool ok = true;
+  int64_t g[6];
+#pragma unroll
+  for (int c = 0; c < 6; c++) g[c] = fx_from_f64<4>(f.sig[c * N + s], rx.sw, &ok) + ufx[c];
+  W[0] = fx_split(g[0] - g[2]);
+  W[1] = fx_split(g[1] - g[2]);
+  W[2] = fx_split(g[3]);
+  W[3] = fx_split(g[4]);
+  W[4] = fx_split(g[5]);
+  a0->hh = rx.c_hh;
+  a0->mid = rx.c_mid;
+  fx_mad(*a0, fx_split(fx_from_f64<2>(f.dF[s], rx.sq, &ok)), rx.nb);
+  const uint64_t y0 = (uint64_t)fx_value<kFxRateShift>(*a0);
+  return ok && y0 - kFxY0Min <= kFxY0Max - kFxY0Min;
+}
+// the uniform stress in the same fixed point
+__device__ __forceinline__ bool g3_fx_u(const RateFx& rx, const double* u, int64_t* ufx) {
+  bool ok = true;
+#pragma unroll
+  for (int c = 0; c < 6; c++) ufx[c] = fx_from_f64<4>(u[c], rx.sw, &ok);
+  return ok;
+}
+__device__ __forceinline__ uint64_t g3_fx_arg(const RateFx& rx, const Fx* W, const FxAcc& a0, int m) {
+  FxAcc a = a0;
+#pragma unroll
+  for (int c = 0; c < 5; c++) fx_mad(a, W[c], rx.m[m][c]);
+  return (uint64_t)fx_value<kFxRateShift>(a);
+}
+__device__ __forceinline__ FxExp fx_cell(const FxExp* t, int j) {  // one 16-byte load
+  const int4 v = *reinterpret_cast<const int4*>(t + j);
+  FxExp q;
+  q.t = (int64_t)((uint64_t)(uint32_t)v.x | ((uint64_t)(uint32_t)v.y << 32));
+  q.ph = v.z;
+  q.pl = v.w;
+  return q;
+}
+
 __device__ __forceinline__ unsigned long long gtimer() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -561,21 +603,34 @@ __device__ double block_incl_scan(double v, double* sh_inc) {
 }
 
 // Sum of STZ_MODES per-thread accumulators over the block, written to
-// part[m * nblk + b] by threads 0..STZ_MODES-1 in a fixed order.
-__device__ void block_mode_sums(const double* acc, double* part, int nblk, int b) {
+// part[m * nblk + b] by threads 0..STZ_MODES-1 in a fixed order. Within a warp
+// the lanes halve the modes they hold at every step (20, 10, 5, 3, 2, 1): 21
+// FP64 additions per warp instead of the 100 of one butterfly per mode, at 19
+// SM clocks each a fifth of a pass over one site per thread.
+__device__ __forceinline__ void block_mode_sums(const double* acc, double* part, int nblk, int b) {
+  static_assert(STZ_MODES == 20, "the halving below is written for 20 modes");
   __shared__ double red[TH / 32][STZ_MODES];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const bool u4 = lane & 16, u3 = lane & 8, u2 = lane & 4, u1 = lane & 2, u0 = lane & 1;
+  double a[10], c[5], d[3];
 #pragma unroll
-  for (int m = 0; m < STZ_MODES; m++) {
-    double v = acc[m];
+  for (int i = 0; i < 10; i++)
+    a[i] = (u4 ? acc[i + 10] : acc[i]) + __shfl_xor_sync(FULL, u4 ? acc[i] : acc[i + 10], 16);
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(FULL, v, off);
-    if (lane == 0) red[w][m] = v;
-  }
+  for (int i = 0; i < 5; i++) c[i] = (u3 ? a[i + 5] : a[i]) + __shfl_xor_sync(FULL, u3 ? a[i] : a[i + 5], 8);
+#pragma unroll
+  for (int i = 0; i < 2; i++) d[i] = (u2 ? c[i + 3] : c[i]) + __shfl_xor_sync(FULL, u2 ? c[i] : c[i + 3], 4);
+  d[2] = c[2] + __shfl_xor_sync(FULL, c[2], 4);  // kept by the lanes with u2 clear
+  const double e0 = (u1 ? d[1] : d[0]) + __shfl_xor_sync(FULL, u1 ? d[0] : d[1], 2);
+  const double e1 = d[2] + __shfl_xor_sync(FULL, d[2], 2);
+  const double t = (u0 ? e1 : e0) + __shfl_xor_sync(FULL, u0 ? e0 : e1, 1);
+  // lane bits 2, 1, 0: 000 -> 0, 010 -> 1, 001 -> 2, 100 -> 3, 110 -> 4 of the lane's five modes
+  const int k = (u2 ? 3 : 0) + (u1 ? 1 : 0) + (u0 ? 2 : 0);
+  if (!u0 || (!u1 && !u2)) red[w][(u4 ? 10 : 0) + (u3 ? 5 : 0) + k] = t;
   __syncthreads();
   if (threadIdx.x < STZ_MODES) {
     double s = 0;
-    for (int k = 0; k < TH / 32; k++) s += red[k][threadIdx.x];
+    for (int q = 0; q < TH / 32; q++) s += red[q][threadIdx.x];
     part[(long long)threadIdx.x * nblk + b] = s;
   }
 }
@@ -691,20 +746,22 @@ __device__ bool group_reduce(const KParams& kp, const Fields& f, int b) {
 // ----------------------------------------------------------- selection
 // Rate of (site, mode) exactly as the main pass computed it (raw units).
 template <int MODEL>
-__device__ __forceinline__ double site_rate(const KParams& kp, const Fields& f, const double* u, double totime,
-                                            long long s, int m) {
+__device__ __forceinline__ double site_rate(const KParams& kp, const Fields& f, const RateFx& rx, const double* u,
+                                            double totime, long long s, int m) {
   if (MODEL == 0) {
     const R2Site d = r2_load(kp, f, u, totime, s);
     return kp.vt * exp_tang(r2_arg(kp, f, d, s, m));
   } else if (MODEL == 1) {
+    int64_t ufx[6];
+    Fx W[5];
+    FxAcc a0;
+    if (rx.on && g3_fx_u(rx, u, ufx) && g3_fx_site(rx, f, kp.N, ufx, s, W, &a0)) {
+      const uint64_t Y = g3_fx_arg(rx, W, a0, m);
+      return fx_double(fx_exp2_bits(Y, fx_cell(rx.tab, fx_exp_cell(Y))));
+    }
     double sg[6];
     g3_load(kp, f, u, s, sg);
     return kp.vt * exp_tang(g3_arg(kp, g3_arg_site(kp, sg, f.dF[s]), m));
-  } else {
-    float sv[5];
-    mx_site(kp, f, s, sv);
-    const float a = (kp.q_ref - f.dF32[s]) * kp.a_scale;
-    return (double)ex2_approx(mx_x(kp, sv, a, m));
   }
 }
 
@@ -732,8 +789,8 @@ __device__ double site_Q(const KParams& kp, const Fields& f, const double* u, do
 // scan the caller left in sh_inc; level 2: the rates of the chosen mode in the
 // chosen block, recomputed into registers and scanned. Whole block.
 template <int MODEL>
-__device__ void search_event(const KParams& kp, const Fields& f, const double* u, double totime, double T,
-                             const double* sh_inc, long long* site_out, int* mode_out, double* margin_out) {
+__device__ void search_event(const KParams& kp, const Fields& f, const RateFx& rx, const double* u, double totime,
+                             double T, const double* sh_inc, long long* site_out, int* mode_out, double* margin_out) {
   __shared__ double sh_inc2[TH];
   __shared__ long long sh_p;
   __shared__ double sh_cb;
@@ -817,7 +874,7 @@ __device__ void search_event(const KParams& kp, const Fields& f, const double* u
 #pragma unroll
   for (int k = 0; k < kMaxPer; k++) {
     const long long s = a0 + k;
-    rr[k] = (k < per && s < s1) ? site_rate<MODEL>(kp, f, u, totime, s, m) : 0.0;
+    rr[k] = (k < per && s < s1) ? site_rate<MODEL>(kp, f, rx, u, totime, s, m) : 0.0;
     loc += rr[k];
   }
   const double I2 = block_incl_scan(loc, sh_inc2);
@@ -910,7 +967,7 @@ __device__ __forceinline__ void ctl_copy(Ctl* dst, const Ctl* src) {
 // Last block of a rate kernel: total rate, step kind, dice, event search and
 // commit. MODEL 0 REF2D FP64, 1 GLOBAL3D FP64.
 template <int MODEL>
-__device__ void finish_step(const KParams& kp, const Fields& f) {
+__device__ __noinline__ void finish_step(const KParams& kp, const Fields& f, const RateFx& rx) {
   __shared__ Ctl sc;
   __shared__ double sh_inc[TH];
   __shared__ int sh_kind;
@@ -976,7 +1033,7 @@ __device__ void finish_step(const KParams& kp, const Fields& f) {
   const unsigned long long t_dec = gtimer();
   const int kind = sh_kind;
   if (kind == kThermal) {
-    search_event<MODEL>(kp, f, sh_u, sh_tot, sh_T, sh_inc, &sh_site, &sh_mode, &sh_margin);
+    search_event<MODEL>(kp, f, rx, sh_u, sh_tot, sh_T, sh_inc, &sh_site, &sh_mode, &sh_margin);
     __syncthreads();
   }
   const unsigned long long t_search = gtimer();
@@ -1020,16 +1077,12 @@ __device__ void finish_step(const KParams& kp, const Fields& f) {
 }
 
 // ------------------------------------------------------------ FP64 rates
+// The rates of the sites s0 .. s1-1 of chunk b by the FP64 chain: their
+// per-mode sums to part, the number of negative barriers returned (every
+// thread of the block calls it).
 template <int MODEL>
-__global__ void __launch_bounds__(TH) k_rate64(KParams kp, Fields f) {
-  Ctl* ctl = f.ctl;
-  if (ctl->halt) return;
-  const int b = blockIdx.x;
-  const long long s0 = (long long)b * kp.bsites;
-  const long long s1 = min(s0 + (long long)kp.bsites, kp.N);
-  double u[6];
-  for (int c = 0; c < 6; c++) u[c] = ctl->u[c];
-  const double totime = ctl->totime;
+__device__ __noinline__ unsigned rate_chunk_fp64(const KParams& kp, const Fields& f, const double* u, double totime,
+                                                 int b, long long s0, long long s1) {
   double acc[STZ_MODES];
 #pragma unroll
   for (int m = 0; m < STZ_MODES; m++) acc[m] = 0;
@@ -1056,11 +1109,140 @@ __global__ void __launch_bounds__(TH) k_rate64(KParams kp, Fields f) {
     }
   }
   block_mode_sums(acc, f.part, kp.nblk, b);
+  return neg;
+}
+
+// What every chunk ends with: its count of negative barriers, the group's and
+// the grid's last-block tests. True in the block that finishes the step.
+__device__ __forceinline__ bool chunk_done(const KParams& kp, const Fields& f, int b, unsigned neg) {
   const unsigned nb = block_sum_u(neg);
-  if (threadIdx.x == 0 && nb) atomicAdd(&ctl->neg_count, (unsigned long long)nb);
-  if (!group_reduce(kp, f, b)) return;
-  if (!last_block(ctl, kp.ngroups)) return;
-  finish_step<MODEL>(kp, f);
+  if (threadIdx.x == 0 && nb) atomicAdd(&f.ctl->neg_count, (unsigned long long)nb);
+  return group_reduce(kp, f, b) && last_block(f.ctl, kp.ngroups);
+}
+
+template <int MODEL>
+__global__ void __launch_bounds__(TH) k_rate64(KParams kp, Fields f, RateFx rx) {
+  Ctl* ctl = f.ctl;
+  if (ctl->halt) return;
+  const int b = blockIdx.x;
+  const long long s0 = (long long)b * kp.bsites;
+  const long long s1 = min(s0 + (long long)kp.bsites, kp.N);
+  double u[6];
+  for (int c = 0; c < 6; c++) u[c] = ctl->u[c];
+  const unsigned neg = rate_chunk_fp64<MODEL>(kp, f, u, ctl->totime, b, s0, s1);
+  if (chunk_done(kp, f, b, neg)) finish_step<MODEL>(kp, f, rx);
+}
+
+// Sums of N values per lane over the warp, the lanes halving the values they
+// hold at every step (N + 2 or so FP64 additions per lane instead of 5 N).
+// Returns this lane's sum; *idx is the value it belongs to, or -1.
+template <int N, int OFF>
+struct WarpSums {
+  static __device__ __forceinline__ double run(const double* v, int lane, int* idx) {
+    constexpr int H = (N + 1) / 2;
+    const bool up = lane & OFF;
+    double w[H];
+#pragma unroll
+    for (int i = 0; i < H; i++) {
+      if (i + H < N) w[i] = (up ? v[i + H] : v[i]) + __shfl_xor_sync(FULL, up ? v[i] : v[i + H], OFF);
+      else w[i] = v[i] + __shfl_xor_sync(FULL, v[i], OFF);  // both halves have it; the lower keeps it
+    }
+    const double t = WarpSums<H, OFF / 2>::run(w, lane, idx);
+    if (up) *idx = *idx >= 0 && *idx + H < N ? *idx + H : -1;
+    return t;
+  }
+};
+template <int N>
+struct WarpSums<N, 0> {
+  static __device__ __forceinline__ double run(const double* v, int, int* idx) {
+    *idx = 0;
+    return v[0];
+  }
+};
+
+// The 3D rates in 64-bit fixed point (RateFx; fixp.cuh): the FP64 pipe, which
+// bounded this pass (26 FP64 operations per site and mode, 85% busy), is left
+// with the per-warp sums. A thread holds the operands of its Q sites and walks
+// the modes, whose constants are kernel parameters; the Q rates of a mode are
+// added as integers before the one conversion to FP64, and G modes share a
+// halving reduction. Blocks run through the chunks b, b + gridDim.x, ... so that
+// the 32 KB exponential table is copied to shared memory once per resident
+// block. A chunk with a value outside the fixed point's range (or a NaN) goes
+// through the FP64 chain as a whole. Measured against the FP64 chain, kernel
+// with selection: 294 -> 66 us at 64^3, 1800 -> 277 us at 128^3 (100
+// instructions per site and mode; integer dispatch bounds it now). Blocks per
+// SM: at four sites per thread 128 registers (two blocks) and 80 (three, 156
+// bytes of spills) measured the same, 277 and 275 us.
+template <int Q>
+__global__ void __launch_bounds__(TH, Q == 4 ? 2 : 3) k_rate64_fx(KParams kp, Fields f, RateFx rx) {
+  constexpr int G = Q == 1 ? 10 : (Q == 2 ? 5 : 4);  // modes per reduction
+  __shared__ FxExp tab[kFxExpCells];
+  __shared__ int64_t sh_u[6];
+  __shared__ int sh_uok;
+  __shared__ double red[TH / 32][STZ_MODES];
+  Ctl* ctl = f.ctl;
+  if (ctl->halt) return;
+  {
+    const int4* src = reinterpret_cast<const int4*>(rx.tab);
+    int4* dst = reinterpret_cast<int4*>(tab);
+#pragma unroll
+    for (int i = 0; i < kFxExpCells / TH; i++) dst[i * TH + threadIdx.x] = __ldg(src + i * TH + threadIdx.x);
+  }
+  if (threadIdx.x == 0) sh_uok = g3_fx_u(rx, ctl->u, sh_u);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int b = blockIdx.x; b < kp.nblk; b += gridDim.x) {
+    const long long s0 = (long long)b * kp.bsites;
+    const long long s1 = min(s0 + (long long)kp.bsites, kp.N);
+    bool ok = sh_uok;
+    unsigned neg = 0;
+    Fx W[Q][5];
+    FxAcc a0[Q];
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      const long long s = s0 + threadIdx.x + q * TH;
+      if (s < s1) {
+        ok &= g3_fx_site(rx, f, kp.N, sh_u, s, W[q], &a0[q]);
+      } else {
+        // no site: the smallest representable rate, 2^-1021
+        for (int c = 0; c < 5; c++) W[q][c] = Fx{0, 0};
+        a0[q] = FxAcc{(int64_t)1 << (53 - kFxRateShift), 0};
+      }
+    }
+    if (!__syncthreads_or(!ok)) {
+#pragma unroll 1
+      for (int g = 0; g < STZ_MODES; g += G) {
+        double v[G];
+#pragma unroll
+        for (int i = 0; i < G; i++) {
+          uint64_t Y[Q];
+          FxExp c[Q];
+#pragma unroll
+          for (int q = 0; q < Q; q++) {
+            Y[q] = g3_fx_arg(rx, W[q], a0[q], g + i);
+            neg += Y[q] > rx.neg;
+            c[q] = fx_cell(tab, fx_exp_cell(Y[q]));
+          }
+          v[i] = fx_double(fx_exp2_sum_bits<Q>(Y, c));
+        }
+        int idx;
+        const double t = WarpSums<G, 16>::run(v, lane, &idx);
+        if (idx >= 0) red[w][g + idx] = t;
+      }
+      __syncthreads();
+      if (threadIdx.x < STZ_MODES) {
+        double t = 0;
+#pragma unroll
+        for (int k = 0; k < TH / 32; k++) t += red[k][threadIdx.x];
+        f.part[(long long)threadIdx.x * kp.nblk + b] = t;
+      }
+    } else {
+      double u[6];
+      for (int c = 0; c < 6; c++) u[c] = ctl->u[c];
+      neg = rate_chunk_fp64<1>(kp, f, u, ctl->totime, b, s0, s1);
+    }
+    if (chunk_done(kp, f, b, neg)) finish_step<1>(kp, f, rx);
+  }
 }
 
 // ------------------------------------------------------------ athermal
@@ -2766,9 +2948,22 @@ __global__ void k_hold(unsigned long long ns) {
 
 }  // namespace
 
-void launch_rate_fp64(const KParams& kp, const Fields& f, cudaStream_t st) {
-  if (kp.model == STZ_MODEL_REF2D) k_rate64<0><<<kp.nblk, TH, 0, st>>>(kp, f);
-  else k_rate64<1><<<kp.nblk, TH, 0, st>>>(kp, f);
+int rate_fx_blocks_per_sm(int spt) {
+  int occ = 0;
+  const void* k = spt == 1 ? (const void*)k_rate64_fx<1> : spt == 2 ? (const void*)k_rate64_fx<2> : (const void*)k_rate64_fx<4>;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, TH, 0) != cudaSuccess || occ < 1) {
+    (void)cudaGetLastError();
+    occ = 1;
+  }
+  return occ;
+}
+
+void launch_rate_fp64(const KParams& kp, const Fields& f, const RateFx& rx, cudaStream_t st) {
+  if (kp.model == STZ_MODEL_REF2D) k_rate64<0><<<kp.nblk, TH, 0, st>>>(kp, f, rx);
+  else if (!rx.on) k_rate64<1><<<kp.nblk, TH, 0, st>>>(kp, f, rx);
+  else if (kp.bsites == TH) k_rate64_fx<1><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
+  else if (kp.bsites == 2 * TH) k_rate64_fx<2><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
+  else k_rate64_fx<4><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
 }
 
 // The staged lines of the mixed-form main kernels are dynamic shared memory,

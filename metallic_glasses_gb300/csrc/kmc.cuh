@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "fixp.cuh"
 #include "stz_internal.h"
 
 namespace stz {
@@ -12,7 +13,10 @@ constexpr int kGroup = 32;     // blocks per group in the two-level rate sums
 
 // Rate kernel of the FP64 forms (ActEnergy + KMC rates + selection/commit in
 // the last block). model: STZ_MODEL_REF2D or STZ_MODEL_GLOBAL3D.
-void launch_rate_fp64(const KParams& kp, const Fields& f, cudaStream_t st);
+void launch_rate_fp64(const KParams& kp, const Fields& f, const RateFx& rx, cudaStream_t st);
+// Resident blocks per SM of the fixed-point rate kernel (occupancy query) at
+// spt (1, 2 or 4) sites per thread.
+int rate_fx_blocks_per_sm(int spt);
 // Mixed form: incremental stress update + rates + selection/commit.
 // update_only: apply the pending transformation and uniform change, nothing else.
 void launch_mixed(const KParams& kp, const Fields& f, int update_only, cudaStream_t st);

@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "../../include/stz_api.h"
+#include "fixp.cuh"
 #include "mt19937.cuh"
 
 #ifdef __CUDACC__
@@ -151,6 +152,7 @@ struct KParams {
   long long N, Nk;
   int nblk, bsites;          // rate kernel: blocks and sites per block
   int ngroups;               // groups of kGroup blocks
+  int rate_grid;             // resident blocks of the fixed-point rate kernel (at most nblk)
   int mx_c1, mx_units;       // mixed form: d1 chunks per d0, units (kt0 * mx_c1)
   unsigned c1_magic;         // ceil(2^32 / mx_c1), for the division of unit indices
   int adv_q2, adv_r2;        // kRateThreads sites = adv_q2 rows of n2 plus adv_r2 sites
@@ -193,6 +195,9 @@ struct ModeSet {
   float mdev_raw[STZ_MODES][5];
 };
 
+// The constants of a 3D FP64 context's fixed-point rates (fixp.cpp).
+void rate_fx_constants(const KParams& kp, RateFx* x);
+
 struct BatchDesc {
   KParams kp;
   Fields f;
@@ -211,6 +216,8 @@ struct stz_ctx {
   stz_params p{};
   stz::KParams kp{};
   stz::Fields f{};
+  stz::RateFx rx{};                  // 3D FP64 forms: constants of the fixed-point rates
+  stz::FxExp* exptab = nullptr;      // its exponential table on the device
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;

@@ -433,3 +433,43 @@ def test_inhomogeneous_medium_steps(engine_lib):
     assert sc2["status"] == 0 and sc2["kstep"] == 30
     assert np.all(np.isfinite(sc2["stress"]))
     assert not np.array_equal(ev0["site"], ev2["site"])
+
+
+# ------------------------------------------------- fixed-point 3D rates
+@pytest.mark.parametrize("shape,barrier", [
+    ((2, 2, 2), None), ((6, 9, 12), None), ((16, 16, 16), None),   # one chunk and less, a ragged last chunk
+    ((64, 72, 108), None), ((96, 96, 96), None),                  # two and four sites per thread
+    ((6, 9, 12), 40.0), ((6, 9, 12), 1e4), ((6, 9, 12), -0.5),    # barriers outside the fixed point's range, below zero
+])
+def test_fixed_point_rates_match_fp64_rates(engine_lib, shape, barrier):
+    """The total rate of a step against the sum over all sites and modes of
+    vt exp(-Q/kT) in extended precision, Q read back from the engine (its FP64
+    chain, which the fixed-point pass does not use), under a stress field of
+    about 1 GPa. Q carries a few roundings of 2^-53 of a few eV, 3e-14 of a
+    rate at 455 K (kT = 0.039 eV); the bar is 1e-13. A barrier out of range
+    sends its chunk through the FP64 chain; a negative one is an avalanche."""
+    p = configs.stress32(n=shape[2])
+    p.n[0], p.n[1], p.n[2] = shape
+    eng = api.Engine(p)
+    rng = np.random.default_rng(7)
+    for c in range(6):
+        eng.set_field(api.FIELD_EPS0, c, rng.standard_normal(eng.N) * 0.006)
+    if barrier is not None:
+        dF = eng.field(api.FIELD_DF)
+        dF[eng.N // 2] = barrier
+        eng.set_field(api.FIELD_DF, 0, dF)
+    eng.solve()
+    kT = p.temperature * 1.380658e-23 / 1.60217733e-19
+    R = np.longdouble(0)
+    neg = 0
+    for m in range(20):
+        Q = eng.field(api.FIELD_Q, m)
+        neg += int((Q < 0).sum())
+        R += np.exp(-Q.astype(np.longdouble) / np.longdouble(kT)).sum()
+    R *= np.longdouble(p.voxel_volume * p.trial_frequency)
+    eng.run(max_steps=1)
+    ev, sc = eng.events(), eng.scalars()
+    assert (sc["astep"] == 1) == (neg > 0)
+    if neg == 0:
+        assert abs(ev["total_rate"][0] / R - 1) < 1e-13
+    eng.close()
