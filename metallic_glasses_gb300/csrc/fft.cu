@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "fft.cuh"
+#include "fftx.cuh"
 
 namespace stz {
 namespace {
@@ -721,7 +722,8 @@ __global__ void __launch_bounds__(256) k_c2r_dev(const typename VT<T>::V* __rest
                                                  const typename VT<T>::V* __restrict__ tw_h,
                                                  const typename VT<T>::V* __restrict__ tw_p, double invN,
                                                  float* __restrict__ sdev, const double* __restrict__ uadd,
-                                                 double* __restrict__ err, const int* gate) {
+                                                 double* __restrict__ err, const int* gate,
+                                                 const double* __restrict__ ebar, double lambda, double mu) {
   using V = typename VT<T>::V;
   if (gate && *gate == 0) return;
   constexpr int NC = 6;
@@ -768,6 +770,9 @@ __global__ void __launch_bounds__(256) k_c2r_dev(const typename VT<T>::V* __rest
   using A = typename ErrAcc<T>::A;
   T ua[NC];
   for (int c = 0; c < NC; c++) ua[c] = uadd ? from_f64<T>(uadd[c]) : (T)0.0;
+  if (ebar)
+    for (int c = 0; c < NC; c++)
+      ua[c] = ua[c] + from_f64<T>((c < 3 ? lambda * (ebar[0] + ebar[1] + ebar[2]) : 0.0) + 2.0 * mu * ebar[c]);
   A mxa = 0, ssa = 0, sra = 0, mra = 0;
   for (int idx = threadIdx.x, q = 0; idx < L * n2; idx += blockDim.x, q++) {
     const int l = idx / n2, i = idx - l * n2;
@@ -875,10 +880,12 @@ Sched make_sched_rev(int n) {
   return s;
 }
 
-int upload_twiddles(int n, int count, double2** d64, float2** d32, float4** dpair) {
+int upload_twiddles(int n, int count, double2** d64, float2** d32, float4** dpair, FxTwiddle** dfx) {
   std::vector<double2> h(count > 0 ? count : 1);
   std::vector<float2> hf(h.size());
   std::vector<float4> hp(h.size());
+  std::vector<FxTwiddle> hx(h.size());
+  fx_twiddles(n, count, hx.data());
   for (int k = 0; k < count; k++) {
     double ang = -2.0 * M_PI * (double)k / (double)n;
     h[k] = make_double2(std::cos(ang), std::sin(ang));
@@ -889,6 +896,8 @@ int upload_twiddles(int n, int count, double2** d64, float2** d32, float4** dpai
   if (cudaMalloc(d64, sizeof(double2) * h.size()) != cudaSuccess) return STZ_ERR_NOMEM;
   if (cudaMalloc(d32, sizeof(float2) * h.size()) != cudaSuccess) return STZ_ERR_NOMEM;
   if (cudaMalloc(dpair, sizeof(float4) * h.size()) != cudaSuccess) return STZ_ERR_NOMEM;
+  if (cudaMalloc(dfx, sizeof(FxTwiddle) * h.size()) != cudaSuccess) return STZ_ERR_NOMEM;
+  cudaMemcpy(*dfx, hx.data(), sizeof(FxTwiddle) * h.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(*d64, h.data(), sizeof(double2) * h.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(*d32, hf.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(*dpair, hp.data(), sizeof(float4) * h.size(), cudaMemcpyHostToDevice);
@@ -955,6 +964,25 @@ struct Tw<dfl> {
   static const df2* post(const FFTPlan& p) { return reinterpret_cast<const df2*>(p.tw_pd); }
 };
 
+// The C2R pass of a kOutDev32 solve; factor multiplies its sums (1 / N). With
+// ebar, the uniform stress C:ebar is added (a spectrum without its mean part).
+template <typename T>
+void c2r_dev(const FFTPlan& p, const SolveArgs& a, double factor, const double* ebar, cudaStream_t st,
+             int64_t* launches) {
+  using V = typename VT<T>::V;
+  const long long rows = (long long)p.n0 * p.n1;
+  // the deviatoric epilogue stages the block's six real rows: a row tile of
+  // its own, kept within 72 KB of shared memory so that several blocks share
+  // an SM (the tuned tile is timed without this staging)
+  int L = p.L_x;
+  auto dev_smem = [&](int l) { return 2 * (size_t)p.nc * l * (p.h + 2) * sizeof(V); };
+  while (L > 1 && dev_smem(L) > 72 * 1024) L /= 2;
+  k_c2r_dev<T><<<(unsigned)((rows + L - 1) / L), 256, dev_smem(L), st>>>(
+      reinterpret_cast<const V*>(a.spec), p.n2, p.h, p.nh, rows, p.N, p.Nk, L, p.sh, Tw<T>::h(p), Tw<T>::post(p), factor,
+      a.sdev, a.uadd, a.err, a.gate, ebar, a.lambda, a.mu);
+  if (launches) *launches += 1;
+}
+
 template <typename T>
 int solve_t(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* launches) {
   using V = typename VT<T>::V;
@@ -1008,14 +1036,7 @@ int solve_t(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* laun
     nl += 1;
   }
   const double invN = 1.0 / (double)p.N;
-  size_t sc = p.smem_c2r;
-  // the deviatoric epilogue stages the block's six real rows: a row tile of
-  // its own, kept within 72 KB of shared memory so that several blocks share
-  // an SM (the tuned tile is timed without this staging)
-  int Ld = p.L_x;
-  auto dev_smem = [&](int L) { return 2 * (size_t)p.nc * L * (p.h + 2) * sizeof(V); };
-  while (a.out == kOutDev32 && Ld > 1 && dev_smem(Ld) > 72 * 1024) Ld /= 2;
-  if (a.out == kOutDev32) sc = dev_smem(Ld);
+  const size_t sc = p.smem_c2r;
   if (a.out == kOutSig64)
     k_c2r_x<T, kOutSig64><<<gx.x, TH, sc, st>>>(spec, nco, p.n2, p.h, p.nh, rows, p.N, p.Nk, p.L_x, p.sh,
                                                Tw<T>::h(p), Tw<T>::post(p), invN, a.sig64, nullptr, nullptr,
@@ -1025,9 +1046,7 @@ int solve_t(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* laun
                                                Tw<T>::h(p), Tw<T>::post(p), invN, nullptr, a.sig32, nullptr,
                                                nullptr, nullptr, nullptr, a.gate);
   else if (p.nc == 6)
-    k_c2r_dev<T><<<(unsigned)((rows + Ld - 1) / Ld), TH, sc, st>>>(spec, p.n2, p.h, p.nh, rows, p.N, p.Nk, Ld, p.sh,
-                                                                     Tw<T>::h(p), Tw<T>::post(p), invN, a.sdev,
-                                                                     a.uadd, a.err, a.gate);
+    c2r_dev<T>(p, a, invN, nullptr, st, nullptr);
   else
     k_c2r_x<T, kOutDev32><<<gx.x, TH, p.smem_c2r + sizeof(double) * (size_t)p.nc * p.L_x * p.n2, st>>>(
         spec, p.nc, p.n2, p.h, p.nh, rows, p.N, p.Nk, p.L_x, p.sh, Tw<T>::h(p), Tw<T>::post(p), invN, nullptr,
@@ -1038,6 +1057,46 @@ int solve_t(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* laun
 }
 
 }  // namespace
+
+// Tiles (lines per block) of the three kinds of pass and their shared memory,
+// in FP64 (the FP32 and pair transforms use the same tiles) and in fixed point
+// (padded lines); false if a pass would not fit in `limit` bytes.
+static bool plan_set_tiles(FFTPlan* p, int Lx, int Ly, int Lg, size_t limit = 200 * 1024) {
+  const size_t cz = sizeof(double2);
+  const int ng = p->n0 > 1 ? p->n0 : p->n1;
+  const size_t sx = 2 * (size_t)Lx * (p->h + 1) * cz, sc = 2 * (size_t)Lx * (p->h + 2) * cz;
+  const size_t sy = 2 * (size_t)Ly * (p->n1 + 1) * cz, sg = 2 * (size_t)p->nc * Lg * (ng + 1) * cz;
+  const size_t rx = 2 * (size_t)Lx * fx_ld(p->h + 1) * cz + sizeof(int) * Lx, ry = 2 * (size_t)Ly * fx_ld(p->n1) * cz,
+               rg = 2 * (size_t)p->nc * Lg * fx_ld(ng) * cz;
+  if (Lx < 1 || Ly < 1 || Lg < 1 || (Ly > 1 && Ly * p->n1 > 2048)) return false;
+  if (sc + sizeof(double) * p->nc * Lx * p->n2 > limit || ry > limit || rg > limit || rx > limit) return false;
+  p->L_x = Lx;
+  p->L_y = Ly;
+  p->L_g = Lg;
+  p->smem_x = sx;
+  p->smem_c2r = sc;
+  p->smem_y = sy;
+  p->smem_g = sg;
+  p->smem_xr = rx;
+  p->smem_yr = ry;
+  p->smem_gr = rg;
+  return true;
+}
+
+// The tiles a plan starts with: 1024 complex values of rows, eight lines of the
+// other axes (four or fewer where shared memory asks for it).
+static bool default_tiles(FFTPlan* p) {
+  p->e_x = 4;
+  p->e_y = 4;
+  p->e_g = 2;
+  const size_t cz = sizeof(double2);
+  const int ng = p->n0 > 1 ? p->n0 : p->n1;
+  int Lx = std::max(1, 1024 / p->h), Ly = 8, Lg = 8;
+  while (Lx > 1 && 2 * (size_t)Lx * fx_ld(p->h + 1) * cz + sizeof(double) * p->nc * Lx * p->n2 > 200 * 1024) Lx /= 2;
+  while (Ly > 1 && (2 * (size_t)Ly * fx_ld(p->n1) * cz > 100 * 1024 || Ly * p->n1 > 2048)) Ly /= 2;
+  while (Lg > 1 && 2 * (size_t)p->nc * Lg * fx_ld(ng) * cz > 200 * 1024) Lg /= 2;
+  return plan_set_tiles(p, Lx, Ly, Lg, 224 * 1024);
+}
 
 int fft_plan_create(FFTPlan* p, int n0, int n1, int n2, int nc) {
   std::memset((void*)p, 0, sizeof(*p));
@@ -1053,53 +1112,22 @@ int fft_plan_create(FFTPlan* p, int n0, int n1, int n2, int nc) {
   if (p->sh.nst < 0 || p->s1.nst < 0 || p->s0.nst < 0) return STZ_ERR_INVALID;
   if (p->h > 4096 || n1 > 1024 || n0 > 1024) return STZ_ERR_INVALID;
   int st;
-  if ((st = upload_twiddles(p->h, p->h, &p->tw_h, &p->tw_hf, &p->tw_hd))) return st;
-  if ((st = upload_twiddles(n1, n1, &p->tw_1, &p->tw_1f, &p->tw_1d))) return st;
-  if ((st = upload_twiddles(n0, n0, &p->tw_0, &p->tw_0f, &p->tw_0d))) return st;
-  if ((st = upload_twiddles(n2, p->nh, &p->tw_p, &p->tw_pf, &p->tw_pd))) return st;
-  // tiles (FP64 sizes; the FP32 transform uses the same tiles)
-  const size_t cz = sizeof(double2);
-  p->L_x = std::max(1, 1024 / p->h);
-  while (p->L_x > 1 && 2 * (size_t)p->L_x * (p->h + 2) * cz + sizeof(double) * nc * p->L_x * n2 > 200 * 1024) p->L_x /= 2;
-  p->L_y = 8;
-  while (p->L_y > 1 && 2 * (size_t)p->L_y * (n1 + 1) * cz > 100 * 1024) p->L_y /= 2;
-  const int ng = n0 > 1 ? n0 : n1;
-  p->L_g = 8;
-  while (p->L_g > 1 && 2 * (size_t)nc * p->L_g * (ng + 1) * cz > 200 * 1024) p->L_g /= 2;
-  p->smem_x = 2 * (size_t)p->L_x * (p->h + 1) * cz;
-  p->smem_c2r = 2 * (size_t)p->L_x * (p->h + 2) * cz;
-  p->smem_y = 2 * (size_t)p->L_y * (n1 + 1) * cz;
-  p->smem_g = 2 * (size_t)nc * p->L_g * (ng + 1) * cz;
-  if (p->smem_g > 227 * 1024) return STZ_ERR_INVALID;
+  if ((st = upload_twiddles(p->h, p->h, &p->tw_h, &p->tw_hf, &p->tw_hd, &p->tx_h))) return st;
+  if ((st = upload_twiddles(n1, n1, &p->tw_1, &p->tw_1f, &p->tw_1d, &p->tx_1))) return st;
+  if ((st = upload_twiddles(n0, n0, &p->tw_0, &p->tw_0f, &p->tw_0d, &p->tx_0))) return st;
+  if ((st = upload_twiddles(n2, p->nh, &p->tw_p, &p->tw_pf, &p->tw_pd, &p->tx_p))) return st;
+  if (!default_tiles(p)) return STZ_ERR_INVALID;
   size_t sc_max = p->smem_c2r + sizeof(double) * nc * p->L_x * n2;
   set_smem_attrs<double>(p->smem_x, p->smem_y, p->smem_g, sc_max);
   set_smem_attrs<float>(p->smem_x, p->smem_y, p->smem_g, sc_max);
   set_smem_attrs<dfl>(p->smem_x, p->smem_y, p->smem_g, sc_max);
+  fftx_init();
   return STZ_OK;
-}
-
-// Tiles (lines per block) of the three kinds of pass and their shared memory;
-// false if a pass would not fit.
-static bool plan_set_tiles(FFTPlan* p, int Lx, int Ly, int Lg) {
-  const size_t cz = sizeof(double2);
-  const int ng = p->n0 > 1 ? p->n0 : p->n1;
-  const size_t sx = 2 * (size_t)Lx * (p->h + 1) * cz, sc = 2 * (size_t)Lx * (p->h + 2) * cz;
-  const size_t sy = 2 * (size_t)Ly * (p->n1 + 1) * cz, sg = 2 * (size_t)p->nc * Lg * (ng + 1) * cz;
-  if (Lx < 1 || Ly < 1 || Lg < 1) return false;
-  if (sc + sizeof(double) * p->nc * Lx * p->n2 > 200 * 1024 || sy > 200 * 1024 || sg > 200 * 1024) return false;
-  p->L_x = Lx;
-  p->L_y = Ly;
-  p->L_g = Lg;
-  p->smem_x = sx;
-  p->smem_c2r = sc;
-  p->smem_y = sy;
-  p->smem_g = sg;
-  return true;
 }
 
 namespace {
 struct Tuned {
-  int Lx, Ly, Lg;
+  int Lx, Ly, Lg, ex, ey, eg;
   Sched sh, s1, s0;
   int rejected;  // candidates whose result differed from the default schedule's
 };
@@ -1108,9 +1136,12 @@ std::map<std::array<int, 6>, Tuned> g_tuned;
 
 float time_solve(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1) {
   float best = 1e30f;
-  for (int rep = 0; rep < 2; rep++) {
+  // small grids: enough solves that the events bracket device time and not the
+  // host's launches
+  const int n = p.N * p.nc < (1 << 21) ? 12 : 3;
+  for (int rep = 0; rep < (n > 3 ? 4 : 2); rep++) {
     cudaEventRecord(e0, st);
-    for (int i = 0; i < 3; i++) fft_solve(p, a, st, nullptr);
+    for (int i = 0; i < n; i++) fft_solve(p, a, st, nullptr);
     cudaEventRecord(e1, st);
     cudaEventSynchronize(e1);
     float ms = 0;
@@ -1133,6 +1164,9 @@ int fft_autotune(FFTPlan* p, cudaStream_t st, int* chosen, int pair) {
       p->sh = it->second.sh;
       p->s1 = it->second.s1;
       p->s0 = it->second.s0;
+      p->e_x = it->second.ex;
+      p->e_y = it->second.ey;
+      p->e_g = it->second.eg;
       if (chosen) { chosen[0] = p->L_x; chosen[1] = p->L_y; chosen[2] = p->L_g; chosen[3] = it->second.rejected; }
       return STZ_OK;
     }
@@ -1197,11 +1231,11 @@ int fft_autotune(FFTPlan* p, cudaStream_t st, int* chosen, int pair) {
     FFTPlan q = best;
     if (Lx >= 1 && plan_set_tiles(&q, Lx, q.L_y, q.L_g)) consider(q);
   }
-  for (int Ly : {2, 4, 16}) {
+  for (int Ly : {2, 4, 16, 32}) {
     FFTPlan q = best;
     if (Ly != best.L_y && plan_set_tiles(&q, q.L_x, Ly, q.L_g)) consider(q);
   }
-  for (int Lg : {2, 4, 16}) {
+  for (int Lg : {1, 2, 4, 16}) {
     FFTPlan q = best;
     if (Lg != best.L_g && plan_set_tiles(&q, q.L_x, q.L_y, Lg)) consider(q);
   }
@@ -1212,16 +1246,36 @@ int fft_autotune(FFTPlan* p, cudaStream_t st, int* chosen, int pair) {
     q.s0 = v ? make_sched_rev(p->n0) : make_sched_r4(p->n0);
     if (q.sh.nst > 0 && q.s1.nst > 0 && q.s0.nst > 0) consider(q);
   }
+  if (!pair) {  // threads per tile of the fixed-point passes
+    for (int e : {2, 8}) {
+      FFTPlan q = best;
+      q.e_x = e;
+      consider(q);
+    }
+    for (int e : {2, 8}) {
+      FFTPlan q = best;
+      q.e_y = e;
+      if (p->n0 > 1) consider(q);
+    }
+    for (int e : {1, 4}) {
+      FFTPlan q = best;
+      q.e_g = e;
+      consider(q);
+    }
+  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaFree(eps); cudaFree(ref); cudaFree(out); cudaFree(spec);
+  p->e_x = best.e_x;
+  p->e_y = best.e_y;
+  p->e_g = best.e_g;
   plan_set_tiles(p, best.L_x, best.L_y, best.L_g);
   p->sh = best.sh;
   p->s1 = best.s1;
   p->s0 = best.s0;
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tuned[key] = Tuned{p->L_x, p->L_y, p->L_g, p->sh, p->s1, p->s0, rejected};
+    g_tuned[key] = Tuned{p->L_x, p->L_y, p->L_g, p->e_x, p->e_y, p->e_g, p->sh, p->s1, p->s0, rejected};
   }
   if (chosen) { chosen[0] = p->L_x; chosen[1] = p->L_y; chosen[2] = p->L_g; chosen[3] = rejected; }
   return cudaGetLastError() == cudaSuccess ? STZ_OK : STZ_ERR_CUDA;
@@ -1229,7 +1283,7 @@ int fft_autotune(FFTPlan* p, cudaStream_t st, int* chosen, int pair) {
 
 // Plan whose twiddle tables live in caller-provided device storage (for the
 // allocation-free entry point). FP64 transforms only; no device allocation.
-size_t fft_twiddle_count(int n0, int n1, int n2) { return (size_t)(n2 / 2) + n1 + n0 + (n2 / 2 + 1); }
+size_t fft_twiddle_count(int n0, int n1, int n2) { return 2 * ((size_t)(n2 / 2) + n1 + n0 + (n2 / 2 + 1)); }
 
 int fft_plan_init_in(FFTPlan* p, int n0, int n1, int n2, int nc, double2* storage, size_t cap, cudaStream_t st) {
   std::memset((void*)p, 0, sizeof(*p));
@@ -1258,24 +1312,19 @@ int fft_plan_init_in(FFTPlan* p, int n0, int n1, int n2, int nc, double2* storag
     *dst[t] = storage + off;
     off += counts[t];
   }
+  FxTwiddle** dfx[4] = {&p->tx_h, &p->tx_1, &p->tx_0, &p->tx_p};
+  for (int t = 0; t < 4; t++) {
+    fx_twiddles(lens[t], counts[t], reinterpret_cast<FxTwiddle*>(host.data() + off));
+    *dfx[t] = reinterpret_cast<FxTwiddle*>(storage + off);
+    off += counts[t];
+  }
   if (cudaMemcpyAsync(storage, host.data(), sizeof(double2) * host.size(), cudaMemcpyHostToDevice, st) !=
       cudaSuccess)
     return STZ_ERR_CUDA;
   if (cudaStreamSynchronize(st) != cudaSuccess) return STZ_ERR_CUDA;
-  const size_t cz = sizeof(double2);
-  p->L_x = std::max(1, 1024 / p->h);
-  while (p->L_x > 1 && 2 * (size_t)p->L_x * (p->h + 2) * cz + sizeof(double) * nc * p->L_x * n2 > 200 * 1024) p->L_x /= 2;
-  p->L_y = 8;
-  while (p->L_y > 1 && 2 * (size_t)p->L_y * (n1 + 1) * cz > 100 * 1024) p->L_y /= 2;
-  const int ng = n0 > 1 ? n0 : n1;
-  p->L_g = 8;
-  while (p->L_g > 1 && 2 * (size_t)nc * p->L_g * (ng + 1) * cz > 200 * 1024) p->L_g /= 2;
-  p->smem_x = 2 * (size_t)p->L_x * (p->h + 1) * cz;
-  p->smem_c2r = 2 * (size_t)p->L_x * (p->h + 2) * cz;
-  p->smem_y = 2 * (size_t)p->L_y * (n1 + 1) * cz;
-  p->smem_g = 2 * (size_t)nc * p->L_g * (ng + 1) * cz;
-  if (p->smem_g > 227 * 1024) return STZ_ERR_INVALID;
+  if (!default_tiles(p)) return STZ_ERR_INVALID;
   set_smem_attrs<double>(p->smem_x, p->smem_y, p->smem_g, p->smem_c2r + sizeof(double) * nc * p->L_x * n2);
+  fftx_init();
   return STZ_OK;
 }
 
@@ -1285,11 +1334,20 @@ void fft_plan_destroy(FFTPlan* p) {
   cudaFree(p->tw_h); cudaFree(p->tw_1); cudaFree(p->tw_0); cudaFree(p->tw_p);
   cudaFree(p->tw_hf); cudaFree(p->tw_1f); cudaFree(p->tw_0f); cudaFree(p->tw_pf);
   cudaFree(p->tw_hd); cudaFree(p->tw_1d); cudaFree(p->tw_0d); cudaFree(p->tw_pd);
+  cudaFree(p->tx_h); cudaFree(p->tx_1); cudaFree(p->tx_0); cudaFree(p->tx_p);
   std::memset((void*)p, 0, sizeof(*p));
 }
 
 int fft_solve(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* launches) {
   if (a.pair) return solve_t<dfl>(p, a, st, launches);
+  // FP64 solves run in fixed point (fftx.cu), but for the displacement (a
+  // print-time solve) and media whose moduli are out of its range
+  if (!a.fp32 && !a.disp && (a.out == kOutSig64 || (a.out == kOutDev32 && p.nc == 6)) && fftx_fits(a.lambda, a.mu)) {
+    fftx_spectrum(p, a, st, launches);
+    if (a.out == kOutSig64) fftx_c2r(p, a, st, launches);
+    else c2r_dev<double>(p, a, fftx_factor(p, a.mu), a.ebar, st, launches);
+    return STZ_OK;
+  }
   return a.fp32 ? solve_t<float>(p, a, st, launches) : solve_t<double>(p, a, st, launches);
 }
 

@@ -35,6 +35,10 @@ struct FFTPlan {
   // tiles (lines per block) of each pass
   int L_x = 0, L_y = 0, L_g = 0;
   size_t smem_x = 0, smem_y = 0, smem_g = 0, smem_c2r = 0;
+  // the fixed-point passes (fftx.cu): split twiddles and shared memory
+  FxTwiddle *tx_h = nullptr, *tx_1 = nullptr, *tx_0 = nullptr, *tx_p = nullptr;
+  size_t smem_xr = 0, smem_yr = 0, smem_gr = 0;
+  int e_x = 0, e_y = 0, e_g = 0;  // values of a tile (e_g: of each component) per thread
 };
 
 int fft_plan_create(FFTPlan* p, int n0, int n1, int n2, int nc);

@@ -2,6 +2,7 @@
 // the constants of a context.
 #include "fixp.cuh"
 
+#include <algorithm>
 #include <cmath>
 
 #include "stz_internal.h"
@@ -49,6 +50,59 @@ void fx_exp_table(FxExp* t) {
     t[j].ph = s.h;
     t[j].pl = s.l;
   }
+}
+
+void fx_twiddles(int n, int count, FxTwiddle* out) {
+  const long double pi2 = 6.28318530717958647692528676655900577L;
+  for (int k = 0; k < count; k++) {
+    // the angle folded to an eighth of a turn, so that exact values stay exact
+    // and symmetric values are equal
+    const int k8 = (int)((8LL * k / n) & 7);
+    long double c, s;
+    auto cs = [&](long long num) {  // angle num / (8 n) of a turn, num in [0, n]
+      c = std::cos(pi2 * num / (8.0L * n));
+      s = std::sin(pi2 * num / (8.0L * n));
+    };
+    const long long num = 8LL * k - (long long)k8 * n;  // within the octant
+    if (k8 & 1) cs(n - num); else cs(num);
+    long double re, im;
+    switch (k8) {
+      case 0: re = c; im = s; break;
+      case 1: re = s; im = c; break;
+      case 2: re = -s; im = c; break;
+      case 3: re = -c; im = s; break;
+      case 4: re = -c; im = -s; break;
+      case 5: re = -s; im = -c; break;
+      case 6: re = s; im = -c; break;
+      default: re = c; im = -s; break;
+    }
+    auto fix = [](long double v) {
+      Fx f = fx_split((int64_t)std::llrint(std::ldexp(v, 62)));
+      if (f.l == INT32_MIN) f.l++;  // so that the halves can be negated
+      return f;
+    };
+    out[k] = FxTwiddle{fix(re), fix(-im)};
+  }
+}
+
+void fx_green_constants(int n0, int n1, int n2, double lambda, double mu, GreenFx* g) {
+  GreenFx& ga = *g;
+  ga.is3d = n0 > 1;
+  ga.n0 = n0; ga.n1 = n1; ga.n2 = n2; ga.nh = n2 / 2 + 1;
+  const long double lam = lambda, m = mu, al = (lam + m) / (lam + 2 * m);
+  const long double l2 = lam / (2 * m), c1 = (1 - al) * lam / m;
+  // constants at most 2^62; the operator's growth (1 + 3 |lambda| / (2 mu) for
+  // tau, then three more bits) as headroom
+  const long double big = std::max(std::fabs(l2), std::fabs(c1));
+  ga.lams = 2;
+  while (std::ldexp(1.0L, ga.lams - 2) < big) ga.lams++;
+  ga.lam = fx_split(fixed(l2, 64 - ga.lams));
+  ga.c1 = fx_split(fixed(c1, 64 - ga.lams));
+  ga.al2 = fx_split(fixed(2 * al, 60));
+  ga.kb = 3;
+  while (std::ldexp(1.0L, ga.kb) < 8 * (1 + 3 * std::fabs(l2))) ga.kb++;
+  const int nn[3] = {n0, n1, n2};
+  for (int i = 0; i < 3; i++) ga.inv[i] = fixed(1.0L / nn[i], 61);
 }
 
 // The constants of a 3D FP64 context (see RateFx); on = 0 when they do not fit.

@@ -209,4 +209,23 @@ constexpr int kFxRateShift = 5;
 // the smallest and largest Y of a site before its stress terms
 constexpr uint64_t kFxY0Min = (uint64_t)514 << 53, kFxY0Max = (uint64_t)1533 << 53;
 
+// exp(-2 pi i k / n), k = 0 .. count-1, as split fixed point (x 2^62): the
+// halves of the real part, then of the imaginary part (fixp.cpp).
+struct alignas(16) FxTwiddle {
+  Fx r, i;
+};
+void fx_twiddles(int n, int count, FxTwiddle* out);
+
+// Constants of the fixed-point Green's pass (fftx.cu).
+struct GreenFx {
+  int is3d, n0, n1, n2, nh;
+  int kb;            // headroom of the operator: inputs enter shifted right by kb bits
+  int lams;          // lam and c1 carry 2^(64 - lams)
+  Fx lam;            // lambda / (2 mu)
+  Fx c1;             // (1 - alpha) lambda / mu, alpha = (lambda + mu) / (lambda + 2 mu)
+  Fx al2;            // 2 alpha, x 2^60
+  int64_t inv[3];    // 2^61 / n0, n1, n2
+};
+void fx_green_constants(int n0, int n1, int n2, double lambda, double mu, GreenFx* g);
+
 }  // namespace stz

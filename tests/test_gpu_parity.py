@@ -473,3 +473,78 @@ def test_fixed_point_rates_match_fp64_rates(engine_lib, shape, barrier):
     if neg == 0:
         assert abs(ev["total_rate"][0] / R - 1) < 1e-13
     eng.close()
+
+
+# ------------------------------------------------- fixed-point solve
+def _noalloc(lib, dim, shape, lam, mu, eps, ebar):
+    import ctypes as C
+    torch = pytest.importorskip("torch")
+    d = torch.tensor(eps, dtype=torch.float64, device="cuda")
+    s = torch.full_like(d, 7.0)
+    eb = (C.c_double * len(ebar))(*ebar)
+    st = lib.stz_solve_noalloc(dim, *shape, lam, mu, d.data_ptr(), eb, s.data_ptr(), None)
+    assert st == api.OK, lib.stz_last_error().decode()
+    return s.cpu().numpy()
+
+
+@pytest.mark.parametrize("shape", [
+    (2, 2, 2), (2, 3, 4), (1, 2, 2), (1, 1, 2), (3, 1, 6), (1, 512, 2), (2, 2, 512), (64, 2, 54),
+    (1, 1024, 32), (1, 32, 1024), (2, 16, 648), (27, 9, 18),   # long lines: the passes' general forms
+])
+def test_fixed_point_solve_edges(engine_lib, oracle_lib, shape):
+    """The solve in fixed point on lines of one value up to 1024, odd lengths and
+    tiles with idle lanes, against the oracle's complex FP64 solve (the bar of
+    test_fft_green_solve_matches_oracle)."""
+    dim = 2 if shape[0] == 1 else 3
+    p = configs.ref2d(shape[1], shape[2]) if dim == 2 else configs.shear64(seed=2)
+    p.n[0], p.n[1], p.n[2] = shape
+    ora = oracle_lib.Model(p)
+    nc, N = 3 * (dim - 1), int(np.prod(shape))
+    rng = np.random.default_rng(11)
+    eps = rng.standard_normal((nc, N)) * 0.02
+    for c in range(nc):
+        ora.set_field(api.FIELD_EPS0, c, eps[c])
+    ora.solve()
+    want = np.stack([ora.field(api.FIELD_SIGMA, c) for c in range(nc)])
+    ebar = ora.scalars()["eps_avg"][:nc]
+    got = _noalloc(engine_lib, dim, shape, p.lambda_, p.mu, eps, ebar)
+    assert rel_err(got, want) < 1e-11
+
+
+@pytest.mark.parametrize("scale", [1e-200, 1e-30, 1e30, 1e200])
+def test_fixed_point_solve_is_scale_free(engine_lib, scale):
+    """A power of ten times the eigenstrain gives that times the stress to a few
+    roundings, inside and outside the range of the FP32 line sums."""
+    shape = (6, 8, 12)
+    rng = np.random.default_rng(3)
+    eps = rng.standard_normal((6, 576)) * 0.02
+    a = _noalloc(engine_lib, 3, shape, 80.0, 35.0, eps, [0.0] * 6)
+    b = _noalloc(engine_lib, 3, shape, 80.0, 35.0, eps * scale, [0.0] * 6) / scale
+    assert np.abs(a - b).max() <= 1e-14 * np.abs(a).max()
+    assert not _noalloc(engine_lib, 3, shape, 80.0, 35.0, eps * 0.0, [0.0] * 6).any()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_fixed_point_solve_keeps_nan(engine_lib, bad):
+    """A value that is not finite makes every site's stress NaN, as it does in
+    FP64 arithmetic (it enters every wave vector)."""
+    eps = np.zeros((6, 16 * 12 * 8))
+    eps[2, 77] = bad
+    assert np.isnan(_noalloc(engine_lib, 3, (16, 12, 8), 80.0, 35.0, eps, [0.0] * 6)[2]).all()
+
+
+@pytest.mark.parametrize("lam", [-30.0, 0.0, 35.0, 8000.0, 1e6])
+def test_solve_for_extreme_media(engine_lib, oracle_lib, lam):
+    """Lame constants at the ends of the fixed point's range and (1e6) beyond
+    it, where the FP64 passes run. The rounding of FP64 grows with lambda / mu."""
+    p = configs.shear64(seed=2, n=8)
+    p.lambda_, p.mu = lam, 35.0
+    ora = oracle_lib.Model(p)
+    rng = np.random.default_rng(5)
+    eps = rng.standard_normal((6, 512)) * 0.02
+    for c in range(6):
+        ora.set_field(api.FIELD_EPS0, c, eps[c])
+    ora.solve()
+    want = np.stack([ora.field(api.FIELD_SIGMA, c) for c in range(6)])
+    got = _noalloc(engine_lib, 3, (8, 8, 8), lam, 35.0, eps, ora.scalars()["eps_avg"])
+    assert rel_err(got, want) < 1e-11 * max(1.0, abs(lam) / 35.0)
