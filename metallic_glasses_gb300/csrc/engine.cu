@@ -500,7 +500,7 @@ void enqueue_plain_step(stz_ctx* c, cudaEvent_t t0 = nullptr, cudaEvent_t t1 = n
   if (t0) cudaEventRecord(t0, c->stream);
   launch_rate_fp64(kp, f, c->rx, c->stream);
   if (t1) cudaEventRecord(t1, c->stream);
-  launch_athermal(kp, f, 0, c->stream);
+  launch_athermal(kp, f, c->rx, 0, c->stream);
   solve_plain(c, gate, ebar);
   if (kp.incr64) {
     launch_incr64(kp, f, c->stream);
@@ -509,7 +509,7 @@ void enqueue_plain_step(stz_ctx* c, cudaEvent_t t0 = nullptr, cudaEvent_t t1 = n
   launch_post_a(kp, f, c->stream);
   solve_plain(c, gate, ebar);
   if (f.Q1) {
-    launch_q0_reset(kp, f, c->stream);
+    launch_q0_reset(kp, f, c->rx, c->stream);
     c->launches += 1;
   }
   launch_post_b(kp, f, c->stream);
@@ -595,7 +595,7 @@ int mixed_service(stz_ctx* c, int* done) {
   if (h.step_kind == kAthermal) {
     // the avalanche, the reference's re-solve with the current mean strain,
     // the athermal correction and the print check, then the stop checks
-    launch_athermal(kp, f, 1, c->stream);
+    launch_athermal(kp, f, c->rx, 1, c->stream);
     solve_dev(c, f.ctl->eps_avg, nullptr, f.scratch);
     launch_mixed_after_resolve(kp, f, 0, c->stream);
     launch_post_a(kp, f, c->stream);
@@ -847,7 +847,7 @@ int stz::create_ctx(const stz_params* pin, stz_ctx** out, int units_per_block) {
   st = ref2d ? init_ref2d(c, &rng) : init_global3d(c, &rng);
   if (st) return fail(st);
   if (mixed) mixed_constants(c);
-  if (!mixed && !ref2d) {
+  if (!mixed) {
     std::vector<FxExp> tab(kFxExpCells);
     fx_exp_table(tab.data());
     if ((st = dalloc(&c->exptab, tab.size()))) return fail(st);
@@ -857,7 +857,15 @@ int stz::create_ctx(const stz_params* pin, stz_ctx** out, int units_per_block) {
     c->rx.tab = c->exptab;
     int sms = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device);
-    kp.rate_grid = std::min(kp.nblk, sms * rate_fx_blocks_per_sm(kp.bsites / kRateThreads));
+    kp.rate_grid = std::min(kp.nblk, sms * rate_fx_blocks_per_sm(p.model, kp.bsites / kRateThreads));
+    if (ref2d && c->rx.on) {
+      const size_t nm = (size_t)STZ_MODES * N;
+      if ((st = dalloc(&f.cq, nm)) || (st = dalloc(&f.dx, nm)) || (st = dalloc(&f.dxy, nm))) return fail(st);
+      if (p.softening &&
+          ((st = dalloc(&f.ux, nm)) || (st = dalloc(&f.uxy, nm)) || (st = dalloc(&f.pn, (size_t)2 * N))))
+        return fail(st);
+      launch_r2_fixed(kp, f, c->rx, 0, STZ_MODES, 1, c->stream);
+    }
   }
 
   // control block
@@ -908,7 +916,8 @@ extern "C" void stz_destroy(stz_ctx* c) {
   void* ptrs[] = {f.eps0, f.sig, f.sdev, f.dF, f.dF32, f.Q0, f.Q1, f.deps, f.dnorm, f.rtab64, f.mro, f.prev_deps, f.perm_soft, f.temp_soft,
                   f.tlast, f.amark, f.part, f.gsum, f.gticket, f.lsum, f.lbnd, f.psum, f.spec, f.ktab, f.log,
                   f.ctl, f.scratch, f.msum, c->err_dev, c->l2buf, c->qbuf, f.lam_site, f.mu_site,
-                  f.inh_tau0, f.inh_eeff, f.inh_last, f.inh_part, c->exptab};
+                  f.inh_tau0, f.inh_eeff, f.inh_last, f.inh_part, c->exptab,
+                  f.cq, f.dx, f.dxy, f.ux, f.uxy, f.pn};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->fft) {
@@ -1241,6 +1250,9 @@ extern "C" int stz_set_field(stz_ctx* c, int32_t which, int32_t comp, const doub
   CK(cudaMemcpyAsync(d64, host, sizeof(double) * c->kp.N, cudaMemcpyHostToDevice, c->stream));
   if (which == STZ_FIELD_DF && c->f.dF32) launch_fill_f32(c->f.dF, c->f.dF32, c->kp.N, c->stream);
   if (which == STZ_FIELD_DEPS && c->f.dnorm) launch_mode_norms(c->kp, c->f, c->stream);
+  if (c->f.cq && (which == STZ_FIELD_DEPS || which == STZ_FIELD_DF || which == STZ_FIELD_PREV_DEPS))
+    launch_r2_fixed(c->kp, c->f, c->rx, which == STZ_FIELD_DEPS ? comp / 3 : which == STZ_FIELD_DF ? comp : 0,
+                    which != STZ_FIELD_PREV_DEPS, which == STZ_FIELD_PREV_DEPS, c->stream);
   CK(cudaStreamSynchronize(c->stream));
   return STZ_OK;
 }

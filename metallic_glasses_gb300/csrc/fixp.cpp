@@ -105,36 +105,53 @@ void fx_green_constants(int n0, int n1, int n2, double lambda, double mu, GreenF
   for (int i = 0; i < 3; i++) ga.inv[i] = fixed(1.0L / nn[i], 61);
 }
 
-// The constants of a 3D FP64 context (see RateFx); on = 0 when they do not fit.
+// The constants of an FP64 context (see RateFx); on = 0 when they do not fit.
 void rate_fx_constants(const KParams& kp, RateFx* x) {
   x->on = 0;
+  const bool d2 = kp.model == STZ_MODEL_REF2D;
   const long double kT = kp.kT, w = (long double)kp.V0 * 1e-18L * (long double)kJInEv / (2 * kT) * kLog2e;
   const long double b = kLog2e / kT, c = std::log2((long double)kp.vt) + 1022;
-  long double M[STZ_MODES][5], smax = 0;
-  for (int m = 0; m < STZ_MODES; m++) {
-    const double* d = kp.modes[m];
-    M[m][0] = w * d[0];
-    M[m][1] = w * d[1];
-    for (int k = 2; k < 5; k++) M[m][k] = 2 * w * d[k + 1];
-    long double s = 0;
-    for (int k = 0; k < 5; k++) s += std::fabs(M[m][k]);
-    // the trace of a mode is rounding; a mode set with one is not represented
-    if (!(std::fabs((long double)d[0] + d[1] + d[2]) <= 1e-15L * (std::fabs(d[0]) + std::fabs(d[1]) + std::fabs(d[2]))))
-      return;
-    if (!(s <= 1e15L)) return;
-    smax = std::max(smax, s);
+  if (!(b > 1e-15L && b < 1e15L) || !(w > 1e-15L && w < 1e15L) || !(c > 600 && c < 1440)) return;
+  if (d2) {
+    const int LW = (int)std::ceil(std::log2(w));
+    x->sw = 48 + LW;
+    x->w2 = fx_split(fixed(w, 60 - LW));
+    x->l2e = fx_split(fixed(kLog2e, 61));
+    const long double ft[3] = {0.1L, 0.01L, 0.9L};
+    for (int t = 0; t < 3; t++)
+      for (int m = 0; m < STZ_MODES; m++) x->ftp[t][m] = fx_split(fixed(std::pow(ft[t], (long double)(m + 2)), 62));
+    x->decayed = 746 * kp.t_temp;
+  } else {
+    long double M[STZ_MODES][5], smax = 0;
+    for (int m = 0; m < STZ_MODES; m++) {
+      const double* d = kp.modes[m];
+      M[m][0] = w * d[0];
+      M[m][1] = w * d[1];
+      for (int k = 2; k < 5; k++) M[m][k] = 2 * w * d[k + 1];
+      long double s = 0;
+      for (int k = 0; k < 5; k++) s += std::fabs(M[m][k]);
+      // the trace of a mode is rounding; a mode set with one is not represented
+      if (!(std::fabs((long double)d[0] + d[1] + d[2]) <=
+            1e-15L * (std::fabs(d[0]) + std::fabs(d[1]) + std::fabs(d[2]))))
+        return;
+      if (!(s <= 1e15L)) return;
+      smax = std::max(smax, s);
+    }
+    if (!(smax > 1e-15L)) return;
+    const int L = (int)std::ceil(std::log2(smax));
+    x->sw = 51 + L;
+    for (int m = 0; m < STZ_MODES; m++)
+      for (int k = 0; k < 5; k++) x->m[m][k] = fx_split(fixed(M[m][k], 61 - L));
   }
-  if (!(smax > 1e-15L) || !(b > 1e-15L && b < 1e15L) || !(c > 600 && c < 1440)) return;
-  const int L = (int)std::ceil(std::log2(smax)), LB = (int)std::ceil(std::log2(b));
-  x->sw = 51 + L;
+  const int LB = (int)std::ceil(std::log2(b));
   x->sq = 51 + LB;
-  for (int m = 0; m < STZ_MODES; m++)
-    for (int k = 0; k < 5; k++) x->m[m][k] = fx_split(fixed(M[m][k], 61 - L));
   x->nb = fx_split(fixed(-b, 61 - LB));
   const uint64_t c53 = (uint64_t)fixed(c - 1024, 53) + ((uint64_t)1024 << 53);  // c 2^53 may exceed 2^63
   x->c_hh = (int64_t)(c53 >> kFxRateShift);
   x->c_mid = (int64_t)(c53 & ((1u << kFxRateShift) - 1)) << (32 - kFxRateShift);
   x->neg = c53;
+  if (!(0.33L * b < 500)) return;
+  x->mark = c53 - (uint64_t)fixed(0.33L * b, 53);
   x->on = 1;
 }
 

@@ -186,7 +186,7 @@ FX_HD uint64_t fx_exp2_sum_bits(const uint64_t* Y, const FxExp* q) {
 // point (integer arithmetic only: the same bits on every host; fixp.cpp).
 void fx_exp_table(FxExp* t);
 
-// Constants of the fixed-point rates of one context (3D FP64 forms). The rate
+// Constants of the fixed-point rates of one FP64 context. In 3D the rate
 // argument in log2 units, y = log2(vt) - dF log2(e)/kT + sum_c W_c M_mc, with
 // W = (s_xx - s_zz, s_yy - s_zz, s_yz, s_xz, s_xy) (the modes are traceless)
 // and M the modes times V0 1e-18 J log2(e) / (2 kT) (shears doubled), is held
@@ -202,8 +202,16 @@ struct RateFx {
   Fx nb;              // -log2(e)/kT
   int64_t c_hh, c_mid;  // log2(vt) + 1022
   uint64_t neg;       // Y above this: a positive rate argument (a negative barrier)
+  uint64_t mark;      // Y above this: a barrier below 0.33 eV (the avalanche's marks)
   const FxExp* tab;   // device table
   Fx m[20][5];
+  // 2D model (see R2Fx in kmc.cu): the work scale V0 1e-18 J log2(e) / (2 kT)
+  // of the stress coordinates and log2(e) x 2^61; the powers ft^(m + 2) of the
+  // crystal-like types' factors x 2^62; the decay of the temporary softening
+  // underflows beyond this time
+  Fx w2, l2e;
+  Fx ftp[3][20];
+  double decayed;
 };
 constexpr int kFxRateShift = 5;
 // the smallest and largest Y of a site before its stress terms

@@ -535,6 +535,158 @@ __device__ __forceinline__ FxExp fx_cell(const FxExp* t, int j) {  // one 16-byt
   return q;
 }
 
+// REF2D in fixed point. A site's operands: W0 = (s_xx - s_yy) w and W2 = 2 s_xy w
+// (x 2^49, below 2^12), w = V0 1e-18 J log2(e) / (2 kT), so that the work term of
+// mode m is W0 dx + W2 dxy (its modes are traceless); for a softened site the
+// normalised last increment and soft = (permanent + temporary softening)
+// log2(e) (x 2^57, below 2^4).
+struct R2Fx {
+  Fx W0, W2, p0, p2, soft;
+  int mro;         // crystal-like type under NO_SF_XTAL_MRO, else 0
+  bool softened;
+};
+constexpr int kFxR2Shift = 8;
+__device__ __forceinline__ Fx fx_load(const Fx* p) {
+  const int2 v = *reinterpret_cast<const int2*>(p);
+  return Fx{v.x, v.y};
+}
+__device__ __forceinline__ bool nonzero(double x) { return (__double_as_longlong(x) << 1) != 0; }
+
+// The site's softening: permanent plus decayed temporary (init.c:711-739). A
+// term whose decay underflows, or without temporary softening, is +0 exactly.
+__device__ __forceinline__ double r2_softening(const KParams& kp, const Fields& f, double totime, double decayed,
+                                               long long s) {
+  if (!kp.softening) return 0.0;
+  double soft = f.perm_soft[s];
+  const double ts = f.temp_soft[s];
+  if (nonzero(ts)) {
+    const double age = totime - f.tlast[s];
+    if (!(age >= decayed)) soft += ts * exp_tang(-age / kp.t_temp);
+  }
+  return soft;
+}
+__device__ __forceinline__ bool r2_fx_site(const KParams& kp, const RateFx& rx, const Fields& f, const int64_t* ufx,
+                                           double totime, long long s, R2Fx* d) {
+  bool ok = true;
+  const long long N = kp.N;
+  int64_t g[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) g[c] = fx_from_f64<3>(f.sig[c * N + s], rx.sw, &ok) + ufx[c];
+  FxAcc a{0, 0}, b{0, 0};
+  fx_mad(a, fx_split(g[0] - g[1]), rx.w2);
+  fx_mad(b, fx_split(g[2]), rx.w2);
+  const int64_t W0 = fx_value<5>(a), W2 = fx_value<6>(b);
+  ok &= (uint64_t)(W0 + (1ll << 61)) < (1ull << 62) && (uint64_t)(W2 + (1ll << 61)) < (1ull << 62) &&
+        (uint64_t)(g[2] + (1ll << 60)) < (1ull << 61);
+  d->W0 = fx_split(W0);
+  d->W2 = fx_split(W2);
+  const double soft = r2_softening(kp, f, totime, rx.decayed, s);
+  d->softened = nonzero(soft);
+  d->mro = 0;
+  d->soft = d->p0 = d->p2 = Fx{0, 0};
+  if (d->softened) {
+    ok &= __double_as_longlong(soft) >= 0;
+    FxAcc q{0, 0};
+    fx_mad(q, fx_split(fx_from_f64<3>(soft, 57, &ok)), rx.l2e);
+    d->soft = fx_split(fx_value<3>(q));
+    d->p0 = fx_load(f.pn + s);
+    d->p2 = fx_load(f.pn + N + s);
+    ok &= d->p0.h != INT32_MIN;
+    if (f.mro && kp.no_sf_xtal_mro) d->mro = f.mro[s];
+  }
+  return ok;
+}
+__device__ __forceinline__ bool r2_fx_u(const RateFx& rx, const double* u, int64_t* ufx) {
+  bool ok = true;
+#pragma unroll
+  for (int c = 0; c < 3; c++) ufx[c] = fx_from_f64<3>(u[c], rx.sw, &ok);
+  return ok;
+}
+// a b / 2^(64 - S)
+template <int S>
+__device__ __forceinline__ int64_t fx_mul(int64_t a, Fx b) {
+  FxAcc q{0, 0};
+  fx_mad(q, fx_split(a), b);
+  return fx_value<S>(q);
+}
+// 2^(-z) for z >= 0 in units of 2^-59, as R 2^-62 2^-n: the exponential's table
+// takes z to 2^-53; the rest enters to first order (a barrier of 100 kT takes
+// the factor's relative error a hundredfold into the rate's argument).
+__device__ __forceinline__ int64_t fx_exp2_neg(int64_t z, const FxExp* tab, int* n) {
+  const uint64_t Y = ((uint64_t)1022 << 53) - (uint64_t)(z >> 6);
+  const int64_t R = fx_exp2_mant<false>(Y, fx_cell(tab, fx_exp_cell(Y)));
+  *n = min(63, 1022 - (int)(Y >> 53));
+  return R - (fx_wide((int32_t)(R >> 32), ((int)z & 63) * 45426, 0) >> 43);  // ln 2 2^16
+}
+// The constant part of a softened site's argument: C - (C - cq) 2^(-z), z =
+// modifier (x 2^62) soft; the direction modifiers of init.c:590-642, a
+// crystal-like site's scaled by its factor to the power m + 2.
+__device__ __forceinline__ uint64_t r2_fx_soften(const KParams& kp, const RateFx& rx, const Fields& f, const FxExp* tab,
+                                                 const R2Fx& d, long long i, int m, uint64_t cq) {
+  FxAcc p{0, 0};
+  fx_mad(p, d.p0, fx_load(f.ux + i));
+  fx_mad(p, d.p2, fx_load(f.uxy + i));
+  constexpr int64_t one = 1ll << 62;
+  int64_t DM = fx_value<6>(p);  // x 2^62
+  DM = DM > one ? one : (DM < -one ? -one : DM);
+  const int64_t a = (DM >> 1) + (one >> 1);  // (1 + DM) / 2
+  int64_t mod;
+  switch (kp.sf_scheme) {
+    case STZ_SF_LINEAR_FWD: mod = a; break;
+    case STZ_SF_LINEAR_BWD: mod = one - a; break;
+    case STZ_SF_EVEN: mod = one >> 1; break;
+    case STZ_SF_SQUARE_FWD: mod = fx_mul<2>(a, fx_split(a)); break;
+    case STZ_SF_CUBIC_FWD: mod = fx_mul<2>(fx_mul<2>(a, fx_split(a)), fx_split(a)); break;
+    default: {  // exp(-DM^2 9 / 2); DM^2 log2(e) x 2^61 before the factor
+      int n;
+      mod = fx_exp2_neg((fx_mul<2>(fx_mul<2>(DM, fx_split(DM)), rx.l2e) >> 3) * 9, tab, &n) >> n;
+    }
+  }
+  if (d.mro) mod = fx_mul<2>(mod, rx.ftp[d.mro - 1][m]);
+  int n;
+  const int64_t R = fx_exp2_neg(fx_mul<4>(mod, d.soft), tab, &n);
+  return rx.neg - (uint64_t)(fx_mul<3>((int64_t)(rx.neg - cq), fx_split(R >> 1)) >> n);
+}
+__device__ __forceinline__ uint64_t r2_fx_arg(const KParams& kp, const RateFx& rx, const Fields& f, const FxExp* tab,
+                                              const R2Fx& d, long long s, int m, bool* ok) {
+  const long long i = (long long)m * kp.N + s;
+  uint64_t cq = f.cq[i];
+  FxAcc a{0, 0};
+  fx_mad(a, d.W0, fx_load(f.dx + i));
+  fx_mad(a, d.W2, fx_load(f.dxy + i));
+  // the work term within 2^8 in magnitude
+  *ok &= cq != 0 && (uint32_t)((int32_t)(a.hh >> 32) + (1 << 21)) < (1u << 22);
+  if (d.softened) cq = r2_fx_soften(kp, rx, f, tab, d, i, m, cq);
+  return cq + (uint64_t)fx_value<kFxR2Shift>(a);
+}
+
+// The stored fixed-point operands of one (mode, site) and of a site's last
+// increment, from the FP64 fields.
+__device__ __forceinline__ void r2_fx_store_mode(const RateFx& rx, const Fields& f, long long i, double q0, double d0,
+                                                 double d1, double d2, double rnorm) {
+  bool ok = d1 == -d0;
+  FxAcc a{rx.c_hh, rx.c_mid};
+  fx_mad(a, fx_split(fx_from_f64<2>(q0, rx.sq, &ok)), rx.nb);
+  const uint64_t y = (uint64_t)fx_value<kFxRateShift>(a);
+  ok &= y - kFxY0Min <= kFxY0Max - kFxY0Min && rx.neg - y + (1ull << 62) < (1ull << 63);  // |Q0 log2(e)/kT| < 512
+  f.dx[i] = fx_split(fx_from_f64<3>(d0, 60, &ok));
+  f.dxy[i] = fx_split(fx_from_f64<3>(d2, 60, &ok));
+  if (f.ux) {
+    f.ux[i] = fx_split(fx_from_f64<3>(d0 * rnorm, 60, &ok));
+    f.uxy[i] = fx_split(fx_from_f64<3>(d2 * rnorm, 60, &ok));
+  }
+  f.cq[i] = ok ? y : 0;
+}
+__device__ __forceinline__ void r2_fx_store_prev(const Fields& f, long long N, long long s, double p0, double p1,
+                                                 double p2) {
+  const double r = 1.0 / (sqrt(p0 * p0 + p1 * p1 + 2 * p2 * p2) + kEpsilon);
+  bool ok = true;
+  Fx a = fx_split(fx_from_f64<2>((p0 - p1) * r, 60, &ok)), b = fx_split(fx_from_f64<2>(2 * p2 * r, 60, &ok));
+  if (!ok) a = Fx{INT32_MIN, 0};
+  f.pn[s] = a;
+  f.pn[N + s] = b;
+}
+
 __device__ __forceinline__ unsigned long long gtimer() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -749,6 +901,13 @@ template <int MODEL>
 __device__ __forceinline__ double site_rate(const KParams& kp, const Fields& f, const RateFx& rx, const double* u,
                                             double totime, long long s, int m) {
   if (MODEL == 0) {
+    int64_t ufx[3];
+    R2Fx x;
+    if (rx.on && r2_fx_u(rx, u, ufx) && r2_fx_site(kp, rx, f, ufx, totime, s, &x)) {
+      bool ok = true;
+      const uint64_t Y = r2_fx_arg(kp, rx, f, rx.tab, x, s, m, &ok);
+      if (ok) return fx_double(fx_exp2_bits(Y, fx_cell(rx.tab, fx_exp_cell(Y))));
+    }
     const R2Site d = r2_load(kp, f, u, totime, s);
     return kp.vt * exp_tang(r2_arg(kp, f, d, s, m));
   } else if (MODEL == 1) {
@@ -909,7 +1068,7 @@ __device__ void search_event(const KParams& kp, const Fields& f, const RateFx& r
 // ------------------------------------------------------------ commits
 // VoxelShearTransform (elastic.c:361-520) for the FP64 models; thread 0 only.
 template <int MODEL>
-__device__ void transform(const KParams& kp, const Fields& f, Ctl* ctl, int mm, long long s, MT* rng) {
+__device__ void transform(const KParams& kp, const Fields& f, const RateFx& rx, Ctl* ctl, int mm, long long s, MT* rng) {
   const long long N = kp.N;
   double d[6];
   if (MODEL == 0) {
@@ -932,13 +1091,19 @@ __device__ void transform(const KParams& kp, const Fields& f, Ctl* ctl, int mm, 
     f.perm_soft[s] = ps;
     f.temp_soft[s] = ds * (ty == 1 ? kp.temp_soft_mro : kp.temp_soft);
     f.tlast[s] = ctl->totime;
+    if (f.pn) r2_fx_store_prev(f, N, s, d[0], d[1], d[2]);
     if (ty) {
       // a crystal-like site keeps its modes and draws new barriers
       // xQ0amp (1 - RandomRatio + RandomRatio u) (elastic.c:451-500)
       for (int i = 0; i < STZ_MODES; i++) {
         const double u = mt_uniform(rng);
-        f.Q0[(long long)i * N + s] =
-            __dmul_rn(kp.xq0amp, __dadd_rn(1.0 - kp.random_ratio, __dmul_rn(kp.random_ratio, u)));
+        const long long j = (long long)i * N + s;
+        const double q0 = __dmul_rn(kp.xq0amp, __dadd_rn(1.0 - kp.random_ratio, __dmul_rn(kp.random_ratio, u)));
+        f.Q0[j] = q0;
+        if (f.cq) {
+          const double* dd = f.deps + (long long)i * 3 * N;
+          r2_fx_store_mode(rx, f, j, q0, dd[s], dd[N + s], dd[2 * N + s], f.dnorm[j]);
+        }
       }
       return;
     }
@@ -950,7 +1115,10 @@ __device__ void transform(const KParams& kp, const Fields& f, Ctl* ctl, int mm, 
       dd[s] = a;
       dd[N + s] = -a;
       dd[2 * N + s] = c2;
-      f.dnorm[(long long)i * N + s] = mode_rnorm(a, -a, c2);
+      const long long j = (long long)i * N + s;
+      const double rn = mode_rnorm(a, -a, c2);
+      f.dnorm[j] = rn;
+      if (f.cq) r2_fx_store_mode(rx, f, j, f.Q0[j], a, -a, c2, rn);
     }
   }
 }
@@ -1053,7 +1221,7 @@ __device__ __noinline__ void finish_step(const KParams& kp, const Fields& f, con
         c->sel_site = s;
         c->sel_mode = m;
         c->sel_q = q;
-        transform<MODEL>(kp, f, c, m, s, &c->rng);
+        transform<MODEL>(kp, f, rx, c, m, s, &c->rng);
         if (kp.incr64) {
           c->incr_req = 1;  // the incremental update instead of the re-solve
           c->pend_site = s;
@@ -1245,18 +1413,119 @@ __global__ void __launch_bounds__(TH, Q == 4 ? 2 : 3) k_rate64_fx(KParams kp, Fi
   }
 }
 
+// The rates of the 2D model in fixed point: per (mode, site) the stored operands
+// (24 bytes, 40 at a softened site) in place of the FP64 barrier, increments and
+// norm. Otherwise as k_rate64_fx.
+template <int Q>
+__global__ void __launch_bounds__(TH, 3) k_rate64_fx2(KParams kp, Fields f, RateFx rx) {
+  constexpr int G = Q == 1 ? 10 : (Q == 2 ? 5 : 4);  // modes per reduction
+  __shared__ FxExp tab[kFxExpCells];
+  __shared__ int64_t sh_u[3];
+  __shared__ int sh_uok;
+  __shared__ double red[TH / 32][STZ_MODES];
+  Ctl* ctl = f.ctl;
+  if (ctl->halt) return;
+  {
+    const int4* src = reinterpret_cast<const int4*>(rx.tab);
+    int4* dst = reinterpret_cast<int4*>(tab);
+#pragma unroll
+    for (int i = 0; i < kFxExpCells / TH; i++) dst[i * TH + threadIdx.x] = __ldg(src + i * TH + threadIdx.x);
+  }
+  const double totime = ctl->totime;
+  if (threadIdx.x == 0) sh_uok = r2_fx_u(rx, ctl->u, sh_u);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int b = blockIdx.x; b < kp.nblk; b += gridDim.x) {
+    const long long s0 = (long long)b * kp.bsites;
+    const long long s1 = min(s0 + (long long)kp.bsites, kp.N);
+    bool ok = sh_uok;
+    unsigned neg = 0;
+    R2Fx d[Q];
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      const long long s = s0 + threadIdx.x + q * TH;
+      if (s < s1) ok &= r2_fx_site(kp, rx, f, sh_u, totime, s, &d[q]);
+    }
+#pragma unroll 1
+    for (int g = 0; g < STZ_MODES; g += G) {
+      double v[G];
+#pragma unroll
+      for (int i = 0; i < G; i++) {
+        uint64_t Y[Q];
+        FxExp c[Q];
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+          const long long s = s0 + threadIdx.x + q * TH;
+          Y[q] = (uint64_t)1 << 53;  // no site: the smallest representable rate, 2^-1021
+          if (s < s1) Y[q] = r2_fx_arg(kp, rx, f, tab, d[q], s, g + i, &ok);
+          neg += Y[q] > rx.neg;
+          c[q] = fx_cell(tab, fx_exp_cell(Y[q]));
+        }
+        v[i] = fx_double(fx_exp2_sum_bits<Q>(Y, c));
+      }
+      int idx;
+      const double t = WarpSums<G, 16>::run(v, lane, &idx);
+      if (idx >= 0) red[w][g + idx] = t;
+    }
+    if (!__syncthreads_or(!ok)) {
+      if (threadIdx.x < STZ_MODES) {
+        double t = 0;
+#pragma unroll
+        for (int k = 0; k < TH / 32; k++) t += red[k][threadIdx.x];
+        f.part[(long long)threadIdx.x * kp.nblk + b] = t;
+      }
+    } else {
+      double u[6];
+      for (int c = 0; c < 6; c++) u[c] = ctl->u[c];
+      neg = rate_chunk_fp64<0>(kp, f, u, totime, b, s0, s1);
+    }
+    if (chunk_done(kp, f, b, neg)) finish_step<0>(kp, f, rx);
+  }
+}
+
 // ------------------------------------------------------------ athermal
 // Mark every site whose lowest-barrier mode has Q < 0 or |Q| < 0.33
-// (evolution.c:55-65). mixed: Q from the FP32 deviatoric field.
-__global__ void k_ath_mark(KParams kp, Fields f, int mixed) {
+// (evolution.c:55-65). mixed: Q from the FP32 deviatoric field. The FP64 forms
+// find the lowest barrier as the largest fixed-point rate argument (their FP64
+// Q's of a site out of its range).
+__global__ void k_ath_mark(KParams kp, Fields f, RateFx rx, int mixed) {
   Ctl* ctl = f.ctl;
   if (ctl->step_kind != kAthermal) return;
   double u[6];
   for (int c = 0; c < 6; c++) u[c] = ctl->u[c];
   const double totime = ctl->totime;
+  const bool r2 = kp.model == STZ_MODEL_REF2D;
+  int64_t ufx[6];
+  const bool fx = rx.on && !mixed && (r2 ? r2_fx_u(rx, u, ufx) : g3_fx_u(rx, u, ufx));
   for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < kp.N; s += (long long)gridDim.x * blockDim.x) {
     int mm = 0;
     double minQ = 0;
+    if (fx) {
+      uint64_t top = 0;
+      bool ok;
+      if (r2) {
+        R2Fx d;
+        ok = r2_fx_site(kp, rx, f, ufx, totime, s, &d);
+        for (int m = 0; m < STZ_MODES; m++) {
+          const uint64_t Y = r2_fx_arg(kp, rx, f, rx.tab, d, s, m, &ok);
+          if (Y > top) { mm = m; top = Y; }
+        }
+      } else {
+        Fx W[5];
+        FxAcc a0;
+        ok = g3_fx_site(rx, f, kp.N, ufx, s, W, &a0);
+#pragma unroll 4
+        for (int m = 0; m < STZ_MODES; m++) {
+          const uint64_t Y = g3_fx_arg(rx, W, a0, m);
+          if (Y > top) { mm = m; top = Y; }
+        }
+      }
+      if (ok) {
+        f.amark[s] = top > rx.mark ? (signed char)(mm + 1) : (signed char)0;  // Q < 0.33
+        continue;
+      }
+      mm = 0;
+    }
     for (int m = 0; m < STZ_MODES; m++) {
       double Q;
       if (kp.model == STZ_MODEL_REF2D) Q = site_Q<0>(kp, f, u, totime, s, m);
@@ -1270,7 +1539,7 @@ __global__ void k_ath_mark(KParams kp, Fields f, int mixed) {
 
 // Transform the marked sites in index order (the RNG stream order of the
 // reference's space_loop); one block, thread 0 commits.
-__global__ void k_ath_commit(KParams kp, Fields f, int mixed) {
+__global__ void k_ath_commit(KParams kp, Fields f, RateFx rx, int mixed) {
   Ctl* ctl = f.ctl;
   if (ctl->step_kind != kAthermal) return;
   __shared__ unsigned ballot[TH / 32];
@@ -1303,8 +1572,8 @@ __global__ void k_ath_commit(KParams kp, Fields f, int mixed) {
           if (kp.model == STZ_MODEL_REF2D) q = site_Q<0>(kp, f, u, totime, site, mm);
           else if (mixed) q = site_Q<2>(kp, f, u, totime, site, mm);
           else q = site_Q<1>(kp, f, u, totime, site, mm);
-          if (kp.model == STZ_MODEL_REF2D) transform<0>(kp, f, ctl, mm, site, &srng);
-          else transform<1>(kp, f, ctl, mm, site, &srng);
+          if (kp.model == STZ_MODEL_REF2D) transform<0>(kp, f, rx, ctl, mm, site, &srng);
+          else transform<1>(kp, f, rx, ctl, mm, site, &srng);
           log_event(kp, f, ctl, STZ_EV_ATHERMAL, site, mm, ctl->totime, 0.0, q, 0.0);
         }
       }
@@ -1413,11 +1682,18 @@ __global__ void k_post_print(KParams kp, Fields f) {
 
 // The print's reset of the barriers to their initial copy (bmg.c:214-221),
 // when this step printed. Only REF2D grids with crystal-like sites have Q1.
-__global__ void k_q0_reset(KParams kp, Fields f) {
+__global__ void k_q0_reset(KParams kp, Fields f, RateFx rx) {
   if (!f.ctl->print_done || f.ctl->step_kind == kNone) return;
   const long long total = (long long)STZ_MODES * kp.N;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
-    f.Q0[i] = f.Q1[i];
+    if (f.Q0[i] != f.Q1[i]) {
+      f.Q0[i] = f.Q1[i];
+      if (f.cq) {
+        const long long m = i / kp.N, s = i - m * kp.N;
+        const double* dd = f.deps + m * 3 * kp.N;
+        r2_fx_store_mode(rx, f, i, f.Q1[i], dd[s], dd[kp.N + s], dd[2 * kp.N + s], f.dnorm[i]);
+      }
+    }
 }
 
 // One block of TH threads, as k_post_a.
@@ -2948,9 +3224,18 @@ __global__ void k_hold(unsigned long long ns) {
 
 }  // namespace
 
-int rate_fx_blocks_per_sm(int spt) {
+namespace {
+template <int MODEL>
+const void* rate_fx_kernel(int spt) {
+  if (MODEL == 0)
+    return spt == 1 ? (const void*)k_rate64_fx2<1> : spt == 2 ? (const void*)k_rate64_fx2<2> : (const void*)k_rate64_fx2<4>;
+  return spt == 1 ? (const void*)k_rate64_fx<1> : spt == 2 ? (const void*)k_rate64_fx<2> : (const void*)k_rate64_fx<4>;
+}
+}  // namespace
+
+int rate_fx_blocks_per_sm(int model, int spt) {
   int occ = 0;
-  const void* k = spt == 1 ? (const void*)k_rate64_fx<1> : spt == 2 ? (const void*)k_rate64_fx<2> : (const void*)k_rate64_fx<4>;
+  const void* k = model == STZ_MODEL_REF2D ? rate_fx_kernel<0>(spt) : rate_fx_kernel<1>(spt);
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, TH, 0) != cudaSuccess || occ < 1) {
     (void)cudaGetLastError();
     occ = 1;
@@ -2959,11 +3244,18 @@ int rate_fx_blocks_per_sm(int spt) {
 }
 
 void launch_rate_fp64(const KParams& kp, const Fields& f, const RateFx& rx, cudaStream_t st) {
-  if (kp.model == STZ_MODEL_REF2D) k_rate64<0><<<kp.nblk, TH, 0, st>>>(kp, f, rx);
-  else if (!rx.on) k_rate64<1><<<kp.nblk, TH, 0, st>>>(kp, f, rx);
-  else if (kp.bsites == TH) k_rate64_fx<1><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
-  else if (kp.bsites == 2 * TH) k_rate64_fx<2><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
-  else k_rate64_fx<4><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
+  if (!rx.on) {
+    if (kp.model == STZ_MODEL_REF2D) k_rate64<0><<<kp.nblk, TH, 0, st>>>(kp, f, rx);
+    else k_rate64<1><<<kp.nblk, TH, 0, st>>>(kp, f, rx);
+  } else if (kp.model == STZ_MODEL_REF2D) {
+    if (kp.bsites == TH) k_rate64_fx2<1><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
+    else if (kp.bsites == 2 * TH) k_rate64_fx2<2><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
+    else k_rate64_fx2<4><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
+  } else {
+    if (kp.bsites == TH) k_rate64_fx<1><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
+    else if (kp.bsites == 2 * TH) k_rate64_fx<2><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
+    else k_rate64_fx<4><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
+  }
 }
 
 // The staged lines of the mixed-form main kernels are dynamic shared memory,
@@ -3120,6 +3412,26 @@ void launch_mode_norms(const KParams& kp, const Fields& f, cudaStream_t st) {
   k_mode_norms<<<nb, TH, 0, st>>>(kp, f);
 }
 
+// The fixed-point operands of the modes m0 .. m0 + nm - 1 at every site and, with
+// prev, of every site's last increment (REF2D), from the FP64 fields.
+__global__ void k_r2_fixed(KParams kp, Fields f, RateFx rx, int m0, int nm, int prev) {
+  const long long N = kp.N, total = nm * N;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+  for (long long k = t; k < total; k += nt) {
+    const long long i = m0 * N + k, m = i / N, s = i - m * N;
+    const double* dd = f.deps + m * 3 * N;
+    r2_fx_store_mode(rx, f, i, f.Q0[i], dd[s], dd[N + s], dd[2 * N + s], f.dnorm[i]);
+  }
+  if (prev && f.pn)
+    for (long long s = t; s < N; s += nt)
+      r2_fx_store_prev(f, N, s, f.prev_deps[s], f.prev_deps[N + s], f.prev_deps[2 * N + s]);
+}
+
+void launch_r2_fixed(const KParams& kp, const Fields& f, const RateFx& rx, int m0, int nm, int prev, cudaStream_t st) {
+  const long long total = std::max(nm, 1) * kp.N;
+  k_r2_fixed<<<(unsigned)std::min<long long>((total + TH - 1) / TH, 152LL * 16), TH, 0, st>>>(kp, f, rx, m0, nm, prev);
+}
+
 int wait_selftest(int tries, int* status_dev, int* kmax, cudaStream_t st) {
   *kmax = kMbarTries;
   k_wait_selftest<<<1, 32, 0, st>>>(tries, status_dev);
@@ -3131,10 +3443,10 @@ void launch_mixed(const KParams& kp, const Fields& f, int update_only, cudaStrea
   launch_mixed_tail(kp, f, update_only, st);
 }
 
-void launch_athermal(const KParams& kp, const Fields& f, int mixed, cudaStream_t st) {
+void launch_athermal(const KParams& kp, const Fields& f, const RateFx& rx, int mixed, cudaStream_t st) {
   const long long nb = std::min<long long>((kp.N + TH - 1) / TH, 152LL * 8);
-  k_ath_mark<<<(unsigned)nb, TH, 0, st>>>(kp, f, mixed);
-  k_ath_commit<<<1, TH, 0, st>>>(kp, f, mixed);
+  k_ath_mark<<<(unsigned)nb, TH, 0, st>>>(kp, f, rx, mixed);
+  k_ath_commit<<<1, TH, 0, st>>>(kp, f, rx, mixed);
 }
 
 void launch_post_a(const KParams& kp, const Fields& f, cudaStream_t st) {
@@ -3154,10 +3466,10 @@ void launch_note_solve(const Fields& f, const int* gate, const double* ebar, cud
   k_note_solve<<<1, 1, 0, st>>>(f, gate, ebar);
 }
 
-void launch_q0_reset(const KParams& kp, const Fields& f, cudaStream_t st) {
+void launch_q0_reset(const KParams& kp, const Fields& f, const RateFx& rx, cudaStream_t st) {
   const long long total = (long long)STZ_MODES * kp.N;
   const unsigned nb = (unsigned)std::min<long long>((total + TH - 1) / TH, 152LL * 8);
-  k_q0_reset<<<nb, TH, 0, st>>>(kp, f);
+  k_q0_reset<<<nb, TH, 0, st>>>(kp, f, rx);
 }
 
 void launch_mixed_after_resolve(const KParams& kp, const Fields& f, int kind, cudaStream_t st) {

@@ -16,7 +16,7 @@ constexpr int kGroup = 32;     // blocks per group in the two-level rate sums
 void launch_rate_fp64(const KParams& kp, const Fields& f, const RateFx& rx, cudaStream_t st);
 // Resident blocks per SM of the fixed-point rate kernel (occupancy query) at
 // spt (1, 2 or 4) sites per thread.
-int rate_fx_blocks_per_sm(int spt);
+int rate_fx_blocks_per_sm(int model, int spt);
 // Mixed form: incremental stress update + rates + selection/commit.
 // update_only: apply the pending transformation and uniform change, nothing else.
 void launch_mixed(const KParams& kp, const Fields& f, int update_only, cudaStream_t st);
@@ -47,6 +47,9 @@ int mixed_blocks_per_sm(int n2);
 size_t mixed_smem(int n2);
 // the stored mode norms of the 2D model, after its mode increments were written
 void launch_mode_norms(const KParams& kp, const Fields& f, cudaStream_t st);
+// the fixed-point operands of the 2D model's modes and barriers m0 .. m0 + nm - 1
+// and (prev) of its sites' last increments, after the FP64 fields were written
+void launch_r2_fixed(const KParams& kp, const Fields& f, const RateFx& rx, int m0, int nm, int prev, cudaStream_t st);
 // bounded-wait self-test kernel (one block); *kmax receives the kernels' limit
 int wait_selftest(int tries, int* status_dev, int* kmax, cudaStream_t st);
 // The two halves of launch_mixed: the grid-wide update/rate kernel and the
@@ -54,7 +57,7 @@ int wait_selftest(int tries, int* status_dev, int* kmax, cudaStream_t st);
 void launch_mixed_main(const KParams& kp, const Fields& f, int update_only, cudaStream_t st);
 void launch_mixed_tail(const KParams& kp, const Fields& f, int update_only, cudaStream_t st);
 // Athermal avalanche (evolution.c:47-100): mark sites, then commit in order.
-void launch_athermal(const KParams& kp, const Fields& f, int mixed, cudaStream_t st);
+void launch_athermal(const KParams& kp, const Fields& f, const RateFx& rx, int mixed, cudaStream_t st);
 // Bookkeeping after the solve of a step (loading, clock, print check) and
 // after the optional print re-solve (stop checks, targets).
 void launch_post_a(const KParams& kp, const Fields& f, cudaStream_t st);
@@ -65,7 +68,7 @@ void launch_post_b(const KParams& kp, const Fields& f, cudaStream_t st);
 void launch_incr64(const KParams& kp, const Fields& f, cudaStream_t st);
 void launch_note_solve(const Fields& f, const int* gate, const double* ebar, cudaStream_t st);
 // REF2D with crystal-like sites: restore the initial barriers when the step printed
-void launch_q0_reset(const KParams& kp, const Fields& f, cudaStream_t st);
+void launch_q0_reset(const KParams& kp, const Fields& f, const RateFx& rx, cudaStream_t st);
 // Reset of the incremental state after a full re-solve (mixed form).
 // kind 0: field solved with the current mean strain (print / athermal);
 // kind 1: periodic re-solve with the applied mean strain (field unchanged).

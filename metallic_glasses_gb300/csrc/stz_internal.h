@@ -111,6 +111,14 @@ struct Fields {
   double* Q0 = nullptr;      // [MODES][N] (REF2D)
   double* deps = nullptr;    // [MODES][3][N] (REF2D)
   double* dnorm = nullptr;   // [MODES][N] 1 / (|deps| + eps) of each mode (REF2D), kept with deps
+  // REF2D in fixed point (R2Fx), kept with Q0, deps and prev_deps
+  uint64_t* cq = nullptr;    // [MODES][N] log2(vt) + 1022 - Q0 log2(e)/kT, x 2^53; 0: a value of
+                             // the (mode, site) does not fit
+  Fx* dx = nullptr;          // [MODES][N] deps xx and xy, x 2^60 (the modes are traceless)
+  Fx* dxy = nullptr;
+  Fx* ux = nullptr;          // [MODES][N] deps xx and xy over the mode's norm, x 2^60 (softening only)
+  Fx* uxy = nullptr;
+  Fx* pn = nullptr;          // [2][N] (xx - yy) and 2 xy of the last increment over its norm, x 2^60
   double* rtab64 = nullptr;  // [nc][nc][N] FP64 incremental form: stress component c of the
                              // solve of a unit eigenstrain component k at site 0, ebar = 0
   int8_t* mro = nullptr;     // [N] crystal-like MRO type 0..3 (REF2D); null for an all-glass map

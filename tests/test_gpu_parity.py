@@ -548,3 +548,63 @@ def test_solve_for_extreme_media(engine_lib, oracle_lib, lam):
     want = np.stack([ora.field(api.FIELD_SIGMA, c) for c in range(6)])
     got = _noalloc(engine_lib, 3, (8, 8, 8), lam, 35.0, eps, ora.scalars()["eps_avg"])
     assert rel_err(got, want) < 1e-11 * max(1.0, abs(lam) / 35.0)
+
+
+# ------------------------------------------------- fixed-point 2D rates
+@pytest.mark.parametrize("shape,scheme,mro,odd", [
+    ((16, 18), api.SF_SQUARE_FWD, 0.0, None), ((48, 54), api.SF_LINEAR_FWD, 0.15, None),
+    ((48, 54), api.SF_LINEAR_BWD, 0.0, None), ((48, 54), api.SF_EVEN, 0.0, None),
+    ((48, 54), api.SF_CUBIC_FWD, 0.15, None), ((48, 54), api.SF_GAUSS_FWD, 0.0, None),
+    ((576, 576), api.SF_SQUARE_FWD, 0.15, None), ((768, 1024), api.SF_SQUARE_FWD, 0.0, None),  # two, four sites a thread
+    ((48, 54), api.SF_SQUARE_FWD, 0.0, "trace"), ((48, 54), api.SF_SQUARE_FWD, 0.0, "mode"),
+    ((48, 54), api.SF_SQUARE_FWD, 0.0, "barrier"), ((48, 54), api.SF_SQUARE_FWD, 0.0, "soft"),
+    ((48, 54), api.SF_SQUARE_FWD, 0.0, "hardened"),
+])
+def test_fixed_point_2d_rates_match_fp64_rates(engine_lib, shape, scheme, mro, odd):
+    """The total rate of a step of the 2D model, half of its sites softened,
+    against the sum of vt exp(-Q/kT) in extended precision over the engine's own
+    FP64 Q's. Q carries a few roundings of 2^-52 of 2 eV and kT is 0.026 eV, so
+    rates differ by some 1e-13; the bar is 3e-13. `odd`: one value outside the
+    fixed point's range (a mode with a trace, one of strain above 1, a barrier
+    of 30 eV, softening above 8, negative softening), whose chunk takes the FP64
+    chain."""
+    p = configs.ref2d(*shape, xfrac=mro, xq0="1.8")
+    p.sf_scheme = scheme
+    eng = api.Engine(p)
+    N, rng = eng.N, np.random.default_rng(5)
+    for c in range(3):
+        eng.set_field(api.FIELD_EPS0, c, rng.standard_normal(N) * 0.004)
+    hit = rng.random(N) < 0.5
+    pd = np.where(hit, 0.07 * rng.standard_normal((2, N)), 0.0)
+    soft = np.where(hit, np.minimum(p.perm_soft_cap, 26 * (pd ** 2).sum(0)), 0.0)
+    if odd in ("soft", "hardened"):
+        soft[N // 3] = 9.0 if odd == "soft" else -0.01
+    for c, v in ((0, pd[0]), (1, -pd[0]), (2, pd[1])):
+        eng.set_field(api.FIELD_PREV_DEPS, c, v)
+    eng.set_field(api.FIELD_PERM_SOFT, 0, soft)
+    eng.set_field(api.FIELD_TEMP_SOFT, 0, np.where(hit, 0.3, 0.0) * (rng.random(N) < 0.3))
+    eng.set_field(api.FIELD_TLAST, 0, -p.t_temp * rng.uniform(0, 900, N))
+    if odd in ("trace", "mode"):
+        d = eng.field(api.FIELD_DEPS, 3 * 7)
+        d[N // 2] = 0.01 if odd == "trace" else 1.5
+        eng.set_field(api.FIELD_DEPS, 3 * 7, d)
+        if odd == "mode":
+            eng.set_field(api.FIELD_DEPS, 3 * 7 + 1, -d)
+    if odd == "barrier":
+        q = eng.field(api.FIELD_DF, 4)
+        q[N // 2] = 30.0
+        eng.set_field(api.FIELD_DF, 4, q)
+    eng.solve()
+    kT = p.temperature * 1.380658e-23 / 1.60217733e-19
+    R, neg = np.longdouble(0), 0
+    for m in range(20):
+        Q = eng.field(api.FIELD_Q, m)
+        neg += int((Q < 0).sum())
+        R += np.exp(-Q.astype(np.longdouble) / np.longdouble(kT)).sum()
+    R *= np.longdouble(p.voxel_volume * p.trial_frequency)
+    eng.run(max_steps=1)
+    ev, sc = eng.events(), eng.scalars()
+    assert (sc["astep"] == 1) == (neg > 0)
+    if neg == 0:
+        assert abs(ev["total_rate"][0] / R - 1) < 3e-13
+    eng.close()
