@@ -207,7 +207,7 @@ int init_ref2d(stz_ctx* c, MT* rng) {
   }
   if ((st = upload(c->f.Q0, Q0.data(), sizeof(double) * Q0.size(), c->stream))) return st;
   if ((st = upload(c->f.deps, deps.data(), sizeof(double) * deps.size(), c->stream))) return st;
-  launch_mode_norms(c->kp, c->f, c->stream);
+  launch_mode_norms(c->kp, c->f, 0, STZ_MODES, c->stream);
   CK(cudaGetLastError());
   std::vector<double> tl((size_t)N, -100 * p.t_temp);
   if ((st = upload(c->f.tlast, tl.data(), sizeof(double) * N, c->stream))) return st;
@@ -794,7 +794,10 @@ int stz::create_ctx(const stz_params* pin, stz_ctx** out, int units_per_block) {
   if ((st = dalloc(&f.ctl, 1))) return fail(st);
   if ((st = dalloc(&f.eps0, (size_t)nc * N))) return fail(st);
   if ((st = dalloc(&f.prev_deps, (size_t)nc * N))) return fail(st);
-  if ((st = dalloc(&f.amark, (size_t)N))) return fail(st);
+  {
+    const size_t chunks = (size_t)((N + kRateThreads - 1) / kRateThreads);
+    if ((st = dalloc(&f.amark, chunks * (kRateThreads + sizeof(short))))) return fail(st);
+  }
   if (mixed) {
     if ((st = dalloc(&f.lsum, (size_t)STZ_MODES * kp.n0 * kp.n1))) return fail(st);
     if ((st = dalloc(&f.lbnd, (size_t)STZ_MODES * kp.n0 * kp.n1))) return fail(st);
@@ -848,8 +851,11 @@ int stz::create_ctx(const stz_params* pin, stz_ctx** out, int units_per_block) {
   if (st) return fail(st);
   if (mixed) mixed_constants(c);
   if (!mixed) {
-    std::vector<FxExp> tab(kFxExpCells);
-    fx_exp_table(tab.data());
+    static const std::vector<FxExp> tab = [] {
+      std::vector<FxExp> t(kFxExpCells);
+      fx_exp_table(t.data());
+      return t;
+    }();
     if ((st = dalloc(&c->exptab, tab.size()))) return fail(st);
     if ((st = upload(c->exptab, tab.data(), sizeof(FxExp) * tab.size(), c->stream))) return fail(st);
     CK(cudaStreamSynchronize(c->stream));
@@ -857,12 +863,12 @@ int stz::create_ctx(const stz_params* pin, stz_ctx** out, int units_per_block) {
     c->rx.tab = c->exptab;
     int sms = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device);
-    kp.rate_grid = std::min(kp.nblk, sms * rate_fx_blocks_per_sm(p.model, kp.bsites / kRateThreads));
+    c->rx.grid = std::min(kp.nblk, sms * rate_fx_blocks_per_sm(p.model, kp.bsites / kRateThreads));
     if (ref2d && c->rx.on) {
       const size_t nm = (size_t)STZ_MODES * N;
-      if ((st = dalloc(&f.cq, nm)) || (st = dalloc(&f.dx, nm)) || (st = dalloc(&f.dxy, nm))) return fail(st);
+      if ((st = dalloc(&c->rx.cq, nm)) || (st = dalloc(&c->rx.dx, nm)) || (st = dalloc(&c->rx.dxy, nm))) return fail(st);
       if (p.softening &&
-          ((st = dalloc(&f.ux, nm)) || (st = dalloc(&f.uxy, nm)) || (st = dalloc(&f.pn, (size_t)2 * N))))
+          ((st = dalloc(&c->rx.ux, nm)) || (st = dalloc(&c->rx.uxy, nm)) || (st = dalloc(&c->rx.pn, (size_t)2 * N))))
         return fail(st);
       launch_r2_fixed(kp, f, c->rx, 0, STZ_MODES, 1, c->stream);
     }
@@ -917,7 +923,7 @@ extern "C" void stz_destroy(stz_ctx* c) {
                   f.tlast, f.amark, f.part, f.gsum, f.gticket, f.lsum, f.lbnd, f.psum, f.spec, f.ktab, f.log,
                   f.ctl, f.scratch, f.msum, c->err_dev, c->l2buf, c->qbuf, f.lam_site, f.mu_site,
                   f.inh_tau0, f.inh_eeff, f.inh_last, f.inh_part, c->exptab,
-                  f.cq, f.dx, f.dxy, f.ux, f.uxy, f.pn};
+                  c->rx.cq, c->rx.dx, c->rx.dxy, c->rx.ux, c->rx.uxy, c->rx.pn};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->fft) {
@@ -1249,8 +1255,8 @@ extern "C" int stz_set_field(stz_ctx* c, int32_t which, int32_t comp, const doub
   if (st) return st;
   CK(cudaMemcpyAsync(d64, host, sizeof(double) * c->kp.N, cudaMemcpyHostToDevice, c->stream));
   if (which == STZ_FIELD_DF && c->f.dF32) launch_fill_f32(c->f.dF, c->f.dF32, c->kp.N, c->stream);
-  if (which == STZ_FIELD_DEPS && c->f.dnorm) launch_mode_norms(c->kp, c->f, c->stream);
-  if (c->f.cq && (which == STZ_FIELD_DEPS || which == STZ_FIELD_DF || which == STZ_FIELD_PREV_DEPS))
+  if (which == STZ_FIELD_DEPS && c->f.dnorm) launch_mode_norms(c->kp, c->f, comp / 3, 1, c->stream);
+  if (c->rx.cq && (which == STZ_FIELD_DEPS || which == STZ_FIELD_DF || which == STZ_FIELD_PREV_DEPS))
     launch_r2_fixed(c->kp, c->f, c->rx, which == STZ_FIELD_DEPS ? comp / 3 : which == STZ_FIELD_DF ? comp : 0,
                     which != STZ_FIELD_PREV_DEPS, which == STZ_FIELD_PREV_DEPS, c->stream);
   CK(cudaStreamSynchronize(c->stream));

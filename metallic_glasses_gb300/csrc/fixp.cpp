@@ -130,18 +130,19 @@ void rate_fx_constants(const KParams& kp, RateFx* x) {
       for (int k = 2; k < 5; k++) M[m][k] = 2 * w * d[k + 1];
       long double s = 0;
       for (int k = 0; k < 5; k++) s += std::fabs(M[m][k]);
-      // the trace of a mode is rounding; a mode set with one is not represented
-      if (!(std::fabs((long double)d[0] + d[1] + d[2]) <=
-            1e-15L * (std::fabs(d[0]) + std::fabs(d[1]) + std::fabs(d[2]))))
-        return;
       if (!(s <= 1e15L)) return;
       smax = std::max(smax, s);
     }
     if (!(smax > 1e-15L)) return;
     const int L = (int)std::ceil(std::log2(smax));
     x->sw = 51 + L;
-    for (int m = 0; m < STZ_MODES; m++)
+    for (int m = 0; m < STZ_MODES; m++) {
       for (int k = 0; k < 5; k++) x->m[m][k] = fx_split(fixed(M[m][k], 61 - L));
+      const double* d = kp.modes[m];
+      const long double t = std::ldexp(w * ((long double)d[0] + d[1] + d[2]), 61 - L);
+      if (!(std::fabs(t) < 2e9L)) return;  // a trace far beyond rounding
+      x->mt[m] = (int32_t)std::llrint(t);
+    }
   }
   const int LB = (int)std::ceil(std::log2(b));
   x->sq = 51 + LB;

@@ -188,8 +188,8 @@ void fx_exp_table(FxExp* t);
 
 // Constants of the fixed-point rates of one FP64 context. In 3D the rate
 // argument in log2 units, y = log2(vt) - dF log2(e)/kT + sum_c W_c M_mc, with
-// W = (s_xx - s_zz, s_yy - s_zz, s_yz, s_xz, s_xy) (the modes are traceless)
-// and M the modes times V0 1e-18 J log2(e) / (2 kT) (shears doubled), is held
+// W = (s_xx - s_zz, s_yy - s_zz, s_yz, s_xz, s_xy) and M the modes times V0
+// 1e-18 J log2(e) / (2 kT) (shears doubled), is held
 // as (y + 1022) 2^53 = 2^5 (hh 2^64 + mid 2^32) / 2^64 of an FxAcc.
 // Scales: with L = ceil(log2(max_m sum_c |M_mc|)) stresses carry 2^(51 + L) and
 // modes 2^(61 - L), so stresses below 2^(8 - L) GPa (32 GPa at 455 K and 1 nm^3)
@@ -205,6 +205,7 @@ struct RateFx {
   uint64_t mark;      // Y above this: a barrier below 0.33 eV (the avalanche's marks)
   const FxExp* tab;   // device table
   Fx m[20][5];
+  int32_t mt[20];     // the modes' traces (rounding, some 1e-17), which s_zz multiplies
   // 2D model (see R2Fx in kmc.cu): the work scale V0 1e-18 J log2(e) / (2 kT)
   // of the stress coordinates and log2(e) x 2^61; the powers ft^(m + 2) of the
   // crystal-like types' factors x 2^62; the decay of the temporary softening
@@ -212,6 +213,13 @@ struct RateFx {
   Fx w2, l2e;
   Fx ftp[3][20];
   double decayed;
+  // ... and its stored operands, kept with Q0, deps and prev_deps
+  uint64_t* cq;       // [MODES][N] log2(vt) + 1022 - Q0 log2(e)/kT, x 2^53; 0: a value of the
+                      // (mode, site) does not fit
+  Fx *dx, *dxy;       // [MODES][N] deps xx and xy, x 2^60 (the modes are traceless)
+  Fx *ux, *uxy;       // [MODES][N] deps xx and xy over the mode's norm, x 2^60 (softening only)
+  Fx* pn;             // [2][N] (xx - yy) and 2 xy of the last increment over its norm, x 2^60
+  int grid;           // resident blocks of the rate kernel (at most nblk)
 };
 constexpr int kFxRateShift = 5;
 // the smallest and largest Y of a site before its stress terms

@@ -507,6 +507,7 @@ __device__ __forceinline__ bool g3_fx_site(const RateFx& rx, const Fields& f, lo
   W[2] = fx_split(g[3]);
   W[3] = fx_split(g[4]);
   W[4] = fx_split(g[5]);
+  W[5] = fx_split(g[2]);
   a0->hh = rx.c_hh;
   a0->mid = rx.c_mid;
   fx_mad(*a0, fx_split(fx_from_f64<2>(f.dF[s], rx.sq, &ok)), rx.nb);
@@ -524,6 +525,7 @@ __device__ __forceinline__ uint64_t g3_fx_arg(const RateFx& rx, const Fx* W, con
   FxAcc a = a0;
 #pragma unroll
   for (int c = 0; c < 5; c++) fx_mad(a, W[c], rx.m[m][c]);
+  a.mid = fx_wide(W[5].h, rx.mt[m], a.mid);
   return (uint64_t)fx_value<kFxRateShift>(a);
 }
 __device__ __forceinline__ FxExp fx_cell(const FxExp* t, int j) {  // one 16-byte load
@@ -589,8 +591,8 @@ __device__ __forceinline__ bool r2_fx_site(const KParams& kp, const RateFx& rx, 
     FxAcc q{0, 0};
     fx_mad(q, fx_split(fx_from_f64<3>(soft, 57, &ok)), rx.l2e);
     d->soft = fx_split(fx_value<3>(q));
-    d->p0 = fx_load(f.pn + s);
-    d->p2 = fx_load(f.pn + N + s);
+    d->p0 = fx_load(rx.pn + s);
+    d->p2 = fx_load(rx.pn + N + s);
     ok &= d->p0.h != INT32_MIN;
     if (f.mro && kp.no_sf_xtal_mro) d->mro = f.mro[s];
   }
@@ -624,8 +626,8 @@ __device__ __forceinline__ int64_t fx_exp2_neg(int64_t z, const FxExp* tab, int*
 __device__ __forceinline__ uint64_t r2_fx_soften(const KParams& kp, const RateFx& rx, const Fields& f, const FxExp* tab,
                                                  const R2Fx& d, long long i, int m, uint64_t cq) {
   FxAcc p{0, 0};
-  fx_mad(p, d.p0, fx_load(f.ux + i));
-  fx_mad(p, d.p2, fx_load(f.uxy + i));
+  fx_mad(p, d.p0, fx_load(rx.ux + i));
+  fx_mad(p, d.p2, fx_load(rx.uxy + i));
   constexpr int64_t one = 1ll << 62;
   int64_t DM = fx_value<6>(p);  // x 2^62
   DM = DM > one ? one : (DM < -one ? -one : DM);
@@ -650,10 +652,10 @@ __device__ __forceinline__ uint64_t r2_fx_soften(const KParams& kp, const RateFx
 __device__ __forceinline__ uint64_t r2_fx_arg(const KParams& kp, const RateFx& rx, const Fields& f, const FxExp* tab,
                                               const R2Fx& d, long long s, int m, bool* ok) {
   const long long i = (long long)m * kp.N + s;
-  uint64_t cq = f.cq[i];
+  uint64_t cq = rx.cq[i];
   FxAcc a{0, 0};
-  fx_mad(a, d.W0, fx_load(f.dx + i));
-  fx_mad(a, d.W2, fx_load(f.dxy + i));
+  fx_mad(a, d.W0, fx_load(rx.dx + i));
+  fx_mad(a, d.W2, fx_load(rx.dxy + i));
   // the work term within 2^8 in magnitude
   *ok &= cq != 0 && (uint32_t)((int32_t)(a.hh >> 32) + (1 << 21)) < (1u << 22);
   if (d.softened) cq = r2_fx_soften(kp, rx, f, tab, d, i, m, cq);
@@ -662,29 +664,29 @@ __device__ __forceinline__ uint64_t r2_fx_arg(const KParams& kp, const RateFx& r
 
 // The stored fixed-point operands of one (mode, site) and of a site's last
 // increment, from the FP64 fields.
-__device__ __forceinline__ void r2_fx_store_mode(const RateFx& rx, const Fields& f, long long i, double q0, double d0,
+__device__ __forceinline__ void r2_fx_store_mode(const RateFx& rx, long long i, double q0, double d0,
                                                  double d1, double d2, double rnorm) {
   bool ok = d1 == -d0;
   FxAcc a{rx.c_hh, rx.c_mid};
   fx_mad(a, fx_split(fx_from_f64<2>(q0, rx.sq, &ok)), rx.nb);
   const uint64_t y = (uint64_t)fx_value<kFxRateShift>(a);
   ok &= y - kFxY0Min <= kFxY0Max - kFxY0Min && rx.neg - y + (1ull << 62) < (1ull << 63);  // |Q0 log2(e)/kT| < 512
-  f.dx[i] = fx_split(fx_from_f64<3>(d0, 60, &ok));
-  f.dxy[i] = fx_split(fx_from_f64<3>(d2, 60, &ok));
-  if (f.ux) {
-    f.ux[i] = fx_split(fx_from_f64<3>(d0 * rnorm, 60, &ok));
-    f.uxy[i] = fx_split(fx_from_f64<3>(d2 * rnorm, 60, &ok));
+  rx.dx[i] = fx_split(fx_from_f64<3>(d0, 60, &ok));
+  rx.dxy[i] = fx_split(fx_from_f64<3>(d2, 60, &ok));
+  if (rx.ux) {
+    rx.ux[i] = fx_split(fx_from_f64<3>(d0 * rnorm, 60, &ok));
+    rx.uxy[i] = fx_split(fx_from_f64<3>(d2 * rnorm, 60, &ok));
   }
-  f.cq[i] = ok ? y : 0;
+  rx.cq[i] = ok ? y : 0;
 }
-__device__ __forceinline__ void r2_fx_store_prev(const Fields& f, long long N, long long s, double p0, double p1,
+__device__ __forceinline__ void r2_fx_store_prev(const RateFx& rx, long long N, long long s, double p0, double p1,
                                                  double p2) {
   const double r = 1.0 / (sqrt(p0 * p0 + p1 * p1 + 2 * p2 * p2) + kEpsilon);
   bool ok = true;
   Fx a = fx_split(fx_from_f64<2>((p0 - p1) * r, 60, &ok)), b = fx_split(fx_from_f64<2>(2 * p2 * r, 60, &ok));
   if (!ok) a = Fx{INT32_MIN, 0};
-  f.pn[s] = a;
-  f.pn[N + s] = b;
+  rx.pn[s] = a;
+  rx.pn[N + s] = b;
 }
 
 __device__ __forceinline__ unsigned long long gtimer() {
@@ -912,7 +914,7 @@ __device__ __forceinline__ double site_rate(const KParams& kp, const Fields& f, 
     return kp.vt * exp_tang(r2_arg(kp, f, d, s, m));
   } else if (MODEL == 1) {
     int64_t ufx[6];
-    Fx W[5];
+    Fx W[6];
     FxAcc a0;
     if (rx.on && g3_fx_u(rx, u, ufx) && g3_fx_site(rx, f, kp.N, ufx, s, W, &a0)) {
       const uint64_t Y = g3_fx_arg(rx, W, a0, m);
@@ -1066,59 +1068,176 @@ __device__ void search_event(const KParams& kp, const Fields& f, const RateFx& r
 }
 
 // ------------------------------------------------------------ commits
-// VoxelShearTransform (elastic.c:361-520) for the FP64 models; thread 0 only.
-template <int MODEL>
-__device__ void transform(const KParams& kp, const Fields& f, const RateFx& rx, Ctl* ctl, int mm, long long s, MT* rng) {
-  const long long N = kp.N;
-  double d[6];
-  if (MODEL == 0) {
-    const double* dd = f.deps + (long long)mm * 3 * N;
-    d[0] = dd[s]; d[1] = dd[N + s]; d[2] = dd[2 * N + s];
-  } else {
-    for (int c = 0; c < 6; c++) d[c] = kp.modes[mm][c];
-  }
-  for (int c = 0; c < kp.nc; c++) {
-    f.prev_deps[c * N + s] = d[c];
-    f.eps0[c * N + s] += d[c];
-    ctl->eps0_sum[c] += d[c];
-    ctl->pend_deps[c] = d[c];
-  }
-  if (MODEL == 0) {
-    const int ty = f.mro ? f.mro[s] : 0;
-    const double ds = d[0] * d[0] + d[1] * d[1] + 2 * d[2] * d[2];
-    double ps = f.perm_soft[s] + ds * (ty == 1 ? kp.perm_soft_mro : kp.perm_soft);
-    if (ps > kp.perm_soft_cap) ps = kp.perm_soft_cap;
-    f.perm_soft[s] = ps;
-    f.temp_soft[s] = ds * (ty == 1 ? kp.temp_soft_mro : kp.temp_soft);
-    f.tlast[s] = ctl->totime;
-    if (f.pn) r2_fx_store_prev(f, N, s, d[0], d[1], d[2]);
-    if (ty) {
-      // a crystal-like site keeps its modes and draws new barriers
-      // xQ0amp (1 - RandomRatio + RandomRatio u) (elastic.c:451-500)
-      for (int i = 0; i < STZ_MODES; i++) {
-        const double u = mt_uniform(rng);
-        const long long j = (long long)i * N + s;
-        const double q0 = __dmul_rn(kp.xq0amp, __dadd_rn(1.0 - kp.random_ratio, __dmul_rn(kp.random_ratio, u)));
-        f.Q0[j] = q0;
-        if (f.cq) {
-          const double* dd = f.deps + (long long)i * 3 * N;
-          r2_fx_store_mode(rx, f, j, q0, dd[s], dd[N + s], dd[2 * N + s], f.dnorm[j]);
-        }
+// VoxelShearTransform (elastic.c:361-520) of the FP64 models, shared out over
+// warps: one thread doing it took 60 to 100 us of the 2D model's event (40
+// Gaussians, each a rejection loop with a logarithm and a square root on a pipe
+// with a latency of some 70 clocks per operation).
+
+// The generator's refill by one warp (block_twist's four phases).
+__device__ void warp_twist(MT* g) {
+  const uint32_t UP = 0x80000000u, LO = 0x7fffffffu, A = 0x9908b0dfu;
+  const int lane = threadIdx.x & 31;
+  uint32_t* mt = g->mt;
+  const int k0[4] = {0, 227, 454, 623}, k1[4] = {227, 454, 623, 624};
+  __syncwarp();
+  for (int ph = 0; ph < 4; ph++)
+    for (int b = k0[ph]; b < k1[ph]; b += 32) {
+      const int q = b + lane;
+      const bool mine = q < k1[ph];
+      uint32_t v = 0;
+      if (mine) {
+        const uint32_t y = (mt[q] & UP) | (mt[q == 623 ? 0 : q + 1] & LO);
+        v = (q < 227 ? mt[q + 397] : mt[q - 227]) ^ (y >> 1) ^ ((y & 1u) ? A : 0u);
       }
-      return;
+      __syncwarp();
+      if (mine) mt[q] = v;
+      __syncwarp();
     }
-    // re-draw the site's modes, glass branch (elastic.c:508-512)
-    for (int i = 0; i < STZ_MODES; i++) {
-      double* dd = f.deps + (long long)i * 3 * N;
-      const double a = 0.5 * kp.gamma0 * mt_gaussian(rng, 1.0);
-      const double c2 = 0.5 * kp.gamma0 * mt_gaussian(rng, 1.0);
-      dd[s] = a;
-      dd[N + s] = -a;
-      dd[2 * N + s] = c2;
-      const long long j = (long long)i * N + s;
-      const double rn = mode_rnorm(a, -a, c2);
-      f.dnorm[j] = rn;
-      if (f.cq) r2_fx_store_mode(rx, f, j, f.Q0[j], a, -a, c2, rn);
+  if (lane == 0) g->mti = 0;
+  __syncwarp();
+}
+
+// One pair of the polar method: x, y uniform on (-1, 1), accepted inside the
+// unit circle (mt_gaussian's test).
+struct Polar {
+  double y, r2;
+  bool ok;
+};
+__device__ __forceinline__ Polar polar(uint32_t wx, uint32_t wy) {
+  const double x = -1 + 2 * (wx / 4294967296.0), y = -1 + 2 * (wy / 4294967296.0);
+  const double r2 = __dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y));
+  return Polar{y, r2, !(r2 > 1.0 || r2 == 0)};
+}
+__device__ __forceinline__ double polar_value(const Polar& p) {  // sigma = 1
+  return __dmul_rn(__dmul_rn(1.0, p.y), sqrt(-2.0 * log(p.r2) / p.r2));
+}
+
+// The next n values of mt_gaussian(g, 1.0) in order, by one warp: a round takes
+// up to 32 pairs of the generator's next words, and the words up to the last
+// value taken are consumed. A zero word, which the method rejects singly, sends
+// the round's first value through the serial form.
+__device__ void warp_gaussians(MT* g, double* out, int n) {
+  const int lane = threadIdx.x & 31;
+  int have = 0;
+  while (have < n) {
+    __syncwarp();
+    int at = g->mti;
+    __syncwarp();
+    if (at >= 624) {
+      warp_twist(g);
+      continue;
+    }
+    uint32_t wx = 1, wy = 1;
+    int pairs;
+    if (at == 623) {  // a pair across the refill
+      wx = mt_temper(g->mt[623]);
+      warp_twist(g);
+      wy = mt_temper(g->mt[0]);
+      pairs = 1;
+      at = -1;
+    } else {
+      pairs = min(32, (624 - at) / 2);
+      if (lane < pairs) {
+        wx = mt_temper(g->mt[at + 2 * lane]);
+        wy = mt_temper(g->mt[at + 2 * lane + 1]);
+      }
+    }
+    if (__any_sync(FULL, wx == 0 || wy == 0)) {
+      if (lane == 0) {
+        double v;
+        if (at < 0 && wx != 0) {  // the pair's first word is spent
+          for (;;) {
+            do { wy = mt_next(g); } while (wy == 0);
+            const Polar p = polar(wx, wy);
+            if (p.ok) { v = polar_value(p); break; }
+            do { wx = mt_next(g); } while (wx == 0);
+          }
+        } else {
+          v = mt_gaussian(g, 1.0);  // (at < 0: the first word was the rejected one)
+        }
+        out[have] = v;
+      }
+      have++;
+      continue;
+    }
+    const Polar p = polar(wx, wy);
+    const unsigned acc = __ballot_sync(FULL, lane < pairs && p.ok);
+    const int take = min(__popc(acc), n - have), rank = __popc(acc & ((1u << lane) - 1u));
+    const bool mine = (acc >> lane & 1u) && rank < take;
+    if (mine) out[have + rank] = polar_value(p);
+    const unsigned last = __ballot_sync(FULL, mine && rank == n - have - 1);
+    if (lane == 0) g->mti = at + 2 * (last ? __ffs(last) : pairs);
+    have += take;
+  }
+  __syncwarp();
+}
+
+// The random numbers of a transformation at a site of MRO type ty into sh (40
+// values): a glass site's 40 Gaussians (elastic.c:508-512), a crystal-like
+// site's 20 uniforms (elastic.c:451-500). One warp.
+__device__ void draw_site(MT* g, int ty, double* sh) {
+  if (ty == 0) {
+    warp_gaussians(g, sh, 2 * STZ_MODES);
+    return;
+  }
+  if ((threadIdx.x & 31) == 0)
+    for (int i = 0; i < STZ_MODES; i++) sh[i] = mt_uniform(g);
+  __syncwarp();
+}
+// ... and the new modes or barriers they give, lane i mode i. One warp.
+__device__ void redraw_modes(const KParams& kp, const Fields& f, const RateFx& rx, long long s, int ty,
+                             const double* sh) {
+  const int i = threadIdx.x & 31;
+  if (i >= STZ_MODES) return;
+  const long long N = kp.N, j = (long long)i * N + s;
+  double* dd = f.deps + (long long)i * 3 * N;
+  if (ty) {
+    // a crystal-like site keeps its modes and draws new barriers
+    // xQ0amp (1 - RandomRatio + RandomRatio u)
+    const double q0 = __dmul_rn(kp.xq0amp, __dadd_rn(1.0 - kp.random_ratio, __dmul_rn(kp.random_ratio, sh[i])));
+    f.Q0[j] = q0;
+    if (rx.cq) r2_fx_store_mode(rx, j, q0, dd[s], dd[N + s], dd[2 * N + s], f.dnorm[j]);
+    return;
+  }
+  const double a = 0.5 * kp.gamma0 * sh[2 * i], c2 = 0.5 * kp.gamma0 * sh[2 * i + 1];
+  dd[s] = a;
+  dd[N + s] = -a;
+  dd[2 * N + s] = c2;
+  const double rn = mode_rnorm(a, -a, c2);
+  f.dnorm[j] = rn;
+  if (rx.cq) r2_fx_store_mode(rx, j, f.Q0[j], a, -a, c2, rn);
+}
+
+// The increment of mode mm at site s: component c in lane c (before the modes
+// are redrawn).
+template <int MODEL>
+__device__ __forceinline__ double site_increment(const KParams& kp, const Fields& f, int mm, long long s) {
+  const int c = threadIdx.x & 31;
+  if (c >= kp.nc) return 0.0;
+  return MODEL == 0 ? f.deps[((long long)mm * 3 + c) * kp.N + s] : kp.modes[mm][c];
+}
+// The site's state after a transformation of increment d (lane c component c):
+// eigenstrain, last increment and softening. One warp.
+template <int MODEL>
+__device__ void transform_site(const KParams& kp, const Fields& f, const RateFx& rx, Ctl* ctl, long long s, double d, int ty) {
+  const long long N = kp.N;
+  const int c = threadIdx.x & 31;
+  if (c < kp.nc) {
+    f.prev_deps[c * N + s] = d;
+    f.eps0[c * N + s] += d;
+    ctl->eps0_sum[c] += d;
+    ctl->pend_deps[c] = d;
+  }
+  if (MODEL == 0) {
+    const double d0 = __shfl_sync(FULL, d, 0), d1 = __shfl_sync(FULL, d, 1), d2 = __shfl_sync(FULL, d, 2);
+    if (c == 0) {
+      const double ds = d0 * d0 + d1 * d1 + 2 * d2 * d2;
+      double ps = f.perm_soft[s] + ds * (ty == 1 ? kp.perm_soft_mro : kp.perm_soft);
+      if (ps > kp.perm_soft_cap) ps = kp.perm_soft_cap;
+      f.perm_soft[s] = ps;
+      f.temp_soft[s] = ds * (ty == 1 ? kp.temp_soft_mro : kp.temp_soft);
+      f.tlast[s] = ctl->totime;
+      if (rx.pn) r2_fx_store_prev(rx, N, s, d0, d1, d2);
     }
   }
 }
@@ -1145,7 +1264,6 @@ __device__ __noinline__ void finish_step(const KParams& kp, const Fields& f, con
   __shared__ long long sh_site;
   __shared__ int sh_mode;
   __shared__ double sh_margin;
-  const unsigned long long t_tail = gtimer();
   Ctl* const g = f.ctl;
   ctl_copy(&sc, g);
   // per-thread contiguous chunks of the per-(mode, group) sums, fixed order
@@ -1155,8 +1273,7 @@ __device__ __noinline__ void finish_step(const KParams& kp, const Fields& f, con
   double S = 0;
   for (long long p = p0; p < p1; p++) S += f.gsum[p];
   block_incl_scan(S, sh_inc);  // also orders the copy above
-  const unsigned long long t_sums = gtimer();
-  if (MODEL != 0) block_twist_if_needed(&sc.rng);
+  block_twist_if_needed(&sc.rng);
   Ctl* c = &sc;
   if (threadIdx.x == 0) {
     c->ticket = 0;
@@ -1198,44 +1315,51 @@ __device__ __noinline__ void finish_step(const KParams& kp, const Fields& f, con
     sh_kind = kind;
   }
   __syncthreads();
-  const unsigned long long t_dec = gtimer();
   const int kind = sh_kind;
   if (kind == kThermal) {
     search_event<MODEL>(kp, f, rx, sh_u, sh_tot, sh_T, sh_inc, &sh_site, &sh_mode, &sh_margin);
     __syncthreads();
   }
-  const unsigned long long t_search = gtimer();
-  if (threadIdx.x == 0) {
-    const double Rtrue = sh_R;
-    if (kind == kThermal) {
-      const long long s = sh_site;
-      const int m = sh_mode;
-      if (s < 0) {
-        c->status = STZ_ERR_NO_EVENT;
-        c->halt = 1;
-        c->halt_reason = kHaltError;
-        c->step_kind = kNone;
+  if (kind == kThermal && sh_site >= 0) {
+    // warp 0 draws the new modes, warp 1 the event's Q (both from the state
+    // before the transformation), warp 2 reads the increment; then each writes
+    __shared__ double sh_draw[2 * STZ_MODES];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long s = sh_site;
+    const int m = sh_mode;
+    const int ty = MODEL == 0 && f.mro ? f.mro[s] : 0;
+    double q = 0, d = 0;
+    if (MODEL == 0 && w == 0) draw_site(&c->rng, ty, sh_draw);
+    if (w == 1) q = site_Q<MODEL>(kp, f, sh_u, sh_tot, s, m);
+    if (w == 2) d = site_increment<MODEL>(kp, f, m, s);
+    __syncthreads();
+    if (MODEL == 0 && w == 0) redraw_modes(kp, f, rx, s, ty, sh_draw);
+    if (w == 1 && lane == 0) {
+      if (sh_margin < 1e-12 * sh_R) c->near_ties++;
+      c->sel_site = s;
+      c->sel_mode = m;
+      c->sel_q = q;
+      if (kp.incr64) {
+        c->incr_req = 1;  // the incremental update instead of the re-solve
+        c->pend_site = s;
       } else {
-        if (sh_margin < 1e-12 * sh_R) c->near_ties++;
-        const double q = site_Q<MODEL>(kp, f, sh_u, sh_tot, s, m);
-        c->sel_site = s;
-        c->sel_mode = m;
-        c->sel_q = q;
-        transform<MODEL>(kp, f, rx, c, m, s, &c->rng);
-        if (kp.incr64) {
-          c->incr_req = 1;  // the incremental update instead of the re-solve
-          c->pend_site = s;
-        } else {
-          c->solve_req = 1;
-        }
-        log_event(kp, f, c, STZ_EV_THERMAL, s, m, c->totime + c->t_kmc, c->t_kmc, q, Rtrue, sh_margin / sh_R, 1);
+        c->solve_req = 1;
       }
+      log_event(kp, f, c, STZ_EV_THERMAL, s, m, c->totime + c->t_kmc, c->t_kmc, q, sh_R, sh_margin / sh_R, 1);
+    }
+    if (w == 2) transform_site<MODEL>(kp, f, rx, c, s, d, ty);
+  } else if (threadIdx.x == 0) {
+    if (kind == kThermal) {
+      c->status = STZ_ERR_NO_EVENT;
+      c->halt = 1;
+      c->halt_reason = kHaltError;
+      c->step_kind = kNone;
     } else if (kind == kElastic) {
       c->estep++;
       c->totime += kp.dt;
       elastic_step(kp, c);
       c->solve_req = 0;
-      log_event(kp, f, c, STZ_EV_ELASTIC, -1, -1, c->totime, kp.dt, 0.0, Rtrue);
+      log_event(kp, f, c, STZ_EV_ELASTIC, -1, -1, c->totime, kp.dt, 0.0, sh_R);
     } else if (kind == kAthermal) {
       c->solve_req = 0;  // the athermal commit requests the solve
     }
@@ -1364,7 +1488,7 @@ __global__ void __launch_bounds__(TH, Q == 4 ? 2 : 3) k_rate64_fx(KParams kp, Fi
     const long long s1 = min(s0 + (long long)kp.bsites, kp.N);
     bool ok = sh_uok;
     unsigned neg = 0;
-    Fx W[Q][5];
+    Fx W[Q][6];
     FxAcc a0[Q];
 #pragma unroll
     for (int q = 0; q < Q; q++) {
@@ -1373,7 +1497,7 @@ __global__ void __launch_bounds__(TH, Q == 4 ? 2 : 3) k_rate64_fx(KParams kp, Fi
         ok &= g3_fx_site(rx, f, kp.N, sh_u, s, W[q], &a0[q]);
       } else {
         // no site: the smallest representable rate, 2^-1021
-        for (int c = 0; c < 5; c++) W[q][c] = Fx{0, 0};
+        for (int c = 0; c < 6; c++) W[q][c] = Fx{0, 0};
         a0[q] = FxAcc{(int64_t)1 << (53 - kFxRateShift), 0};
       }
     }
@@ -1484,10 +1608,53 @@ __global__ void __launch_bounds__(TH, 3) k_rate64_fx2(KParams kp, Fields f, Rate
 }
 
 // ------------------------------------------------------------ athermal
-// Mark every site whose lowest-barrier mode has Q < 0 or |Q| < 0.33
-// (evolution.c:55-65). mixed: Q from the FP32 deviatoric field. The FP64 forms
-// find the lowest barrier as the largest fixed-point rate argument (their FP64
-// Q's of a site out of its range).
+// Mode + 1 of a site that joins the avalanche, else 0: the mode of lowest
+// barrier, when that is below 0 or within 0.33 of it (evolution.c:55-65).
+// mixed: Q from the FP32 deviatoric field. The FP64 forms find the lowest
+// barrier as the largest fixed-point rate argument (ufx not null; their FP64
+// Q's at a site out of its range).
+__device__ int ath_site(const KParams& kp, const Fields& f, const RateFx& rx, const double* u, double totime,
+                        const int64_t* ufx, long long s, int mixed) {
+  int mm = 0;
+  if (ufx) {
+    uint64_t top = 0;
+    bool ok;
+    if (kp.model == STZ_MODEL_REF2D) {
+      R2Fx d;
+      ok = r2_fx_site(kp, rx, f, ufx, totime, s, &d);
+      for (int m = 0; m < STZ_MODES; m++) {
+        const uint64_t Y = r2_fx_arg(kp, rx, f, rx.tab, d, s, m, &ok);
+        if (Y > top) { mm = m; top = Y; }
+      }
+    } else {
+      Fx W[6];
+      FxAcc a0;
+      ok = g3_fx_site(rx, f, kp.N, ufx, s, W, &a0);
+#pragma unroll 4
+      for (int m = 0; m < STZ_MODES; m++) {
+        const uint64_t Y = g3_fx_arg(rx, W, a0, m);
+        if (Y > top) { mm = m; top = Y; }
+      }
+    }
+    if (ok) return top > rx.mark ? mm + 1 : 0;  // Q < 0.33
+    mm = 0;
+  }
+  double minQ = 0;
+  for (int m = 0; m < STZ_MODES; m++) {
+    double Q;
+    if (kp.model == STZ_MODEL_REF2D) Q = site_Q<0>(kp, f, u, totime, s, m);
+    else if (mixed) Q = site_Q<2>(kp, f, u, totime, s, m);
+    else Q = site_Q<1>(kp, f, u, totime, s, m);
+    if (m == 0 || minQ > Q) { mm = m; minQ = Q; }
+  }
+  return (minQ < 0 || fabs(minQ) < 0.33) ? mm + 1 : 0;
+}
+
+// The marks per chunk of TH sites, behind the marks.
+__device__ __forceinline__ short* mark_counts(const KParams& kp, const Fields& f) {
+  return reinterpret_cast<short*>(f.amark + (kp.N + TH - 1) / TH * TH);
+}
+// Mark the sites that join the avalanche, with the count of each chunk of TH sites.
 __global__ void k_ath_mark(KParams kp, Fields f, RateFx rx, int mixed) {
   Ctl* ctl = f.ctl;
   if (ctl->step_kind != kAthermal) return;
@@ -1497,89 +1664,76 @@ __global__ void k_ath_mark(KParams kp, Fields f, RateFx rx, int mixed) {
   const bool r2 = kp.model == STZ_MODEL_REF2D;
   int64_t ufx[6];
   const bool fx = rx.on && !mixed && (r2 ? r2_fx_u(rx, u, ufx) : g3_fx_u(rx, u, ufx));
-  for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < kp.N; s += (long long)gridDim.x * blockDim.x) {
-    int mm = 0;
-    double minQ = 0;
-    if (fx) {
-      uint64_t top = 0;
-      bool ok;
-      if (r2) {
-        R2Fx d;
-        ok = r2_fx_site(kp, rx, f, ufx, totime, s, &d);
-        for (int m = 0; m < STZ_MODES; m++) {
-          const uint64_t Y = r2_fx_arg(kp, rx, f, rx.tab, d, s, m, &ok);
-          if (Y > top) { mm = m; top = Y; }
-        }
-      } else {
-        Fx W[5];
-        FxAcc a0;
-        ok = g3_fx_site(rx, f, kp.N, ufx, s, W, &a0);
-#pragma unroll 4
-        for (int m = 0; m < STZ_MODES; m++) {
-          const uint64_t Y = g3_fx_arg(rx, W, a0, m);
-          if (Y > top) { mm = m; top = Y; }
-        }
-      }
-      if (ok) {
-        f.amark[s] = top > rx.mark ? (signed char)(mm + 1) : (signed char)0;  // Q < 0.33
-        continue;
-      }
-      mm = 0;
-    }
-    for (int m = 0; m < STZ_MODES; m++) {
-      double Q;
-      if (kp.model == STZ_MODEL_REF2D) Q = site_Q<0>(kp, f, u, totime, s, m);
-      else if (mixed) Q = site_Q<2>(kp, f, u, totime, s, m);
-      else Q = site_Q<1>(kp, f, u, totime, s, m);
-      if (m == 0 || minQ > Q) { mm = m; minQ = Q; }
-    }
-    f.amark[s] = (minQ < 0 || fabs(minQ) < 0.33) ? (signed char)(mm + 1) : (signed char)0;
+  // one chunk of TH sites per block and turn; its marks counted
+  for (long long ch = blockIdx.x; ch * TH < kp.N; ch += gridDim.x) {
+    const long long s = ch * TH + threadIdx.x;
+    int mark = 0;
+    if (s < kp.N) mark = ath_site(kp, f, rx, u, totime, fx ? ufx : nullptr, s, mixed);
+    if (s < kp.N) f.amark[s] = (signed char)mark;
+    const int n = __syncthreads_count(mark != 0);
+    if (threadIdx.x == 0) mark_counts(kp, f)[ch] = (short)n;
   }
 }
 
 // Transform the marked sites in index order (the RNG stream order of the
-// reference's space_loop); one block, thread 0 commits.
-__global__ void k_ath_commit(KParams kp, Fields f, RateFx rx, int mixed) {
+// reference's space_loop); one block. The chunks' counts lead to the marks: a
+// block-wide walk of every site's mark took 1.1 ms at 512^2.
+__global__ void __launch_bounds__(TH) k_ath_commit(KParams kp, Fields f, RateFx rx, int mixed) {
   Ctl* ctl = f.ctl;
   if (ctl->step_kind != kAthermal) return;
-  __shared__ unsigned ballot[TH / 32];
+  __shared__ unsigned ballot[TH / 32], chunks[TH / 32];
   __shared__ MT srng;
+  __shared__ double sh_draw[2 * STZ_MODES];
   {
     const uint32_t* src = reinterpret_cast<const uint32_t*>(&ctl->rng);
     uint32_t* dst = reinterpret_cast<uint32_t*>(&srng);
     for (int i = threadIdx.x; i < (int)(sizeof(MT) / 4); i += blockDim.x) dst[i] = src[i];
   }
-  __syncthreads();
   double u[6];
   for (int c = 0; c < 6; c++) u[c] = ctl->u[c];
   const double totime = ctl->totime;
   if (threadIdx.x == 0) ctl->astep++;
-  for (long long base = 0; base < kp.N; base += TH) {
-    const long long s = base + threadIdx.x;
-    const bool mk = s < kp.N && f.amark[s] != 0;
-    const unsigned bal = __ballot_sync(FULL, mk);
-    if ((threadIdx.x & 31) == 0) ballot[threadIdx.x >> 5] = bal;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool r2 = kp.model == STZ_MODEL_REF2D;
+  const long long nch = (kp.N + TH - 1) / TH;
+  for (long long cb = 0; cb < nch; cb += TH) {
+    const unsigned cbal = __ballot_sync(FULL, cb + threadIdx.x < nch && mark_counts(kp, f)[cb + threadIdx.x] != 0);
     __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int w = 0; w < TH / 32; w++) {
-        unsigned bb = ballot[w];
-        while (bb) {
-          const int lane = __ffs(bb) - 1;
-          bb &= bb - 1;
-          const long long site = base + w * 32 + lane;
-          const int mm = f.amark[site] - 1;
-          double q;
-          if (kp.model == STZ_MODEL_REF2D) q = site_Q<0>(kp, f, u, totime, site, mm);
-          else if (mixed) q = site_Q<2>(kp, f, u, totime, site, mm);
-          else q = site_Q<1>(kp, f, u, totime, site, mm);
-          if (kp.model == STZ_MODEL_REF2D) transform<0>(kp, f, rx, ctl, mm, site, &srng);
-          else transform<1>(kp, f, rx, ctl, mm, site, &srng);
-          log_event(kp, f, ctl, STZ_EV_ATHERMAL, site, mm, ctl->totime, 0.0, q, 0.0);
-        }
+    if (lane == 0) chunks[w] = cbal;
+    __syncthreads();
+    for (int cw = 0; cw < TH / 32; cw++)
+      for (unsigned cm = chunks[cw]; cm; cm &= cm - 1) {  // the same in every thread
+        const long long base = (cb + cw * 32 + __ffs(cm) - 1) * TH;
+        const long long s0 = base + threadIdx.x;
+        const unsigned bal = __ballot_sync(FULL, s0 < kp.N && f.amark[s0] != 0);
+        __syncthreads();
+        if (lane == 0) ballot[w] = bal;
+        __syncthreads();
+        for (int bw = 0; bw < TH / 32; bw++)
+          for (unsigned bb = ballot[bw]; bb; bb &= bb - 1) {
+            const long long s = base + bw * 32 + __ffs(bb) - 1;
+            const int mm = f.amark[s] - 1;
+            const int ty = r2 && f.mro ? f.mro[s] : 0;
+            double q = 0, d = 0;
+            if (r2 && w == 0) draw_site(&srng, ty, sh_draw);
+            if (w == 1) {
+              if (r2) q = site_Q<0>(kp, f, u, totime, s, mm);
+              else if (mixed) q = site_Q<2>(kp, f, u, totime, s, mm);
+              else q = site_Q<1>(kp, f, u, totime, s, mm);
+            }
+            if (w == 2) d = r2 ? site_increment<0>(kp, f, mm, s) : site_increment<1>(kp, f, mm, s);
+            __syncthreads();
+            if (r2 && w == 0) redraw_modes(kp, f, rx, s, ty, sh_draw);
+            if (w == 1 && lane == 0) log_event(kp, f, ctl, STZ_EV_ATHERMAL, s, mm, ctl->totime, 0.0, q, 0.0);
+            if (w == 2) {
+              if (r2) transform_site<0>(kp, f, rx, ctl, s, d, ty);
+              else transform_site<1>(kp, f, rx, ctl, s, d, ty);
+            }
+            __syncthreads();
+          }
       }
-    }
-    __syncthreads();
   }
+  __syncthreads();
   {
     const uint32_t* src = reinterpret_cast<const uint32_t*>(&srng);
     uint32_t* dst = reinterpret_cast<uint32_t*>(&ctl->rng);
@@ -1688,10 +1842,10 @@ __global__ void k_q0_reset(KParams kp, Fields f, RateFx rx) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
     if (f.Q0[i] != f.Q1[i]) {
       f.Q0[i] = f.Q1[i];
-      if (f.cq) {
+      if (rx.cq) {
         const long long m = i / kp.N, s = i - m * kp.N;
         const double* dd = f.deps + m * 3 * kp.N;
-        r2_fx_store_mode(rx, f, i, f.Q1[i], dd[s], dd[kp.N + s], dd[2 * kp.N + s], f.dnorm[i]);
+        r2_fx_store_mode(rx, i, f.Q1[i], dd[s], dd[kp.N + s], dd[2 * kp.N + s], f.dnorm[i]);
       }
     }
 }
@@ -3248,13 +3402,13 @@ void launch_rate_fp64(const KParams& kp, const Fields& f, const RateFx& rx, cuda
     if (kp.model == STZ_MODEL_REF2D) k_rate64<0><<<kp.nblk, TH, 0, st>>>(kp, f, rx);
     else k_rate64<1><<<kp.nblk, TH, 0, st>>>(kp, f, rx);
   } else if (kp.model == STZ_MODEL_REF2D) {
-    if (kp.bsites == TH) k_rate64_fx2<1><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
-    else if (kp.bsites == 2 * TH) k_rate64_fx2<2><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
-    else k_rate64_fx2<4><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
+    if (kp.bsites == TH) k_rate64_fx2<1><<<rx.grid, TH, 0, st>>>(kp, f, rx);
+    else if (kp.bsites == 2 * TH) k_rate64_fx2<2><<<rx.grid, TH, 0, st>>>(kp, f, rx);
+    else k_rate64_fx2<4><<<rx.grid, TH, 0, st>>>(kp, f, rx);
   } else {
-    if (kp.bsites == TH) k_rate64_fx<1><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
-    else if (kp.bsites == 2 * TH) k_rate64_fx<2><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
-    else k_rate64_fx<4><<<kp.rate_grid, TH, 0, st>>>(kp, f, rx);
+    if (kp.bsites == TH) k_rate64_fx<1><<<rx.grid, TH, 0, st>>>(kp, f, rx);
+    else if (kp.bsites == 2 * TH) k_rate64_fx<2><<<rx.grid, TH, 0, st>>>(kp, f, rx);
+    else k_rate64_fx<4><<<rx.grid, TH, 0, st>>>(kp, f, rx);
   }
 }
 
@@ -3395,21 +3549,21 @@ void launch_mixed_tail(const KParams& kp, const Fields& f, int update_only, cuda
   else launch_pdl(k_mixed_select, dim3(kp.n0), 0, st, kp, f);
 }
 
-// The stored mode norms of every (mode, site) from the mode increments.
-__global__ void k_mode_norms(KParams kp, Fields f) {
-  const long long N = kp.N, total = (long long)STZ_MODES * N;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long m = i / N, s = i - m * N;
+// The stored norms of the modes m0 .. m0 + nm - 1 at every site, from the mode
+// increments.
+__global__ void k_mode_norms(KParams kp, Fields f, int m0, int nm) {
+  const long long N = kp.N, total = nm * N;
+  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < total;
+       k += (long long)gridDim.x * blockDim.x) {
+    const long long i = m0 * N + k, m = i / N, s = i - m * N;
     const double* dd = f.deps + m * 3 * N;
     f.dnorm[i] = mode_rnorm(dd[s], dd[N + s], dd[2 * N + s]);
   }
 }
 
-void launch_mode_norms(const KParams& kp, const Fields& f, cudaStream_t st) {
-  const long long total = (long long)STZ_MODES * kp.N;
-  const unsigned nb = (unsigned)std::min<long long>((total + TH - 1) / TH, 152LL * 16);
-  k_mode_norms<<<nb, TH, 0, st>>>(kp, f);
+void launch_mode_norms(const KParams& kp, const Fields& f, int m0, int nm, cudaStream_t st) {
+  const unsigned nb = (unsigned)std::min<long long>((nm * kp.N + TH - 1) / TH, 152LL * 16);
+  k_mode_norms<<<nb, TH, 0, st>>>(kp, f, m0, nm);
 }
 
 // The fixed-point operands of the modes m0 .. m0 + nm - 1 at every site and, with
@@ -3420,11 +3574,11 @@ __global__ void k_r2_fixed(KParams kp, Fields f, RateFx rx, int m0, int nm, int 
   for (long long k = t; k < total; k += nt) {
     const long long i = m0 * N + k, m = i / N, s = i - m * N;
     const double* dd = f.deps + m * 3 * N;
-    r2_fx_store_mode(rx, f, i, f.Q0[i], dd[s], dd[N + s], dd[2 * N + s], f.dnorm[i]);
+    r2_fx_store_mode(rx, i, f.Q0[i], dd[s], dd[N + s], dd[2 * N + s], f.dnorm[i]);
   }
-  if (prev && f.pn)
+  if (prev && rx.pn)
     for (long long s = t; s < N; s += nt)
-      r2_fx_store_prev(f, N, s, f.prev_deps[s], f.prev_deps[N + s], f.prev_deps[2 * N + s]);
+      r2_fx_store_prev(rx, N, s, f.prev_deps[s], f.prev_deps[N + s], f.prev_deps[2 * N + s]);
 }
 
 void launch_r2_fixed(const KParams& kp, const Fields& f, const RateFx& rx, int m0, int nm, int prev, cudaStream_t st) {

@@ -45,8 +45,9 @@ void launch_mixed_batched(const BatchDesc* d, const int* blk_rep, const int* rep
 int mixed_blocks_per_sm(int n2);
 // Dynamic shared memory of one mixed-form main block for lines of n2 sites.
 size_t mixed_smem(int n2);
-// the stored mode norms of the 2D model, after its mode increments were written
-void launch_mode_norms(const KParams& kp, const Fields& f, cudaStream_t st);
+// the stored norms of the 2D model's modes m0 .. m0 + nm - 1, after their
+// increments were written
+void launch_mode_norms(const KParams& kp, const Fields& f, int m0, int nm, cudaStream_t st);
 // the fixed-point operands of the 2D model's modes and barriers m0 .. m0 + nm - 1
 // and (prev) of its sites' last increments, after the FP64 fields were written
 void launch_r2_fixed(const KParams& kp, const Fields& f, const RateFx& rx, int m0, int nm, int prev, cudaStream_t st);

@@ -111,14 +111,6 @@ struct Fields {
   double* Q0 = nullptr;      // [MODES][N] (REF2D)
   double* deps = nullptr;    // [MODES][3][N] (REF2D)
   double* dnorm = nullptr;   // [MODES][N] 1 / (|deps| + eps) of each mode (REF2D), kept with deps
-  // REF2D in fixed point (R2Fx), kept with Q0, deps and prev_deps
-  uint64_t* cq = nullptr;    // [MODES][N] log2(vt) + 1022 - Q0 log2(e)/kT, x 2^53; 0: a value of
-                             // the (mode, site) does not fit
-  Fx* dx = nullptr;          // [MODES][N] deps xx and xy, x 2^60 (the modes are traceless)
-  Fx* dxy = nullptr;
-  Fx* ux = nullptr;          // [MODES][N] deps xx and xy over the mode's norm, x 2^60 (softening only)
-  Fx* uxy = nullptr;
-  Fx* pn = nullptr;          // [2][N] (xx - yy) and 2 xy of the last increment over its norm, x 2^60
   double* rtab64 = nullptr;  // [nc][nc][N] FP64 incremental form: stress component c of the
                              // solve of a unit eigenstrain component k at site 0, ebar = 0
   int8_t* mro = nullptr;     // [N] crystal-like MRO type 0..3 (REF2D); null for an all-glass map
@@ -128,7 +120,8 @@ struct Fields {
   double* perm_soft = nullptr;
   double* temp_soft = nullptr;
   double* tlast = nullptr;
-  signed char* amark = nullptr; // [N] athermal marks (mode+1, 0 = none)
+  signed char* amark = nullptr; // [N] athermal marks (mode+1, 0 = none), then the marks per chunk
+                                // of kRateThreads sites (mark_counts, kmc.cu)
   double* part = nullptr;    // [MODES][nblk] per (mode, block) rate sums
   double* gsum = nullptr;    // [MODES][ngroups] per (mode, group of blocks) sums
   unsigned* gticket = nullptr;  // [ngroups] last-block counters of the groups
@@ -160,7 +153,6 @@ struct KParams {
   long long N, Nk;
   int nblk, bsites;          // rate kernel: blocks and sites per block
   int ngroups;               // groups of kGroup blocks
-  int rate_grid;             // resident blocks of the fixed-point rate kernel (at most nblk)
   int mx_c1, mx_units;       // mixed form: d1 chunks per d0, units (kt0 * mx_c1)
   unsigned c1_magic;         // ceil(2^32 / mx_c1), for the division of unit indices
   int adv_q2, adv_r2;        // kRateThreads sites = adv_q2 rows of n2 plus adv_r2 sites
