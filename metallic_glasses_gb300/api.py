@@ -214,9 +214,10 @@ class Engine:
         return scalars_dict(s)
 
     def events(self, first=0, count=None):
-        total = self.scalars()["n_events_logged"]
         if count is None:
-            count = max(0, total - first)
+            s = Scalars()
+            _check(self.lib.stz_get_scalars(self.h, C.byref(s)))
+            count = max(0, s.n_events_logged - first)
         out = np.zeros(count, dtype=EVENT_DTYPE)
         n = C.c_int64()
         _check(self.lib.stz_get_events(self.h, first, out.ctypes.data, count, C.byref(n)))

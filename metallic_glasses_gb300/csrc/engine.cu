@@ -513,7 +513,7 @@ void enqueue_plain_step(stz_ctx* c, cudaEvent_t t0 = nullptr, cudaEvent_t t1 = n
     c->launches += 1;
   }
   launch_post_b(kp, f, c->stream);
-  c->launches += 1 + 2 + 2 + 1;
+  c->launches += 1 + 2 + 1 + 1;
 }
 
 int sync_ctl(stz_ctx* c) {
@@ -522,17 +522,28 @@ int sync_ctl(stz_ctx* c) {
   CK(cudaMemcpyAsync(&c->host_ctl, c->f.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   c->d2h_bytes += sizeof(Ctl);
+  c->ctl_clean = true;
   return STZ_OK;
 }
 
-int drain_log(stz_ctx* c) {
+// Steps (events) that a run may do between two looks at the log, at most.
+constexpr int kRunSteps = 64;
+
+// The log entries that `steps` steps write at most: an avalanche logs each site once.
+long long log_need(const stz_ctx* c, long long steps) { return steps * (c->kp.N + 1); }
+
+// New log entries to the host. The device learns that their slots are free at
+// once, or, when `later` is set, as long as the ring holds what the next part
+// of the run may write, when the next run starts.
+int drain_log(stz_ctx* c, bool later = false) {
   Ctl& h = c->host_ctl;
   const long long cap = c->kp.log_cap;
-  long long from = h.log_base, to = h.nlog;
-  if (to > from) {
+  long long i = c->drained;
+  const long long to = h.nlog;
+  if (to > i) {
     const size_t old = c->host_log.size();
+    const long long from = i;
     c->host_log.resize(old + (size_t)(to - from));
-    long long i = from;
     while (i < to) {
       const long long slot = i % cap;
       const long long n = std::min(to - i, cap - slot);
@@ -541,6 +552,10 @@ int drain_log(stz_ctx* c) {
       c->d2h_bytes += (int64_t)sizeof(stz_event) * n;
       i += n;
     }
+    c->drained = to;
+    CK(cudaStreamSynchronize(c->stream));
+  }
+  if (h.log_base < to && !(later && cap - (to - h.log_base) >= log_need(c, kRunSteps))) {
     h.log_base = to;
     CK(cudaMemcpyAsync(&c->f.ctl->log_base, &h.log_base, sizeof(long long), cudaMemcpyHostToDevice, c->stream));
     c->h2d_bytes += sizeof(long long);
@@ -549,38 +564,123 @@ int drain_log(stz_ctx* c) {
   return STZ_OK;
 }
 
+// The control block and the new log entries after a part of a run, with one
+// wait in the usual case: the next kPinEvents slots of the ring travel along
+// with the control block (88 bytes each), into pinned memory.
+constexpr int kPinEvents = 64;
+}  // namespace
+}  // namespace stz
+struct Pinned {
+  stz::Ctl ctl;
+  stz_event ev[stz::kPinEvents];
+};
+namespace stz {
+namespace {
+int sync_run(stz_ctx* c) {
+  if (!c->pin) {
+    const int st = sync_ctl(c);
+    return st ? st : drain_log(c);
+  }
+  CK(cudaGetLastError());
+  const long long cap = c->kp.log_cap, slot = c->drained % cap, n = std::min<long long>(kPinEvents, cap - slot);
+  CK(cudaMemcpyAsync(&c->pin->ctl, c->f.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(c->pin->ev, c->f.log + slot, sizeof(stz_event) * n, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  c->d2h_bytes += sizeof(Ctl) + (int64_t)sizeof(stz_event) * n;
+  c->host_ctl = c->pin->ctl;
+  c->ctl_clean = true;
+  const long long have = std::min(n, c->host_ctl.nlog - c->drained);
+  if (have > 0) {
+    c->host_log.insert(c->host_log.end(), c->pin->ev, c->pin->ev + have);
+    c->drained += have;
+  }
+  return drain_log(c, true);
+}
+
 int set_targets(stz_ctx* c, long long max_kstep, long long max_step) {
   Ctl& h = c->host_ctl;
+  h.log_base = c->drained;
   h.max_kstep = max_kstep;
   h.max_step = max_step;
   h.halt = h.stopped ? 1 : 0;
   h.halt_reason = h.stopped ? kHaltStop : kHaltNone;
-  CK(cudaMemcpyAsync(&c->f.ctl->max_kstep, &h.max_kstep, sizeof(long long) * 2, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(&c->f.ctl->halt, &h.halt, sizeof(int) * 2, cudaMemcpyHostToDevice, c->stream));
-  c->h2d_bytes += sizeof(long long) * 2 + sizeof(int) * 2;
+  const RunTargets t{h.log_base, h.max_kstep, h.max_step, h.halt, h.halt_reason};
+  static_assert(offsetof(Ctl, halt_reason) - offsetof(Ctl, log_base) == offsetof(RunTargets, halt_reason), "one copy");
+  CK(cudaMemcpyAsync(&c->f.ctl->log_base, &t, sizeof(t), cudaMemcpyHostToDevice, c->stream));
+  c->h2d_bytes += sizeof(t);
+  c->ctl_clean = false;
   return STZ_OK;
 }
 
-int capture_plain_graph(stz_ctx* c, int steps) {
-  if (c->graph && c->graph_batch == steps) return STZ_OK;
-  if (c->graph) { cudaGraphExecDestroy(c->graph); c->graph = nullptr; }
-  cudaGraph_t g;
-  const int64_t l0 = c->launches;
-  CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-  for (int i = 0; i < steps; i++) {
-    if (c->kp.nc == 6 && c->f.sdev) {
+// Steps of the graphs that a run of the FP64 forms is launched in.
+constexpr int kGraphSteps[3] = {1, 4, 16};
+
+// `n` driver steps (mixed: events), one after another.
+void enqueue_each(stz_ctx* c, int n) {
+  for (int i = 0; i < n; i++) {
+    if (c->f.sdev) {
       launch_mixed(c->kp, c->f, 0, c->stream);
       c->launches += kMixedLaunches;
     } else {
       enqueue_plain_step(c);
     }
   }
-  CK(cudaStreamEndCapture(c->stream, &g));
-  c->graph_launches = c->launches - l0;
-  c->launches = l0;
-  CK(cudaGraphInstantiate(&c->graph, g, 0));
-  cudaGraphDestroy(g);
-  c->graph_batch = steps;
+}
+
+// `n` copies of graph `which` of `steps` steps. The first time the steps are
+// launched one by one and the graph is captured while the device works on them
+// (0.5 ms for 64 mixed events, which a first run would wait for otherwise).
+int enqueue_graph(stz_ctx* c, int which, int steps, int n) {
+  if (n <= 0) return STZ_OK;
+  if (!c->use_graph) {
+    enqueue_each(c, n * steps);
+    return STZ_OK;
+  }
+  if (!c->graph[which]) {
+    enqueue_each(c, steps);
+    n--;
+    cudaGraph_t g;
+    const int64_t l0 = c->launches;
+    CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+    enqueue_each(c, steps);
+    CK(cudaStreamEndCapture(c->stream, &g));
+    c->graph_launches[which] = c->launches - l0;
+    c->launches = l0;
+    CK(cudaGraphInstantiate(&c->graph[which], g, 0));
+    cudaGraphDestroy(g);
+  }
+  for (int i = 0; i < n; i++) {
+    if (cudaGraphLaunch(c->graph[which], c->stream) != cudaSuccess) {
+      set_error("graph launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+      return STZ_ERR_CUDA;
+    }
+    c->launches += c->graph_launches[which];
+  }
+  return STZ_OK;
+}
+
+// Enqueues the next part of a run of which at least `left` steps (events) are
+// to be done (< 0: no limit). Steps past the target return at once, but each
+// costs its kernels' launches (about 1 us each: eleven in an FP64 step), so a
+// short run takes the small graphs: a single step of the 2D model at 64^2
+// took 371 us with the other 15 steps of one 16-step graph behind it, 127 us
+// now. The mixed form has one wait per 64 events (its re-solves and prints are
+// serviced there), and launches fewer than 33 events one by one: the host
+// enqueues an event in less time than the device needs for it.
+int enqueue_run(stz_ctx* c, long long left) {
+  if (c->f.sdev) {
+    if (left < 0 || left > kRunSteps / 2) return enqueue_graph(c, 2, kRunSteps, 1);
+    enqueue_each(c, (int)left);
+    return STZ_OK;
+  }
+  // as many as the log ring holds the avalanches of (16 where it does not hold
+  // that many either)
+  const int most = c->kp.log_cap >= log_need(c, kRunSteps) ? kRunSteps : 16;
+  int n = left < 0 || left > most ? most : (int)left, st;
+  for (int g = 2; g >= 0; g--) {
+    if ((st = enqueue_graph(c, g, kGraphSteps[g], n / kGraphSteps[g]))) return st;
+    n %= kGraphSteps[g];
+  }
   return STZ_OK;
 }
 
@@ -588,6 +688,7 @@ int capture_plain_graph(stz_ctx* c, int steps) {
 // must stop (target, stop condition or error).
 int mixed_service(stz_ctx* c, int* done) {
   Ctl& h = c->host_ctl;
+  c->ctl_clean = false;
   const KParams& kp = c->kp;
   const Fields& f = c->f;
   *done = 0;
@@ -606,7 +707,7 @@ int mixed_service(stz_ctx* c, int* done) {
       launch_mixed_after_resolve(kp, f, 0, c->stream);
     }
     launch_post_b(kp, f, c->stream);
-    c->launches += 6;
+    c->launches += 5;
   } else {
     if (kp.resolve_period > 0 && h.kstep >= h.next_resolve) {
       // periodic full re-solve: bring the FP32 field up to date, re-solve it
@@ -792,6 +893,10 @@ int stz::create_ctx(const stz_params* pin, stz_ctx** out, int units_per_block) {
     return code;
   };
   if ((st = dalloc(&f.ctl, 1))) return fail(st);
+  if (units_per_block == 0 && cudaHostAlloc((void**)&c->pin, sizeof(Pinned), cudaHostAllocDefault) != cudaSuccess) {
+    (void)cudaGetLastError();  // runs read back through pageable memory then
+    c->pin = nullptr;
+  }
   if ((st = dalloc(&f.eps0, (size_t)nc * N))) return fail(st);
   if ((st = dalloc(&f.prev_deps, (size_t)nc * N))) return fail(st);
   {
@@ -930,7 +1035,9 @@ extern "C" void stz_destroy(stz_ctx* c) {
     fft_plan_destroy(plan_of(c));
     delete plan_of(c);
   }
-  if (c->graph) cudaGraphExecDestroy(c->graph);
+  for (cudaGraphExec_t g : c->graph)
+    if (g) cudaGraphExecDestroy(g);
+  if (c->pin) cudaFreeHost(c->pin);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   if (c->kev0) cudaEventDestroy(c->kev0);
@@ -943,30 +1050,20 @@ extern "C" int stz_run(stz_ctx* c, int64_t max_steps, int64_t max_events) {
   if (!c) return STZ_ERR_INVALID;
   int st;
   cudaSetDevice(c->p.device);
-  if ((st = sync_ctl(c))) return st;
+  if (!c->ctl_clean && (st = sync_ctl(c))) return st;
   Ctl& h = c->host_ctl;
   if (h.status) return h.status;
   const long long tk = max_events > 0 ? h.kstep + max_events : -1;
   const long long ts = max_steps > 0 ? h.step + max_steps : -1;
   if ((st = set_targets(c, tk, ts))) return st;
   const bool mixed = c->f.sdev != nullptr;
-  const int batch = mixed ? 64 : 16;
-  if (c->use_graph && (st = capture_plain_graph(c, batch))) return st;
   for (;;) {
-    if (c->use_graph) {
-      if (cudaGraphLaunch(c->graph, c->stream) != cudaSuccess) {
-        set_error("graph launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-        return STZ_ERR_CUDA;
-      }
-      c->launches += c->graph_launches;
-    } else {
-      for (int i = 0; i < batch; i++) {
-        if (mixed) { launch_mixed(c->kp, c->f, 0, c->stream); c->launches += kMixedLaunches; }
-        else enqueue_plain_step(c);
-      }
-    }
-    if ((st = sync_ctl(c))) return st;
-    if ((st = drain_log(c))) return st;
+    // steps still to do: to the nearer of the two targets at least
+    long long left = ts >= 0 ? ts - h.step : -1;
+    if (tk >= 0 && (left < 0 || tk - h.kstep < left)) left = tk - h.kstep;
+    c->ctl_clean = false;
+    if ((st = enqueue_run(c, left < 0 ? left : std::max<long long>(left, 1)))) return st;
+    if ((st = sync_run(c))) return st;
     if (h.status) { set_error("device reported status %d", h.status); return h.status; }
     if (mixed && h.halt) {
       int done = 0;
@@ -982,6 +1079,7 @@ extern "C" int stz_run(stz_ctx* c, int64_t max_steps, int64_t max_events) {
 
 extern "C" int stz_solve(stz_ctx* c) {
   if (!c) return STZ_ERR_INVALID;
+  c->ctl_clean = false;
   cudaSetDevice(c->p.device);
   if (c->f.sdev) {
     solve_dev(c, c->f.ctl->eps_avg, nullptr, c->f.scratch);
@@ -1009,7 +1107,7 @@ extern "C" int stz_solve(stz_ctx* c) {
 extern "C" int stz_get_scalars(stz_ctx* c, stz_scalars* o) {
   if (!c || !o) return STZ_ERR_INVALID;
   cudaSetDevice(c->p.device);
-  int st = sync_ctl(c);
+  const int st = c->ctl_clean ? STZ_OK : sync_ctl(c);
   if (st) return st;
   const Ctl& h = c->host_ctl;
   std::memset(o, 0, sizeof(*o));
@@ -1110,6 +1208,7 @@ extern "C" int stz_get_field(stz_ctx* c, int32_t which, int32_t comp, double* ho
   }
   if (which == STZ_FIELD_SDEV) {
     if (!c->f.sdev || comp < 0 || comp >= 5) return STZ_ERR_INVALID;
+    c->ctl_clean = false;
     launch_mixed(c->kp, c->f, 1, c->stream);  // apply the pending update
     std::vector<float> hf((size_t)N);
     CK(cudaMemcpyAsync(hf.data(), c->f.sdev + (size_t)comp * N, sizeof(float) * N, cudaMemcpyDeviceToHost, c->stream));
@@ -1134,7 +1233,7 @@ extern "C" int stz_get_field(stz_ctx* c, int32_t which, int32_t comp, double* ho
     cudaMemcpyAsync(host, tmp + (size_t)comp * N, sizeof(double) * N, cudaMemcpyDeviceToHost, c->stream);
     CK(cudaStreamSynchronize(c->stream));
     cudaFree(tmp);
-    sync_ctl(c);
+    if (!c->ctl_clean) sync_ctl(c);
     for (long long s = 0; s < N; s++) host[s] += c->host_ctl.u[comp];
     return STZ_OK;
   }
@@ -1145,7 +1244,7 @@ extern "C" int stz_get_field(stz_ctx* c, int32_t which, int32_t comp, double* ho
   CK(cudaMemcpyAsync(host, d64, sizeof(double) * N, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   if (which == STZ_FIELD_SIGMA) {
-    sync_ctl(c);
+    if (!c->ctl_clean) sync_ctl(c);
     for (long long s = 0; s < N; s++) host[s] += c->host_ctl.u[comp];
   }
   return STZ_OK;
@@ -1393,6 +1492,7 @@ extern "C" int stz_kernel_time(stz_ctx* c, int32_t which, double* ms_avg, int64_
   cudaSetDevice(c->p.device);
   int st = sync_ctl(c);
   if (st) return st;
+  c->ctl_clean = false;
   const int steps = launches && *launches > 0 ? (int)*launches : 64;
   const bool mixed = c->f.sdev != nullptr;
   if (!mixed) {
@@ -1414,6 +1514,7 @@ extern "C" int stz_kernel_time(stz_ctx* c, int32_t which, double* ms_avg, int64_
       if ((st = sync_ctl(c))) return st;
       if ((st = drain_log(c))) return st;
       if (h.status) return h.status;
+      c->ctl_clean = false;
     }
     *ms_avg = n ? tot / n : 0;
     if (launches) *launches = n;
@@ -1632,7 +1733,10 @@ extern "C" int stz_batch_run(stz_batch* b, int64_t events) {
       return STZ_ERR_CUDA;
     }
     b->launches += kMixedLaunches * rounds;
-    for (stz_ctx* c : b->reps) c->launches += kMixedLaunches * rounds;
+    for (stz_ctx* c : b->reps) {
+      c->launches += kMixedLaunches * rounds;
+      c->ctl_clean = false;
+    }
     since_drain += rounds;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(b->h_status.data(), b->d_status, sizeof(stz::BatchStatus) * n, cudaMemcpyDeviceToHost,

@@ -1768,12 +1768,10 @@ __global__ void k_post_a(KParams kp, Fields f) {
       subtract_error(kp, ctl, 1, ts);
       for (int c = 0; c < kp.nc; c++) ctl->eps_avg[c] -= ts[c];
     }
-  } else {
-    ctl->solve_req = 0;
-    return;
   }
-  ctl->print_done = 0;
-  ctl->solve_req = 0;
+  // the print check after every step kind; requests the print's re-solve
+  ctl->print_done = kind != kNone ? print_check(kp, ctl) : 0;
+  ctl->solve_req = ctl->print_done;
 }
 
 // FP64 incremental form, after a thermal event: the field the re-solve would
@@ -1824,14 +1822,6 @@ __global__ void k_incr64_done(Fields f) {
 __global__ void k_note_solve(Fields f, const int* gate, const double* ebar) {
   if (gate && !*gate) return;
   for (int c = 0; c < 6; c++) f.ctl->ebar_solved[c] = ebar[c];
-}
-
-// print check after every step kind; requests the print re-solve
-__global__ void k_post_print(KParams kp, Fields f) {
-  Ctl* ctl = f.ctl;
-  if (ctl->step_kind == kNone) return;
-  ctl->print_done = print_check(kp, ctl);
-  ctl->solve_req = ctl->print_done;
 }
 
 // The print's reset of the barriers to their initial copy (bmg.c:214-221),
@@ -3605,7 +3595,6 @@ void launch_athermal(const KParams& kp, const Fields& f, const RateFx& rx, int m
 
 void launch_post_a(const KParams& kp, const Fields& f, cudaStream_t st) {
   k_post_a<<<1, TH, 0, st>>>(kp, f);
-  k_post_print<<<1, 1, 0, st>>>(kp, f);
 }
 
 void launch_post_b(const KParams& kp, const Fields& f, cudaStream_t st) { k_post_b<<<1, TH, 0, st>>>(kp, f); }

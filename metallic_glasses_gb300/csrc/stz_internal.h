@@ -70,8 +70,12 @@ struct Ctl {
   double sel_q;              // Q of the last selected (site, mode)
   long long step, kstep, astep, estep, n_print;
   long long nlog, nlog_dropped, near_ties;
-  long long log_base;        // first log entry not yet copied to the host
-  long long max_kstep, max_step;  // halt targets (absolute), < 0 = none
+  // written by the host before a run, in one copy (RunTargets): the first log entry
+  // whose slot may not be reused yet, the halt targets (absolute, < 0 = none) and
+  // the halt state
+  long long log_base;
+  long long max_kstep, max_step;
+  int halt, halt_reason;
   long long next_resolve;    // mixed: kstep at which the periodic re-solve is due
   unsigned long long neg_count;   // (mode, site) pairs with Q < 0 this step
   int step_kind;
@@ -79,7 +83,6 @@ struct Ctl {
   int print_done;            // the print of this step re-solved the field
   int stopped;
   int status;                // sticky STZ_* error
-  int halt, halt_reason;
   int has_pend;              // incremental path: a transformation is pending
   int pend_mode;
   long long pend_site;
@@ -98,6 +101,11 @@ struct Ctl {
   unsigned long long prof_part_ns[8];  // tail: copy-in+sums, twist+decision, search, commit,
                                        // search levels (mode, plane), line, site
   MT rng;
+};
+
+struct RunTargets {
+  long long log_base, max_kstep, max_step;
+  int halt, halt_reason;
 };
 
 // Device fields. Layout: component-major structure of arrays, site index
@@ -225,7 +233,7 @@ struct stz_ctx {
   void* fft = nullptr;               // FFT plan (fft.cu)
   int64_t launches = 0;
   std::vector<stz_event> host_log;   // drained events
-  long long drained = 0;
+  long long drained = 0;             // log entries copied to host_log
   stz::Ctl host_ctl{};
   double ktime_ms = 0;
   int64_t ktime_n = 0;
@@ -234,9 +242,10 @@ struct stz_ctx {
   std::vector<double> lam_h, mu_h;    // host copies of the site moduli (empty until set)
   std::vector<int8_t> mro_h;          // REF2D crystal-like MRO map (types) and its angles
   std::vector<double> mro_theta_h;
-  cudaGraphExec_t graph = nullptr;
-  int graph_batch = 0;
-  int64_t graph_launches = 0;        // kernels per graph launch
+  cudaGraphExec_t graph[3] = {};     // graphs of 1, 4 and 16 FP64 steps, or [2] of 64 mixed events,
+  int64_t graph_launches[3] = {};    // captured when a run first wants them; kernels of each
+  struct Pinned* pin = nullptr;      // landing area of what a run reads back (not for batch members)
+  bool ctl_clean = false;            // host_ctl is the device's control block
   void* l2buf = nullptr;
   size_t l2flush_bytes = 0;
   double* qbuf = nullptr;            // [N] activation energies of one mode (stz_get_field)

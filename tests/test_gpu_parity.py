@@ -608,3 +608,34 @@ def test_fixed_point_2d_rates_match_fp64_rates(engine_lib, shape, scheme, mro, o
     if neg == 0:
         assert abs(ev["total_rate"][0] / R - 1) < 3e-13
     eng.close()
+
+
+@pytest.mark.parametrize("form", ["ref2d", "incremental", "mixed"])
+@pytest.mark.parametrize("cap", [0, 256])
+def test_runs_of_any_length_join(engine_lib, form, cap):
+    """A run in parts that take every size of launch (one step, the graphs, a
+    whole turn and its remainders) and one run of the same length give the same
+    events and the same state, with the default ring of log entries and with a
+    ring that wraps."""
+    p = configs.ref2d(36, 48) if form == "ref2d" else configs.shear64(n=24)
+    if form != "ref2d":
+        p.solver = api.SOLVER_KERNEL
+    if form == "mixed":
+        p.precision = api.PREC_MIXED
+    p.log_capacity = cap
+    one, parts = api.Engine(p), api.Engine(p)
+    lengths = [1, 1, 3, 5, 16, 17, 33, 64, 65, 129, 1]
+    one.run(max_steps=sum(lengths))
+    for n in lengths:
+        parts.run(max_steps=n)
+        assert len(parts.events()) == parts.scalars()["n_events_logged"]
+    a, b = one.scalars(), parts.scalars()
+    assert a["step"] == b["step"] == sum(lengths)
+    assert a["n_events_logged"] == b["n_events_logged"]
+    assert a["log_dropped"] == b["log_dropped"] == 0
+    assert (one.events() == parts.events()).all()
+    for k in ("time", "kstep", "astep"):
+        assert a[k] == b[k]
+    assert (one.field(api.FIELD_SIGMA, 0) == parts.field(api.FIELD_SIGMA, 0)).all()
+    one.close()
+    parts.close()
