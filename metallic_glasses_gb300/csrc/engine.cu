@@ -506,14 +506,12 @@ void enqueue_plain_step(stz_ctx* c, cudaEvent_t t0 = nullptr, cudaEvent_t t1 = n
     launch_incr64(kp, f, c->stream);
     c->launches += 2;
   }
-  launch_post_a(kp, f, c->stream);
-  solve_plain(c, gate, ebar);
+  launch_post(kp, f, c->stream);
   if (f.Q1) {
     launch_q0_reset(kp, f, c->rx, c->stream);
     c->launches += 1;
   }
-  launch_post_b(kp, f, c->stream);
-  c->launches += 1 + 2 + 1 + 1;
+  c->launches += 1 + 2 + 1;
 }
 
 int sync_ctl(stz_ctx* c) {
@@ -663,7 +661,7 @@ int enqueue_graph(stz_ctx* c, int which, int steps, int n) {
 // to be done (< 0: no limit). Steps past the target return at once, but each
 // costs its kernels' launches (about 1 us each: eleven in an FP64 step), so a
 // short run takes the small graphs: a single step of the 2D model at 64^2
-// took 371 us with the other 15 steps of one 16-step graph behind it, 127 us
+// took 371 us with the other 15 steps of one 16-step graph behind it, 123 us
 // now. The mixed form has one wait per 64 events (its re-solves and prints are
 // serviced there), and launches fewer than 33 events one by one: the host
 // enqueues an event in less time than the device needs for it.
@@ -699,14 +697,14 @@ int mixed_service(stz_ctx* c, int* done) {
     launch_athermal(kp, f, c->rx, 1, c->stream);
     solve_dev(c, f.ctl->eps_avg, nullptr, f.scratch);
     launch_mixed_after_resolve(kp, f, 0, c->stream);
-    launch_post_a(kp, f, c->stream);
+    launch_post(kp, f, c->stream);
     int st = sync_ctl(c);
     if (st) return st;
     if (h.print_done) {
       solve_dev(c, f.ctl->eps_avg, nullptr, f.scratch);
       launch_mixed_after_resolve(kp, f, 0, c->stream);
+      launch_post(kp, f, c->stream);
     }
-    launch_post_b(kp, f, c->stream);
     c->launches += 5;
   } else {
     if (kp.resolve_period > 0 && h.kstep >= h.next_resolve) {
@@ -734,7 +732,7 @@ int mixed_service(stz_ctx* c, int* done) {
     if (h.print_done) {
       solve_dev(c, f.ctl->eps_avg, nullptr, f.scratch);
       launch_mixed_after_resolve(kp, f, 0, c->stream);
-      launch_post_b(kp, f, c->stream);
+      launch_post(kp, f, c->stream);
       c->launches += 2;
     }
   }
@@ -1504,13 +1502,16 @@ extern "C" int stz_kernel_time(stz_ctx* c, int32_t which, double* ms_avg, int64_
     if ((st = set_targets(c, -1, h.step + steps))) return st;
     double tot = 0;
     int n = 0;
-    for (int i = 0; i < steps && !h.halt && !h.stopped; i++) {
+    for (int i = 0; i < 2 * steps && !h.halt && !h.stopped; i++) {
+      const bool print = h.step_kind == kPrint;  // the second half of a step
       enqueue_plain_step(c, c->kev0, c->kev1);
       CK(cudaStreamSynchronize(c->stream));
       float ms = 0;
       CK(cudaEventElapsedTime(&ms, c->kev0, c->kev1));
-      tot += ms;
-      n++;
+      if (!print) {
+        tot += ms;
+        n++;
+      }
       if ((st = sync_ctl(c))) return st;
       if ((st = drain_log(c))) return st;
       if (h.status) return h.status;

@@ -9,9 +9,10 @@
 //                (evolution.c:136-193) and commits it (elastic.c:361-520)
 //   k_ath_mark, k_ath_commit   athermal avalanche (evolution.c:47-100)
 //   FFT solve    fft.cu
-//   k_post_a     loading, clock and print check (evolution.c:262-358, bmg.c:181-187)
-//   FFT solve    print re-solve (bmg.c:292-295), skipped unless printing
-//   k_post_b     stop conditions (bmg.c:382-410) and run targets
+//   k_post       loading, clock and print check (evolution.c:262-358, bmg.c:181-187),
+//                stop conditions (bmg.c:382-410) and run targets. A step that
+//                prints takes a second iteration for the print's re-solve
+//                (bmg.c:292-295): only the solve and k_post work in it.
 // Kernels after the first read their work flags from the control block and
 // return at once when the step does not need them.
 //
@@ -1415,7 +1416,7 @@ __device__ __forceinline__ bool chunk_done(const KParams& kp, const Fields& f, i
 template <int MODEL>
 __global__ void __launch_bounds__(TH) k_rate64(KParams kp, Fields f, RateFx rx) {
   Ctl* ctl = f.ctl;
-  if (ctl->halt) return;
+  if (ctl->halt || ctl->step_kind == kPrint) return;
   const int b = blockIdx.x;
   const long long s0 = (long long)b * kp.bsites;
   const long long s1 = min(s0 + (long long)kp.bsites, kp.N);
@@ -1473,7 +1474,7 @@ __global__ void __launch_bounds__(TH, Q == 4 ? 2 : 3) k_rate64_fx(KParams kp, Fi
   __shared__ int sh_uok;
   __shared__ double red[TH / 32][STZ_MODES];
   Ctl* ctl = f.ctl;
-  if (ctl->halt) return;
+  if (ctl->halt || ctl->step_kind == kPrint) return;
   {
     const int4* src = reinterpret_cast<const int4*>(rx.tab);
     int4* dst = reinterpret_cast<int4*>(tab);
@@ -1548,7 +1549,7 @@ __global__ void __launch_bounds__(TH, 3) k_rate64_fx2(KParams kp, Fields f, Rate
   __shared__ int sh_uok;
   __shared__ double red[TH / 32][STZ_MODES];
   Ctl* ctl = f.ctl;
-  if (ctl->halt) return;
+  if (ctl->halt || ctl->step_kind == kPrint) return;
   {
     const int4* src = reinterpret_cast<const int4*>(rx.tab);
     int4* dst = reinterpret_cast<int4*>(tab);
@@ -1743,35 +1744,57 @@ __global__ void __launch_bounds__(TH) k_ath_commit(KParams kp, Fields f, RateFx 
 }
 
 // ------------------------------------------------------------ post steps
+// The step after its solve: loading, clock, the print check, and, unless the
+// step prints, the stop conditions. A step that prints asks for its re-solve
+// and leaves the rest of itself to the next iteration, whose other kernels
+// return at once (kPrint): its solve is the print's, and the mean stress and
+// the stop conditions follow it. Few steps print, and a second solve in every
+// iteration costs three (2D) to five launches of grids that return at once,
+// 1 to 7 us each.
 // One block of TH threads: the field mean by the block, the rest by thread 0.
-__global__ void k_post_a(KParams kp, Fields f) {
+__global__ void k_post(KParams kp, Fields f) {
   Ctl* ctl = f.ctl;
-  if (ctl->halt && ctl->step_kind == kNone) return;
   const int kind = ctl->step_kind;
+  if (kind == kNone) {
+    if (threadIdx.x == 0 && !ctl->halt) ctl->solve_req = 0;
+    return;
+  }
+  const bool print = ctl->print_done != 0;
   // the mean of the solved field; after an incremental update, C:(ebar - <eps*>)
   // of the same linear solve
-  const bool fieldmean = f.msum != nullptr && !(kp.incr64 && kind == kThermal);
-  if ((kind == kThermal || kind == kAthermal) && fieldmean) field_mean_stress(kp, f, ctl->stress);
+  const bool solved = print || kind == kThermal || kind == kAthermal;
+  const bool fieldmean = f.msum != nullptr && (print || !(kp.incr64 && kind == kThermal));
+  __syncthreads();
+  if (solved && fieldmean) field_mean_stress(kp, f, ctl->stress);
   if (threadIdx.x != 0) return;
-  if (kind == kThermal) {
+  if (solved) {
     if (!fieldmean) solved_mean_stress(kp, ctl, ctl->eps_avg, ctl->stress);
     for (int c = 0; c < 6; c++) ctl->u[c] = 0;
-    load_after_event(kp, ctl, ctl->t_kmc);
-    ctl->totime += ctl->t_kmc;
-  } else if (kind == kAthermal) {
-    if (!fieldmean) solved_mean_stress(kp, ctl, ctl->eps_avg, ctl->stress);
-    for (int c = 0; c < 6; c++) ctl->u[c] = 0;
-    if (kp.loading == STZ_LOAD_STRESS) {
-      hold_stress(kp, ctl);
-    } else {
-      double ts[6];
-      subtract_error(kp, ctl, 1, ts);
-      for (int c = 0; c < kp.nc; c++) ctl->eps_avg[c] -= ts[c];
+  }
+  if (!print) {
+    if (kind == kThermal) {
+      load_after_event(kp, ctl, ctl->t_kmc);
+      ctl->totime += ctl->t_kmc;
+    } else if (kind == kAthermal) {
+      if (kp.loading == STZ_LOAD_STRESS) {
+        hold_stress(kp, ctl);
+      } else {
+        double ts[6];
+        subtract_error(kp, ctl, 1, ts);
+        for (int c = 0; c < kp.nc; c++) ctl->eps_avg[c] -= ts[c];
+      }
+    }
+    if (print_check(kp, ctl)) {
+      ctl->print_done = 1;
+      ctl->solve_req = 1;
+      ctl->step_kind = kPrint;
+      return;
     }
   }
-  // the print check after every step kind; requests the print's re-solve
-  ctl->print_done = kind != kNone ? print_check(kp, ctl) : 0;
-  ctl->solve_req = ctl->print_done;
+  ctl->print_done = 0;
+  ctl->solve_req = 0;
+  ctl->step_kind = kNone;
+  stop_check(kp, ctl);
 }
 
 // FP64 incremental form, after a thermal event: the field the re-solve would
@@ -1827,7 +1850,7 @@ __global__ void k_note_solve(Fields f, const int* gate, const double* ebar) {
 // The print's reset of the barriers to their initial copy (bmg.c:214-221),
 // when this step printed. Only REF2D grids with crystal-like sites have Q1.
 __global__ void k_q0_reset(KParams kp, Fields f, RateFx rx) {
-  if (!f.ctl->print_done || f.ctl->step_kind == kNone) return;
+  if (f.ctl->step_kind != kPrint) return;
   const long long total = (long long)STZ_MODES * kp.N;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
     if (f.Q0[i] != f.Q1[i]) {
@@ -1838,23 +1861,6 @@ __global__ void k_q0_reset(KParams kp, Fields f, RateFx rx) {
         r2_fx_store_mode(rx, i, f.Q1[i], dd[s], dd[kp.N + s], dd[2 * kp.N + s], f.dnorm[i]);
       }
     }
-}
-
-// One block of TH threads, as k_post_a.
-__global__ void k_post_b(KParams kp, Fields f) {
-  Ctl* ctl = f.ctl;
-  if (ctl->step_kind == kNone) return;
-  if (ctl->print_done && f.msum) field_mean_stress(kp, f, ctl->stress);
-  if (threadIdx.x != 0) return;
-  if (ctl->print_done) {
-    if (!f.msum) solved_mean_stress(kp, ctl, ctl->eps_avg, ctl->stress);
-    for (int c = 0; c < 6; c++) ctl->u[c] = 0;
-  }
-  ctl->print_done = 0;
-  ctl->solve_req = 0;
-  ctl->step_kind = kNone;
-  stop_check(kp, ctl);
-  (void)f;
 }
 
 // ------------------------------------------------------------ mixed form
@@ -3593,11 +3599,7 @@ void launch_athermal(const KParams& kp, const Fields& f, const RateFx& rx, int m
   k_ath_commit<<<1, TH, 0, st>>>(kp, f, rx, mixed);
 }
 
-void launch_post_a(const KParams& kp, const Fields& f, cudaStream_t st) {
-  k_post_a<<<1, TH, 0, st>>>(kp, f);
-}
-
-void launch_post_b(const KParams& kp, const Fields& f, cudaStream_t st) { k_post_b<<<1, TH, 0, st>>>(kp, f); }
+void launch_post(const KParams& kp, const Fields& f, cudaStream_t st) { k_post<<<1, TH, 0, st>>>(kp, f); }
 
 void launch_incr64(const KParams& kp, const Fields& f, cudaStream_t st) {
   const unsigned nb = (unsigned)std::min<long long>((kp.N + TH - 1) / TH, 152LL * 8);

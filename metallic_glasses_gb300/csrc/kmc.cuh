@@ -61,8 +61,7 @@ void launch_mixed_tail(const KParams& kp, const Fields& f, int update_only, cuda
 void launch_athermal(const KParams& kp, const Fields& f, const RateFx& rx, int mixed, cudaStream_t st);
 // Bookkeeping after the solve of a step (loading, clock, print check) and
 // after the optional print re-solve (stop checks, targets).
-void launch_post_a(const KParams& kp, const Fields& f, cudaStream_t st);
-void launch_post_b(const KParams& kp, const Fields& f, cudaStream_t st);
+void launch_post(const KParams& kp, const Fields& f, cudaStream_t st);
 // FP64 incremental form: the thermal event's update of the field (two kernels,
 // gated on the control block), and the mean strain of an FFT solve (gated as
 // the solve)

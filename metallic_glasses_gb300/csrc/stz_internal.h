@@ -28,7 +28,8 @@ constexpr double kJInEv = 1 / kEvInJ;
 constexpr double kBoltz = 1.380658e-23;
 constexpr double kEpsilon = 1e-17;
 
-enum StepKind { kThermal = 0, kAthermal = 1, kElastic = 2, kNone = -1 };
+// kPrint: a step that printed, whose re-solve is the next iteration's
+enum StepKind { kThermal = 0, kAthermal = 1, kElastic = 2, kPrint = 3, kNone = -1 };
 
 enum HaltReason {
   kHaltNone = 0,
