@@ -321,22 +321,25 @@ int solve_plain(stz_ctx* c, const int* gate, const double* ebar) {
   a.lambda = c->kp.lambda;
   a.mu = c->kp.mu;
   a.gate = gate;
+  a.rare = gate && c->kp.incr64;
   a.out = kOutSig64;
   a.sig64 = c->f.sig;
   a.msum = c->f.msum;
   a.spec = c->f.spec;
   a.fp32 = 0;
   const int st = fft_solve(*plan_of(c), a, c->stream, &c->launches);
-  if (!st && c->kp.incr64) {
-    // the incremental updates start from the mean strain of this solve
-    launch_note_solve(c->f, gate, ebar, c->stream);
+  if (!st && c->kp.incr64 && !gate) {
+    // the incremental updates start from the mean strain of this solve (k_post
+    // notes it for the solves of the steps)
+    launch_note_solve(c->f, ebar, c->stream);
     c->launches += 1;
   }
   return st;
 }
 
 // FP64 incremental form: the solve of a unit eigenstrain component k at site
-// 0 with zero mean strain, for each k, as the stress table rtab64 [k][c][N].
+// 0 with zero mean strain, for each k, as the stress table rtab64 (2D: all of
+// it; 3D: the octant and the index pairs that the symmetry leaves).
 // The solve is linear in the eigenstrain and the mean strain, so a transformed
 // voxel's increment d and a mean-strain change adds sum_k d_k R_k (shifted to
 // the voxel) plus C:(change) to the field.
@@ -345,7 +348,8 @@ int build_response_table64(stz_ctx* c) {
   const long long N = kp.N;
   const int nc = kp.nc;
   int st;
-  if ((st = dalloc(&c->f.rtab64, (size_t)nc * nc * N))) return st;
+  const bool oct = kp.n0 > 1;
+  if ((st = dalloc(&c->f.rtab64, oct ? oct_table_len(kp) : (size_t)nc * nc * N))) return st;
   double *eps = nullptr, *zero = nullptr;
   if ((st = dalloc(&eps, (size_t)nc * N))) return st;
   if ((st = dalloc(&zero, 6))) { cudaFree(eps); return st; }
@@ -363,10 +367,12 @@ int build_response_table64(stz_ctx* c) {
     a.lambda = kp.lambda;
     a.mu = kp.mu;
     a.out = kOutSig64;
-    a.sig64 = c->f.rtab64 + (size_t)k * nc * N;
+    a.sig64 = oct ? c->f.sig : c->f.rtab64 + (size_t)k * nc * N;  // the stress is solved after this
     a.msum = c->f.msum;
     a.spec = c->f.spec;
     if ((st = fft_solve(*plan_of(c), a, c->stream, &c->launches))) break;
+    if (oct) launch_oct_column(kp, c->f.sig, c->f.rtab64, k, c->stream);
+    if (oct && k == nc - 1) launch_oct_fix(kp, c->f.rtab64, c->stream);
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
       set_error("response table: %s", cudaGetErrorString(cudaGetLastError()));
       st = STZ_ERR_CUDA;
@@ -504,7 +510,7 @@ void enqueue_plain_step(stz_ctx* c, cudaEvent_t t0 = nullptr, cudaEvent_t t1 = n
   solve_plain(c, gate, ebar);
   if (kp.incr64) {
     launch_incr64(kp, f, c->stream);
-    c->launches += 2;
+    c->launches += 1;
   }
   launch_post(kp, f, c->stream);
   if (f.Q1) {

@@ -63,6 +63,7 @@ struct SolveArgs {
   const double* uadd;    // device: uniform stress added after the solve (nc), or null
   double lambda, mu;
   const int* gate;       // device: skip everything when *gate == 0 (null = always run)
+  int rare;              // gated and seldom run: grids of one wave
   int out;               // SolveOut
   double* sig64;         // kOutSig64
   float* sig32;          // kOutSig32

@@ -305,18 +305,17 @@ struct RowMap {
 
 // ---------------------------------------------------------------- R2C, axis 2
 template <int U>
-__global__ void __launch_bounds__(kMaxTh) k_r2c_fx(const double* __restrict__ in, double2* __restrict__ out, int h,
-                                                   int nh, long long rows, long long N, long long Nk, int L, int lgp,
-                                                   FxSched sh, const FxTwiddle* __restrict__ tw_h,
-                                                   const FxTwiddle* __restrict__ tw_p, const int* gate) {
-  if (gate && *gate == 0) return;
+__device__ __forceinline__ void r2c_tile(int tile, const double* __restrict__ in, double2* __restrict__ out, int h,
+                                         int nh, long long rows, long long N, long long Nk, int L, int lgp,
+                                         const FxSched& sh, const FxTwiddle* __restrict__ tw_h,
+                                         const FxTwiddle* __restrict__ tw_p) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int ld = fx_ld(h);
   cx* a = reinterpret_cast<cx*>(smraw);
   cx* b = a + L * ld;
   int* lsc = reinterpret_cast<int*>(b + L * ld);
   const int c = blockIdx.y;
-  const long long r0 = (long long)blockIdx.x * L;
+  const long long r0 = (long long)tile * L;
   const int Lr = (int)min((long long)L, rows - r0);
   const int lpr = 1 << lgp, j0 = threadIdx.x & (lpr - 1), g0 = threadIdx.x >> lgp, ng = blockDim.x >> lgp;
   const double2* src = reinterpret_cast<const double2*>(in + (long long)c * N) + r0 * h + j0;
@@ -389,16 +388,28 @@ __global__ void __launch_bounds__(kMaxTh) k_r2c_fx(const double* __restrict__ in
   }
 }
 
+// A launch of fewer blocks than tiles (a gated solve that rarely runs) takes
+// the tiles in turns; so do the other passes.
+template <int U>
+__global__ void __launch_bounds__(kMaxTh) k_r2c_fx(const double* __restrict__ in, double2* __restrict__ out, int h,
+                                                   int nh, long long rows, long long N, long long Nk, int L, int lgp,
+                                                   FxSched sh, const FxTwiddle* __restrict__ tw_h,
+                                                   const FxTwiddle* __restrict__ tw_p, int tiles, const int* gate) {
+  if (gate && *gate == 0) return;
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    if (t != (int)blockIdx.x) __syncthreads();
+    r2c_tile<U>(t, in, out, h, nh, rows, N, Nk, L, lgp, sh, tw_h, tw_p);
+  }
+}
+
 // ------------------------------------------------------- C2C along axis 1
 // Columns are numbered through all planes (q = i0 nh + k2), so that a tile may
 // straddle two of them: nh is one past a multiple of the tile, and a tile per
 // plane's remainder would leave up to half of the lanes idle. U values of a
 // column per thread, held in registers between load and conversion.
 template <bool INV, int U>
-__global__ void __launch_bounds__(kMaxTh) k_c2c_fx(double2* __restrict__ data, int n, int nh, int columns, long long Nk,
-                                                   int L, int lgL, FxSched sc,
-                                                   const FxTwiddle* __restrict__ tw, const int* gate) {
-  if (gate && *gate == 0) return;
+__device__ __forceinline__ void c2c_tile(int tile, double2* __restrict__ data, int n, int nh, int columns, long long Nk,
+                                         int L, int lgL, const FxSched& sc, const FxTwiddle* __restrict__ tw) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ int lsc[32];
   const int ld = fx_ld(n);
@@ -406,7 +417,7 @@ __global__ void __launch_bounds__(kMaxTh) k_c2c_fx(double2* __restrict__ data, i
   cx* b = a + L * ld;
   const int c = blockIdx.y;
   const int l = threadIdx.x & (L - 1), p0 = threadIdx.x >> lgL, dp = blockDim.x >> lgL;
-  const int q = blockIdx.x * L + l;
+  const int q = tile * L + l;
   const int o = (int)((unsigned)q / (unsigned)nh);
   const int pe = q < columns ? n : 0;  // columns past the last hold nothing
   double2* base = data + (long long)c * Nk + (long long)o * n * nh + (q - o * nh) + (long long)p0 * nh;
@@ -434,6 +445,17 @@ __global__ void __launch_bounds__(kMaxTh) k_c2c_fx(double2* __restrict__ data, i
       const cx r = res[pad(p0 + u * dp)];
       base[u * step] = unscale(INV ? cx{r.y, r.x} : r, -s, s == kBad);
     }
+}
+
+template <bool INV, int U>
+__global__ void __launch_bounds__(kMaxTh) k_c2c_fx(double2* __restrict__ data, int n, int nh, int columns, long long Nk,
+                                                   int L, int lgL, FxSched sc, const FxTwiddle* __restrict__ tw,
+                                                   int tiles, const int* gate) {
+  if (gate && *gate == 0) return;
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    if (t != (int)blockIdx.x) __syncthreads();
+    c2c_tile<INV, U>(t, data, n, nh, columns, Nk, L, lgL, sc, tw);
+  }
 }
 
 // ------------------------------------------------------------- Green's pass
@@ -520,17 +542,16 @@ __device__ __forceinline__ void green_part(const GreenFx& ga, const Fx* g, const
 // U values per thread of each component's line in registers between load and
 // conversion (0: through shared memory).
 template <int NC, int U>
-__global__ void __launch_bounds__(kMaxTh, 2) k_green_fx(double2* __restrict__ spec, int n, int stride, int inner,
-                                                        long long Nk, int L, int lgL, FxSched sc,
-                                                        const FxTwiddle* __restrict__ tw, GreenFx ga, const int* gate) {
-  if (gate && *gate == 0) return;
+__device__ __forceinline__ void green_tile(int tile, double2* __restrict__ spec, int n, int stride, int inner,
+                                           long long Nk, int L, int lgL, const FxSched& sc,
+                                           const FxTwiddle* __restrict__ tw, const GreenFx& ga) {
   constexpr int ND = NC == 3 ? 2 : 3;
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ int lsc[32], lsh[32], lkb[32];
   const int ld = fx_ld(n);
   cx* a = reinterpret_cast<cx*>(smraw);
   cx* b = a + NC * L * ld;
-  const int q0 = blockIdx.x * L;
+  const int q0 = tile * L;
   const int l = threadIdx.x & (L - 1), p0 = threadIdx.x >> lgL, dp = blockDim.x >> lgL;
   const int q = q0 + l;
   const bool in = q < inner;
@@ -723,19 +744,28 @@ __global__ void __launch_bounds__(kMaxTh, 2) k_green_fx(double2* __restrict__ sp
       }
 }
 
+template <int NC, int U>
+__global__ void __launch_bounds__(kMaxTh, 2) k_green_fx(double2* __restrict__ spec, int n, int stride, int inner,
+                                                        long long Nk, int L, int lgL, FxSched sc,
+                                                        const FxTwiddle* __restrict__ tw, GreenFx ga, int tiles,
+                                                        const int* gate) {
+  if (gate && *gate == 0) return;
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    if (t != (int)blockIdx.x) __syncthreads();
+    green_tile<NC, U>(t, spec, n, stride, inner, Nk, L, lgL, sc, tw, ga);
+  }
+}
+
 // ---------------------------------------------------------------- C2R, axis 2
 // Rows of one component (blockIdx.y), the block's sum of the component to msum.
 // The factor 2 mu / N of the solve and the mean strain's uniform stress are
 // applied here, in FP64 (three operations per value on an otherwise idle pipe).
 template <int U>
-__global__ void __launch_bounds__(kMaxTh) k_c2r_fx(const double2* __restrict__ in, int nc, int h, int nh,
-                                                   long long rows, long long N, long long Nk, int L, int lgp,
-                                                   FxSched sh, const FxTwiddle* __restrict__ tw_h,
-                                                   const FxTwiddle* __restrict__ tw_p, double factor,
-                                                   const double* __restrict__ ebar, double lambda, double mu,
-                                                   double* __restrict__ sig, double* __restrict__ msum,
-                                                   const int* gate) {
-  if (gate && *gate == 0) return;
+__device__ __forceinline__ void c2r_tile(int tile, int tiles, const double2* __restrict__ in, int nc, int h, int nh,
+                                         long long rows, long long N, long long Nk, int L, int lgp, const FxSched& sh,
+                                         const FxTwiddle* __restrict__ tw_h, const FxTwiddle* __restrict__ tw_p,
+                                         double factor, const double* __restrict__ ebar, double lambda, double mu,
+                                         double* __restrict__ sig, double* __restrict__ msum) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ double red[kMaxTh / 32];
   const int ld = fx_ld(h + 1);
@@ -743,7 +773,7 @@ __global__ void __launch_bounds__(kMaxTh) k_c2r_fx(const double2* __restrict__ i
   cx* b = a + L * ld;
   int* lsc = reinterpret_cast<int*>(b + L * ld);
   const int c = blockIdx.y;
-  const long long r0 = (long long)blockIdx.x * L;
+  const long long r0 = (long long)tile * L;
   const int Lr = (int)min((long long)L, rows - r0);
   const int lpr = 1 << lgp, j0 = threadIdx.x & (lpr - 1), g0 = threadIdx.x >> lgp, ng = blockDim.x >> lgp;
   // C:<eps> of this component
@@ -849,8 +879,23 @@ __global__ void __launch_bounds__(kMaxTh) k_c2r_fx(const double2* __restrict__ i
     if (threadIdx.x == 0) {
       double t = 0;
       for (int k = 0; k < (int)(blockDim.x >> 5); k++) t += red[k];
-      msum[(long long)c * gridDim.x + blockIdx.x] = t;
+      msum[(long long)c * tiles + tile] = t;
     }
+  }
+}
+
+template <int U>
+__global__ void __launch_bounds__(kMaxTh) k_c2r_fx(const double2* __restrict__ in, int nc, int h, int nh,
+                                                   long long rows, long long N, long long Nk, int L, int lgp,
+                                                   FxSched sh, const FxTwiddle* __restrict__ tw_h,
+                                                   const FxTwiddle* __restrict__ tw_p, double factor,
+                                                   const double* __restrict__ ebar, double lambda, double mu,
+                                                   double* __restrict__ sig, double* __restrict__ msum, int tiles,
+                                                   const int* gate) {
+  if (gate && *gate == 0) return;
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    if (t != (int)blockIdx.x) __syncthreads();
+    c2r_tile<U>(t, tiles, in, nc, h, nh, rows, N, Nk, L, lgp, sh, tw_h, tw_p, factor, ebar, lambda, mu, sig, msum);
   }
 }
 
@@ -897,27 +942,40 @@ void raise_limit(F* k, int optin) {
     (void)cudaGetLastError();
 }
 
+// Blocks of a pass over `tiles` tiles of `comps` components. A block each; for a
+// gated solve that rarely runs, two blocks per SM in all: a grid whose blocks
+// return at once takes 6 to 7 us with 2000 blocks of 100 KB, 1.5 us then.
+dim3 fx_grid(const SolveArgs& a, int tiles, int comps) {
+  const int most = 304 / comps;
+  return dim3((unsigned)(a.rare && tiles > most ? most : tiles), (unsigned)comps);
+}
+
 template <int NC>
-void launch_green(const FFTPlan& p, int n, int inner, double2* spec, const FxSched& x, const FxTwiddle* tw,
-                  const GreenFx& ga, const int* gate, cudaStream_t st) {
+void launch_green(const FFTPlan& p, int n, int inner, const SolveArgs& a, const FxSched& x, const FxTwiddle* tw,
+                  const GreenFx& ga, cudaStream_t st) {
+  double2* spec = reinterpret_cast<double2*>(a.spec);
+  const int* gate = a.gate;
   const ColLaunch c = col_launch(n, p.L_g, p.e_g);
-  const unsigned grid = (unsigned)((inner + p.L_g - 1) / p.L_g);
+  const int tiles = (inner + p.L_g - 1) / p.L_g;
+  const dim3 grid = fx_grid(a, tiles, 1);
   const int lg = ilog2(p.L_g);
   if (c.U == 1)
-    k_green_fx<NC, 1><<<grid, c.threads, p.smem_gr, st>>>(spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, gate);
+    k_green_fx<NC, 1><<<grid, c.threads, p.smem_gr, st>>>(spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, tiles, gate);
   else if (c.U == 2)
-    k_green_fx<NC, 2><<<grid, c.threads, p.smem_gr, st>>>(spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, gate);
+    k_green_fx<NC, 2><<<grid, c.threads, p.smem_gr, st>>>(spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, tiles, gate);
   else
-    k_green_fx<NC, 0><<<grid, c.threads, p.smem_gr, st>>>(spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, gate);
+    k_green_fx<NC, 0><<<grid, c.threads, p.smem_gr, st>>>(spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, tiles, gate);
 }
 
 template <bool INV>
-void launch_c2c(const FFTPlan& p, double2* spec, const FxSched& x, const int* gate, cudaStream_t st) {
+void launch_c2c(const FFTPlan& p, const SolveArgs& a, const FxSched& x, cudaStream_t st) {
   const ColLaunch c = col_launch(p.n1, p.L_y, p.e_y);
   const int columns = p.n0 * p.nh, lg = ilog2(p.L_y);
-  const dim3 grid((unsigned)((columns + p.L_y - 1) / p.L_y), (unsigned)p.nc);
+  const int tiles = (columns + p.L_y - 1) / p.L_y;
+  const dim3 grid = fx_grid(a, tiles, p.nc);
   auto go = [&](auto* k) {
-    k<<<grid, c.threads, p.smem_yr, st>>>(spec, p.n1, p.nh, columns, p.Nk, p.L_y, lg, x, p.tx_1, gate);
+    k<<<grid, c.threads, p.smem_yr, st>>>(reinterpret_cast<double2*>(a.spec), p.n1, p.nh, columns, p.Nk, p.L_y, lg, x,
+                                          p.tx_1, tiles, a.gate);
   };
   if (c.U <= 2) go(k_c2c_fx<INV, 2>);
   else if (c.U == 4) go(k_c2c_fx<INV, 4>);
@@ -965,10 +1023,12 @@ void fftx_spectrum(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_
   double2* spec = reinterpret_cast<double2*>(a.spec);
   const long long rows = (long long)p.n0 * p.n1;
   const FxSched xh = fx_sched(p.sh), x1 = fx_sched(p.s1), x0 = fx_sched(p.s0);
-  const dim3 gx((unsigned)((rows + p.L_x - 1) / p.L_x), (unsigned)p.nc);
+  const int tiles = (int)((rows + p.L_x - 1) / p.L_x);
+  const dim3 gx = fx_grid(a, tiles, p.nc);
   const RowLaunch r = row_launch(p.h, p.L_x, p.e_x);
   auto r2c = [&](auto* k) {
-    k<<<gx, r.threads, p.smem_xr, st>>>(a.eps, spec, p.h, p.nh, rows, p.N, p.Nk, p.L_x, r.lgp, xh, p.tx_h, p.tx_p, a.gate);
+    k<<<gx, r.threads, p.smem_xr, st>>>(a.eps, spec, p.h, p.nh, rows, p.N, p.Nk, p.L_x, r.lgp, xh, p.tx_h,
+                                        p.tx_p, tiles, a.gate);
   };
   if (r.U == 1) r2c(k_r2c_fx<1>);
   else if (r.U == 2) r2c(k_r2c_fx<2>);
@@ -978,11 +1038,11 @@ void fftx_spectrum(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_
   GreenFx ga;
   fx_green_constants(p.n0, p.n1, p.n2, a.lambda, a.mu, &ga);
   if (p.n0 > 1) {
-    launch_c2c<false>(p, spec, x1, a.gate, st);
-    launch_green<6>(p, p.n0, p.n1 * p.nh, spec, x0, p.tx_0, ga, a.gate, st);
-    launch_c2c<true>(p, spec, x1, a.gate, st);
+    launch_c2c<false>(p, a, x1, st);
+    launch_green<6>(p, p.n0, p.n1 * p.nh, a, x0, p.tx_0, ga, st);
+    launch_c2c<true>(p, a, x1, st);
   } else {
-    launch_green<3>(p, p.n1, p.nh, spec, x1, p.tx_1, ga, a.gate, st);
+    launch_green<3>(p, p.n1, p.nh, a, x1, p.tx_1, ga, st);
   }
   if (launches) *launches += p.n0 > 1 ? 4 : 2;
 }
@@ -991,12 +1051,13 @@ double fftx_factor(const FFTPlan& p, double mu) { return (double)(2 * (long doub
 
 void fftx_c2r(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* launches) {
   const long long rows = (long long)p.n0 * p.n1;
-  const dim3 gx((unsigned)((rows + p.L_x - 1) / p.L_x), (unsigned)p.nc);
+  const int tiles = (int)((rows + p.L_x - 1) / p.L_x);
+  const dim3 gx = fx_grid(a, tiles, p.nc);
   const RowLaunch r = row_launch(p.h, p.L_x, p.e_x);
   auto go = [&](auto* k) {
     k<<<gx, r.threads, p.smem_xr, st>>>(reinterpret_cast<const double2*>(a.spec), p.nc, p.h, p.nh, rows, p.N, p.Nk, p.L_x,
                                         r.lgp, fx_sched(p.sh), p.tx_h, p.tx_p, fftx_factor(p, a.mu), a.ebar, a.lambda,
-                                        a.mu, a.sig64, a.msum, a.gate);
+                                        a.mu, a.sig64, a.msum, tiles, a.gate);
   };
   if (r.U == 1) go(k_c2r_fx<1>);
   else if (r.U == 2) go(k_c2r_fx<2>);

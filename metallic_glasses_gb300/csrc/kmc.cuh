@@ -66,7 +66,12 @@ void launch_post(const KParams& kp, const Fields& f, cudaStream_t st);
 // gated on the control block), and the mean strain of an FFT solve (gated as
 // the solve)
 void launch_incr64(const KParams& kp, const Fields& f, cudaStream_t st);
-void launch_note_solve(const Fields& f, const int* gate, const double* ebar, cudaStream_t st);
+void launch_note_solve(const Fields& f, const double* ebar, cudaStream_t st);
+// The 3D octant table: its doubles (the offsets' scales behind the values), a column from
+// a solved unit response, and its turn into fixed point.
+size_t oct_table_len(const KParams& kp);
+void launch_oct_column(const KParams& kp, const double* sig, double* tab, int k, cudaStream_t st);
+void launch_oct_fix(const KParams& kp, double* tab, cudaStream_t st);
 // REF2D with crystal-like sites: restore the initial barriers when the step printed
 void launch_q0_reset(const KParams& kp, const Fields& f, const RateFx& rx, cudaStream_t st);
 // Reset of the incremental state after a full re-solve (mixed form).

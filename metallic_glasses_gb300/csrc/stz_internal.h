@@ -120,8 +120,9 @@ struct Fields {
   double* Q0 = nullptr;      // [MODES][N] (REF2D)
   double* deps = nullptr;    // [MODES][3][N] (REF2D)
   double* dnorm = nullptr;   // [MODES][N] 1 / (|deps| + eps) of each mode (REF2D), kept with deps
-  double* rtab64 = nullptr;  // [nc][nc][N] FP64 incremental form: stress component c of the
-                             // solve of a unit eigenstrain component k at site 0, ebar = 0
+  double* rtab64 = nullptr;  // FP64 incremental form: stress component c of the solve of a unit
+                             // eigenstrain component k at site 0, ebar = 0. 2D: [k][c][N];
+                             // 3D: 64-bit fixed point [21][kt0][kt1][kt2], then the scales
   int8_t* mro = nullptr;     // [N] crystal-like MRO type 0..3 (REF2D); null for an all-glass map
   double* Q1 = nullptr;      // [MODES][N] the initial Q0, restored at every print (bmg.c:214-221);
                              // only with crystal-like sites (glass sites never change Q0)
