@@ -46,7 +46,7 @@ void fx_exp_table(FxExp* t) {
     for (int i = 0; i < 12; i++)
       if (h >> (11 - i) & 1) v = mul_q126(v, (u128)kRoots[i][0] << 64 | kRoots[i][1]);
     t[j].t = (int64_t)((uint64_t)(v >> 64) + ((uint64_t)(v >> 63) & 1));
-    const Fx s = fx_split((int64_t)((mul_q126(v, ln2) + ((u128)1 << 64)) >> 65));
+    const Fx s = fx_split((int64_t)((mul_q126(v, ln2) + ((u128)1 << 74)) >> 75));
     t[j].ph = s.h;
     t[j].pl = s.l;
   }

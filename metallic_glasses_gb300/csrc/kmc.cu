@@ -66,6 +66,19 @@ __device__ void iso_inv(const KParams& kp, const double* s, double* e) {
     for (int c = 3; c < 6; c++) e[c] = s[c] / 2 / mu;
   }
 }
+// Component `lane` of the same, its s in every lane of a warp (0 beyond the
+// last): the divisions side by side, some 900 clocks each.
+__device__ double iso_inv_lane(const KParams& kp, double s, int lane) {
+  const double s0 = __shfl_sync(FULL, s, 0), s1 = __shfl_sync(FULL, s, 1), s2 = __shfl_sync(FULL, s, 2);
+  const double lam = kp.lambda, mu = kp.mu;
+  const bool d2 = kp.nc == 3;
+  if (kp.fast_inv) {
+    const double tr = d2 ? s0 + s1 : s0 + s1 + s2;
+    return (lane < ndiag(kp.nc) ? -kp.inv_lam_coef * tr : 0.0) + s * kp.inv_2mu;
+  }
+  const double tra = -lam / 2 / mu / ((d2 ? 2 : 3) * lam + 2 * mu) * (d2 ? s0 + s1 : s0 + s1 + s2);
+  return lane < ndiag(kp.nc) ? tra + s / 2 / mu : s / 2 / mu;
+}
 
 // AvgStress (elastic.c:733-752): mean of the solved field, from the per-block
 // sums the C2R pass left in msum (fixed summation order)
@@ -74,30 +87,24 @@ __device__ void iso_inv(const KParams& kp, const double* s, double* e) {
 // the warps in order (a dependent chain of FP64 additions in one thread took
 // about 1 ms at 128^3: GB300 runs FP64 at 1/64 of the FP32 rate). Thread 0
 // writes out; every thread of the block must call it.
+// A warp per component, eight loads at a time (a block of TH threads).
 __device__ void field_mean_stress(const KParams& kp, const Fields& f, double* out) {
-  __shared__ double red[TH / 32][6];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  double s[6] = {0, 0, 0, 0, 0, 0};
-  for (int c = 0; c < kp.nc; c++)
-    for (int b = threadIdx.x; b < kp.c2r_blocks; b += blockDim.x) s[c] += f.msum[(long long)c * kp.c2r_blocks + b];
-  for (int c = 0; c < kp.nc; c++) {
-    for (int off = 16; off > 0; off >>= 1) s[c] += __shfl_xor_sync(FULL, s[c], off);
-    if (lane == 0) red[w][c] = s[c];
+  const int lane = threadIdx.x & 31;
+  static_assert(TH / 32 >= 6, "a warp per component");
+  if ((int)threadIdx.x >> 5 < kp.nc) {
+    const int c = threadIdx.x >> 5, nb = kp.c2r_blocks;
+    const double* src = f.msum + (long long)c * nb;
+    double s = 0;
+    for (int b = lane; b < nb; b += 8 * 32) {
+      double v[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) v[i] = b + i * 32 < nb ? src[b + i * 32] : 0.0;
+      s += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+    }
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(FULL, s, off);
+    if (lane == 0) out[c] = s / (double)kp.N;
   }
   __syncthreads();
-  if (threadIdx.x == 0)
-    for (int c = 0; c < kp.nc; c++) {
-      double t = 0;
-      for (int k = 0; k < nw; k++) t += red[k][c];
-      out[c] = t / (double)kp.N;
-    }
-  __syncthreads();
-}
-
-__device__ void solved_mean_stress(const KParams& kp, const Ctl* ctl, const double* ebar, double* out) {
-  double e[6];
-  for (int c = 0; c < kp.nc; c++) e[c] = ebar[c] - ctl->eps0_sum[c] * kp.invN;
-  apply_C(kp, e, out);
 }
 
 __device__ __forceinline__ int shear_comp(const KParams& kp) { return kp.nc == 3 ? 2 : STZ_XY; }
@@ -117,10 +124,14 @@ __device__ void subtract_error(const KParams& kp, const Ctl* ctl, int athermal, 
   iso_inv(kp, ts, tmpStrain);
 }
 
-__device__ void hold_stress(const KParams& kp, Ctl* ctl) {
+// `inv` (optional, here and below): the strain of the stress difference, formed
+// by the caller
+__device__ void hold_stress(const KParams& kp, Ctl* ctl, const double* inv = nullptr) {
   double d[6] = {0, 0, 0, 0, 0, 0}, de[6];
   for (int c = 0; c < kp.nc; c++) d[c] = kp.applied[c] - ctl->stress[c];
-  iso_inv(kp, d, de);
+  if (inv)
+    for (int c = 0; c < kp.nc; c++) de[c] = inv[c];
+  else iso_inv(kp, d, de);
   for (int c = 0; c < kp.nc; c++) {
     ctl->eps_avg[c] += de[c];
     ctl->u[c] += d[c];
@@ -130,13 +141,17 @@ __device__ void hold_stress(const KParams& kp, Ctl* ctl) {
 
 // loading after a thermal event (evolution.c:262-317); ctl->stress holds the
 // mean stress of the field solved right after the transformation
-__device__ void load_after_event(const KParams& kp, Ctl* ctl, double t_kmc) {
+__device__ void load_after_event(const KParams& kp, Ctl* ctl, double t_kmc, const double* inv = nullptr) {
   double ts[6];
+  if (kp.loading != STZ_LOAD_STRESS) {
+    if (inv)
+      for (int c = 0; c < kp.nc; c++) ts[c] = inv[c];
+    else subtract_error(kp, ctl, 0, ts);
+  }
   const double rate = kp.strain_rate, nu = kp.poisson, E = kp.young, mu = kp.mu;
   const bool d2 = kp.nc == 3;
   switch (kp.loading) {
     case STZ_LOAD_TENSION:
-      subtract_error(kp, ctl, 0, ts);
       ctl->eps_avg[0] += (rate * t_kmc * 1 - ts[0]);
       ctl->eps_avg[1] += (rate * t_kmc * (-nu) - ts[1]);
       if (d2) {
@@ -149,7 +164,6 @@ __device__ void load_after_event(const KParams& kp, Ctl* ctl, double t_kmc) {
       ctl->u[0] += E * rate * t_kmc;
       break;
     case STZ_LOAD_COMPRESSION:
-      subtract_error(kp, ctl, 0, ts);
       ctl->eps_avg[0] += (-rate * t_kmc * 1);
       ctl->eps_avg[1] += (rate * t_kmc * (nu));
       ctl->eps_avg[0] += (-rate * t_kmc * 1 - ts[0]);
@@ -160,7 +174,6 @@ __device__ void load_after_event(const KParams& kp, Ctl* ctl, double t_kmc) {
       break;
     case STZ_LOAD_SHEAR: {
       const int sc = shear_comp(kp);
-      subtract_error(kp, ctl, 0, ts);
       for (int c = 0; c < kp.nc; c++)
         if (c != sc) ctl->eps_avg[c] += -ts[c];
       ctl->eps_avg[sc] += rate * t_kmc;
@@ -169,7 +182,7 @@ __device__ void load_after_event(const KParams& kp, Ctl* ctl, double t_kmc) {
       break;
     }
     case STZ_LOAD_STRESS:
-      hold_stress(kp, ctl);
+      hold_stress(kp, ctl, inv);
       break;
   }
 }
@@ -538,6 +551,19 @@ __device__ __forceinline__ FxExp fx_cell(const FxExp* t, int j) {  // one 16-byt
   return q;
 }
 
+// the same from the table in shared memory at `tab`: cell j of Y's high word
+// (left to itself the compiler makes two 8-byte loads, twice the bank conflicts)
+__device__ __forceinline__ FxExp fx_cell_shared(unsigned tab, uint64_t Y) {
+  FxExp q;
+  uint32_t lo, hi;
+  const unsigned at = tab + ((unsigned)(Y >> 38) & ((kFxExpCells - 1) * (unsigned)sizeof(FxExp)));
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(lo), "=r"(hi), "=r"(q.ph), "=r"(q.pl)
+               : "r"(at));
+  q.t = (int64_t)((uint64_t)lo | ((uint64_t)hi << 32));
+  return q;
+}
+
 // REF2D in fixed point. A site's operands: W0 = (s_xx - s_yy) w and W2 = 2 s_xy w
 // (x 2^49, below 2^12), w = V0 1e-18 J log2(e) / (2 kT), so that the work term of
 // mode m is W0 dx + W2 dxy (its modes are traceless); for a softened site the
@@ -730,7 +756,7 @@ __device__ __forceinline__ void mx_site(const KParams& kp, const Fields& f, long
 // ---------------------------------------------------- block-level helpers
 // Inclusive scan of one double per thread over a 256-thread block; returns the
 // inclusive value and leaves every thread's inclusive value in sh_inc.
-__device__ double block_incl_scan(double v, double* sh_inc) {
+__device__ __noinline__ double block_incl_scan(double v, double* sh_inc) {
   __shared__ double wsum[TH / 32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   double x = v;
@@ -1033,10 +1059,12 @@ __device__ void search_event(const KParams& kp, const Fields& f, const RateFx& r
   constexpr int kMaxPer = kSptFp64;  // sites per thread
   double rr[kMaxPer];
   double loc = 0;
-#pragma unroll
-  for (int k = 0; k < kMaxPer; k++) {
+  // not unrolled, here and below: one block runs this once, and fetching the
+  // instructions of four copies took 20 us of the 25 us they ran (128^3)
+#pragma unroll 1
+  for (int k = 0; k < per; k++) {
     const long long s = a0 + k;
-    rr[k] = (k < per && s < s1) ? site_rate<MODEL>(kp, f, rx, u, totime, s, m) : 0.0;
+    rr[k] = s < s1 ? site_rate<MODEL>(kp, f, rx, u, totime, s, m) : 0.0;
     loc += rr[k];
   }
   const double I2 = block_incl_scan(loc, sh_inc2);
@@ -1048,8 +1076,8 @@ __device__ void search_event(const KParams& kp, const Fields& f, const RateFx& r
     double run = E2;
     int hit = -1, lastk = -1;
     double hb = E2, ha = E2, lb = E2, la = E2;
-#pragma unroll
-    for (int k = 0; k < kMaxPer; k++) {
+#pragma unroll 1
+    for (int k = 0; k < per; k++) {
       const double before = run;
       run += rr[k];
       const bool pos = rr[k] > 0;
@@ -1266,13 +1294,20 @@ __device__ __noinline__ void finish_step(const KParams& kp, const Fields& f, con
   __shared__ int sh_mode;
   __shared__ double sh_margin;
   Ctl* const g = f.ctl;
-  ctl_copy(&sc, g);
-  // per-thread contiguous chunks of the per-(mode, group) sums, fixed order
+  // per-thread contiguous chunks of the per-(mode, group) sums, fixed order; the
+  // first loads together with those of the control block
   const long long P = (long long)STZ_MODES * kp.ngroups;
   const long long ch = (P + TH - 1) / TH;
   const long long p0 = threadIdx.x * ch, p1 = min(p0 + ch, P);
+  constexpr int kFirst = 6;
+  double v[kFirst];
+#pragma unroll
+  for (int i = 0; i < kFirst; i++) v[i] = p0 + i < p1 ? f.gsum[p0 + i] : 0.0;
+  ctl_copy(&sc, g);
   double S = 0;
-  for (long long p = p0; p < p1; p++) S += f.gsum[p];
+#pragma unroll
+  for (int i = 0; i < kFirst; i++) S += v[i];
+  for (long long p = p0 + kFirst; p < p1; p++) S += f.gsum[p];
   block_incl_scan(S, sh_inc);  // also orders the copy above
   block_twist_if_needed(&sc.rng);
   Ctl* c = &sc;
@@ -1483,12 +1518,13 @@ __global__ void __launch_bounds__(TH, Q == 4 ? 2 : 3) k_rate64_fx(KParams kp, Fi
   }
   if (threadIdx.x == 0) sh_uok = g3_fx_u(rx, ctl->u, sh_u);
   __syncthreads();
+  const unsigned tab_at = (unsigned)__cvta_generic_to_shared(tab);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int b = blockIdx.x; b < kp.nblk; b += gridDim.x) {
     const long long s0 = (long long)b * kp.bsites;
     const long long s1 = min(s0 + (long long)kp.bsites, kp.N);
     bool ok = sh_uok;
-    unsigned neg = 0;
+    unsigned neg = 0, top = 0;  // negative barriers; the largest argument's high word
     Fx W[Q][6];
     FxAcc a0[Q];
 #pragma unroll
@@ -1513,14 +1549,20 @@ __global__ void __launch_bounds__(TH, Q == 4 ? 2 : 3) k_rate64_fx(KParams kp, Fi
 #pragma unroll
           for (int q = 0; q < Q; q++) {
             Y[q] = g3_fx_arg(rx, W[q], a0[q], g + i);
-            neg += Y[q] > rx.neg;
-            c[q] = fx_cell(tab, fx_exp_cell(Y[q]));
+            top = max(top, (unsigned)(Y[q] >> 32));
+            c[q] = fx_cell_shared(tab_at, Y[q]);
           }
           v[i] = fx_double(fx_exp2_sum_bits<Q>(Y, c));
         }
         int idx;
         const double t = WarpSums<G, 16>::run(v, lane, &idx);
         if (idx >= 0) red[w][g + idx] = t;
+      }
+      if (top >= (unsigned)(rx.neg >> 32)) {  // seldom: a negative barrier, or nearly one
+#pragma unroll
+        for (int q = 0; q < Q; q++)
+#pragma unroll 1
+          for (int m = 0; m < STZ_MODES; m++) neg += g3_fx_arg(rx, W[q], a0[q], m) > rx.neg;
       }
       __syncthreads();
       if (threadIdx.x < STZ_MODES) {
@@ -1559,12 +1601,13 @@ __global__ void __launch_bounds__(TH, 3) k_rate64_fx2(KParams kp, Fields f, Rate
   const double totime = ctl->totime;
   if (threadIdx.x == 0) sh_uok = r2_fx_u(rx, ctl->u, sh_u);
   __syncthreads();
+  const unsigned tab_at = (unsigned)__cvta_generic_to_shared(tab);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int b = blockIdx.x; b < kp.nblk; b += gridDim.x) {
     const long long s0 = (long long)b * kp.bsites;
     const long long s1 = min(s0 + (long long)kp.bsites, kp.N);
     bool ok = sh_uok;
-    unsigned neg = 0;
+    unsigned neg = 0, top = 0;  // negative barriers; the largest argument's high word
     R2Fx d[Q];
 #pragma unroll
     for (int q = 0; q < Q; q++) {
@@ -1583,14 +1626,23 @@ __global__ void __launch_bounds__(TH, 3) k_rate64_fx2(KParams kp, Fields f, Rate
           const long long s = s0 + threadIdx.x + q * TH;
           Y[q] = (uint64_t)1 << 53;  // no site: the smallest representable rate, 2^-1021
           if (s < s1) Y[q] = r2_fx_arg(kp, rx, f, tab, d[q], s, g + i, &ok);
-          neg += Y[q] > rx.neg;
-          c[q] = fx_cell(tab, fx_exp_cell(Y[q]));
+          top = max(top, (unsigned)(Y[q] >> 32));
+          c[q] = fx_cell_shared(tab_at, Y[q]);
         }
         v[i] = fx_double(fx_exp2_sum_bits<Q>(Y, c));
       }
       int idx;
       const double t = WarpSums<G, 16>::run(v, lane, &idx);
       if (idx >= 0) red[w][g + idx] = t;
+    }
+    if (top >= (unsigned)(rx.neg >> 32)) {  // as in 3D
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        const long long s = s0 + threadIdx.x + q * TH;
+        if (s < s1)
+#pragma unroll 1
+          for (int m = 0; m < STZ_MODES; m++) neg += r2_fx_arg(kp, rx, f, tab, d[q], s, m, &ok) > rx.neg;
+      }
     }
     if (!__syncthreads_or(!ok)) {
       if (threadIdx.x < STZ_MODES) {
@@ -1744,50 +1796,23 @@ __global__ void __launch_bounds__(TH) k_ath_commit(KParams kp, Fields f, RateFx 
 }
 
 // ------------------------------------------------------------ post steps
-// The step after its solve: loading, clock, the print check, and, unless the
-// step prints, the stop conditions. A step that prints asks for its re-solve
-// and leaves the rest of itself to the next iteration, whose other kernels
-// return at once (kPrint): its solve is the print's, and the mean stress and
-// the stop conditions follow it. Few steps print, and a second solve in every
-// iteration costs three (2D) to five launches of grids that return at once,
-// 1 to 7 us each.
-// One block of TH threads: the field mean by the block, the rest by thread 0.
-__global__ void k_post(KParams kp, Fields f) {
-  Ctl* ctl = f.ctl;
+__device__ void post_step(const KParams& kp, Ctl* ctl, bool print, bool solved, const double* inv) {
   const int kind = ctl->step_kind;
-  if (kind == kNone) {
-    if (threadIdx.x == 0 && !ctl->halt) ctl->solve_req = 0;
-    return;
-  }
-  const bool print = ctl->print_done != 0;
-  // the mean of the solved field; after an incremental update, C:(ebar - <eps*>)
-  // of the same linear solve
-  const bool solved = print || kind == kThermal || kind == kAthermal;
-  const bool fieldmean = f.msum != nullptr && (print || !(kp.incr64 && kind == kThermal));
-  __syncthreads();
-  if (solved && fieldmean) field_mean_stress(kp, f, ctl->stress);
-  if (threadIdx.x != 0) return;
   if (kp.incr64 && (ctl->incr_req || ctl->solve_req)) {
     // the field now holds the solve at the current mean strain
     for (int c = 0; c < 6; c++) ctl->ebar_solved[c] = ctl->eps_avg[c];
     ctl->incr_req = 0;
   }
-  if (solved) {
-    if (!fieldmean) solved_mean_stress(kp, ctl, ctl->eps_avg, ctl->stress);
+  if (solved)
     for (int c = 0; c < 6; c++) ctl->u[c] = 0;
-  }
   if (!print) {
     if (kind == kThermal) {
-      load_after_event(kp, ctl, ctl->t_kmc);
+      load_after_event(kp, ctl, ctl->t_kmc, inv);
       ctl->totime += ctl->t_kmc;
     } else if (kind == kAthermal) {
-      if (kp.loading == STZ_LOAD_STRESS) {
-        hold_stress(kp, ctl);
-      } else {
-        double ts[6];
-        subtract_error(kp, ctl, 1, ts);
-        for (int c = 0; c < kp.nc; c++) ctl->eps_avg[c] -= ts[c];
-      }
+      if (kp.loading == STZ_LOAD_STRESS) hold_stress(kp, ctl, inv);
+      else
+        for (int c = 0; c < kp.nc; c++) ctl->eps_avg[c] -= inv[c];
     }
     if (print_check(kp, ctl)) {
       ctl->print_done = 1;
@@ -1800,6 +1825,63 @@ __global__ void k_post(KParams kp, Fields f) {
   ctl->solve_req = 0;
   ctl->step_kind = kNone;
   stop_check(kp, ctl);
+}
+
+// The step after its solve: loading, clock, the print check, and, unless the
+// step prints, the stop conditions. A step that prints asks for its re-solve
+// and leaves the rest of itself to the next iteration, whose other kernels
+// return at once (kPrint): its solve is the print's, and the mean stress and
+// the stop conditions follow it. Few steps print, and a second solve in every
+// iteration costs three (2D) to five launches of grids that return at once,
+// 1 to 7 us each.
+// One block of TH threads on a shared copy of the control block (without the
+// generator, its last member): the field mean by a warp per component, the
+// tensors by a lane per component, the rest by thread 0. By one thread on the
+// control block in L2 it took 7 to 10 us, and the field mean 12 at 64^3.
+__global__ void __launch_bounds__(TH) k_post(KParams kp, Fields f) {
+  constexpr int kWords = (int)(offsetof(Ctl, rng) / 4);
+  __shared__ __align__(16) uint32_t words[sizeof(Ctl) / 4];
+  Ctl* const ctl = reinterpret_cast<Ctl*>(words);
+  uint32_t* const g = reinterpret_cast<uint32_t*>(f.ctl);
+  for (int i = threadIdx.x; i < kWords; i += TH) words[i] = g[i];
+  __syncthreads();
+  const int kind = ctl->step_kind;
+  if (kind == kNone) {
+    if (threadIdx.x == 0 && !ctl->halt) f.ctl->solve_req = 0;
+    return;
+  }
+  const bool print = ctl->print_done != 0;
+  // the mean of the solved field; after an incremental update, C:(ebar - <eps*>)
+  // of the same linear solve
+  const bool solved = print || kind == kThermal || kind == kAthermal;
+  const bool fieldmean = f.msum != nullptr && (print || !(kp.incr64 && kind == kThermal));
+  if (solved && fieldmean) field_mean_stress(kp, f, ctl->stress);
+  if (threadIdx.x < 32) {
+    // a lane per component: the mean stress, and the strain of its difference
+    // from the applied stress or of the error to subtract
+    __shared__ double inv[6];
+    const int c = threadIdx.x;
+    if (solved && !fieldmean) {
+      const double e = c < kp.nc ? ctl->eps_avg[c] - ctl->eps0_sum[c] * kp.invN : 0.0;
+      const double e0 = __shfl_sync(FULL, e, 0), e1 = __shfl_sync(FULL, e, 1), e2 = __shfl_sync(FULL, e, 2);
+      const double tr = kp.nc == 3 ? e0 + e1 : e0 + e1 + e2;
+      if (c < kp.nc) ctl->stress[c] = (c < ndiag(kp.nc) ? kp.lambda * tr : 0.0) + 2.0 * kp.mu * e;
+      __syncwarp();
+    }
+    double s = 0;
+    if (kp.loading == STZ_LOAD_STRESS) {
+      if (c < kp.nc) s = kp.applied[c] - ctl->stress[c];
+    } else if (!kp.no_subtract_error) {
+      const int zc = kind == kAthermal && kp.nc == 3 ? 0 : loaded_comp(kp);
+      if (c < kp.nc && c != zc) s = ctl->stress[c];
+    }
+    s = iso_inv_lane(kp, s, c);
+    if (c < kp.nc) inv[c] = s;
+    __syncwarp();
+    if (c == 0) post_step(kp, ctl, print, solved, inv);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kWords; i += TH) g[i] = words[i];
 }
 
 // FP64 incremental form, after a thermal event: the field the re-solve would
