@@ -494,6 +494,18 @@ int build_response_table(stz_ctx* c) {
   return STZ_OK;
 }
 
+// Parts (1, 2 or 4) that the rate kernel splits the modes of a block's sites
+// into, on grids of one site per thread: as many as leave one round of resident
+// blocks. A 64^2 grid has 16 blocks for 304 places (21 us in four parts, 25.5
+// whole). Beyond one round a part's own operands and sums cost more than the
+// evener rounds give: 512^2, seven rounds of half the modes in place of four,
+// 111 us against 102; 64^3 64 against 57.
+int rate_fx_split(int nblk, int resident) {
+  int s = 1;
+  while (s < 4 && nblk * 2 * s <= resident) s *= 2;
+  return s;
+}
+
 // ------------------------------------------------------------- stepping
 // One driver-loop iteration of the FP64 forms, as a fixed kernel sequence.
 // One driver step of the FP64 forms; t0/t1 (optional) are recorded around the
@@ -972,7 +984,9 @@ int stz::create_ctx(const stz_params* pin, stz_ctx** out, int units_per_block) {
     c->rx.tab = c->exptab;
     int sms = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device);
-    c->rx.grid = std::min(kp.nblk, sms * rate_fx_blocks_per_sm(p.model, kp.bsites / kRateThreads));
+    const int spt = kp.bsites / kRateThreads;
+    c->rx.split = spt == 1 ? rate_fx_split(kp.nblk, sms * rate_fx_blocks_per_sm(p.model, 1, 2)) : 1;
+    c->rx.grid = std::min(kp.nblk * c->rx.split, sms * rate_fx_blocks_per_sm(p.model, spt, c->rx.split));
     if (ref2d && c->rx.on) {
       const size_t nm = (size_t)STZ_MODES * N;
       if ((st = dalloc(&c->rx.cq, nm)) || (st = dalloc(&c->rx.dx, nm)) || (st = dalloc(&c->rx.dxy, nm))) return fail(st);

@@ -228,7 +228,8 @@ struct RateFx {
   Fx *dx, *dxy;       // [MODES][N] deps xx and xy, x 2^60 (the modes are traceless)
   Fx *ux, *uxy;       // [MODES][N] deps xx and xy over the mode's norm, x 2^60 (softening only)
   Fx* pn;             // [2][N] (xx - yy) and 2 xy of the last increment over its norm, x 2^60
-  int grid;           // resident blocks of the rate kernel (at most nblk)
+  int grid;           // resident blocks of the rate kernel (at most nblk split)
+  int split;          // parts that a block's modes are split into (rate_fx_split)
 };
 constexpr int kFxRateShift = 5;
 // the smallest and largest Y of a site before its stress terms

@@ -574,6 +574,11 @@ struct R2Fx {
   int mro;         // crystal-like type under NO_SF_XTAL_MRO, else 0
   bool softened;
 };
+// ... and the stored operands of one of its modes
+struct R2Mode {
+  uint64_t cq;
+  Fx dx, dxy, ux, uxy;
+};
 constexpr int kFxR2Shift = 8;
 __device__ __forceinline__ Fx fx_load(const Fx* p) {
   const int2 v = *reinterpret_cast<const int2*>(p);
@@ -650,11 +655,12 @@ __device__ __forceinline__ int64_t fx_exp2_neg(int64_t z, const FxExp* tab, int*
 // The constant part of a softened site's argument: C - (C - cq) 2^(-z), z =
 // modifier (x 2^62) soft; the direction modifiers of init.c:590-642, a
 // crystal-like site's scaled by its factor to the power m + 2.
-__device__ __forceinline__ uint64_t r2_fx_soften(const KParams& kp, const RateFx& rx, const Fields& f, const FxExp* tab,
-                                                 const R2Fx& d, long long i, int m, uint64_t cq) {
+__device__ __forceinline__ uint64_t r2_fx_soften(const KParams& kp, const RateFx& rx, const FxExp* tab, const R2Fx& d,
+                                                 const R2Mode& q, int m) {
+  const uint64_t cq = q.cq;
   FxAcc p{0, 0};
-  fx_mad(p, d.p0, fx_load(rx.ux + i));
-  fx_mad(p, d.p2, fx_load(rx.uxy + i));
+  fx_mad(p, d.p0, q.ux);
+  fx_mad(p, d.p2, q.uxy);
   constexpr int64_t one = 1ll << 62;
   int64_t DM = fx_value<6>(p);  // x 2^62
   DM = DM > one ? one : (DM < -one ? -one : DM);
@@ -676,17 +682,33 @@ __device__ __forceinline__ uint64_t r2_fx_soften(const KParams& kp, const RateFx
   const int64_t R = fx_exp2_neg(fx_mul<4>(mod, d.soft), tab, &n);
   return rx.neg - (uint64_t)(fx_mul<3>((int64_t)(rx.neg - cq), fx_split(R >> 1)) >> n);
 }
-__device__ __forceinline__ uint64_t r2_fx_arg(const KParams& kp, const RateFx& rx, const Fields& f, const FxExp* tab,
-                                              const R2Fx& d, long long s, int m, bool* ok) {
+__device__ __forceinline__ R2Mode r2_fx_mode(const KParams& kp, const RateFx& rx, const R2Fx& d, long long s, int m) {
   const long long i = (long long)m * kp.N + s;
-  uint64_t cq = rx.cq[i];
+  R2Mode q;
+  q.cq = rx.cq[i];
+  q.dx = fx_load(rx.dx + i);
+  q.dxy = fx_load(rx.dxy + i);
+  q.ux = q.uxy = Fx{0, 0};
+  if (d.softened) {
+    q.ux = fx_load(rx.ux + i);
+    q.uxy = fx_load(rx.uxy + i);
+  }
+  return q;
+}
+__device__ __forceinline__ uint64_t r2_fx_arg(const KParams& kp, const RateFx& rx, const FxExp* tab, const R2Fx& d,
+                                              const R2Mode& q, int m, bool* ok) {
+  uint64_t cq = q.cq;
   FxAcc a{0, 0};
-  fx_mad(a, d.W0, fx_load(rx.dx + i));
-  fx_mad(a, d.W2, fx_load(rx.dxy + i));
+  fx_mad(a, d.W0, q.dx);
+  fx_mad(a, d.W2, q.dxy);
   // the work term within 2^8 in magnitude
   *ok &= cq != 0 && (uint32_t)((int32_t)(a.hh >> 32) + (1 << 21)) < (1u << 22);
-  if (d.softened) cq = r2_fx_soften(kp, rx, f, tab, d, i, m, cq);
+  if (d.softened) cq = r2_fx_soften(kp, rx, tab, d, q, m);
   return cq + (uint64_t)fx_value<kFxR2Shift>(a);
+}
+__device__ __forceinline__ uint64_t r2_fx_arg(const KParams& kp, const RateFx& rx, const FxExp* tab, const R2Fx& d,
+                                              long long s, int m, bool* ok) {
+  return r2_fx_arg(kp, rx, tab, d, r2_fx_mode(kp, rx, d, s, m), m, ok);
 }
 
 // The stored fixed-point operands of one (mode, site) and of a site's last
@@ -788,7 +810,7 @@ __device__ __noinline__ double block_incl_scan(double v, double* sh_inc) {
 // the lanes halve the modes they hold at every step (20, 10, 5, 3, 2, 1): 21
 // FP64 additions per warp instead of the 100 of one butterfly per mode, at 19
 // SM clocks each a fifth of a pass over one site per thread.
-__device__ __forceinline__ void block_mode_sums(const double* acc, double* part, int nblk, int b) {
+__device__ __forceinline__ void block_mode_sums(const double* acc, double* part, int nblk, int b, int m0, int m1) {
   static_assert(STZ_MODES == 20, "the halving below is written for 20 modes");
   __shared__ double red[TH / 32][STZ_MODES];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -809,7 +831,7 @@ __device__ __forceinline__ void block_mode_sums(const double* acc, double* part,
   const int k = (u2 ? 3 : 0) + (u1 ? 1 : 0) + (u0 ? 2 : 0);
   if (!u0 || (!u1 && !u2)) red[w][(u4 ? 10 : 0) + (u3 ? 5 : 0) + k] = t;
   __syncthreads();
-  if (threadIdx.x < STZ_MODES) {
+  if ((int)threadIdx.x >= m0 && (int)threadIdx.x < m1) {
     double s = 0;
     for (int q = 0; q < TH / 32; q++) s += red[q][threadIdx.x];
     part[(long long)threadIdx.x * nblk + b] = s;
@@ -900,7 +922,7 @@ __device__ void block_twist(MT* g) {
 // blocks reduces the group's per-(mode, block) sums to per-(mode, group) sums
 // with a fixed warp butterfly (every lane ends with the same bits). Returns
 // true in that block.
-__device__ bool group_reduce(const KParams& kp, const Fields& f, int b) {
+__device__ bool group_reduce(const KParams& kp, const Fields& f, int b, int split) {
   __shared__ bool is_last;
   const int g = b / kGroup;
   const int g0 = g * kGroup, g1 = min(g0 + kGroup, kp.nblk);
@@ -908,7 +930,7 @@ __device__ bool group_reduce(const KParams& kp, const Fields& f, int b) {
   __syncthreads();
   if (threadIdx.x == 0) {
     const unsigned t = atomicAdd(&f.gticket[g], 1u);
-    is_last = (t == (unsigned)(g1 - g0 - 1));
+    is_last = (t == (unsigned)((g1 - g0) * split - 1));
   }
   __syncthreads();
   if (!is_last) return false;
@@ -934,7 +956,7 @@ __device__ __forceinline__ double site_rate(const KParams& kp, const Fields& f, 
     R2Fx x;
     if (rx.on && r2_fx_u(rx, u, ufx) && r2_fx_site(kp, rx, f, ufx, totime, s, &x)) {
       bool ok = true;
-      const uint64_t Y = r2_fx_arg(kp, rx, f, rx.tab, x, s, m, &ok);
+      const uint64_t Y = r2_fx_arg(kp, rx, rx.tab, x, s, m, &ok);
       if (ok) return fx_double(fx_exp2_bits(Y, fx_cell(rx.tab, fx_exp_cell(Y))));
     }
     const R2Site d = r2_load(kp, f, u, totime, s);
@@ -1410,7 +1432,7 @@ __device__ __noinline__ void finish_step(const KParams& kp, const Fields& f, con
 // thread of the block calls it).
 template <int MODEL>
 __device__ __noinline__ unsigned rate_chunk_fp64(const KParams& kp, const Fields& f, const double* u, double totime,
-                                                 int b, long long s0, long long s1) {
+                                                 int b, long long s0, long long s1, int m0, int m1) {
   double acc[STZ_MODES];
 #pragma unroll
   for (int m = 0; m < STZ_MODES; m++) acc[m] = 0;
@@ -1436,16 +1458,16 @@ __device__ __noinline__ unsigned rate_chunk_fp64(const KParams& kp, const Fields
       }
     }
   }
-  block_mode_sums(acc, f.part, kp.nblk, b);
+  block_mode_sums(acc, f.part, kp.nblk, b, m0, m1);
   return neg;
 }
 
 // What every chunk ends with: its count of negative barriers, the group's and
 // the grid's last-block tests. True in the block that finishes the step.
-__device__ __forceinline__ bool chunk_done(const KParams& kp, const Fields& f, int b, unsigned neg) {
+__device__ __forceinline__ bool chunk_done(const KParams& kp, const Fields& f, int b, unsigned neg, int split) {
   const unsigned nb = block_sum_u(neg);
   if (threadIdx.x == 0 && nb) atomicAdd(&f.ctl->neg_count, (unsigned long long)nb);
-  return group_reduce(kp, f, b) && last_block(f.ctl, kp.ngroups);
+  return group_reduce(kp, f, b, split) && last_block(f.ctl, kp.ngroups);
 }
 
 template <int MODEL>
@@ -1457,8 +1479,8 @@ __global__ void __launch_bounds__(TH) k_rate64(KParams kp, Fields f, RateFx rx) 
   const long long s1 = min(s0 + (long long)kp.bsites, kp.N);
   double u[6];
   for (int c = 0; c < 6; c++) u[c] = ctl->u[c];
-  const unsigned neg = rate_chunk_fp64<MODEL>(kp, f, u, ctl->totime, b, s0, s1);
-  if (chunk_done(kp, f, b, neg)) finish_step<MODEL>(kp, f, rx);
+  const unsigned neg = rate_chunk_fp64<MODEL>(kp, f, u, ctl->totime, b, s0, s1, 0, STZ_MODES);
+  if (chunk_done(kp, f, b, neg, 1)) finish_step<MODEL>(kp, f, rx);
 }
 
 // Sums of N values per lane over the warp, the lanes halving the values they
@@ -1501,9 +1523,9 @@ struct WarpSums<N, 0> {
 // instructions per site and mode; integer dispatch bounds it now). Blocks per
 // SM: at four sites per thread 128 registers (two blocks) and 80 (three, 156
 // bytes of spills) measured the same, 277 and 275 us.
-template <int Q>
+template <int Q, bool SPLIT = false>
 __global__ void __launch_bounds__(TH, Q == 4 ? 2 : 3) k_rate64_fx(KParams kp, Fields f, RateFx rx) {
-  constexpr int G = Q == 1 ? 10 : (Q == 2 ? 5 : 4);  // modes per reduction
+  constexpr int G = Q == 4 ? 4 : Q == 2 || SPLIT ? 5 : 10;  // modes per reduction
   __shared__ FxExp tab[kFxExpCells];
   __shared__ int64_t sh_u[6];
   __shared__ int sh_uok;
@@ -1520,7 +1542,9 @@ __global__ void __launch_bounds__(TH, Q == 4 ? 2 : 3) k_rate64_fx(KParams kp, Fi
   __syncthreads();
   const unsigned tab_at = (unsigned)__cvta_generic_to_shared(tab);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int b = blockIdx.x; b < kp.nblk; b += gridDim.x) {
+  const int nm = STZ_MODES / rx.split;
+  for (int it = blockIdx.x; it < kp.nblk * rx.split; it += gridDim.x) {
+    const int part = it / kp.nblk, b = it - part * kp.nblk, m0 = part * nm, m1 = m0 + nm;
     const long long s0 = (long long)b * kp.bsites;
     const long long s1 = min(s0 + (long long)kp.bsites, kp.N);
     bool ok = sh_uok;
@@ -1540,7 +1564,7 @@ __global__ void __launch_bounds__(TH, Q == 4 ? 2 : 3) k_rate64_fx(KParams kp, Fi
     }
     if (!__syncthreads_or(!ok)) {
 #pragma unroll 1
-      for (int g = 0; g < STZ_MODES; g += G) {
+      for (int g = m0; g < m1; g += G) {
         double v[G];
 #pragma unroll
         for (int i = 0; i < G; i++) {
@@ -1562,10 +1586,10 @@ __global__ void __launch_bounds__(TH, Q == 4 ? 2 : 3) k_rate64_fx(KParams kp, Fi
 #pragma unroll
         for (int q = 0; q < Q; q++)
 #pragma unroll 1
-          for (int m = 0; m < STZ_MODES; m++) neg += g3_fx_arg(rx, W[q], a0[q], m) > rx.neg;
+          for (int m = m0; m < m1; m++) neg += g3_fx_arg(rx, W[q], a0[q], m) > rx.neg;
       }
       __syncthreads();
-      if (threadIdx.x < STZ_MODES) {
+      if ((int)threadIdx.x >= m0 && (int)threadIdx.x < m1) {
         double t = 0;
 #pragma unroll
         for (int k = 0; k < TH / 32; k++) t += red[k][threadIdx.x];
@@ -1574,18 +1598,19 @@ __global__ void __launch_bounds__(TH, Q == 4 ? 2 : 3) k_rate64_fx(KParams kp, Fi
     } else {
       double u[6];
       for (int c = 0; c < 6; c++) u[c] = ctl->u[c];
-      neg = rate_chunk_fp64<1>(kp, f, u, ctl->totime, b, s0, s1);
+      neg = rate_chunk_fp64<1>(kp, f, u, ctl->totime, b, s0, s1, m0, m1);
     }
-    if (chunk_done(kp, f, b, neg)) finish_step<1>(kp, f, rx);
+    if (chunk_done(kp, f, b, neg, rx.split)) finish_step<1>(kp, f, rx);
   }
 }
 
 // The rates of the 2D model in fixed point: per (mode, site) the stored operands
 // (24 bytes, 40 at a softened site) in place of the FP64 barrier, increments and
 // norm. Otherwise as k_rate64_fx.
-template <int Q>
-__global__ void __launch_bounds__(TH, 3) k_rate64_fx2(KParams kp, Fields f, RateFx rx) {
-  constexpr int G = Q == 1 ? 10 : (Q == 2 ? 5 : 4);  // modes per reduction
+template <int Q, bool SPLIT = false>
+__global__ void __launch_bounds__(TH, 2) k_rate64_fx2(KParams kp, Fields f, RateFx rx) {
+  constexpr int G = Q > 1 ? 4 : SPLIT ? 5 : 10;     // modes per reduction
+  constexpr int B = Q == 1 ? 5 : (Q == 2 ? 2 : 1);  // modes whose operands are loaded together
   __shared__ FxExp tab[kFxExpCells];
   __shared__ int64_t sh_u[3];
   __shared__ int sh_uok;
@@ -1603,7 +1628,9 @@ __global__ void __launch_bounds__(TH, 3) k_rate64_fx2(KParams kp, Fields f, Rate
   __syncthreads();
   const unsigned tab_at = (unsigned)__cvta_generic_to_shared(tab);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int b = blockIdx.x; b < kp.nblk; b += gridDim.x) {
+  const int nm = STZ_MODES / rx.split;
+  for (int it = blockIdx.x; it < kp.nblk * rx.split; it += gridDim.x) {
+    const int part = it / kp.nblk, b = it - part * kp.nblk, m0 = part * nm, m1 = m0 + nm;
     const long long s0 = (long long)b * kp.bsites;
     const long long s1 = min(s0 + (long long)kp.bsites, kp.N);
     bool ok = sh_uok;
@@ -1615,21 +1642,34 @@ __global__ void __launch_bounds__(TH, 3) k_rate64_fx2(KParams kp, Fields f, Rate
       if (s < s1) ok &= r2_fx_site(kp, rx, f, sh_u, totime, s, &d[q]);
     }
 #pragma unroll 1
-    for (int g = 0; g < STZ_MODES; g += G) {
+    for (int g = m0; g < m1; g += G) {
       double v[G];
+      // the operands of B modes in flight together: one mode at a time, between
+      // the softened sites' branches, waited on each (120 us at 512^2, 102 so)
 #pragma unroll
-      for (int i = 0; i < G; i++) {
-        uint64_t Y[Q];
-        FxExp c[Q];
+      for (int h = 0; h < G; h += B) {
+        R2Mode o[B][Q];
 #pragma unroll
-        for (int q = 0; q < Q; q++) {
-          const long long s = s0 + threadIdx.x + q * TH;
-          Y[q] = (uint64_t)1 << 53;  // no site: the smallest representable rate, 2^-1021
-          if (s < s1) Y[q] = r2_fx_arg(kp, rx, f, tab, d[q], s, g + i, &ok);
-          top = max(top, (unsigned)(Y[q] >> 32));
-          c[q] = fx_cell_shared(tab_at, Y[q]);
+        for (int i = 0; i < B; i++)
+#pragma unroll
+          for (int q = 0; q < Q; q++) {
+            const long long s = s0 + threadIdx.x + q * TH;
+            if (s < s1) o[i][q] = r2_fx_mode(kp, rx, d[q], s, g + h + i);
+          }
+#pragma unroll
+        for (int i = 0; i < B; i++) {
+          uint64_t Y[Q];
+          FxExp c[Q];
+#pragma unroll
+          for (int q = 0; q < Q; q++) {
+            const long long s = s0 + threadIdx.x + q * TH;
+            Y[q] = (uint64_t)1 << 53;  // no site: the smallest representable rate, 2^-1021
+            if (s < s1) Y[q] = r2_fx_arg(kp, rx, tab, d[q], o[i][q], g + h + i, &ok);
+            top = max(top, (unsigned)(Y[q] >> 32));
+            c[q] = fx_cell_shared(tab_at, Y[q]);
+          }
+          v[h + i] = fx_double(fx_exp2_sum_bits<Q>(Y, c));
         }
-        v[i] = fx_double(fx_exp2_sum_bits<Q>(Y, c));
       }
       int idx;
       const double t = WarpSums<G, 16>::run(v, lane, &idx);
@@ -1641,11 +1681,11 @@ __global__ void __launch_bounds__(TH, 3) k_rate64_fx2(KParams kp, Fields f, Rate
         const long long s = s0 + threadIdx.x + q * TH;
         if (s < s1)
 #pragma unroll 1
-          for (int m = 0; m < STZ_MODES; m++) neg += r2_fx_arg(kp, rx, f, tab, d[q], s, m, &ok) > rx.neg;
+          for (int m = m0; m < m1; m++) neg += r2_fx_arg(kp, rx, tab, d[q], s, m, &ok) > rx.neg;
       }
     }
     if (!__syncthreads_or(!ok)) {
-      if (threadIdx.x < STZ_MODES) {
+      if ((int)threadIdx.x >= m0 && (int)threadIdx.x < m1) {
         double t = 0;
 #pragma unroll
         for (int k = 0; k < TH / 32; k++) t += red[k][threadIdx.x];
@@ -1654,9 +1694,9 @@ __global__ void __launch_bounds__(TH, 3) k_rate64_fx2(KParams kp, Fields f, Rate
     } else {
       double u[6];
       for (int c = 0; c < 6; c++) u[c] = ctl->u[c];
-      neg = rate_chunk_fp64<0>(kp, f, u, totime, b, s0, s1);
+      neg = rate_chunk_fp64<0>(kp, f, u, totime, b, s0, s1, m0, m1);
     }
-    if (chunk_done(kp, f, b, neg)) finish_step<0>(kp, f, rx);
+    if (chunk_done(kp, f, b, neg, rx.split)) finish_step<0>(kp, f, rx);
   }
 }
 
@@ -1676,7 +1716,7 @@ __device__ int ath_site(const KParams& kp, const Fields& f, const RateFx& rx, co
       R2Fx d;
       ok = r2_fx_site(kp, rx, f, ufx, totime, s, &d);
       for (int m = 0; m < STZ_MODES; m++) {
-        const uint64_t Y = r2_fx_arg(kp, rx, f, rx.tab, d, s, m, &ok);
+        const uint64_t Y = r2_fx_arg(kp, rx, rx.tab, d, s, m, &ok);
         if (Y > top) { mm = m; top = Y; }
       }
     } else {
@@ -3623,16 +3663,16 @@ __global__ void k_hold(unsigned long long ns) {
 
 namespace {
 template <int MODEL>
-const void* rate_fx_kernel(int spt) {
+auto rate_fx_kernel(int spt, int split) -> void (*)(KParams, Fields, RateFx) {
   if (MODEL == 0)
-    return spt == 1 ? (const void*)k_rate64_fx2<1> : spt == 2 ? (const void*)k_rate64_fx2<2> : (const void*)k_rate64_fx2<4>;
-  return spt == 1 ? (const void*)k_rate64_fx<1> : spt == 2 ? (const void*)k_rate64_fx<2> : (const void*)k_rate64_fx<4>;
+    return spt == 4 ? k_rate64_fx2<4> : spt == 2 ? k_rate64_fx2<2> : split > 1 ? k_rate64_fx2<1, true> : k_rate64_fx2<1>;
+  return spt == 4 ? k_rate64_fx<4> : spt == 2 ? k_rate64_fx<2> : split > 1 ? k_rate64_fx<1, true> : k_rate64_fx<1>;
 }
 }  // namespace
 
-int rate_fx_blocks_per_sm(int model, int spt) {
+int rate_fx_blocks_per_sm(int model, int spt, int split) {
   int occ = 0;
-  const void* k = model == STZ_MODEL_REF2D ? rate_fx_kernel<0>(spt) : rate_fx_kernel<1>(spt);
+  const auto k = model == STZ_MODEL_REF2D ? rate_fx_kernel<0>(spt, split) : rate_fx_kernel<1>(spt, split);
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, TH, 0) != cudaSuccess || occ < 1) {
     (void)cudaGetLastError();
     occ = 1;
@@ -3644,14 +3684,10 @@ void launch_rate_fp64(const KParams& kp, const Fields& f, const RateFx& rx, cuda
   if (!rx.on) {
     if (kp.model == STZ_MODEL_REF2D) k_rate64<0><<<kp.nblk, TH, 0, st>>>(kp, f, rx);
     else k_rate64<1><<<kp.nblk, TH, 0, st>>>(kp, f, rx);
-  } else if (kp.model == STZ_MODEL_REF2D) {
-    if (kp.bsites == TH) k_rate64_fx2<1><<<rx.grid, TH, 0, st>>>(kp, f, rx);
-    else if (kp.bsites == 2 * TH) k_rate64_fx2<2><<<rx.grid, TH, 0, st>>>(kp, f, rx);
-    else k_rate64_fx2<4><<<rx.grid, TH, 0, st>>>(kp, f, rx);
   } else {
-    if (kp.bsites == TH) k_rate64_fx<1><<<rx.grid, TH, 0, st>>>(kp, f, rx);
-    else if (kp.bsites == 2 * TH) k_rate64_fx<2><<<rx.grid, TH, 0, st>>>(kp, f, rx);
-    else k_rate64_fx<4><<<rx.grid, TH, 0, st>>>(kp, f, rx);
+    const int spt = kp.bsites / TH;
+    const auto k = kp.model == STZ_MODEL_REF2D ? rate_fx_kernel<0>(spt, rx.split) : rate_fx_kernel<1>(spt, rx.split);
+    k<<<rx.grid, TH, 0, st>>>(kp, f, rx);
   }
 }
 

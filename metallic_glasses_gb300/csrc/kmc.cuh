@@ -16,7 +16,7 @@ constexpr int kGroup = 32;     // blocks per group in the two-level rate sums
 void launch_rate_fp64(const KParams& kp, const Fields& f, const RateFx& rx, cudaStream_t st);
 // Resident blocks per SM of the fixed-point rate kernel (occupancy query) at
 // spt (1, 2 or 4) sites per thread.
-int rate_fx_blocks_per_sm(int model, int spt);
+int rate_fx_blocks_per_sm(int model, int spt, int split);
 // Mixed form: incremental stress update + rates + selection/commit.
 // update_only: apply the pending transformation and uniform change, nothing else.
 void launch_mixed(const KParams& kp, const Fields& f, int update_only, cudaStream_t st);

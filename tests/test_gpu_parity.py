@@ -669,3 +669,18 @@ def test_octant_update_is_the_solve(engine_lib, shape, shift):
         d = a[c] - b[c]
         assert np.abs(d - d.mean()).max() < 1e-14 * size
     eng.close()
+
+
+@pytest.mark.parametrize("odd", [None, "mode"])
+@pytest.mark.parametrize("shape", [(72, 96), (162, 192), (192, 216)])
+def test_split_2d_rates_match_fp64_rates(engine_lib, shape, odd):
+    """The same on grids whose blocks' modes are split into four, two and one
+    parts (up to 76, 152 and more blocks of 256 sites on 152 multiprocessors);
+    `odd`: a value that sends one part of a block through the FP64 chain."""
+    test_fixed_point_2d_rates_match_fp64_rates(engine_lib, shape, api.SF_SQUARE_FWD, 0.0, odd)
+
+
+@pytest.mark.parametrize("shape", [(36, 36, 36), (48, 48, 54)])
+def test_split_3d_rates_match_fp64_rates(engine_lib, shape):
+    """The 3D rates in two parts and in one (up to 228 and more blocks)."""
+    test_fixed_point_rates_match_fp64_rates(engine_lib, shape, None)
