@@ -629,17 +629,16 @@ __device__ __forceinline__ void green_tile(int tile, double2* __restrict__ spec,
     if (threadIdx.x < L) lkb[threadIdx.x] = max(0, ga.kb - 29 + (32 - __clz(lkb[threadIdx.x])));
     __syncthreads();
   }
-  // The operator in place, a thread per real or imaginary part (even and odd
-  // threads), the parts exchanged for the inverse transform; the lines' new
-  // sums of magnitudes.
+  // The operator in place, both parts of a wave number by one thread (its unit
+  // vector is the larger half of the work), exchanged for the inverse
+  // transform; the lines' new sums of magnitudes.
   float ns[NC];
 #pragma unroll
   for (int c = 0; c < NC; c++) ns[c] = 0.f;
   {
-    const int part = threadIdx.x & 1;
-    const int lg = lgL, items = n << lg;
-    for (int i = threadIdx.x >> 1; i < items; i += blockDim.x >> 1) {
-      const int l1 = i & (L - 1), p = i >> lg, q1 = q0 + l1;
+    const int items = n << lgL;
+    for (int i = threadIdx.x; i < items; i += blockDim.x) {
+      const int l1 = i & (L - 1), p = i >> lgL, q1 = q0 + l1;
       if (q1 >= inner) continue;
       int k0, k1, k2;
       if (NC == 6) {
@@ -651,24 +650,34 @@ __device__ __forceinline__ void green_tile(int tile, double2* __restrict__ spec,
         k1 = p;
         k2 = q1;
       }
-      int64_t* at = reinterpret_cast<int64_t*>(res + l1 * ld + pad(p));
-      const int cstep = 2 * L * ld;
+      cx* at = res + l1 * ld + pad(p);
+      const int cstep = L * ld;
       const int kb = lkb[l1];
-      int64_t t[NC], sg[NC];
-      int64_t tr = 0;
+      int64_t t[2][NC], sg[2][NC];
 #pragma unroll
       for (int c = 0; c < NC; c++) {
-        t[c] = at[c * cstep + part];
-        if (kb > 0) t[c] = shift_round(t[c], kb);
-        if (c < ND) tr += t[c];
+        const cx v = at[c * cstep];
+        t[0][c] = v.x;
+        t[1][c] = v.y;
       }
-      const int64_t lt = rmul_s(tr, ga.lam, ga.lams);
 #pragma unroll
-      for (int c = 0; c < ND; c++) t[c] += lt;
+      for (int h = 0; h < 2; h++) {
+        int64_t tr = 0;
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+          if (kb > 0) t[h][c] = shift_round(t[h][c], kb);
+          if (c < ND) tr += t[h][c];
+        }
+        const int64_t lt = rmul_s(tr, ga.lam, ga.lams);
+#pragma unroll
+        for (int c = 0; c < ND; c++) t[h][c] += lt;
+      }
       if ((k0 | k1 | k2) == 0) {
         // -C:eps_hat; the mean strain's part is added by the last pass
 #pragma unroll
-        for (int c = 0; c < NC; c++) sg[c] = -t[c];
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+          for (int c = 0; c < NC; c++) sg[h][c] = -t[h][c];
       } else {
         Fx g[3];
         unit_wave_fx(k0, k1, k2, ga, g);
@@ -677,7 +686,7 @@ __device__ __forceinline__ void green_tile(int tile, double2* __restrict__ spec,
         // reference's real part)
         const int ny = (2 * k2 == ga.n2 ? 1 : 0) | (2 * k1 == ga.n1 ? 2 : 0) | (NC == 6 && 2 * k0 == ga.n0 ? 4 : 0);
 #pragma unroll
-        for (int c = 0; c < NC; c++) sg[c] = 0;
+        for (int c = 0; c < NC; c++) sg[0][c] = sg[1][c] = 0;
         int nv = 0;
 #pragma unroll 1
         for (int f = 0; f <= ny; f++) {
@@ -685,37 +694,29 @@ __device__ __forceinline__ void green_tile(int tile, double2* __restrict__ spec,
           Fx gm[3];
 #pragma unroll
           for (int k = 0; k < 3; k++) gm[k] = (f >> k & 1) ? Fx{-g[k].h, -g[k].l} : g[k];
-          int64_t s1[NC];
-          green_part<NC>(ga, gm, t, s1);
 #pragma unroll
-          for (int c = 0; c < NC; c++) sg[c] += s1[c];
+          for (int h = 0; h < 2; h++) {
+            int64_t s1[NC];
+            green_part<NC>(ga, gm, t[h], s1);
+#pragma unroll
+            for (int c = 0; c < NC; c++) sg[h][c] += s1[c];
+          }
           nv++;
         }
         if (nv > 1) {
           const int sh = nv == 2 ? 1 : (nv == 4 ? 2 : 3);
 #pragma unroll
-          for (int c = 0; c < NC; c++) sg[c] = shift_round(sg[c], sh);
+          for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int c = 0; c < NC; c++) sg[h][c] = shift_round(sg[h][c], sh);
         }
       }
-      __syncwarp(3u << (threadIdx.x & 30));  // both parts have been read
 #pragma unroll
       for (int c = 0; c < NC; c++) {
-        at[c * cstep + 1 - part] = sg[c];
-        ns[c] += (float)(abs((int)(sg[c] >> 32)) + 1);  // in units of 2^32, rounded up
+        at[c * cstep] = cx{sg[1][c], sg[0][c]};
+        // in units of 2^32, rounded up
+        ns[c] += (float)(abs((int)(sg[0][c] >> 32)) + 1) + (float)(abs((int)(sg[1][c] >> 32)) + 1);
       }
-    }
-  }
-  // the threads of an item's column are i % L = (threadIdx.x / 2) % L: column
-  // sums over threads of equal threadIdx.x % (2 L), then the pair
-#pragma unroll
-  for (int c = 0; c < NC; c++) ns[c] += __shfl_xor_sync(FULL, ns[c], 1);
-  if (L < 32) {
-    // move column j's sum from lanes 2 j to lane j of each group of 2 L lanes
-    const int lane = threadIdx.x & 31, src = (lane & ~(2 * L - 1)) | ((2 * lane) & (2 * L - 1));
-#pragma unroll
-    for (int c = 0; c < NC; c++) {
-      const float v = __shfl_sync(FULL, ns[c], src);
-      ns[c] = (lane & L) ? 0.f : v;  // once per group
     }
   }
   // sums in units of 2^32: a top of 29 puts them below 2^61
