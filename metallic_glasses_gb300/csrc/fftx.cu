@@ -29,7 +29,6 @@
 #include <cmath>
 
 #include "fft.cuh"
-#include "pdl.cuh"
 
 namespace stz {
 
@@ -396,8 +395,6 @@ __global__ void __launch_bounds__(kMaxTh) k_r2c_fx(const double* __restrict__ in
                                                    int nh, long long rows, long long N, long long Nk, int L, int lgp,
                                                    FxSched sh, const FxTwiddle* __restrict__ tw_h,
                                                    const FxTwiddle* __restrict__ tw_p, int tiles, const int* gate) {
-  pdl_wait();
-  pdl_release();
   if (gate && *gate == 0) return;
   for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
     if (t != (int)blockIdx.x) __syncthreads();
@@ -454,8 +451,6 @@ template <bool INV, int U>
 __global__ void __launch_bounds__(kMaxTh) k_c2c_fx(double2* __restrict__ data, int n, int nh, int columns, long long Nk,
                                                    int L, int lgL, FxSched sc, const FxTwiddle* __restrict__ tw,
                                                    int tiles, const int* gate) {
-  pdl_wait();
-  pdl_release();
   if (gate && *gate == 0) return;
   for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
     if (t != (int)blockIdx.x) __syncthreads();
@@ -755,8 +750,6 @@ __global__ void __launch_bounds__(kMaxTh, 2) k_green_fx(double2* __restrict__ sp
                                                         long long Nk, int L, int lgL, FxSched sc,
                                                         const FxTwiddle* __restrict__ tw, GreenFx ga, int tiles,
                                                         const int* gate) {
-  pdl_wait();
-  pdl_release();
   if (gate && *gate == 0) return;
   for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
     if (t != (int)blockIdx.x) __syncthreads();
@@ -900,8 +893,6 @@ __global__ void __launch_bounds__(kMaxTh) k_c2r_fx(const double2* __restrict__ i
                                                    const double* __restrict__ ebar, double lambda, double mu,
                                                    double* __restrict__ sig, double* __restrict__ msum, int tiles,
                                                    const int* gate) {
-  pdl_wait();
-  pdl_release();
   if (gate && *gate == 0) return;
   for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
     if (t != (int)blockIdx.x) __syncthreads();
@@ -960,12 +951,6 @@ dim3 fx_grid(const SolveArgs& a, int tiles, int comps) {
   return dim3((unsigned)(a.rare && tiles > most ? most : tiles), (unsigned)comps);
 }
 
-// Whether a pass may be scheduled while the one before it ends (pdl.cuh): in 2D
-// (a step at 64^2 2.7% faster, at 512^2 1.7%). The 3D passes are several waves of
-// blocks, and the next one's blocks then go to the multiprocessors that finish
-// first: 64^3 steps 4.5% slower.
-int fx_early(const FFTPlan& p) { return p.n0 == 1; }
-
 template <int NC>
 void launch_green(const FFTPlan& p, int n, int inner, const SolveArgs& a, const FxSched& x, const FxTwiddle* tw,
                   const GreenFx& ga, cudaStream_t st) {
@@ -976,14 +961,11 @@ void launch_green(const FFTPlan& p, int n, int inner, const SolveArgs& a, const 
   const dim3 grid = fx_grid(a, tiles, 1);
   const int lg = ilog2(p.L_g);
   if (c.U == 1)
-    launch_pdl(k_green_fx<NC, 1>, grid, c.threads, p.smem_gr, st, fx_early(p), spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, tiles,
-               gate);
+    k_green_fx<NC, 1><<<grid, c.threads, p.smem_gr, st>>>(spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, tiles, gate);
   else if (c.U == 2)
-    launch_pdl(k_green_fx<NC, 2>, grid, c.threads, p.smem_gr, st, fx_early(p), spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, tiles,
-               gate);
+    k_green_fx<NC, 2><<<grid, c.threads, p.smem_gr, st>>>(spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, tiles, gate);
   else
-    launch_pdl(k_green_fx<NC, 0>, grid, c.threads, p.smem_gr, st, fx_early(p), spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, tiles,
-               gate);
+    k_green_fx<NC, 0><<<grid, c.threads, p.smem_gr, st>>>(spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, tiles, gate);
 }
 
 template <bool INV>
@@ -993,7 +975,7 @@ void launch_c2c(const FFTPlan& p, const SolveArgs& a, const FxSched& x, cudaStre
   const int tiles = (columns + p.L_y - 1) / p.L_y;
   const dim3 grid = fx_grid(a, tiles, p.nc);
   auto go = [&](auto* k) {
-    launch_pdl(k, grid, c.threads, p.smem_yr, st, fx_early(p), reinterpret_cast<double2*>(a.spec), p.n1, p.nh, columns, p.Nk, p.L_y, lg, x,
+    k<<<grid, c.threads, p.smem_yr, st>>>(reinterpret_cast<double2*>(a.spec), p.n1, p.nh, columns, p.Nk, p.L_y, lg, x,
                                           p.tx_1, tiles, a.gate);
   };
   if (c.U <= 2) go(k_c2c_fx<INV, 2>);
@@ -1046,8 +1028,7 @@ void fftx_spectrum(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_
   const dim3 gx = fx_grid(a, tiles, p.nc);
   const RowLaunch r = row_launch(p.h, p.L_x, p.e_x);
   auto r2c = [&](auto* k) {
-    // (outside the steps after whatever kernel the caller's stream holds: ordinarily)
-    launch_pdl(k, gx, r.threads, p.smem_xr, st, a.gate && fx_early(p), a.eps, spec, p.h, p.nh, rows, p.N, p.Nk, p.L_x, r.lgp, xh, p.tx_h,
+    k<<<gx, r.threads, p.smem_xr, st>>>(a.eps, spec, p.h, p.nh, rows, p.N, p.Nk, p.L_x, r.lgp, xh, p.tx_h,
                                         p.tx_p, tiles, a.gate);
   };
   if (r.U == 1) r2c(k_r2c_fx<1>);
@@ -1075,7 +1056,7 @@ void fftx_c2r(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* la
   const dim3 gx = fx_grid(a, tiles, p.nc);
   const RowLaunch r = row_launch(p.h, p.L_x, p.e_x);
   auto go = [&](auto* k) {
-    launch_pdl(k, gx, r.threads, p.smem_xr, st, fx_early(p), reinterpret_cast<const double2*>(a.spec), p.nc, p.h, p.nh, rows, p.N, p.Nk, p.L_x,
+    k<<<gx, r.threads, p.smem_xr, st>>>(reinterpret_cast<const double2*>(a.spec), p.nc, p.h, p.nh, rows, p.N, p.Nk, p.L_x,
                                         r.lgp, fx_sched(p.sh), p.tx_h, p.tx_p, fftx_factor(p, a.mu), a.ebar, a.lambda,
                                         a.mu, a.sig64, a.msum, tiles, a.gate);
   };

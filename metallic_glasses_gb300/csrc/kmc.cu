@@ -25,7 +25,6 @@
 #include <cstddef>
 
 #include "kmc.cuh"
-#include "pdl.cuh"
 
 namespace stz {
 namespace {
@@ -744,6 +743,13 @@ __device__ __forceinline__ unsigned long long gtimer() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
+
+// Programmatic dependent launch: wait until the preceding kernel of the
+// stream has completed and its writes are visible (a no-op when the kernel
+// was launched without the attribute), and let the following kernel be
+// scheduled early (it still waits for this one before touching memory).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // 2^x with the hardware approximation (PTX ex2.approx.ftz.f32: one MUFU
 // operation, relative error below 2^-22; results under 2^-126 flush to 0).
@@ -1525,16 +1531,13 @@ __global__ void __launch_bounds__(TH, Q == 4 ? 2 : 3) k_rate64_fx(KParams kp, Fi
   __shared__ int sh_uok;
   __shared__ double red[TH / 32][STZ_MODES];
   Ctl* ctl = f.ctl;
+  if (ctl->halt || ctl->step_kind == kPrint) return;
   {
     const int4* src = reinterpret_cast<const int4*>(rx.tab);
     int4* dst = reinterpret_cast<int4*>(tab);
 #pragma unroll
     for (int i = 0; i < kFxExpCells / TH; i++) dst[i * TH + threadIdx.x] = __ldg(src + i * TH + threadIdx.x);
   }
-  // the table is constant; what follows is the previous kernels' work
-  pdl_wait();
-  pdl_release();
-  if (ctl->halt || ctl->step_kind == kPrint) return;
   if (threadIdx.x == 0) sh_uok = g3_fx_u(rx, ctl->u, sh_u);
   __syncthreads();
   const unsigned tab_at = (unsigned)__cvta_generic_to_shared(tab);
@@ -1613,16 +1616,13 @@ __global__ void __launch_bounds__(TH, 2) k_rate64_fx2(KParams kp, Fields f, Rate
   __shared__ int sh_uok;
   __shared__ double red[TH / 32][STZ_MODES];
   Ctl* ctl = f.ctl;
+  if (ctl->halt || ctl->step_kind == kPrint) return;
   {
     const int4* src = reinterpret_cast<const int4*>(rx.tab);
     int4* dst = reinterpret_cast<int4*>(tab);
 #pragma unroll
     for (int i = 0; i < kFxExpCells / TH; i++) dst[i * TH + threadIdx.x] = __ldg(src + i * TH + threadIdx.x);
   }
-  // the table is constant; what follows is the previous kernels' work
-  pdl_wait();
-  pdl_release();
-  if (ctl->halt || ctl->step_kind == kPrint) return;
   const double totime = ctl->totime;
   if (threadIdx.x == 0) sh_uok = r2_fx_u(rx, ctl->u, sh_u);
   __syncthreads();
@@ -1749,8 +1749,6 @@ __device__ __forceinline__ short* mark_counts(const KParams& kp, const Fields& f
 }
 // Mark the sites that join the avalanche, with the count of each chunk of TH sites.
 __global__ void k_ath_mark(KParams kp, Fields f, RateFx rx, int mixed) {
-  pdl_wait();
-  pdl_release();
   Ctl* ctl = f.ctl;
   if (ctl->step_kind != kAthermal) return;
   double u[6];
@@ -1774,8 +1772,6 @@ __global__ void k_ath_mark(KParams kp, Fields f, RateFx rx, int mixed) {
 // reference's space_loop); one block. The chunks' counts lead to the marks: a
 // block-wide walk of every site's mark took 1.1 ms at 512^2.
 __global__ void __launch_bounds__(TH) k_ath_commit(KParams kp, Fields f, RateFx rx, int mixed) {
-  pdl_wait();
-  pdl_release();
   Ctl* ctl = f.ctl;
   if (ctl->step_kind != kAthermal) return;
   __shared__ unsigned ballot[TH / 32], chunks[TH / 32];
@@ -1883,8 +1879,6 @@ __device__ void post_step(const KParams& kp, Ctl* ctl, bool print, bool solved, 
 // tensors by a lane per component, the rest by thread 0. By one thread on the
 // control block in L2 it took 7 to 10 us, and the field mean 12 at 64^3.
 __global__ void __launch_bounds__(TH) k_post(KParams kp, Fields f) {
-  pdl_wait();
-  pdl_release();
   constexpr int kWords = (int)(offsetof(Ctl, rng) / 4);
   __shared__ __align__(16) uint32_t words[sizeof(Ctl) / 4];
   Ctl* const ctl = reinterpret_cast<Ctl*>(words);
@@ -1940,8 +1934,6 @@ __global__ void __launch_bounds__(TH) k_post(KParams kp, Fields f) {
 //
 // 2D: every response of every offset is read (nine values a site).
 __global__ void k_incr64(KParams kp, Fields f) {
-  pdl_wait();
-  pdl_release();
   const Ctl* ctl = f.ctl;
   if (!ctl->incr_req) return;
   const int nc = kp.nc, nd = nc == 3 ? 2 : 3;
@@ -2024,8 +2016,6 @@ __global__ void k_oct_fix(double* tab, int tn) {
 }
 
 __global__ void __launch_bounds__(TH, 2) k_incr64_oct(KParams kp, Fields f) {
-  pdl_wait();
-  pdl_release();
   const Ctl* ctl = f.ctl;
   if (!ctl->incr_req) return;
   __shared__ Fx sd[9];         // the increment's normal components, its shear components twice and once
@@ -2147,8 +2137,6 @@ __global__ void k_note_solve(Fields f, const double* ebar) {
 // The print's reset of the barriers to their initial copy (bmg.c:214-221),
 // when this step printed. Only REF2D grids with crystal-like sites have Q1.
 __global__ void k_q0_reset(KParams kp, Fields f, RateFx rx) {
-  pdl_wait();
-  pdl_release();
   if (f.ctl->step_kind != kPrint) return;
   const long long total = (long long)STZ_MODES * kp.N;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
@@ -3699,7 +3687,7 @@ void launch_rate_fp64(const KParams& kp, const Fields& f, const RateFx& rx, cuda
   } else {
     const int spt = kp.bsites / TH;
     const auto k = kp.model == STZ_MODEL_REF2D ? rate_fx_kernel<0>(spt, rx.split) : rate_fx_kernel<1>(spt, rx.split);
-    launch_pdl(k, rx.grid, TH, 0, st, 1, kp, f, rx);
+    k<<<rx.grid, TH, 0, st>>>(kp, f, rx);
   }
 }
 
@@ -3753,6 +3741,25 @@ int mixed_blocks_per_sm(int n2) {
   return occ;
 }
 
+namespace {
+// Launch with the programmatic-stream-serialization attribute: the kernel may
+// be scheduled while the previous kernel of the stream finishes; it waits for
+// it with griddepcontrol.wait.
+template <typename... A>
+void launch_pdl(void (*kern)(A...), dim3 grid, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(TH);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, args...);
+}
+}  // namespace
 
 int batch_class(int n2) {
   for (int c = 0; c < kBatchClasses - 1; c++)
@@ -3807,18 +3814,18 @@ void launch_mixed_batched(const BatchDesc* d, const int* blk_rep, const int* rep
 void launch_mixed_main(const KParams& kp, const Fields& f, int update_only, cudaStream_t st) {
   mixed_smem_init();
   if (update_only) k_mixed<1><<<kp.nblk, TH, mix_smem_bytes(kp.n2), st>>>(kp, f);
-  else if (kp.general_pass) launch_pdl(k_mixed<0>, dim3(kp.nblk), TH, mix_smem_bytes(kp.n2), st, 1, kp, f);
-  else if (kp.n2 == 256) launch_pdl(k_mixed<0, 256>, dim3(kp.nblk), TH, mix_smem_main_bytes(256), st, 1, kp, f);
-  else if (kp.n2 == 128) launch_pdl(k_mixed<0, 128>, dim3(kp.nblk), TH, mix_smem_bytes(kp.n2), st, 1, kp, f);
-  else if (kp.n2 == 96) launch_pdl(k_mixed<0, 96>, dim3(kp.nblk), TH, mix_smem_bytes(kp.n2), st, 1, kp, f);
-  else if (kp.n2 == 64) launch_pdl(k_mixed<0, 64>, dim3(kp.nblk), TH, mix_smem_bytes(kp.n2), st, 1, kp, f);
-  else if (kp.n2 == 32) launch_pdl(k_mixed<0, 32>, dim3(kp.nblk), TH, mix_smem_bytes(kp.n2), st, 1, kp, f);
-  else launch_pdl(k_mixed<0>, dim3(kp.nblk), TH, mix_smem_bytes(kp.n2), st, 1, kp, f);
+  else if (kp.general_pass) launch_pdl(k_mixed<0>, dim3(kp.nblk), mix_smem_bytes(kp.n2), st, kp, f);
+  else if (kp.n2 == 256) launch_pdl(k_mixed<0, 256>, dim3(kp.nblk), mix_smem_main_bytes(256), st, kp, f);
+  else if (kp.n2 == 128) launch_pdl(k_mixed<0, 128>, dim3(kp.nblk), mix_smem_bytes(kp.n2), st, kp, f);
+  else if (kp.n2 == 96) launch_pdl(k_mixed<0, 96>, dim3(kp.nblk), mix_smem_bytes(kp.n2), st, kp, f);
+  else if (kp.n2 == 64) launch_pdl(k_mixed<0, 64>, dim3(kp.nblk), mix_smem_bytes(kp.n2), st, kp, f);
+  else if (kp.n2 == 32) launch_pdl(k_mixed<0, 32>, dim3(kp.nblk), mix_smem_bytes(kp.n2), st, kp, f);
+  else launch_pdl(k_mixed<0>, dim3(kp.nblk), mix_smem_bytes(kp.n2), st, kp, f);
 }
 
 void launch_mixed_tail(const KParams& kp, const Fields& f, int update_only, cudaStream_t st) {
   if (update_only) k_mixed_tail<<<1, TH, 0, st>>>(kp, f, update_only);
-  else launch_pdl(k_mixed_select, dim3(kp.n0), TH, 0, st, 1, kp, f);
+  else launch_pdl(k_mixed_select, dim3(kp.n0), 0, st, kp, f);
 }
 
 // The stored norms of the modes m0 .. m0 + nm - 1 at every site, from the mode
@@ -3871,19 +3878,19 @@ void launch_mixed(const KParams& kp, const Fields& f, int update_only, cudaStrea
 
 void launch_athermal(const KParams& kp, const Fields& f, const RateFx& rx, int mixed, cudaStream_t st) {
   const long long nb = std::min<long long>((kp.N + TH - 1) / TH, 152LL * 8);
-  launch_pdl(k_ath_mark, (unsigned)nb, TH, 0, st, 1, kp, f, rx, mixed);
-  launch_pdl(k_ath_commit, 1, TH, 0, st, 1, kp, f, rx, mixed);
+  k_ath_mark<<<(unsigned)nb, TH, 0, st>>>(kp, f, rx, mixed);
+  k_ath_commit<<<1, TH, 0, st>>>(kp, f, rx, mixed);
 }
 
-void launch_post(const KParams& kp, const Fields& f, cudaStream_t st) { launch_pdl(k_post, 1, TH, 0, st, 1, kp, f); }
+void launch_post(const KParams& kp, const Fields& f, cudaStream_t st) { k_post<<<1, TH, 0, st>>>(kp, f); }
 
 void launch_incr64(const KParams& kp, const Fields& f, cudaStream_t st) {
   if (kp.n0 > 1) {
     const long long tn = (long long)kp.kt0 * kp.kt1 * kp.kt2;
-    launch_pdl(k_incr64_oct, (unsigned)std::min<long long>((tn + TH - 1) / TH, 152LL * 4), TH, 0, st, 1, kp, f);
+    k_incr64_oct<<<(unsigned)std::min<long long>((tn + TH - 1) / TH, 152LL * 4), TH, 0, st>>>(kp, f);
     return;
   }
-  launch_pdl(k_incr64, (unsigned)std::min<long long>((kp.N + TH - 1) / TH, 152LL * 8), TH, 0, st, 1, kp, f);
+  k_incr64<<<(unsigned)std::min<long long>((kp.N + TH - 1) / TH, 152LL * 8), TH, 0, st>>>(kp, f);
 }
 
 size_t oct_table_len(const KParams& kp) { return (size_t)(kOctPairs + 1) * kp.kt0 * kp.kt1 * kp.kt2; }
@@ -3901,7 +3908,7 @@ void launch_note_solve(const Fields& f, const double* ebar, cudaStream_t st) { k
 void launch_q0_reset(const KParams& kp, const Fields& f, const RateFx& rx, cudaStream_t st) {
   const long long total = (long long)STZ_MODES * kp.N;
   const unsigned nb = (unsigned)std::min<long long>((total + TH - 1) / TH, 152LL * 8);
-  launch_pdl(k_q0_reset, nb, TH, 0, st, 1, kp, f, rx);
+  k_q0_reset<<<nb, TH, 0, st>>>(kp, f, rx);
 }
 
 void launch_mixed_after_resolve(const KParams& kp, const Fields& f, int kind, cudaStream_t st) {
