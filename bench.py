@@ -445,10 +445,11 @@ def main():
         rp = pl["rate_pass"]
         pl = {k: pl[k] for k in ("grid", "sites", "events", "athermal_steps", "ms", "events_per_s", "us_per_event")}
         if rp and rp["achieved_gbs"]:
-            # the FP64 rate kernel against HBM: far below it, the kernel is
-            # bound by the FP64 pipe (ncu: profiles/k_rate64_64.md)
-            pl["roofline"] = {"kernel": "k_rate64<1> (FP64 rates of 20 modes, per-block sums, selection and commit "
-                                        "in the last block)", "bound": "fp64 pipe (HBM shown for scale)",
+            # the FP64 form's rate kernel against HBM: far below it, the kernel is
+            # bound by issuing integer instructions (ncu: profiles/k_rate64_fx.md)
+            pl["roofline"] = {"kernel": "k_rate64_fx<1> (rates of 20 modes in 64-bit fixed point, per-block sums, "
+                                        "selection and commit in the last block)",
+                              "bound": "integer issue (HBM shown for scale)",
                               "achieved": rp["achieved_gbs"], "peak": peak, "unit": "GB/s",
                               "frac": rp["achieved_gbs"] / peak, "alg_bytes_per_launch": rp["alg_bytes"],
                               "launch_ms": rp["launch_ms"], "launches_timed": rp["launches"],

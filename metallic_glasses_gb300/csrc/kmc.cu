@@ -1,9 +1,10 @@
 // kmc.cu -- the STZ kinetic Monte Carlo step on the device.
 //
 // One driver-loop iteration (bmg.c:139-178) of the FP64 forms is
-//   k_rate64     SofteningFactor + ActEnergy + KMC rates for every (mode, site)
-//                (init.c:561-739, evolution.c:120-128), per-(mode, block) FP64
-//                sums; the last block to finish reduces them, decides athermal
+//   k_rate64_fx, k_rate64_fx2   SofteningFactor + ActEnergy + KMC rates for every
+//                (mode, site) in 64-bit fixed point, 3D and 2D (k_rate64: in FP64,
+//                for constants outside its range; init.c:561-739,
+//                evolution.c:120-128), per-(mode, block) FP64 sums; the last block to finish reduces them, decides athermal
 //                / thermal / elastic, draws the dice, finds the event with a
 //                hierarchical search in the reference's mode-major order
 //                (evolution.c:136-193) and commits it (elastic.c:361-520)
@@ -347,7 +348,7 @@ __device__ __forceinline__ double dire_modifier(int scheme, double dot, double r
 // exp_table.h (generated by exp_table.py) as hi + lo, read through L1 since
 // each lane takes its own entry. Within 1 ulp of the C library's exp (checked
 // for 5 10^7 arguments). Arguments outside (-700, 700), and NaN, take the
-// library routine. As written the FP64 pipe (the bound of the rate kernels)
+// library routine. As written the FP64 pipe (the bound of this form of the rates)
 // does the arithmetic only: the range test compares the bit pattern of |x|,
 // 2^m enters as an integer add to the exponent field, and hi + lo rounds to hi
 // (|lo| is below half an ulp of hi), so S(J) of Tang's reconstruction is hi.
@@ -1518,11 +1519,16 @@ struct WarpSums<N, 0> {
 // halving reduction. Blocks run through the chunks b, b + gridDim.x, ... so that
 // the 32 KB exponential table is copied to shared memory once per resident
 // block. A chunk with a value outside the fixed point's range (or a NaN) goes
-// through the FP64 chain as a whole. Measured against the FP64 chain, kernel
-// with selection: 294 -> 66 us at 64^3, 1800 -> 277 us at 128^3 (100
-// instructions per site and mode; integer dispatch bounds it now). Blocks per
-// SM: at four sites per thread 128 registers (two blocks) and 80 (three, 156
-// bytes of spills) measured the same, 277 and 275 us.
+// through the FP64 chain as a whole; the test for negative barriers is a maximum
+// of the arguments, and only a chunk that passes it is counted. With SPLIT a
+// work item is a part of a chunk's modes (rate_fx_split).
+// Measured against the FP64 chain, kernel with selection: 294 -> 57 us at 64^3,
+// 1800 -> 247 us at 128^3 (74 instructions per site and mode, 21 of them wide
+// multiply-adds at 0.8 SM clocks; 102 instructions before the carry pairs of
+// fx_wide and the shorter exponential: 280 us). A quarter of the time at 128^3
+// and half at 64^3 is the one-block tail. More warps do not help: at four sites
+// per thread two blocks of 128 registers and three of 80 take 280 and 278 us,
+// two sites at four blocks 295, one site 316.
 template <int Q, bool SPLIT = false>
 __global__ void __launch_bounds__(TH, Q == 4 ? 2 : 3) k_rate64_fx(KParams kp, Fields f, RateFx rx) {
   constexpr int G = Q == 4 ? 4 : Q == 2 || SPLIT ? 5 : 10;  // modes per reduction
