@@ -677,10 +677,10 @@ int enqueue_graph(stz_ctx* c, int which, int steps, int n) {
 
 // Enqueues the next part of a run of which at least `left` steps (events) are
 // to be done (< 0: no limit). Steps past the target return at once, but each
-// costs its kernels' launches (about 1 us each: eleven in an FP64 step), so a
+// costs its kernels' launches (about 1 us each: seven to ten in an FP64 step), so a
 // short run takes the small graphs: a single step of the 2D model at 64^2
-// took 371 us with the other 15 steps of one 16-step graph behind it, 123 us
-// now. The mixed form has one wait per 64 events (its re-solves and prints are
+// took 371 us with the other 15 steps of one 16-step graph behind it, 127 us
+// without them. The mixed form has one wait per 64 events (its re-solves and prints are
 // serviced there), and launches fewer than 33 events one by one: the host
 // enqueues an event in less time than the device needs for it.
 int enqueue_run(stz_ctx* c, long long left) {
