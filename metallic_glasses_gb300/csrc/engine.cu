@@ -413,10 +413,10 @@ int solve_inhom(stz_ctx* c, const int* gate, const double* ebar) {
   if (!ebar) CK(cudaMemsetAsync(c->f.scratch, 0, sizeof(double) * 6, c->stream));
   launch_inhom_init(kp, f, d_ebar, c->stream);
   std::vector<double> part(kInhomBlocks);
-  for (int step = 1;; step++) {
-    CK(cudaMemcpyAsync(f.inh_last, f.inh_eeff, sizeof(double) * nc * N, cudaMemcpyDeviceToDevice, c->stream));
+  double *last = f.inh_eeff, *next = f.inh_last;  // the iterate that is solved, and the next one
+  for (int step = 1;; step++, std::swap(last, next)) {
     SolveArgs a{};
-    a.eps = f.inh_last;
+    a.eps = last;
     a.ebar = ebar;
     a.lambda = kp.lambda;
     a.mu = kp.mu;
@@ -426,7 +426,7 @@ int solve_inhom(stz_ctx* c, const int* gate, const double* ebar) {
     a.spec = f.spec;
     int st = fft_solve(*plan_of(c), a, c->stream, &c->launches);
     if (st) return st;
-    launch_inhom_update(kp, f, c->stream);
+    launch_inhom_update(kp, f, last, next, c->stream);
     c->launches += 1;
     CK(cudaMemcpyAsync(part.data(), f.inh_part, sizeof(double) * kInhomBlocks, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));

@@ -43,42 +43,29 @@ __device__ void apply_C(const KParams& kp, const double* e, double* s) {
   for (int c = 0; c < kp.nc; c++) s[c] = (c < nd ? kp.lambda * tr : 0.0) + 2.0 * kp.mu * e[c];
 }
 
-// isotropicinv (elastic.c:522-531) in DIM dimensions. The mixed form uses
-// precomputed coefficients (no divisions on the one-thread commit path); the
-// FP64 forms keep the reference's operation order.
+// s / 2 / mu, correctly rounded, by Markstein's refinement of s RN(1/(2 mu))
+// (as over_kT): three operations in place of a division's ten or so in a row.
+__device__ __forceinline__ double over_2mu(const KParams& kp, double s) {
+  const double q = s * kp.inv_2mu;
+  return isfinite(q) ? __fma_rn(__fma_rn(-q, 2.0 * kp.mu, s), kp.inv_2mu, q) : s / 2 / kp.mu;
+}
+// isotropicinv (elastic.c:522-531) in DIM dimensions, the trace's coefficient
+// from the host. The mixed form multiplies by 1/(2 mu) on its one-thread commit
+// path; the FP64 forms take the quotient. With divisions the update of a varying
+// medium, two of these per site, took 31 us of a 256^2 iteration's 105 (90 now).
 __device__ void iso_inv(const KParams& kp, const double* s, double* e) {
-  const double lam = kp.lambda, mu = kp.mu;
-  if (kp.fast_inv) {
-    const int nd = ndiag(kp.nc);
-    double tr = 0;
-    for (int c = 0; c < nd; c++) tr += s[c];
-    const double t = -kp.inv_lam_coef * tr;
-    for (int c = 0; c < kp.nc; c++) e[c] = (c < nd ? t : 0.0) + s[c] * kp.inv_2mu;
-    return;
-  }
-  if (kp.nc == 3) {
-    double tra = -lam / 2 / mu / (2 * lam + 2 * mu) * (s[0] + s[1]);
-    e[0] = tra + s[0] / 2 / mu;
-    e[1] = tra + s[1] / 2 / mu;
-    e[2] = s[2] / 2 / mu;
-  } else {
-    double tra = -lam / 2 / mu / (3 * lam + 2 * mu) * (s[0] + s[1] + s[2]);
-    for (int c = 0; c < 3; c++) e[c] = tra + s[c] / 2 / mu;
-    for (int c = 3; c < 6; c++) e[c] = s[c] / 2 / mu;
-  }
+  const int nd = ndiag(kp.nc);
+  double tr = 0;
+  for (int c = 0; c < nd; c++) tr += s[c];
+  const double t = -kp.inv_lam_coef * tr;
+  for (int c = 0; c < kp.nc; c++) e[c] = (c < nd ? t : 0.0) + (kp.fast_inv ? s[c] * kp.inv_2mu : over_2mu(kp, s[c]));
 }
 // Component `lane` of the same, its s in every lane of a warp (0 beyond the
-// last): the divisions side by side, some 900 clocks each.
+// last).
 __device__ double iso_inv_lane(const KParams& kp, double s, int lane) {
   const double s0 = __shfl_sync(FULL, s, 0), s1 = __shfl_sync(FULL, s, 1), s2 = __shfl_sync(FULL, s, 2);
-  const double lam = kp.lambda, mu = kp.mu;
-  const bool d2 = kp.nc == 3;
-  if (kp.fast_inv) {
-    const double tr = d2 ? s0 + s1 : s0 + s1 + s2;
-    return (lane < ndiag(kp.nc) ? -kp.inv_lam_coef * tr : 0.0) + s * kp.inv_2mu;
-  }
-  const double tra = -lam / 2 / mu / ((d2 ? 2 : 3) * lam + 2 * mu) * (d2 ? s0 + s1 : s0 + s1 + s2);
-  return lane < ndiag(kp.nc) ? tra + s / 2 / mu : s / 2 / mu;
+  const double t = -kp.inv_lam_coef * (kp.nc == 3 ? s0 + s1 : s0 + s1 + s2);
+  return (lane < ndiag(kp.nc) ? t : 0.0) + (kp.fast_inv ? s * kp.inv_2mu : over_2mu(kp, s));
 }
 
 // AvgStress (elastic.c:733-752): mean of the solved field, from the per-block
@@ -3942,9 +3929,8 @@ void launch_inhom_init(const KParams& kp, const Fields& f, const double* ebar, c
   k_inhom_init<<<kInhomBlocks, TH, 0, st>>>(kp, f.eps0, ebar, f.lam_site, f.mu_site, f.inh_tau0, f.inh_eeff);
 }
 
-void launch_inhom_update(const KParams& kp, const Fields& f, cudaStream_t st) {
-  k_inhom_update<<<kInhomBlocks, TH, 0, st>>>(kp, f.sig, f.inh_last, f.lam_site, f.mu_site, f.inh_tau0, f.inh_eeff,
-                                              f.inh_part);
+void launch_inhom_update(const KParams& kp, const Fields& f, const double* last, double* eeff, cudaStream_t st) {
+  k_inhom_update<<<kInhomBlocks, TH, 0, st>>>(kp, f.sig, last, f.lam_site, f.mu_site, f.inh_tau0, eeff, f.inh_part);
 }
 
 void launch_fill_f32(const double* in, float* out, long long n, cudaStream_t st) {

@@ -152,8 +152,8 @@ struct Fields {
   double* lam_site = nullptr;  // [N] Lambda
   double* mu_site = nullptr;   // [N] Mu
   double* inh_tau0 = nullptr;  // [nc][N] C(x):eps*  of the polarisation fixed point
-  double* inh_eeff = nullptr;  // [nc][N] effective eigenstrain of the reference medium
-  double* inh_last = nullptr;  // [nc][N] its previous iterate
+  double* inh_eeff = nullptr;  // [nc][N] effective eigenstrain of the reference medium: the iterates,
+  double* inh_last = nullptr;  // [nc][N] in turns
   double* inh_part = nullptr;  // [blocks] partial sums of the iterate's squared change
 };
 
