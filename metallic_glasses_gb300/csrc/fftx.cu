@@ -641,7 +641,7 @@ __device__ __forceinline__ void green_tile(int tile, double2* __restrict__ spec,
       const int l1 = i & (L - 1), p = i >> lgL, q1 = q0 + l1;
       if (q1 >= inner) continue;
       int k0, k1, k2;
-      if (NC == 6) {
+      if (NC == 6 && ga.is3d) {
         k0 = p;
         k1 = q1 / ga.nh;
         k2 = q1 - k1 * ga.nh;
@@ -1042,6 +1042,8 @@ void fftx_spectrum(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_
     launch_c2c<false>(p, a, x1, st);
     launch_green<6>(p, p.n0, p.n1 * p.nh, a, x0, p.tx_0, ga, st);
     launch_c2c<true>(p, a, x1, st);
+  } else if (p.nc == 6) {  // six components on a flat grid: no axis 0, Green's pass along axis 1
+    launch_green<6>(p, p.n1, p.nh, a, x1, p.tx_1, ga, st);
   } else {
     launch_green<3>(p, p.n1, p.nh, a, x1, p.tx_1, ga, st);
   }

@@ -684,3 +684,58 @@ def test_split_2d_rates_match_fp64_rates(engine_lib, shape, odd):
 def test_split_3d_rates_match_fp64_rates(engine_lib, shape):
     """The 3D rates in two parts and in one (up to 228 and more blocks)."""
     test_fixed_point_rates_match_fp64_rates(engine_lib, shape, None)
+
+
+FLAT = [(1, 8, 12), (1, 1, 2), (1, 16, 16), (1, 9, 6), (1, 64, 48)]
+
+
+@pytest.mark.parametrize("shape", FLAT)
+def test_flat_3d_grid_solves(engine_lib, oracle_lib, shape):
+    """Six components on a grid without an axis 0: the context's solve and the
+    stand-alone one against the oracle's (the bar of
+    test_fft_green_solve_matches_oracle)."""
+    p = configs.shear64(seed=2)
+    p.n[0], p.n[1], p.n[2] = shape
+    eng, ora = api.Engine(p), oracle_lib.Model(p)
+    rng = np.random.default_rng(11)
+    eps = rng.standard_normal((6, eng.N)) * 0.02
+    for c in range(6):
+        eng.set_field(api.FIELD_EPS0, c, eps[c])
+        ora.set_field(api.FIELD_EPS0, c, eps[c])
+    eng.solve()
+    ora.solve()
+    want = np.stack([ora.field(api.FIELD_SIGMA, c) for c in range(6)])
+    assert rel_err(np.stack([eng.field(api.FIELD_SIGMA, c) for c in range(6)]), want) < 1e-11
+    got = _noalloc(engine_lib, 3, shape, p.lambda_, p.mu, eps, ora.scalars()["eps_avg"])
+    assert rel_err(got, want) < 1e-11
+    eng.close()
+
+
+@pytest.mark.parametrize("shape", FLAT[:1] + FLAT[2:3])
+@pytest.mark.parametrize("form", ["incremental", "mixed"])
+def test_flat_3d_grid_updates(engine_lib, oracle_lib, shape, form):
+    """The updates and the FP64 re-solve on such a grid: the field after 12
+    events against the oracle's solve of the same eigenstrain and mean strain;
+    bars of the octant test (FP64) and of the mixed form (1e-5)."""
+    p = configs.shear64(seed=2, eng_end=1e9)
+    p.n[0], p.n[1], p.n[2] = shape
+    p.solver = api.SOLVER_KERNEL
+    if form == "mixed":
+        p.precision, p.resolve_period, p.resolve_fp64 = api.PREC_MIXED, 5, 1
+    eng, ora = api.Engine(p), oracle_lib.Model(p)
+    eng.run(max_events=12)
+    sc = eng.scalars()
+    for c in range(6):
+        ora.set_field(api.FIELD_EPS0, c, eng.field(api.FIELD_EPS0, c))
+    if form == "mixed":
+        assert sc["n_resolves"] == 2 and sc["stress_err_max_worst"] < 1e-5
+    ora.solve()
+    which, comps, bar = (api.FIELD_SDEV, 5, 1e-5) if form == "mixed" else (api.FIELD_SIGMA, 6, 1e-13)
+    want = np.stack([ora.field(api.FIELD_SIGMA, c) for c in range(6)])
+    if form == "mixed":
+        r2, r6 = 0.5 ** 0.5, 6 ** -0.5
+        want = np.stack([(want[0] - want[1]) * r2, (2 * want[2] - want[0] - want[1]) * r6, *(want[3:] / r2)])
+    for c in range(comps):
+        d = eng.field(which, c) - want[c]  # up to the uniform stress of the loading
+        assert np.abs(d - d.mean()).max() < bar * np.abs(want).max()
+    eng.close()
