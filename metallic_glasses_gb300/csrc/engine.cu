@@ -247,7 +247,10 @@ int init_global3d(stz_ctx* c, MT* rng) {
     for (long long s = 0; s < N; s++) dF[s] = mt_gaussian(rng, 1.0);
     int st;
     if ((st = upload(c->f.dF, dF.data(), sizeof(double) * N, c->stream))) return st;
-    fft_filter_gaussian(*plan_of(c), c->f.dF, p.q0_corr_len, c->f.spec, c->stream);
+    if ((st = fft_filter_gaussian(*plan_of(c), c->f.dF, p.q0_corr_len, c->f.spec, c->stream))) {
+      set_error("filter of the correlated barriers failed on %dx%dx%d", p.n[0], p.n[1], p.n[2]);
+      return st;
+    }
     CK(cudaMemcpyAsync(dF.data(), c->f.dF, sizeof(double) * N, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     double ss = 0;

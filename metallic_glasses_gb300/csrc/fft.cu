@@ -1367,22 +1367,26 @@ int fft_filter_gaussian(const FFTPlan& p, double* field, double corr_len, void* 
   k_c2c_axis<double, -1><<<gy, TH, p.smem_y, st>>>(sp, p.n1, p.nh, inner1, (long long)p.n1 * p.nh, ntile1, p.Nk,
                                                     p.L_y, p.s1, p.tw_1, nullptr);
   const long long inner0 = (long long)p.n1 * p.nh;
-  const int ntile0 = (int)((inner0 + p.L_y - 1) / p.L_y);
-  size_t s0 = 2 * (size_t)p.L_y * (p.n0 + 1) * sizeof(V);
+  // lines per block along axis 0: those of axis 1, fewer where n0 is the longer
+  // (its lines need the shared memory; 32 of 256 values do not fit)
+  int L0 = p.L_y;
+  while (L0 > 1 && 2 * (size_t)L0 * (p.n0 + 1) * sizeof(V) > 200 * 1024) L0 /= 2;
+  const int ntile0 = (int)((inner0 + L0 - 1) / L0);
+  const size_t s0 = 2 * (size_t)L0 * (p.n0 + 1) * sizeof(V);
   if (p.n0 > 1) {
-    k_c2c_axis<double, -1><<<ntile0, TH, s0, st>>>(sp, p.n0, inner0, inner0, 0, ntile0, p.Nk, p.L_y, p.s0, p.tw_0,
+    k_c2c_axis<double, -1><<<ntile0, TH, s0, st>>>(sp, p.n0, inner0, inner0, 0, ntile0, p.Nk, L0, p.s0, p.tw_0,
                                                    nullptr);
   }
   k_gauss_filter<double><<<(unsigned)((p.Nk + 255) / 256), 256, 0, st>>>(sp, p.n0, p.n1, p.n2, p.nh, corr_len, p.Nk);
   if (p.n0 > 1)
-    k_c2c_axis<double, +1><<<ntile0, TH, s0, st>>>(sp, p.n0, inner0, inner0, 0, ntile0, p.Nk, p.L_y, p.s0, p.tw_0,
+    k_c2c_axis<double, +1><<<ntile0, TH, s0, st>>>(sp, p.n0, inner0, inner0, 0, ntile0, p.Nk, L0, p.s0, p.tw_0,
                                                    nullptr);
   k_c2c_axis<double, +1><<<gy, TH, p.smem_y, st>>>(sp, p.n1, p.nh, inner1, (long long)p.n1 * p.nh, ntile1, p.Nk,
                                                     p.L_y, p.s1, p.tw_1, nullptr);
   k_c2r_x<double, kOutSig64><<<gx.x, TH, p.smem_c2r, st>>>(sp, 1, p.n2, p.h, p.nh, rows, p.N, p.Nk, p.L_x, p.sh,
                                                           p.tw_h, p.tw_p, 1.0, field, nullptr, nullptr, nullptr,
                                                           nullptr, nullptr, nullptr);
-  return STZ_OK;
+  return cudaGetLastError() == cudaSuccess ? STZ_OK : STZ_ERR_CUDA;
 }
 
 }  // namespace stz

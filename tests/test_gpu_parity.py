@@ -739,3 +739,24 @@ def test_flat_3d_grid_updates(engine_lib, oracle_lib, shape, form):
         d = eng.field(which, c) - want[c]  # up to the uniform stress of the loading
         assert np.abs(d - d.mean()).max() < bar * np.abs(want).max()
     eng.close()
+
+
+@pytest.mark.parametrize("precision", [api.PREC_FP64, api.PREC_MIXED])
+@pytest.mark.parametrize("shape", [(256, 16, 32), (256, 32, 64), (512, 16, 16), (1024, 2, 8)])
+def test_correlated_barriers_on_long_axis_0(engine_lib, shape, precision):
+    """The barrier filter where axis 0 is longer than axis 1, whatever tile the
+    tuner took for axis 1: neighbours a site apart along axis 0 have the
+    Gaussian covariance's correlation, exp(-1/32) = 0.969 for a length of 4
+    sites (0.01 over a few hundred independent patches; without a filter along
+    the axis it is 0 to 0.06), and the context runs."""
+    p = configs.shear64(seed=3, eng_end=1e9)
+    p.n[0], p.n[1], p.n[2] = shape
+    p.df_kind, p.q0_sd, p.q0_corr_len, p.precision = api.DF_CORRELATED, 0.15, 4.0, precision
+    p.solver = api.SOLVER_KERNEL if precision == api.PREC_MIXED else api.SOLVER_FFT
+    eng = api.Engine(p)
+    q = eng.field(api.FIELD_DF).reshape(shape)
+    q = q - q.mean()
+    assert (q * np.roll(q, 1, 0)).mean() / (q * q).mean() > 0.93
+    eng.run(max_events=2)
+    assert eng.scalars()["kstep"] == 2
+    eng.close()
