@@ -1060,8 +1060,9 @@ int solve_t(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* laun
 
 // Tiles (lines per block) of the three kinds of pass and their shared memory,
 // in FP64 (the FP32 and pair transforms use the same tiles) and in fixed point
-// (padded lines); false if a pass would not fit in `limit` bytes.
-static bool plan_set_tiles(FFTPlan* p, int Lx, int Ly, int Lg, size_t limit = 200 * 1024) {
+// (padded lines); false if a pass would not fit in `limit` bytes, with
+// `staging` the C2R pass beside the real rows of all components.
+static bool plan_set_tiles(FFTPlan* p, int Lx, int Ly, int Lg, size_t limit = 200 * 1024, bool staging = true) {
   const size_t cz = sizeof(double2);
   const int ng = p->n0 > 1 ? p->n0 : p->n1;
   const size_t sx = 2 * (size_t)Lx * (p->h + 1) * cz, sc = 2 * (size_t)Lx * (p->h + 2) * cz;
@@ -1069,7 +1070,8 @@ static bool plan_set_tiles(FFTPlan* p, int Lx, int Ly, int Lg, size_t limit = 20
   const size_t rx = 2 * (size_t)Lx * fx_ld(p->h + 1) * cz + sizeof(int) * Lx, ry = 2 * (size_t)Ly * fx_ld(p->n1) * cz,
                rg = 2 * (size_t)p->nc * Lg * fx_ld(ng) * cz;
   if (Lx < 1 || Ly < 1 || Lg < 1 || (Ly > 1 && Ly * p->n1 > 2048)) return false;
-  if (sc + sizeof(double) * p->nc * Lx * p->n2 > limit || ry > limit || rg > limit || rx > limit) return false;
+  if (sc + (staging ? sizeof(double) * p->nc * Lx * p->n2 : 0) > limit || ry > limit || rg > limit || rx > limit)
+    return false;
   p->L_x = Lx;
   p->L_y = Ly;
   p->L_g = Lg;
@@ -1095,7 +1097,9 @@ static bool default_tiles(FFTPlan* p) {
   while (Lx > 1 && 2 * (size_t)Lx * fx_ld(p->h + 1) * cz + sizeof(double) * p->nc * Lx * p->n2 > 200 * 1024) Lx /= 2;
   while (Ly > 1 && (2 * (size_t)Ly * fx_ld(p->n1) * cz > 100 * 1024 || Ly * p->n1 > 2048)) Ly /= 2;
   while (Lg > 1 && 2 * (size_t)p->nc * Lg * fx_ld(ng) * cz > 200 * 1024) Lg /= 2;
-  return plan_set_tiles(p, Lx, Ly, Lg, 224 * 1024);
+  // the longest lines (8192 values) leave no room for the staging, which no
+  // FP64 output has
+  return plan_set_tiles(p, Lx, Ly, Lg, 224 * 1024, false);
 }
 
 int fft_plan_create(FFTPlan* p, int n0, int n1, int n2, int nc) {

@@ -760,3 +760,32 @@ def test_correlated_barriers_on_long_axis_0(engine_lib, shape, precision):
     eng.run(max_events=2)
     assert eng.scalars()["kstep"] == 2
     eng.close()
+
+
+@pytest.mark.parametrize("shape", [(1, 2, 5832), (1, 16, 8192), (2, 2, 3888), (2, 2, 4096), (2, 4, 8192)])
+def test_contexts_of_long_lines(engine_lib, oracle_lib, shape):
+    """Lines up to the longest accepted, 8192 values, where the passes hold one
+    line a block: the solve against the oracle's (the bar of
+    test_fft_green_solve_matches_oracle), and steps. In 2D without the wave
+    number that is Nyquist's on both axes: the reference's s - round(s) takes
+    either sign there, as (n/2)(1/n) rounds to 1/2 or, for 5832, to less."""
+    p = configs.ref2d(shape[1], shape[2]) if shape[0] == 1 else configs.shear64(seed=2)
+    p.n[0], p.n[1], p.n[2] = shape
+    eng, ora = api.Engine(p), oracle_lib.Model(p)
+    rng = np.random.default_rng(11)
+    for c in range(eng.nc):
+        v = rng.standard_normal(eng.N) * 0.02
+        eng.set_field(api.FIELD_EPS0, c, v)
+        ora.set_field(api.FIELD_EPS0, c, v)
+    eng.solve()
+    ora.solve()
+    alt = 1.0 - 2.0 * (np.indices(shape).sum(0).ravel() % 2)
+    for c in range(eng.nc):
+        want = ora.field(api.FIELD_SIGMA, c)
+        d = eng.field(api.FIELD_SIGMA, c) - want
+        if shape[0] == 1:
+            d -= alt * (alt * d).mean()
+        assert np.abs(d).max() < 1e-11 * np.abs(want).max()
+    eng.run(max_steps=2)
+    assert eng.scalars()["step"] == 2
+    eng.close()
