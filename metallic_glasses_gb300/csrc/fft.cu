@@ -1286,10 +1286,13 @@ int fft_autotune(FFTPlan* p, cudaStream_t st, int* chosen, int pair) {
 }
 
 // Plan whose twiddle tables live in caller-provided device storage (for the
-// allocation-free entry point). FP64 transforms only; no device allocation.
-size_t fft_twiddle_count(int n0, int n1, int n2) { return 2 * ((size_t)(n2 / 2) + n1 + n0 + (n2 / 2 + 1)); }
+// allocation-free entry point). FP64 solves only; no device allocation. The
+// tables are those of the passes that fft_solve takes for the medium: FP64 or
+// fixed point, 16 bytes a value each.
+size_t fft_twiddle_count(int n0, int n1, int n2) { return (size_t)(n2 / 2) + n1 + n0 + (n2 / 2 + 1); }
 
-int fft_plan_init_in(FFTPlan* p, int n0, int n1, int n2, int nc, double2* storage, size_t cap, cudaStream_t st) {
+int fft_plan_init_in(FFTPlan* p, int n0, int n1, int n2, int nc, double lambda, double mu, double2* storage, size_t cap,
+                     cudaStream_t st) {
   std::memset((void*)p, 0, sizeof(*p));
   if (n2 < 2 || n2 % 2 != 0 || n1 < 1 || n0 < 1) return STZ_ERR_INVALID;
   p->n0 = n0; p->n1 = n1; p->n2 = n2; p->nc = nc;
@@ -1303,23 +1306,25 @@ int fft_plan_init_in(FFTPlan* p, int n0, int n1, int n2, int nc, double2* storag
   if (p->sh.nst < 0 || p->s1.nst < 0 || p->s0.nst < 0) return STZ_ERR_INVALID;
   if (p->h > 4096 || n1 > 1024 || n0 > 1024) return STZ_ERR_INVALID;
   if (fft_twiddle_count(n0, n1, n2) > cap) return STZ_ERR_INVALID;
+  const bool fx = fftx_fits(lambda, mu);
   const int lens[4] = {p->h, n1, n0, n2};
   const int counts[4] = {p->h, n1, n0, p->nh};
   double2** dst[4] = {&p->tw_h, &p->tw_1, &p->tw_0, &p->tw_p};
+  FxTwiddle** dfx[4] = {&p->tx_h, &p->tx_1, &p->tx_0, &p->tx_p};
+  static_assert(sizeof(FxTwiddle) == sizeof(double2), "one table size");
   std::vector<double2> host(fft_twiddle_count(n0, n1, n2));
   size_t off = 0;
   for (int t = 0; t < 4; t++) {
-    for (int k = 0; k < counts[t]; k++) {
-      const double ang = -2.0 * M_PI * (double)k / (double)lens[t];
-      host[off + k] = make_double2(std::cos(ang), std::sin(ang));
+    if (fx) {
+      fx_twiddles(lens[t], counts[t], reinterpret_cast<FxTwiddle*>(host.data() + off));
+      *dfx[t] = reinterpret_cast<FxTwiddle*>(storage + off);
+    } else {
+      for (int k = 0; k < counts[t]; k++) {
+        const double ang = -2.0 * M_PI * (double)k / (double)lens[t];
+        host[off + k] = make_double2(std::cos(ang), std::sin(ang));
+      }
+      *dst[t] = storage + off;
     }
-    *dst[t] = storage + off;
-    off += counts[t];
-  }
-  FxTwiddle** dfx[4] = {&p->tx_h, &p->tx_1, &p->tx_0, &p->tx_p};
-  for (int t = 0; t < 4; t++) {
-    fx_twiddles(lens[t], counts[t], reinterpret_cast<FxTwiddle*>(host.data() + off));
-    *dfx[t] = reinterpret_cast<FxTwiddle*>(storage + off);
     off += counts[t];
   }
   if (cudaMemcpyAsync(storage, host.data(), sizeof(double2) * host.size(), cudaMemcpyHostToDevice, st) !=

@@ -49,10 +49,11 @@ int fft_plan_create(FFTPlan* p, int n0, int n1, int n2, int nc);
 // schedule's within 1e-10. chosen (optional, 4 ints): the tiles L_x, L_y, L_g
 // and the number of candidates rejected.
 int fft_autotune(FFTPlan* p, cudaStream_t st, int* chosen, int pair);
-// A plan whose twiddle tables are written into caller-provided device storage
-// of at least fft_twiddle_count() elements (FP64 transforms only).
+// A plan for FP64 solves of one medium whose twiddle tables are written into
+// caller-provided device storage of at least fft_twiddle_count() elements.
 size_t fft_twiddle_count(int n0, int n1, int n2);
-int fft_plan_init_in(FFTPlan* p, int n0, int n1, int n2, int nc, double2* storage, size_t cap, cudaStream_t st);
+int fft_plan_init_in(FFTPlan* p, int n0, int n1, int n2, int nc, double lambda, double mu, double2* storage, size_t cap,
+                     cudaStream_t st);
 // number of blocks of the C2R pass (the length of one component's msum row)
 int fft_c2r_blocks(const FFTPlan& p);
 void fft_plan_destroy(FFTPlan* p);

@@ -71,7 +71,12 @@ extern "C" int stz_solve_noalloc(int32_t dim, int32_t n0, int32_t n1, int32_t n2
   }
   const size_t spec = (size_t)nc * n0 * n1 * (n2 / 2 + 1);
   const size_t tw = stz::fft_twiddle_count(n0, n1, n2);
-  if (spec > kNoAllocSpec || tw + 8 > kNoAllocExtra) {
+  if (tw + 8 > kNoAllocExtra) {
+    stz::set_error("stz_solve_noalloc: grid %dx%dx%d needs %zu twiddles, the fixed scratch holds %zu", n0, n1, n2, tw,
+                   kNoAllocExtra - 8);
+    return STZ_ERR_INVALID;
+  }
+  if (spec > kNoAllocSpec) {
     stz::set_error("stz_solve_noalloc: grid %dx%dx%d needs %zu spectrum values, the fixed scratch holds %zu "
                    "(6 components of 64^3)", n0, n1, n2, spec, kNoAllocSpec);
     return STZ_ERR_INVALID;
@@ -82,7 +87,7 @@ extern "C" int stz_solve_noalloc(int32_t dim, int32_t n0, int32_t n1, int32_t n2
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   double2* extra = base + kNoAllocSpec;
   stz::FFTPlan plan;
-  if ((st = stz::fft_plan_init_in(&plan, n0, n1, n2, nc, extra, kNoAllocExtra - 8, s))) {
+  if ((st = stz::fft_plan_init_in(&plan, n0, n1, n2, nc, lambda, mu, extra, kNoAllocExtra - 8, s))) {
     if (st == STZ_ERR_INVALID)
       stz::set_error("stz_solve_noalloc: grid %dx%dx%d not supported by the FFT", n0, n1, n2);
     else

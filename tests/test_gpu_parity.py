@@ -789,3 +789,23 @@ def test_contexts_of_long_lines(engine_lib, oracle_lib, shape):
     eng.run(max_steps=2)
     assert eng.scalars()["step"] == 2
     eng.close()
+
+
+@pytest.mark.parametrize("shape", [(1, 2, 4096), (1, 32, 6144), (2, 2, 4096), (2, 2, 6144)])
+@pytest.mark.parametrize("lam", [80.0, 1e6])
+def test_noalloc_solves_of_long_lines(engine_lib, oracle_lib, shape, lam):
+    """Lines whose tables fill the fixed scratch, in fixed point and (lambda of
+    1e6) in FP64, against the oracle (the bars of test_solve_for_extreme_media)."""
+    dim = 2 if shape[0] == 1 else 3
+    p = configs.ref2d(shape[1], shape[2]) if dim == 2 else configs.shear64(seed=2)
+    p.n[0], p.n[1], p.n[2] = shape
+    p.lambda_, p.mu = lam, 35.0
+    ora = oracle_lib.Model(p)
+    nc = 3 * (dim - 1)
+    eps = np.random.default_rng(11).standard_normal((nc, int(np.prod(shape)))) * 0.02
+    for c in range(nc):
+        ora.set_field(api.FIELD_EPS0, c, eps[c])
+    ora.solve()
+    want = np.stack([ora.field(api.FIELD_SIGMA, c) for c in range(nc)])
+    got = _noalloc(engine_lib, dim, shape, lam, 35.0, eps, ora.scalars()["eps_avg"][:nc])
+    assert rel_err(got, want) < 1e-11 * max(1.0, lam / 35.0)
