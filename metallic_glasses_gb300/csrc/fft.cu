@@ -1068,7 +1068,7 @@ static bool plan_set_tiles(FFTPlan* p, int Lx, int Ly, int Lg, size_t limit = 20
   const size_t sx = 2 * (size_t)Lx * (p->h + 1) * cz, sc = 2 * (size_t)Lx * (p->h + 2) * cz;
   const size_t sy = 2 * (size_t)Ly * (p->n1 + 1) * cz, sg = 2 * (size_t)p->nc * Lg * (ng + 1) * cz;
   const size_t rx = 2 * (size_t)Lx * fx_ld(p->h + 1) * cz + sizeof(int) * Lx, ry = 2 * (size_t)Ly * fx_ld(p->n1) * cz,
-               rg = 2 * (size_t)p->nc * Lg * fx_ld(ng) * cz;
+               rg = 2 * (size_t)p->nc * Lg * fx_ld(ng) * cz + (size_t)ng * Lg;
   if (Lx < 1 || Ly < 1 || Lg < 1 || (Ly > 1 && Ly * p->n1 > 2048)) return false;
   if (sc + (staging ? sizeof(double) * p->nc * Lx * p->n2 : 0) > limit || ry > limit || rg > limit || rx > limit)
     return false;
@@ -1096,7 +1096,7 @@ static bool default_tiles(FFTPlan* p) {
   int Lx = std::max(1, 1024 / p->h), Ly = 8, Lg = 8;
   while (Lx > 1 && 2 * (size_t)Lx * fx_ld(p->h + 1) * cz + sizeof(double) * p->nc * Lx * p->n2 > 200 * 1024) Lx /= 2;
   while (Ly > 1 && (2 * (size_t)Ly * fx_ld(p->n1) * cz > 100 * 1024 || Ly * p->n1 > 2048)) Ly /= 2;
-  while (Lg > 1 && 2 * (size_t)p->nc * Lg * fx_ld(ng) * cz > 200 * 1024) Lg /= 2;
+  while (Lg > 1 && 2 * (size_t)p->nc * Lg * fx_ld(ng) * cz + (size_t)ng * Lg > 200 * 1024) Lg /= 2;
   // the longest lines (8192 values) leave no room for the staging, which no
   // FP64 output has
   return plan_set_tiles(p, Lx, Ly, Lg, 224 * 1024, false);

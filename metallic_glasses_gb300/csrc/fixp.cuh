@@ -245,7 +245,7 @@ void fx_twiddles(int n, int count, FxTwiddle* out);
 // Constants of the fixed-point Green's pass (fftx.cu).
 struct GreenFx {
   int is3d, n0, n1, n2, nh;  // is3d: the grid has an axis 0 (n0 > 1), whatever its components
-  int kb;            // headroom of the operator: inputs enter shifted right by kb bits
+  int kb;            // headroom of the operator: the largest input is below 2^(61 - kb)
   int lams;          // lam and c1 carry 2^(64 - lams)
   Fx lam;            // lambda / (2 mu)
   Fx c1;             // (1 - alpha) lambda / mu, alpha = (lambda + mu) / (lambda + 2 mu)
