@@ -9,11 +9,14 @@
 //
 // Scale. Every partial sum of a transform of a line is bounded by the line's
 // sum of |re| + |im|. Each line takes that sum (in FP32, rounded up) and the
-// scale that puts it just below the integer range, so no stage can overflow and
-// no stage needs a scale of its own. A line of n values of ordinary spread keeps
-// its values 62 - log2(1.1 n) bits above the integers' unit (55 bits at n = 64,
-// 52 at n = 512), against the 53 bits of every FP64 operation; sparse lines keep
-// more. Roundings are to nearest. A line with an infinity or a NaN becomes NaN.
+// scale that puts it below 2^61 (R2C, whose last step doubles it), 2^62 (column
+// passes) or 2^60 (C2R: 2^62 for the doubled pairs of its half spectrum), so no
+// sum reaches 2^63 and no stage needs a scale of its own. A dense line of n
+// values keeps them some 59.5 - log2(n) bits above the integers' unit (53 at
+// n = 64, 50 at 512), but each value is rounded at that unit three or four times
+// in a pass where an FP64 transform rounds it relative to itself at every
+// operation; sparse lines keep more. Roundings are to nearest. Green's operator
+// works at a scale per wave number. A line with an infinity or a NaN becomes NaN.
 // The mean strain's uniform stress C:<eps> is added to the result in FP64
 // instead of entering the k = 0 term, which it would dominate.
 //
@@ -353,7 +356,7 @@ __device__ __forceinline__ void r2c_tile(int tile, const double* __restrict__ in
         g[i].s += __shfl_xor_sync(FULL, g[i].s, off);
         g[i].hi = max(g[i].hi, __shfl_xor_sync(FULL, g[i].hi, off));
       }
-      const int sc = line_scale(g[i].s, g[i].hi, 2 * h, 60);
+      const int sc = line_scale(g[i].s, g[i].hi, 2 * h, 61);
       if (l < L) {
         if (j0 == 0) lsc[l] = sc;
         if (U > 0) {
@@ -431,7 +434,7 @@ __device__ __forceinline__ void c2c_tile(int tile, double2* __restrict__ data, i
     g.add(v[u].x);
     g.add(v[u].y);
   }
-  column_scales<1>(&g.s, g.hi, L, 2 * n, 61, lsc);
+  column_scales<1>(&g.s, g.hi, L, 2 * n, 62, lsc);
   const int s = lsc[l];
   cx* at = a + l * ld;
 #pragma unroll
@@ -577,7 +580,7 @@ __device__ __forceinline__ void green_tile(int tile, double2* __restrict__ spec,
       cs[c] = g.s;
       hi = max(hi, g.hi);
     }
-    column_scales<NC>(cs, hi, L, 2 * n, 61, lsc);  // the NC lines of a column share a scale
+    column_scales<NC>(cs, hi, L, 2 * n, 62, lsc);  // the NC lines of a column share a scale
     const int s = lsc[l];
 #pragma unroll
     for (int c = 0; c < NC; c++)
@@ -597,7 +600,7 @@ __device__ __forceinline__ void green_tile(int tile, double2* __restrict__ spec,
       cs[c] = g.s;
       hi = max(hi, g.hi);
     }
-    column_scales<NC>(cs, hi, L, 2 * n, 61, lsc);
+    column_scales<NC>(cs, hi, L, 2 * n, 62, lsc);
     const int s = lsc[l];
 #pragma unroll 1
     for (int c = 0; c < NC; c++)
@@ -710,9 +713,9 @@ __device__ __forceinline__ void green_tile(int tile, double2* __restrict__ spec,
       }
     }
   }
-  // sums in units of 2^32: a top of 29 puts them below 2^61. A column of zeros
+  // sums in units of 2^32: a top of 30 puts them below 2^62. A column of zeros
   // has the largest shift.
-  column_scales<NC>(ns, 0x3ff00000u, L, 2 * n, 29, lsh);
+  column_scales<NC>(ns, 0x3ff00000u, L, 2 * n, 30, lsh);
   if (threadIdx.x < L) lsh[threadIdx.x] = min(lsh[threadIdx.x], 62);
   __syncthreads();
   {
@@ -820,7 +823,7 @@ __device__ __forceinline__ void c2r_tile(int tile, int tiles, const double2* __r
         g[i].hi = max(g[i].hi, __shfl_xor_sync(FULL, g[i].hi, off));
       }
       // four times the half spectrum's sum bounds every partial sum of Z
-      const int sc = line_scale(g[i].s, g[i].hi, 2 * nh, 59);
+      const int sc = line_scale(g[i].s, g[i].hi, 2 * nh, 60);
       if (l < L) {
         if (j0 == 0) {
           lsc[l] = sc;

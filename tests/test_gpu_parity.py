@@ -854,3 +854,43 @@ def test_solve_of_nearly_uniform_eigenstrain(engine_lib, shape):
     want = _solve_extended(shape, 80.0, 35.0, eps)
     d = _noalloc(engine_lib, 2 if nc == 3 else 3, shape, 80.0, 35.0, eps, [0.0] * nc) - want
     assert np.sqrt((d ** 2).sum() / (want ** 2).sum()) < 2.5e-16
+
+
+@pytest.mark.parametrize("shape", [(8, 12, 16), (1, 16, 64), (1, 9, 8)])
+def test_solve_at_the_scales_limits(engine_lib, shape):
+    """Fields whose partial sums reach a line's sum of magnitudes, the bound its
+    integer scale is taken from: uniform, alternating, one wave in equal sine and
+    cosine parts along every axis, one site; at 32 amplitudes of an octave, so
+    that the sums lie everywhere up to the scale's limit. 1e-13 of the largest
+    stress: an overflow is of its own size."""
+    nc = 3 if shape[0] == 1 else 6
+    ph = [2 * np.pi * i / n for i, n in zip(np.indices(shape), shape)]
+    alt = (-1.0) ** np.indices(shape).sum(0)
+    delta = np.zeros(shape)
+    delta[0, 1 % shape[1], 2] = 1.0
+    fields = [np.ones(shape), alt, delta] + [np.cos(k * x + np.pi / 4) for x in ph for k in (1, 2)]
+    for sign in (1.0, -1.0):
+        for v in fields:
+            eps = np.stack([v.ravel() * (sign if c % 2 else 1.0) for c in range(nc)])
+            want = _solve_extended(shape, 80.0, 35.0, eps).astype(float)
+            size = np.abs(want).max()
+            for j in range(32):
+                a = 2.0 ** (j / 32)
+                got = _noalloc(engine_lib, 2 if nc == 3 else 3, shape, 80.0, 35.0, eps * a, [0.0] * nc)
+                assert np.abs(got - a * want).max() < 1e-13 * a * max(size, 1.0)
+
+
+def _dense_error(lib, shape):
+    nc = 3 if shape[0] == 1 else 6
+    eps = 0.05 * np.random.default_rng(5).standard_normal((nc, int(np.prod(shape))))
+    want = _solve_extended(shape, 80.0, 35.0, eps)
+    d = _noalloc(lib, 2 if nc == 3 else 3, shape, 80.0, 35.0, eps, [0.0] * nc) - want
+    return np.sqrt((d ** 2).sum() / (want ** 2).sum())
+
+
+@pytest.mark.parametrize("shape", [(2, 2, 1024), (4, 4, 1024), (1024, 2, 16)])
+def test_dense_lines_of_a_thousand_values(engine_lib, shape):
+    """Random eigenstrain on long lines, whose values lie lowest above the
+    integers' unit: within 1e-15 (relative L2) of the solve in extended
+    precision, where FP64 passes come to 0.8e-15 to 0.9e-15."""
+    assert _dense_error(engine_lib, shape) < 1e-15
