@@ -1306,7 +1306,7 @@ int fft_plan_init_in(FFTPlan* p, int n0, int n1, int n2, int nc, double lambda, 
   if (p->sh.nst < 0 || p->s1.nst < 0 || p->s0.nst < 0) return STZ_ERR_INVALID;
   if (p->h > 4096 || n1 > 1024 || n0 > 1024) return STZ_ERR_INVALID;
   if (fft_twiddle_count(n0, n1, n2) > cap) return STZ_ERR_INVALID;
-  const bool fx = fftx_fits(lambda, mu);
+  const bool fx = fftx_fits(n2, lambda, mu);
   const int lens[4] = {p->h, n1, n0, n2};
   const int counts[4] = {p->h, n1, n0, p->nh};
   double2** dst[4] = {&p->tw_h, &p->tw_1, &p->tw_0, &p->tw_p};
@@ -1350,8 +1350,10 @@ void fft_plan_destroy(FFTPlan* p) {
 int fft_solve(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* launches) {
   if (a.pair) return solve_t<dfl>(p, a, st, launches);
   // FP64 solves run in fixed point (fftx.cu), but for the displacement (a
-  // print-time solve) and media whose moduli are out of its range
-  if (!a.fp32 && !a.disp && (a.out == kOutSig64 || (a.out == kOutDev32 && p.nc == 6)) && fftx_fits(a.lambda, a.mu)) {
+  // print-time solve), the longest lines and media whose moduli are out of its
+  // range
+  if (!a.fp32 && !a.disp && (a.out == kOutSig64 || (a.out == kOutDev32 && p.nc == 6)) &&
+      fftx_fits(p.n2, a.lambda, a.mu)) {
     fftx_spectrum(p, a, st, launches);
     if (a.out == kOutSig64) fftx_c2r(p, a, st, launches);
     else c2r_dev<double>(p, a, fftx_factor(p, a.mu), a.ebar, st, launches);

@@ -983,8 +983,8 @@ void launch_c2c(const FFTPlan& p, const SolveArgs& a, const FxSched& x, cudaStre
 
 }  // namespace
 
-bool fftx_fits(double lambda, double mu) {
-  if (!(mu > 0) || !std::isfinite(lambda) || !std::isfinite(mu)) return false;
+bool fftx_fits(int n2, double lambda, double mu) {
+  if (n2 > kFxLongest || !(mu > 0) || !std::isfinite(lambda) || !std::isfinite(mu)) return false;
   const double l = std::fabs(lambda) / mu, al = (lambda + mu) / (lambda + 2 * mu);
   return l <= 256 && std::fabs(al) <= 1.5;
 }

@@ -25,8 +25,15 @@ FxSched fx_sched(const Sched& s);
 // Elements of a line of n in shared memory (padded against bank conflicts).
 __host__ __device__ constexpr int fx_ld(int n) { return (n + (n >> 3)) | 1; }
 
-// True when the medium's constants fit the fixed-point Green's pass.
-bool fftx_fits(double lambda, double mu);
+// The longest lines along axis 2 that the fixed-point passes take (the other axes
+// end at 1024). A dense line's values lie the lower above the integers' unit the
+// longer it is, while an FP64 transform's error hardly grows: random eigenstrain
+// is off by 0.60e-15 of the stress at 16x1296 (FP64 passes 1.08e-15), 0.93e-15 at
+// 2x2x1728 (0.83e-15), 1.3e-15 at 2x2x3072 (0.84e-15), 2.5e-15 at 16x6144 (1.09e-15).
+constexpr int kFxLongest = 1296;
+// True when an FP64 solve of lines of n2 runs in fixed point: the lines are short
+// enough and the medium's constants fit Green's pass.
+bool fftx_fits(int n2, double lambda, double mu);
 // The passes up to the spectrum before the last one (along axis 2), which is
 // the stress's divided by 2 mu; fftx_factor is what a C2R pass multiplies its
 // sums by (2 mu / N).

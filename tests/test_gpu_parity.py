@@ -894,3 +894,31 @@ def test_dense_lines_of_a_thousand_values(engine_lib, shape):
     integers' unit: within 1e-15 (relative L2) of the solve in extended
     precision, where FP64 passes come to 0.8e-15 to 0.9e-15."""
     assert _dense_error(engine_lib, shape) < 1e-15
+
+
+@pytest.mark.parametrize("shape", [(2, 2, 4096), (4, 2, 1728), (1, 16, 6144), (1, 16, 1296)])
+def test_dense_lines_of_thousands_of_values(engine_lib, shape):
+    """Lines on both sides of the longest that the fixed-point passes take: as
+    near to extended precision as FP64 passes, 0.8e-15 to 0.9e-15 (six
+    components) and 1.1e-15 (three)."""
+    assert _dense_error(engine_lib, shape) < (1e-15 if shape[0] > 1 else 1.2e-15)
+
+
+@pytest.mark.parametrize("n2", [1458, 2916])
+def test_nyquist_sign_of_the_reference(engine_lib, oracle_lib, n2):
+    """Lengths whose (n/2)(1/n) rounds below 1/2, so that the reference's
+    s - round(s) gives the Nyquist number its positive sign: with Nyquist's on
+    axis 1 the 2D operator depends on it. Against the oracle, which forms it so
+    (the bar of test_fft_green_solve_matches_oracle)."""
+    p = configs.ref2d(16, n2)
+    eng, ora = api.Engine(p), oracle_lib.Model(p)
+    rng = np.random.default_rng(11)
+    for c in range(3):
+        v = rng.standard_normal(eng.N) * 0.02
+        eng.set_field(api.FIELD_EPS0, c, v)
+        ora.set_field(api.FIELD_EPS0, c, v)
+    eng.solve()
+    ora.solve()
+    for c in range(3):
+        assert rel_err(eng.field(api.FIELD_SIGMA, c), ora.field(api.FIELD_SIGMA, c)) < 1e-11
+    eng.close()
