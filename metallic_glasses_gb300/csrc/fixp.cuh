@@ -201,8 +201,8 @@ void fx_exp_table(FxExp* t);
 // 1e-18 J log2(e) / (2 kT) (shears doubled), is held
 // as (y + 1022) 2^53 = 2^5 (hh 2^64 + mid 2^32) / 2^64 of an FxAcc.
 // Scales: with L = ceil(log2(max_m sum_c |M_mc|)) stresses carry 2^(51 + L) and
-// modes 2^(61 - L), so stresses below 2^(8 - L) GPa (32 GPa at 455 K and 1 nm^3)
-// move y by at most 512; with LB = ceil(log2(log2(e)/kT)) barriers carry
+// modes 2^(61 - L), so stresses (the field's, the uniform one and their sum) below
+// 2^(8 - L) GPa (8 GPa at 455 K and 1 nm^3) move y by at most 512; with LB = ceil(log2(log2(e)/kT)) barriers carry
 // 2^(51 + LB), the constant 2^(61 - LB). A site beyond these limits (or not
 // finite) sends its block through the FP64 chain.
 struct RateFx {

@@ -503,7 +503,10 @@ __device__ __forceinline__ bool g3_fx_site(const RateFx& rx, const Fields& f, lo
   bool ok = true;
   int64_t g[6];
 #pragma unroll
-  for (int c = 0; c < 6; c++) g[c] = fx_from_f64<4>(f.sig[c * N + s], rx.sw, &ok) + ufx[c];
+  for (int c = 0; c < 6; c++) {
+    g[c] = fx_from_f64<4>(f.sig[c * N + s], rx.sw, &ok) + ufx[c];
+    ok &= (uint64_t)(g[c] + (1ll << 59)) < (1ull << 60);
+  }
   W[0] = fx_split(g[0] - g[2]);
   W[1] = fx_split(g[1] - g[2]);
   W[2] = fx_split(g[3]);

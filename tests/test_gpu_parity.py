@@ -922,3 +922,44 @@ def test_nyquist_sign_of_the_reference(engine_lib, oracle_lib, n2):
     for c in range(3):
         assert rel_err(eng.field(api.FIELD_SIGMA, c), ora.field(api.FIELD_SIGMA, c)) < 1e-11
     eng.close()
+
+
+def test_fixed_point_rates_under_two_large_stresses(engine_lib):
+    """A field stress and a uniform stress of the same sign, each within the
+    fixed point's limit of 2^(8 - L) GPa and their sum beyond it, against a mode
+    whose rate argument they take below the representable 2^-1022: the FP64
+    chain's total rate and no avalanche. Barriers of 14 eV, Q to some 1e-15 of
+    them, 1e-12 of a rate at kT = 0.039 eV."""
+    p = configs.stress32(seed=58, n=4)
+    p.applied_stress[api.XY] = 0.0
+    kT = p.temperature * 1.380658e-23 / 1.60217733e-19
+    eng = api.Engine(p)
+    Q = np.empty((7, 20))
+    for k in range(7):
+        for c in range(6):
+            eng.set_field(api.FIELD_SIGMA, c, np.full(eng.N, float(c == k - 1)))
+        Q[k] = [eng.field(api.FIELD_Q, m)[0] for m in range(20)]
+    eng.close()
+    G = (Q[0] - Q[1:]).T * np.log2(np.e) / kT  # work of each mode per GPa, in powers of two
+    # the modes' largest sum of coefficients just below a power of two, 2^L
+    size = np.abs(G[:, [0, 1, 3, 4, 5]]).sum(1).max()
+    L = int(np.ceil(np.log2(size)))
+    p.voxel_volume *= 0.999 * 2.0 ** L / size
+    stress = -np.sign(G[18]) * 0.97 * 2.0 ** (8 - L)
+    for c in range(6):
+        p.applied_stress[c] = stress[c]
+    eng = api.Engine(p)
+    eng.set_mean_strain([0.0] * 6)
+    eng.solve()
+    eng.run(max_events=1)  # the uniform stress now makes up for the applied one
+    for c in range(6):
+        eng.set_field(api.FIELD_SIGMA, c, np.full(eng.N, stress[c]))
+    y0 = 524 - 1022 - np.log2(p.voxel_volume * p.trial_frequency)
+    eng.set_field(api.FIELD_DF, 0, np.full(eng.N, -y0 * kT / np.log2(np.e)))
+    Q = np.stack([eng.field(api.FIELD_Q, m) for m in range(20)])
+    assert Q.min() > 0 and Q[18].min() * np.log2(np.e) / kT > 1070
+    R = np.longdouble(p.voxel_volume * p.trial_frequency) * np.exp(-Q.astype(np.longdouble) / np.longdouble(kT)).sum()
+    eng.run(max_steps=1)
+    assert eng.scalars()["astep"] == 0
+    assert abs(eng.events()["total_rate"][-1] / R - 1) < 1e-12
+    eng.close()
