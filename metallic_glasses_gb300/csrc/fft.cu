@@ -36,6 +36,7 @@
 
 #include "fft.cuh"
 #include "fftx.cuh"
+#include "kmc.cuh"
 
 namespace stz {
 namespace {
@@ -1138,14 +1139,16 @@ struct Tuned {
 std::mutex g_tune_mu;
 std::map<std::array<int, 6>, Tuned> g_tuned;
 
+// The better of two times of three solves. They queue behind a kernel that holds
+// the stream while the host launches them, so that the events bracket device
+// time on the smallest grids too (without it those took four times twelve solves
+// a candidate: 153 ms for the first 64^3 context of a process, 44 so).
 float time_solve(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1) {
   float best = 1e30f;
-  // small grids: enough solves that the events bracket device time and not the
-  // host's launches
-  const int n = p.N * p.nc < (1 << 21) ? 12 : 3;
-  for (int rep = 0; rep < (n > 3 ? 4 : 2); rep++) {
+  for (int rep = 0; rep < 2; rep++) {
+    launch_hold(60000, st);
     cudaEventRecord(e0, st);
-    for (int i = 0; i < n; i++) fft_solve(p, a, st, nullptr);
+    for (int i = 0; i < 3; i++) fft_solve(p, a, st, nullptr);
     cudaEventRecord(e1, st);
     cudaEventSynchronize(e1);
     float ms = 0;
@@ -1250,7 +1253,7 @@ int fft_autotune(FFTPlan* p, cudaStream_t st, int* chosen, int pair) {
     q.s0 = v ? make_sched_rev(p->n0) : make_sched_r4(p->n0);
     if (q.sh.nst > 0 && q.s1.nst > 0 && q.s0.nst > 0) consider(q);
   }
-  if (!pair) {  // threads per tile of the fixed-point passes
+  if (!pair && p->n2 <= kFxLongest) {  // threads per tile of the fixed-point passes
     for (int e : {2, 8}) {
       FFTPlan q = best;
       q.e_x = e;
