@@ -1335,8 +1335,8 @@ int fft_plan_init_in(FFTPlan* p, int n0, int n1, int n2, int nc, double lambda, 
     return STZ_ERR_CUDA;
   if (cudaStreamSynchronize(st) != cudaSuccess) return STZ_ERR_CUDA;
   if (!default_tiles(p)) return STZ_ERR_INVALID;
-  set_smem_attrs<double>(p->smem_x, p->smem_y, p->smem_g, p->smem_c2r + sizeof(double) * nc * p->L_x * n2);
-  fftx_init();
+  if (fx) fftx_init(p);
+  else set_smem_attrs<double>(p->smem_x, p->smem_y, p->smem_g, p->smem_c2r + sizeof(double) * nc * p->L_x * n2);
   return STZ_OK;
 }
 

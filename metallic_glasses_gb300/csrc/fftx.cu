@@ -949,36 +949,42 @@ dim3 fx_grid(const SolveArgs& a, int tiles, int comps) {
   return dim3((unsigned)(a.rare && tiles > most ? most : tiles), (unsigned)comps);
 }
 
-template <int NC>
+// The kernels of a pass by the values a thread holds.
+auto r2c_kernel(int U) {
+  return U == 1 ? k_r2c_fx<1> : U == 2 ? k_r2c_fx<2> : U == 4 ? k_r2c_fx<4> : U == 8 ? k_r2c_fx<8> : k_r2c_fx<0>;
+}
+auto c2r_kernel(int U) {
+  return U == 1 ? k_c2r_fx<1> : U == 2 ? k_c2r_fx<2> : U == 4 ? k_c2r_fx<4> : U == 8 ? k_c2r_fx<8> : k_c2r_fx<0>;
+}
+template <bool INV>
+auto c2c_kernel(int U) {
+  return U == 1 || U == 2 ? k_c2c_fx<INV, 2> : U == 4 ? k_c2c_fx<INV, 4> : k_c2c_fx<INV, 8>;
+}
+auto green_kernel(int nc, int U) {
+  if (nc == 6) return U == 1 ? k_green_fx<6, 1> : U == 2 ? k_green_fx<6, 2> : k_green_fx<6, 0>;
+  return U == 1 ? k_green_fx<3, 1> : U == 2 ? k_green_fx<3, 2> : k_green_fx<3, 0>;
+}
+
+// Green's pass over n values and `inner` columns: along axis 0, or along axis 1
+// of a grid without axis 0 (with three components or six).
 void launch_green(const FFTPlan& p, int n, int inner, const SolveArgs& a, const FxSched& x, const FxTwiddle* tw,
                   const GreenFx& ga, cudaStream_t st) {
-  double2* spec = reinterpret_cast<double2*>(a.spec);
-  const int* gate = a.gate;
   const ColLaunch c = col_launch(n, p.L_g, p.e_g);
   const int tiles = (inner + p.L_g - 1) / p.L_g;
   const dim3 grid = fx_grid(a, tiles, 1);
-  const int lg = ilog2(p.L_g);
-  if (c.U == 1)
-    k_green_fx<NC, 1><<<grid, c.threads, p.smem_gr, st>>>(spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, tiles, gate);
-  else if (c.U == 2)
-    k_green_fx<NC, 2><<<grid, c.threads, p.smem_gr, st>>>(spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, tiles, gate);
-  else
-    k_green_fx<NC, 0><<<grid, c.threads, p.smem_gr, st>>>(spec, n, inner, inner, p.Nk, p.L_g, lg, x, tw, ga, tiles, gate);
+  const auto k = green_kernel(p.nc, c.U);
+  k<<<grid, c.threads, p.smem_gr, st>>>(reinterpret_cast<double2*>(a.spec), n, inner, inner, p.Nk, p.L_g, ilog2(p.L_g), x,
+                                        tw, ga, tiles, a.gate);
 }
 
 template <bool INV>
 void launch_c2c(const FFTPlan& p, const SolveArgs& a, const FxSched& x, cudaStream_t st) {
   const ColLaunch c = col_launch(p.n1, p.L_y, p.e_y);
-  const int columns = p.n0 * p.nh, lg = ilog2(p.L_y);
-  const int tiles = (columns + p.L_y - 1) / p.L_y;
+  const int columns = p.n0 * p.nh, tiles = (columns + p.L_y - 1) / p.L_y;
   const dim3 grid = fx_grid(a, tiles, p.nc);
-  auto go = [&](auto* k) {
-    k<<<grid, c.threads, p.smem_yr, st>>>(reinterpret_cast<double2*>(a.spec), p.n1, p.nh, columns, p.Nk, p.L_y, lg, x,
-                                          p.tx_1, tiles, a.gate);
-  };
-  if (c.U <= 2) go(k_c2c_fx<INV, 2>);
-  else if (c.U == 4) go(k_c2c_fx<INV, 4>);
-  else go(k_c2c_fx<INV, 8>);
+  const auto k = c2c_kernel<INV>(c.U);
+  k<<<grid, c.threads, p.smem_yr, st>>>(reinterpret_cast<double2*>(a.spec), p.n1, p.nh, columns, p.Nk, p.L_y,
+                                        ilog2(p.L_y), x, p.tx_1, tiles, a.gate);
 }
 
 }  // namespace
@@ -989,33 +995,37 @@ bool fftx_fits(int n2, double lambda, double mu) {
   return l <= 256 && std::fabs(al) <= 1.5;
 }
 
-void fftx_init() {
+// Every kernel that a schedule of a grid may take (each pass by the values a
+// thread holds), or with `plan` those of its solve: some calls prepare one solve
+// and cannot afford a look at every kernel (two runtime calls each).
+void fftx_init(const FFTPlan* plan) {
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess || optin <= 0)
     optin = 227 * 1024;
-  raise_limit(k_r2c_fx<0>, optin);
-  raise_limit(k_r2c_fx<1>, optin);
-  raise_limit(k_r2c_fx<2>, optin);
-  raise_limit(k_r2c_fx<4>, optin);
-  raise_limit(k_r2c_fx<8>, optin);
-  raise_limit(k_c2r_fx<0>, optin);
-  raise_limit(k_c2r_fx<1>, optin);
-  raise_limit(k_c2r_fx<2>, optin);
-  raise_limit(k_c2r_fx<4>, optin);
-  raise_limit(k_c2r_fx<8>, optin);
-  raise_limit(k_c2c_fx<false, 2>, optin);
-  raise_limit(k_c2c_fx<false, 4>, optin);
-  raise_limit(k_c2c_fx<false, 8>, optin);
-  raise_limit(k_c2c_fx<true, 2>, optin);
-  raise_limit(k_c2c_fx<true, 4>, optin);
-  raise_limit(k_c2c_fx<true, 8>, optin);
-  raise_limit(k_green_fx<3, 0>, optin);
-  raise_limit(k_green_fx<3, 1>, optin);
-  raise_limit(k_green_fx<3, 2>, optin);
-  raise_limit(k_green_fx<6, 0>, optin);
-  raise_limit(k_green_fx<6, 1>, optin);
-  raise_limit(k_green_fx<6, 2>, optin);
+  if (plan) {
+    const FFTPlan& p = *plan;
+    const int ux = row_launch(p.h, p.L_x, p.e_x).U;
+    raise_limit(r2c_kernel(ux), optin);
+    raise_limit(c2r_kernel(ux), optin);
+    raise_limit(green_kernel(p.nc, col_launch(p.n0 > 1 ? p.n0 : p.n1, p.L_g, p.e_g).U), optin);
+    if (p.n0 > 1) {
+      const int uy = col_launch(p.n1, p.L_y, p.e_y).U;
+      raise_limit(c2c_kernel<false>(uy), optin);
+      raise_limit(c2c_kernel<true>(uy), optin);
+    }
+    return;
+  }
+  for (int u : {0, 1, 2, 4, 8}) {
+    raise_limit(r2c_kernel(u), optin);
+    raise_limit(c2r_kernel(u), optin);
+  }
+  for (int u : {2, 4, 8}) {
+    raise_limit(c2c_kernel<false>(u), optin);
+    raise_limit(c2c_kernel<true>(u), optin);
+  }
+  for (int nc : {3, 6})
+    for (int u : {0, 1, 2}) raise_limit(green_kernel(nc, u), optin);
 }
 
 void fftx_spectrum(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* launches) {
@@ -1025,25 +1035,17 @@ void fftx_spectrum(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_
   const int tiles = (int)((rows + p.L_x - 1) / p.L_x);
   const dim3 gx = fx_grid(a, tiles, p.nc);
   const RowLaunch r = row_launch(p.h, p.L_x, p.e_x);
-  auto r2c = [&](auto* k) {
-    k<<<gx, r.threads, p.smem_xr, st>>>(a.eps, spec, p.h, p.nh, rows, p.N, p.Nk, p.L_x, r.lgp, xh, p.tx_h,
-                                        p.tx_p, tiles, a.gate);
-  };
-  if (r.U == 1) r2c(k_r2c_fx<1>);
-  else if (r.U == 2) r2c(k_r2c_fx<2>);
-  else if (r.U == 4) r2c(k_r2c_fx<4>);
-  else if (r.U == 8) r2c(k_r2c_fx<8>);
-  else r2c(k_r2c_fx<0>);
+  const auto k = r2c_kernel(r.U);
+  k<<<gx, r.threads, p.smem_xr, st>>>(a.eps, spec, p.h, p.nh, rows, p.N, p.Nk, p.L_x, r.lgp, xh, p.tx_h, p.tx_p, tiles,
+                                      a.gate);
   GreenFx ga;
   fx_green_constants(p.n0, p.n1, p.n2, a.lambda, a.mu, &ga);
   if (p.n0 > 1) {
     launch_c2c<false>(p, a, x1, st);
-    launch_green<6>(p, p.n0, p.n1 * p.nh, a, x0, p.tx_0, ga, st);
+    launch_green(p, p.n0, p.n1 * p.nh, a, x0, p.tx_0, ga, st);
     launch_c2c<true>(p, a, x1, st);
-  } else if (p.nc == 6) {  // six components on a flat grid: no axis 0, Green's pass along axis 1
-    launch_green<6>(p, p.n1, p.nh, a, x1, p.tx_1, ga, st);
   } else {
-    launch_green<3>(p, p.n1, p.nh, a, x1, p.tx_1, ga, st);
+    launch_green(p, p.n1, p.nh, a, x1, p.tx_1, ga, st);
   }
   if (launches) *launches += p.n0 > 1 ? 4 : 2;
 }
@@ -1055,16 +1057,10 @@ void fftx_c2r(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* la
   const int tiles = (int)((rows + p.L_x - 1) / p.L_x);
   const dim3 gx = fx_grid(a, tiles, p.nc);
   const RowLaunch r = row_launch(p.h, p.L_x, p.e_x);
-  auto go = [&](auto* k) {
-    k<<<gx, r.threads, p.smem_xr, st>>>(reinterpret_cast<const double2*>(a.spec), p.nc, p.h, p.nh, rows, p.N, p.Nk, p.L_x,
-                                        r.lgp, fx_sched(p.sh), p.tx_h, p.tx_p, fftx_factor(p, a.mu), a.ebar, a.lambda,
-                                        a.mu, a.sig64, a.msum, tiles, a.gate);
-  };
-  if (r.U == 1) go(k_c2r_fx<1>);
-  else if (r.U == 2) go(k_c2r_fx<2>);
-  else if (r.U == 4) go(k_c2r_fx<4>);
-  else if (r.U == 8) go(k_c2r_fx<8>);
-  else go(k_c2r_fx<0>);
+  const auto k = c2r_kernel(r.U);
+  k<<<gx, r.threads, p.smem_xr, st>>>(reinterpret_cast<const double2*>(a.spec), p.nc, p.h, p.nh, rows, p.N, p.Nk, p.L_x,
+                                      r.lgp, fx_sched(p.sh), p.tx_h, p.tx_p, fftx_factor(p, a.mu), a.ebar, a.lambda, a.mu,
+                                      a.sig64, a.msum, tiles, a.gate);
   if (launches) *launches += 1;
 }
 

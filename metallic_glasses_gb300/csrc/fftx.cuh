@@ -41,7 +41,8 @@ void fftx_spectrum(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_
 double fftx_factor(const FFTPlan& p, double mu);
 // The C2R pass of a kOutSig64 solve.
 void fftx_c2r(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* launches);
-// Raises the passes' shared-memory limits on the current device.
-void fftx_init();
+// Raises the passes' shared-memory limits on the current device: of all kernels,
+// or of those that a plan with its present tiles launches.
+void fftx_init(const FFTPlan* plan = nullptr);
 
 }  // namespace stz

@@ -1,9 +1,10 @@
-// fixp.cpp -- host side of the fixed-point rates: the exponential's table and
-// the constants of a context.
+// fixp.cpp -- host side of the fixed-point forms: the exponential's table, the
+// transforms' twiddles and the constants of a context.
 #include "fixp.cuh"
 
 #include <algorithm>
 #include <cmath>
+#include <vector>
 
 #include "stz_internal.h"
 
@@ -52,32 +53,72 @@ void fx_exp_table(FxExp* t) {
   }
 }
 
-void fx_twiddles(int n, int count, FxTwiddle* out) {
-  const long double pi2 = 6.28318530717958647692528676655900577L;
-  for (int k = 0; k < count; k++) {
-    // the angle folded to an eighth of a turn, so that exact values stay exact
-    // and symmetric values are equal
-    const int k8 = (int)((8LL * k / n) & 7);
-    long double c, s;
-    auto cs = [&](long long num) {  // angle num / (8 n) of a turn, num in [0, n]
-      c = std::cos(pi2 * num / (8.0L * n));
-      s = std::sin(pi2 * num / (8.0L * n));
-    };
-    const long long num = 8LL * k - (long long)k8 * n;  // within the octant
-    if (k8 & 1) cs(n - num); else cs(num);
-    long double re, im;
-    switch (k8) {
-      case 0: re = c; im = s; break;
-      case 1: re = s; im = c; break;
-      case 2: re = -s; im = c; break;
-      case 3: re = -c; im = s; break;
-      case 4: re = -c; im = -s; break;
-      case 5: re = -s; im = -c; break;
-      case 6: re = s; im = -c; break;
-      default: re = c; im = -s; break;
+namespace {
+
+// pi / 4 2^126
+const uint64_t kPi4[2] = {0x3243f6a8885a308d, 0x313198a2e0370734};
+
+// 2^126 / m! for m = from, from + 2, ...
+struct Factorials {
+  u128 c[14];
+  constexpr explicit Factorials(int from) : c() {
+    u128 v = (u128)1 << 126;
+    for (int m = 2; m <= from; m++) v /= (unsigned)m;
+    for (int j = 0; j < 14; j++) {
+      c[j] = v;
+      v = v / (unsigned)(from + 2 * j + 1) / (unsigned)(from + 2 * j + 2);
     }
-    auto fix = [](long double v) {
-      Fx f = fx_split((int64_t)std::llrint(std::ldexp(v, 62)));
+  }
+};
+constexpr Factorials kCos(0), kSin(1);
+
+// The alternating series in y (y below 0.62; the 14th term is below 2^-97)
+u128 series(const Factorials& f, u128 y) {
+  u128 s = f.c[13];
+  for (int j = 12; j >= 0; j--) s = f.c[j] - mul_q126(y, s);
+  return s;
+}
+
+}  // namespace
+
+void fx_twiddles(int n, int count, FxTwiddle* out) {
+  // Cosine and sine of an eighth of a turn times num / n, each fraction formed
+  // once: the angles are folded to it, so that exact values stay exact,
+  // symmetric values are equal, and a table takes its series for n/8 of them
+  // (long double functions took 1.1 us a value on the host of a GB300, 160 us of
+  // every stand-alone solve of 48 x 54 x 36).
+  struct CS {
+    int64_t c = 0, s = 0;
+  };
+  std::vector<CS> seen((size_t)n + 1);
+  const u128 pi4 = (u128)kPi4[0] << 64 | kPi4[1], q = pi4 / (unsigned)n, r = pi4 % (unsigned)n;
+  auto round62 = [](u128 v) { return (int64_t)((uint64_t)(v >> 64) + ((uint64_t)(v >> 63) & 1)); };
+  auto cs = [&](long long num) {
+    CS& e = seen[(size_t)num];
+    if (e.c == 0) {  // a cosine is at least sqrt(1/2)
+      const u128 x = q * (unsigned)num + r * (unsigned)num / (unsigned)n, y = mul_q126(x, x);
+      e.c = round62(series(kCos, y));
+      e.s = round62(mul_q126(x, series(kSin, y)));
+    }
+    return e;
+  };
+  for (int k = 0; k < count; k++) {
+    const int k8 = (int)((8LL * k / n) & 7);
+    const long long num = 8LL * k - (long long)k8 * n;  // within the octant
+    const CS v = cs(k8 & 1 ? n - num : num);
+    int64_t re, im;
+    switch (k8) {
+      case 0: re = v.c; im = v.s; break;
+      case 1: re = v.s; im = v.c; break;
+      case 2: re = -v.s; im = v.c; break;
+      case 3: re = -v.c; im = v.s; break;
+      case 4: re = -v.c; im = -v.s; break;
+      case 5: re = -v.s; im = -v.c; break;
+      case 6: re = v.s; im = -v.c; break;
+      default: re = v.c; im = -v.s; break;
+    }
+    auto fix = [](int64_t w) {
+      Fx f = fx_split(w);
       if (f.l == INT32_MIN) f.l++;  // so that the halves can be negated
       return f;
     };

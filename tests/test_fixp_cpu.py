@@ -116,3 +116,23 @@ def test_products_and_conversion(lib):
         assert int(v[0]) == (want if x >= 0 else -want)
     for x in (32.0, -32.0, 1e300, float("inf"), float("-inf"), float("nan")):
         assert lib.t_from(x, 54, p) == 0
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 6, 9, 16, 18, 27, 54, 72, 243, 256, 486, 648, 729, 972, 1024, 1296, 8192])
+def test_twiddles_rounded_to_nearest(tmp_path, n):
+    """exp(-2 pi i k / n) in 2^-62: halves put together are the nearest integers
+    (a low half of -2^31 counts one up), the exact values of quarter turns
+    among them."""
+    src, so = tmp_path / "tw.cpp", tmp_path / "libtw.so"
+    src.write_text('#include "fixp.cuh"\nextern "C" void t_tw(int n, stz::FxTwiddle* t) { stz::fx_twiddles(n, n, t); }\n')
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, "-I", os.path.join(cuda, "include"),
+                    str(src), os.path.join(CSRC, "fixp.cpp"), "-o", str(so)], check=True)
+    t = np.empty((n, 4), np.int32)
+    C.CDLL(str(so)).t_tw(n, t.ctypes.data_as(C.c_void_p))
+    with mpmath.workprec(160):
+        for k in range(0, n, 1 + n // 512):
+            a = -2 * mpmath.pi * k / n
+            for v, (h, l) in ((mpmath.cos(a), t[k, :2]), (mpmath.sin(a), t[k, 2:])):
+                err = abs(mpmath.mpf(int(h) * 2 ** 32 + int(l)) - v * 2 ** 62)
+                assert err <= 0.5 + 1e-9 or (l == 1 - 2 ** 31 and err <= 1.5)
