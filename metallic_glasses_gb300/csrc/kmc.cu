@@ -1667,11 +1667,14 @@ __global__ void __launch_bounds__(TH, 2) k_rate64_fx2(KParams kp, Fields f, Rate
           v[h + i] = fx_double(fx_exp2_sum_bits<Q>(Y, c));
         }
       }
+      // a chunk of the FP64 chain: no use going on (with barriers out of range at
+      // most sites, a 512^2 step at 50 K, the loop's rest cost 7% of the step)
+      if (__any_sync(FULL, !ok)) break;
       int idx;
       const double t = WarpSums<G, 16>::run(v, lane, &idx);
       if (idx >= 0) red[w][g + idx] = t;
     }
-    if (top >= (unsigned)(rx.neg >> 32)) {  // as in 3D
+    if (ok && top >= (unsigned)(rx.neg >> 32)) {  // as in 3D
 #pragma unroll
       for (int q = 0; q < Q; q++) {
         const long long s = s0 + threadIdx.x + q * TH;
