@@ -550,7 +550,8 @@ __device__ __forceinline__ FxExp fx_cell_shared(unsigned tab, uint64_t Y) {
   const unsigned at = tab + ((unsigned)(Y >> 38) & ((kFxExpCells - 1) * (unsigned)sizeof(FxExp)));
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                : "=r"(lo), "=r"(hi), "=r"(q.ph), "=r"(q.pl)
-               : "r"(at));
+               : "r"(at)
+               : "memory");
   q.t = (int64_t)((uint64_t)lo | ((uint64_t)hi << 32));
   return q;
 }
