@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "fft.cuh"
+#include "fftx.cuh"
 #include "kmc.cuh"
 #include "stz_internal.h"
 
@@ -963,7 +964,10 @@ int stz::create_ctx(const stz_params* pin, stz_ctx** out, int units_per_block) {
     return fail(st);
   }
   // tiles and radix order timed for this grid (once per process and shape)
-  if ((st = fft_autotune(plan, c->stream, c->fft_tuned, mixed && !c->p.resolve_fp64 ? 1 : 0))) {
+  const PassKind kind = mixed && !c->p.resolve_fp64            ? kPassPair
+                        : fftx_fits(kp.n2, kp.lambda, kp.mu) ? kPassFx
+                                                             : kPassFp64;
+  if ((st = fft_autotune(plan, c->stream, c->fft_tuned, kind))) {
     set_error("FFT schedule tuning failed: %s", cudaGetErrorString(cudaGetLastError()));
     return fail(st);
   }
@@ -1309,7 +1313,8 @@ extern "C" int stz_fft_schedule(stz_ctx* c, int32_t* tiles, int32_t* radices) {
   if (tiles)
     for (int k = 0; k < 4; k++) tiles[k] = c->fft_tuned[k];
   if (radices) {
-    const Sched* sc[3] = {&p.sh, &p.s1, &p.s0};
+    const bool fx = p.kind == kPassFx;
+    const Sched* sc[3] = {fx ? &p.x.sh : &p.sh, fx ? &p.x.s1 : &p.s1, fx ? &p.x.s0 : &p.s0};
     for (int a = 0; a < 3; a++)
       for (int k = 0; k < 12; k++) radices[a * 12 + k] = k < sc[a]->nst ? sc[a]->r[k] : 0;
   }

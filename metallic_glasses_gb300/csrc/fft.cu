@@ -968,14 +968,13 @@ struct Tw<dfl> {
 // The C2R pass of a kOutDev32 solve; factor multiplies its sums (1 / N). With
 // ebar, the uniform stress C:ebar is added (a spectrum without its mean part).
 template <typename T>
-void c2r_dev(const FFTPlan& p, const SolveArgs& a, double factor, const double* ebar, cudaStream_t st,
+void c2r_dev(const FFTPlan& p, const SolveArgs& a, int L, double factor, const double* ebar, cudaStream_t st,
              int64_t* launches) {
   using V = typename VT<T>::V;
   const long long rows = (long long)p.n0 * p.n1;
   // the deviatoric epilogue stages the block's six real rows: a row tile of
   // its own, kept within 72 KB of shared memory so that several blocks share
   // an SM (the tuned tile is timed without this staging)
-  int L = p.L_x;
   auto dev_smem = [&](int l) { return 2 * (size_t)p.nc * l * (p.h + 2) * sizeof(V); };
   while (L > 1 && dev_smem(L) > 72 * 1024) L /= 2;
   k_c2r_dev<T><<<(unsigned)((rows + L - 1) / L), 256, dev_smem(L), st>>>(
@@ -1047,7 +1046,7 @@ int solve_t(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* laun
                                                Tw<T>::h(p), Tw<T>::post(p), invN, nullptr, a.sig32, nullptr,
                                                nullptr, nullptr, nullptr, a.gate);
   else if (p.nc == 6)
-    c2r_dev<T>(p, a, invN, nullptr, st, nullptr);
+    c2r_dev<T>(p, a, p.L_x, invN, nullptr, st, nullptr);
   else
     k_c2r_x<T, kOutDev32><<<gx.x, TH, p.smem_c2r + sizeof(double) * (size_t)p.nc * p.L_x * p.n2, st>>>(
         spec, p.nc, p.n2, p.h, p.nh, rows, p.N, p.Nk, p.L_x, p.sh, Tw<T>::h(p), Tw<T>::post(p), invN, nullptr,
@@ -1059,20 +1058,17 @@ int solve_t(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* laun
 
 }  // namespace
 
-// Tiles (lines per block) of the three kinds of pass and their shared memory,
-// in FP64 (the FP32 and pair transforms use the same tiles) and in fixed point
-// (padded lines); false if a pass would not fit in `limit` bytes, with
-// `staging` the C2R pass beside the real rows of all components.
+// Tiles (lines per block) of the three kinds of floating-point pass and their
+// shared memory in FP64 (the FP32 and pair transforms use the same tiles);
+// false if a pass, or the C2R pass beside the real rows of all components,
+// would not fit.
 static bool plan_set_tiles(FFTPlan* p, int Lx, int Ly, int Lg, size_t limit = 200 * 1024, bool staging = true) {
   const size_t cz = sizeof(double2);
   const int ng = p->n0 > 1 ? p->n0 : p->n1;
   const size_t sx = 2 * (size_t)Lx * (p->h + 1) * cz, sc = 2 * (size_t)Lx * (p->h + 2) * cz;
   const size_t sy = 2 * (size_t)Ly * (p->n1 + 1) * cz, sg = 2 * (size_t)p->nc * Lg * (ng + 1) * cz;
-  const size_t rx = 2 * (size_t)Lx * fx_ld(p->h + 1) * cz + sizeof(int) * Lx, ry = 2 * (size_t)Ly * fx_ld(p->n1) * cz,
-               rg = 2 * (size_t)p->nc * Lg * fx_ld(ng) * cz + (size_t)ng * Lg;
-  if (Lx < 1 || Ly < 1 || Lg < 1 || (Ly > 1 && Ly * p->n1 > 2048)) return false;
-  if (sc + (staging ? sizeof(double) * p->nc * Lx * p->n2 : 0) > limit || ry > limit || rg > limit || rx > limit)
-    return false;
+  if (Lx < 1 || Ly < 1 || Lg < 1) return false;
+  if (sc + (staging ? sizeof(double) * p->nc * Lx * p->n2 : 0) > limit || sy > limit || sg > limit) return false;
   p->L_x = Lx;
   p->L_y = Ly;
   p->L_g = Lg;
@@ -1080,27 +1076,52 @@ static bool plan_set_tiles(FFTPlan* p, int Lx, int Ly, int Lg, size_t limit = 20
   p->smem_c2r = sc;
   p->smem_y = sy;
   p->smem_g = sg;
-  p->smem_xr = rx;
-  p->smem_yr = ry;
-  p->smem_gr = rg;
   return true;
 }
 
-// The tiles a plan starts with: 1024 complex values of rows, eight lines of the
-// other axes (four or fewer where shared memory asks for it).
-static bool default_tiles(FFTPlan* p) {
-  p->e_x = 4;
-  p->e_y = 4;
-  p->e_g = 2;
+// The same of the fixed-point passes (padded lines; a thread holds at most eight
+// values of a column).
+static bool plan_set_fx_tiles(FFTPlan* p, int Lx, int Ly, int Lg, size_t limit = 200 * 1024) {
   const size_t cz = sizeof(double2);
   const int ng = p->n0 > 1 ? p->n0 : p->n1;
+  const size_t rx = 2 * (size_t)Lx * fx_ld(p->h + 1) * cz + sizeof(int) * Lx, ry = 2 * (size_t)Ly * fx_ld(p->n1) * cz,
+               rg = 2 * (size_t)p->nc * Lg * fx_ld(ng) * cz + (size_t)ng * Lg;
+  if (Lx < 1 || Ly < 1 || Lg < 1 || (Ly > 1 && Ly * p->n1 > 2048)) return false;
+  if (rx > limit || ry > limit || rg > limit) return false;
+  FxPasses& x = p->x;
+  x.Lx = Lx;
+  x.Ly = Ly;
+  x.Lg = Lg;
+  x.smem_x = rx;
+  x.smem_y = ry;
+  x.smem_g = rg;
+  return true;
+}
+
+// The schedule a plan starts with: radices of make_sched, 1024 complex values of
+// rows, eight lines of the other axes (four or fewer where shared memory asks
+// for it).
+static bool default_schedule(FFTPlan* p) {
+  p->sh = p->x.sh = make_sched(p->h);
+  p->s1 = p->x.s1 = make_sched(p->n1);
+  p->s0 = p->x.s0 = make_sched(p->n0);
+  if (p->sh.nst < 0 || p->s1.nst < 0 || p->s0.nst < 0) return false;
+  const size_t cz = sizeof(double2), most = 200 * 1024;
+  const int ng = p->n0 > 1 ? p->n0 : p->n1, nc = p->nc;
   int Lx = std::max(1, 1024 / p->h), Ly = 8, Lg = 8;
-  while (Lx > 1 && 2 * (size_t)Lx * fx_ld(p->h + 1) * cz + sizeof(double) * p->nc * Lx * p->n2 > 200 * 1024) Lx /= 2;
-  while (Ly > 1 && (2 * (size_t)Ly * fx_ld(p->n1) * cz > 100 * 1024 || Ly * p->n1 > 2048)) Ly /= 2;
-  while (Lg > 1 && 2 * (size_t)p->nc * Lg * fx_ld(ng) * cz + (size_t)ng * Lg > 200 * 1024) Lg /= 2;
+  while (Lx > 1 && 2 * (size_t)Lx * (p->h + 2) * cz + sizeof(double) * nc * Lx * p->n2 > most) Lx /= 2;
+  while (Ly > 1 && 2 * (size_t)Ly * (p->n1 + 1) * cz > 100 * 1024) Ly /= 2;
+  while (Lg > 1 && 2 * (size_t)nc * Lg * (ng + 1) * cz > most) Lg /= 2;
   // the longest lines (8192 values) leave no room for the staging, which no
   // FP64 output has
-  return plan_set_tiles(p, Lx, Ly, Lg, 224 * 1024, false);
+  if (!plan_set_tiles(p, Lx, Ly, Lg, 224 * 1024, false)) return false;
+  p->x.ex = 4;
+  p->x.ey = 4;
+  p->x.eg = 2;
+  Lx = std::max(1, 1024 / p->h), Ly = 8, Lg = 8;
+  while (Ly > 1 && (2 * (size_t)Ly * fx_ld(p->n1) * cz > 100 * 1024 || Ly * p->n1 > 2048)) Ly /= 2;
+  while (Lg > 1 && 2 * (size_t)nc * Lg * fx_ld(ng) * cz + (size_t)ng * Lg > most) Lg /= 2;
+  return plan_set_fx_tiles(p, Lx, Ly, Lg, 224 * 1024);
 }
 
 int fft_plan_create(FFTPlan* p, int n0, int n1, int n2, int nc) {
@@ -1111,17 +1132,12 @@ int fft_plan_create(FFTPlan* p, int n0, int n1, int n2, int nc) {
   p->nh = p->h + 1;
   p->N = (long long)n0 * n1 * n2;
   p->Nk = (long long)n0 * n1 * p->nh;
-  p->sh = make_sched(p->h);
-  p->s1 = make_sched(n1);
-  p->s0 = make_sched(n0);
-  if (p->sh.nst < 0 || p->s1.nst < 0 || p->s0.nst < 0) return STZ_ERR_INVALID;
-  if (p->h > 4096 || n1 > 1024 || n0 > 1024) return STZ_ERR_INVALID;
+  if (p->h > 4096 || n1 > 1024 || n0 > 1024 || !default_schedule(p)) return STZ_ERR_INVALID;
   int st;
-  if ((st = upload_twiddles(p->h, p->h, &p->tw_h, &p->tw_hf, &p->tw_hd, &p->tx_h))) return st;
-  if ((st = upload_twiddles(n1, n1, &p->tw_1, &p->tw_1f, &p->tw_1d, &p->tx_1))) return st;
-  if ((st = upload_twiddles(n0, n0, &p->tw_0, &p->tw_0f, &p->tw_0d, &p->tx_0))) return st;
-  if ((st = upload_twiddles(n2, p->nh, &p->tw_p, &p->tw_pf, &p->tw_pd, &p->tx_p))) return st;
-  if (!default_tiles(p)) return STZ_ERR_INVALID;
+  if ((st = upload_twiddles(p->h, p->h, &p->tw_h, &p->tw_hf, &p->tw_hd, &p->x.tw_h))) return st;
+  if ((st = upload_twiddles(n1, n1, &p->tw_1, &p->tw_1f, &p->tw_1d, &p->x.tw_1))) return st;
+  if ((st = upload_twiddles(n0, n0, &p->tw_0, &p->tw_0f, &p->tw_0d, &p->x.tw_0))) return st;
+  if ((st = upload_twiddles(n2, p->nh, &p->tw_p, &p->tw_pf, &p->tw_pd, &p->x.tw_p))) return st;
   size_t sc_max = p->smem_c2r + sizeof(double) * nc * p->L_x * n2;
   set_smem_attrs<double>(p->smem_x, p->smem_y, p->smem_g, sc_max);
   set_smem_attrs<float>(p->smem_x, p->smem_y, p->smem_g, sc_max);
@@ -1131,22 +1147,50 @@ int fft_plan_create(FFTPlan* p, int n0, int n1, int n2, int nc) {
 }
 
 namespace {
+// A tuned schedule: of the fixed-point passes, or tiles and radices of the
+// floating-point ones.
 struct Tuned {
-  int Lx, Ly, Lg, ex, ey, eg;
+  int L[3], ev[3];
   Sched sh, s1, s0;
   int rejected;  // candidates whose result differed from the default schedule's
 };
+bool set_tiles(FFTPlan* p, const int* L) {
+  return p->kind == kPassFx ? plan_set_fx_tiles(p, L[0], L[1], L[2]) : plan_set_tiles(p, L[0], L[1], L[2]);
+}
+Tuned schedule_of(const FFTPlan& p) {
+  const FxPasses& x = p.x;
+  if (p.kind == kPassFx) return Tuned{{x.Lx, x.Ly, x.Lg}, {x.ex, x.ey, x.eg}, x.sh, x.s1, x.s0, 0};
+  return Tuned{{p.L_x, p.L_y, p.L_g}, {0, 0, 0}, p.sh, p.s1, p.s0, 0};
+}
+// false (and the tiles of before) where other tiles do not fit
+bool take_schedule(FFTPlan* p, const Tuned& t) {
+  const Tuned now = schedule_of(*p);
+  const bool ok = std::equal(t.L, t.L + 3, now.L) || set_tiles(p, t.L);
+  if (p->kind == kPassFx) {
+    p->x.ex = t.ev[0];
+    p->x.ey = t.ev[1];
+    p->x.eg = t.ev[2];
+    p->x.sh = t.sh;
+    p->x.s1 = t.s1;
+    p->x.s0 = t.s0;
+  } else {
+    p->sh = t.sh;
+    p->s1 = t.s1;
+    p->s0 = t.s0;
+  }
+  return ok;
+}
 std::mutex g_tune_mu;
 std::map<std::array<int, 6>, Tuned> g_tuned;
 
-// The better of two times of three solves. They queue behind a kernel that holds
-// the stream while the host launches them, so that the events bracket device
-// time on the smallest grids too (without it those took four times twelve solves
-// a candidate: 153 ms for the first 64^3 context of a process, 44 so).
+// The better of two times of three solves. On small grids they queue behind a
+// kernel that holds the stream while the host launches them, so that the events
+// bracket device time (without it those took four times twelve solves a
+// candidate: 153 ms for the first 64^3 context of a process, 45 so).
 float time_solve(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1) {
   float best = 1e30f;
   for (int rep = 0; rep < 2; rep++) {
-    launch_hold(60000, st);
+    if (p.N * p.nc < 1 << 21) launch_hold(40000, st);
     cudaEventRecord(e0, st);
     for (int i = 0; i < 3; i++) fft_solve(p, a, st, nullptr);
     cudaEventRecord(e1, st);
@@ -1159,22 +1203,24 @@ float time_solve(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, cudaEven
 }
 }  // namespace
 
-int fft_autotune(FFTPlan* p, cudaStream_t st, int* chosen, int pair) {
+int fft_autotune(FFTPlan* p, cudaStream_t st, int* chosen, PassKind kind) {
+  p->kind = kind;
   int dev = 0;
   cudaGetDevice(&dev);
-  const std::array<int, 6> key = {dev, p->n0, p->n1, p->n2, p->nc, pair};
+  const std::array<int, 6> key = {dev, p->n0, p->n1, p->n2, p->nc, kind};
+  auto take = [&](const Tuned& t) {
+    take_schedule(p, t);
+    const Tuned now = schedule_of(*p);
+    if (chosen) {
+      for (int i = 0; i < 3; i++) chosen[i] = now.L[i];
+      chosen[3] = t.rejected;
+    }
+  };
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tuned.find(key);
     if (it != g_tuned.end()) {
-      plan_set_tiles(p, it->second.Lx, it->second.Ly, it->second.Lg);
-      p->sh = it->second.sh;
-      p->s1 = it->second.s1;
-      p->s0 = it->second.s0;
-      p->e_x = it->second.ex;
-      p->e_y = it->second.ey;
-      p->e_g = it->second.eg;
-      if (chosen) { chosen[0] = p->L_x; chosen[1] = p->L_y; chosen[2] = p->L_g; chosen[3] = it->second.rejected; }
+      take(it->second);
       return STZ_OK;
     }
   }
@@ -1197,13 +1243,13 @@ int fft_autotune(FFTPlan* p, cudaStream_t st, int* chosen, int pair) {
   cudaMemcpyAsync(eps, h.data(), n * 8, cudaMemcpyHostToDevice, st);
   SolveArgs a{};
   a.eps = eps;
-  a.lambda = 2.0;
+  a.lambda = kind == kPassFp64 ? 1000.0 : 2.0;  // beyond the fixed point's range, or within
   a.mu = 1.0;
   a.out = kOutSig64;
   a.sig64 = ref;
   a.spec = spec;
   a.ortho_mean = 1;
-  a.pair = pair;
+  a.pair = kind == kPassPair;
   fft_solve(*p, a, st, nullptr);
   cudaStreamSynchronize(st);
   std::vector<double> r(n), o(n);
@@ -1228,63 +1274,50 @@ int fft_autotune(FFTPlan* p, cudaStream_t st, int* chosen, int pair) {
   };
   FFTPlan best = *p;
   float tbest = time_solve(best, a, st, e0, e1);
-  auto consider = [&](FFTPlan q) {
-    if (!valid(q)) return;
-    const float t = time_solve(q, a, st, e0, e1);
-    if (t < tbest) { tbest = t; best = q; }
+  auto consider = [&](const Tuned& t) {
+    FFTPlan q = best;
+    if (!take_schedule(&q, t) || !valid(q)) return;
+    const float ms = time_solve(q, a, st, e0, e1);
+    if (ms < tbest) { tbest = ms; best = q; }
   };
-  // coordinate descent over the tiles of each pass, then the radix orders
-  for (int Lx : {p->L_x * 2, p->L_x / 2, p->L_x / 4}) {
-    FFTPlan q = best;
-    if (Lx >= 1 && plan_set_tiles(&q, Lx, q.L_y, q.L_g)) consider(q);
-  }
-  for (int Ly : {2, 4, 16, 32}) {
-    FFTPlan q = best;
-    if (Ly != best.L_y && plan_set_tiles(&q, q.L_x, Ly, q.L_g)) consider(q);
-  }
-  for (int Lg : {1, 2, 4, 16}) {
-    FFTPlan q = best;
-    if (Lg != best.L_g && plan_set_tiles(&q, q.L_x, q.L_y, Lg)) consider(q);
-  }
+  // coordinate descent over the tiles of each pass, the radix orders and, of the
+  // fixed-point passes, the threads per tile
+  const Tuned first = schedule_of(best);
+  auto try_tile = [&](int i, int L) {
+    Tuned t = schedule_of(best);
+    if (L < 1 || L == t.L[i]) return;
+    t.L[i] = L;
+    consider(t);
+  };
+  for (int L : {first.L[0] * 2, first.L[0] / 2, first.L[0] / 4}) try_tile(0, L);
+  for (int L : {2, 4, 16}) try_tile(1, L);
+  if (p->n1 <= 64) try_tile(1, 32);
+  if (kind == kPassFx) try_tile(2, 1);
+  for (int L : {2, 4, 16}) try_tile(2, L);
   for (int v = 0; v < 2; v++) {
-    FFTPlan q = best;
-    q.sh = v ? make_sched_rev(p->h) : make_sched_r4(p->h);
-    q.s1 = v ? make_sched_rev(p->n1) : make_sched_r4(p->n1);
-    q.s0 = v ? make_sched_rev(p->n0) : make_sched_r4(p->n0);
-    if (q.sh.nst > 0 && q.s1.nst > 0 && q.s0.nst > 0) consider(q);
+    Tuned t = schedule_of(best);
+    t.sh = v ? make_sched_rev(p->h) : make_sched_r4(p->h);
+    t.s1 = v ? make_sched_rev(p->n1) : make_sched_r4(p->n1);
+    t.s0 = v ? make_sched_rev(p->n0) : make_sched_r4(p->n0);
+    if (t.sh.nst > 0 && t.s1.nst > 0 && t.s0.nst > 0) consider(t);
   }
-  if (!pair && p->n2 <= kFxLongest) {  // threads per tile of the fixed-point passes
-    for (int e : {2, 8}) {
-      FFTPlan q = best;
-      q.e_x = e;
-      consider(q);
-    }
-    for (int e : {2, 8}) {
-      FFTPlan q = best;
-      q.e_y = e;
-      if (p->n0 > 1) consider(q);
-    }
-    for (int e : {1, 4}) {
-      FFTPlan q = best;
-      q.e_g = e;
-      consider(q);
-    }
-  }
+  if (kind == kPassFx)
+    for (int i = 0; i < 3; i++)
+      for (int ev : {i < 2 ? 2 : 1, i < 2 ? 8 : 4}) {
+        Tuned t = schedule_of(best);
+        t.ev[i] = ev;
+        if (i != 1 || p->n0 > 1) consider(t);
+      }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaFree(eps); cudaFree(ref); cudaFree(out); cudaFree(spec);
-  p->e_x = best.e_x;
-  p->e_y = best.e_y;
-  p->e_g = best.e_g;
-  plan_set_tiles(p, best.L_x, best.L_y, best.L_g);
-  p->sh = best.sh;
-  p->s1 = best.s1;
-  p->s0 = best.s0;
+  Tuned t = schedule_of(best);
+  t.rejected = rejected;
+  take(t);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tuned[key] = Tuned{p->L_x, p->L_y, p->L_g, p->e_x, p->e_y, p->e_g, p->sh, p->s1, p->s0, rejected};
+    g_tuned[key] = t;
   }
-  if (chosen) { chosen[0] = p->L_x; chosen[1] = p->L_y; chosen[2] = p->L_g; chosen[3] = rejected; }
   return cudaGetLastError() == cudaSuccess ? STZ_OK : STZ_ERR_CUDA;
 }
 
@@ -1303,17 +1336,13 @@ int fft_plan_init_in(FFTPlan* p, int n0, int n1, int n2, int nc, double lambda, 
   p->nh = p->h + 1;
   p->N = (long long)n0 * n1 * n2;
   p->Nk = (long long)n0 * n1 * p->nh;
-  p->sh = make_sched(p->h);
-  p->s1 = make_sched(n1);
-  p->s0 = make_sched(n0);
-  if (p->sh.nst < 0 || p->s1.nst < 0 || p->s0.nst < 0) return STZ_ERR_INVALID;
-  if (p->h > 4096 || n1 > 1024 || n0 > 1024) return STZ_ERR_INVALID;
+  if (p->h > 4096 || n1 > 1024 || n0 > 1024 || !default_schedule(p)) return STZ_ERR_INVALID;
   if (fft_twiddle_count(n0, n1, n2) > cap) return STZ_ERR_INVALID;
   const bool fx = fftx_fits(n2, lambda, mu);
   const int lens[4] = {p->h, n1, n0, n2};
   const int counts[4] = {p->h, n1, n0, p->nh};
   double2** dst[4] = {&p->tw_h, &p->tw_1, &p->tw_0, &p->tw_p};
-  FxTwiddle** dfx[4] = {&p->tx_h, &p->tx_1, &p->tx_0, &p->tx_p};
+  FxTwiddle** dfx[4] = {&p->x.tw_h, &p->x.tw_1, &p->x.tw_0, &p->x.tw_p};
   static_assert(sizeof(FxTwiddle) == sizeof(double2), "one table size");
   std::vector<double2> host(fft_twiddle_count(n0, n1, n2));
   size_t off = 0;
@@ -1334,19 +1363,21 @@ int fft_plan_init_in(FFTPlan* p, int n0, int n1, int n2, int nc, double lambda, 
       cudaSuccess)
     return STZ_ERR_CUDA;
   if (cudaStreamSynchronize(st) != cudaSuccess) return STZ_ERR_CUDA;
-  if (!default_tiles(p)) return STZ_ERR_INVALID;
   if (fx) fftx_init(p);
   else set_smem_attrs<double>(p->smem_x, p->smem_y, p->smem_g, p->smem_c2r + sizeof(double) * nc * p->L_x * n2);
   return STZ_OK;
 }
 
-int fft_c2r_blocks(const FFTPlan& p) { return (int)(((long long)p.n0 * p.n1 + p.L_x - 1) / p.L_x); }
+int fft_c2r_blocks(const FFTPlan& p) {
+  const int L = p.kind == kPassFx ? p.x.Lx : p.L_x;
+  return (int)(((long long)p.n0 * p.n1 + L - 1) / L);
+}
 
 void fft_plan_destroy(FFTPlan* p) {
   cudaFree(p->tw_h); cudaFree(p->tw_1); cudaFree(p->tw_0); cudaFree(p->tw_p);
   cudaFree(p->tw_hf); cudaFree(p->tw_1f); cudaFree(p->tw_0f); cudaFree(p->tw_pf);
   cudaFree(p->tw_hd); cudaFree(p->tw_1d); cudaFree(p->tw_0d); cudaFree(p->tw_pd);
-  cudaFree(p->tx_h); cudaFree(p->tx_1); cudaFree(p->tx_0); cudaFree(p->tx_p);
+  cudaFree(p->x.tw_h); cudaFree(p->x.tw_1); cudaFree(p->x.tw_0); cudaFree(p->x.tw_p);
   std::memset((void*)p, 0, sizeof(*p));
 }
 
@@ -1359,7 +1390,7 @@ int fft_solve(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* la
       fftx_fits(p.n2, a.lambda, a.mu)) {
     fftx_spectrum(p, a, st, launches);
     if (a.out == kOutSig64) fftx_c2r(p, a, st, launches);
-    else c2r_dev<double>(p, a, fftx_factor(p, a.mu), a.ebar, st, launches);
+    else c2r_dev<double>(p, a, p.x.Lx, fftx_factor(p, a.mu), a.ebar, st, launches);
     return STZ_OK;
   }
   return a.fp32 ? solve_t<float>(p, a, st, launches) : solve_t<double>(p, a, st, launches);

@@ -23,6 +23,21 @@ enum SolveOut {
                    // field they replace, mixed form re-solve
 };
 
+// The fixed-point passes of a plan (fftx.cu): split twiddles, radix orders,
+// tiles (lines per block), values of a tile (eg: of each component) per thread
+// and shared memory, all apart from the floating-point passes', which a plan
+// may run beside them (the displacement, FP32-pair re-solves, media out of the
+// fixed point's range).
+struct FxPasses {
+  FxTwiddle *tw_h, *tw_1, *tw_0, *tw_p;
+  Sched sh, s1, s0;
+  int Lx, Ly, Lg, ex, ey, eg;
+  size_t smem_x, smem_y, smem_g;
+};
+
+// The passes that a plan's tuning times, and that its mean stress is summed in.
+enum PassKind { kPassFx = 0, kPassPair = 1, kPassFp64 = 2 };
+
 struct FFTPlan {
   int n0, n1, n2, h, nh, nc;
   long long N, Nk;
@@ -35,20 +50,19 @@ struct FFTPlan {
   // tiles (lines per block) of each pass
   int L_x = 0, L_y = 0, L_g = 0;
   size_t smem_x = 0, smem_y = 0, smem_g = 0, smem_c2r = 0;
-  // the fixed-point passes (fftx.cu): split twiddles and shared memory
-  FxTwiddle *tx_h = nullptr, *tx_1 = nullptr, *tx_0 = nullptr, *tx_p = nullptr;
-  size_t smem_xr = 0, smem_yr = 0, smem_gr = 0;
-  int e_x = 0, e_y = 0, e_g = 0;  // values of a tile (e_g: of each component) per thread
+  FxPasses x;
+  int kind = kPassFx;
 };
 
 int fft_plan_create(FFTPlan* p, int n0, int n1, int n2, int nc);
 // Chooses the tiles (lines per block of each pass) and the radix order of the
-// plan by timing solves of a fixed eigenstrain in FP64 (pair = 0) or in FP32
-// pairs (pair = 1), once per device, grid shape and precision per process
-// (cached); a candidate is admitted only if its result equals the default
-// schedule's within 1e-10. chosen (optional, 4 ints): the tiles L_x, L_y, L_g
-// and the number of candidates rejected.
-int fft_autotune(FFTPlan* p, cudaStream_t st, int* chosen, int pair);
+// passes that the plan's solves take (kind) by timing solves of a fixed
+// eigenstrain, once per device, grid shape and kind per process (cached); a
+// candidate is admitted only if its result equals the default schedule's within
+// 1e-10. The other passes keep their default. chosen (optional, 4 ints): the
+// tiles along axis 2, axis 1 and in Green's pass, and the number of candidates
+// rejected.
+int fft_autotune(FFTPlan* p, cudaStream_t st, int* chosen, PassKind kind);
 // A plan for FP64 solves of one medium whose twiddle tables are written into
 // caller-provided device storage of at least fft_twiddle_count() elements.
 size_t fft_twiddle_count(int n0, int n1, int n2);

@@ -969,22 +969,22 @@ auto green_kernel(int nc, int U) {
 // of a grid without axis 0 (with three components or six).
 void launch_green(const FFTPlan& p, int n, int inner, const SolveArgs& a, const FxSched& x, const FxTwiddle* tw,
                   const GreenFx& ga, cudaStream_t st) {
-  const ColLaunch c = col_launch(n, p.L_g, p.e_g);
-  const int tiles = (inner + p.L_g - 1) / p.L_g;
+  const ColLaunch c = col_launch(n, p.x.Lg, p.x.eg);
+  const int tiles = (inner + p.x.Lg - 1) / p.x.Lg;
   const dim3 grid = fx_grid(a, tiles, 1);
   const auto k = green_kernel(p.nc, c.U);
-  k<<<grid, c.threads, p.smem_gr, st>>>(reinterpret_cast<double2*>(a.spec), n, inner, inner, p.Nk, p.L_g, ilog2(p.L_g), x,
+  k<<<grid, c.threads, p.x.smem_g, st>>>(reinterpret_cast<double2*>(a.spec), n, inner, inner, p.Nk, p.x.Lg, ilog2(p.x.Lg), x,
                                         tw, ga, tiles, a.gate);
 }
 
 template <bool INV>
 void launch_c2c(const FFTPlan& p, const SolveArgs& a, const FxSched& x, cudaStream_t st) {
-  const ColLaunch c = col_launch(p.n1, p.L_y, p.e_y);
-  const int columns = p.n0 * p.nh, tiles = (columns + p.L_y - 1) / p.L_y;
+  const ColLaunch c = col_launch(p.n1, p.x.Ly, p.x.ey);
+  const int columns = p.n0 * p.nh, tiles = (columns + p.x.Ly - 1) / p.x.Ly;
   const dim3 grid = fx_grid(a, tiles, p.nc);
   const auto k = c2c_kernel<INV>(c.U);
-  k<<<grid, c.threads, p.smem_yr, st>>>(reinterpret_cast<double2*>(a.spec), p.n1, p.nh, columns, p.Nk, p.L_y,
-                                        ilog2(p.L_y), x, p.tx_1, tiles, a.gate);
+  k<<<grid, c.threads, p.x.smem_y, st>>>(reinterpret_cast<double2*>(a.spec), p.n1, p.nh, columns, p.Nk, p.x.Ly,
+                                        ilog2(p.x.Ly), x, p.x.tw_1, tiles, a.gate);
 }
 
 }  // namespace
@@ -1005,12 +1005,12 @@ void fftx_init(const FFTPlan* plan) {
     optin = 227 * 1024;
   if (plan) {
     const FFTPlan& p = *plan;
-    const int ux = row_launch(p.h, p.L_x, p.e_x).U;
+    const int ux = row_launch(p.h, p.x.Lx, p.x.ex).U;
     raise_limit(r2c_kernel(ux), optin);
     raise_limit(c2r_kernel(ux), optin);
-    raise_limit(green_kernel(p.nc, col_launch(p.n0 > 1 ? p.n0 : p.n1, p.L_g, p.e_g).U), optin);
+    raise_limit(green_kernel(p.nc, col_launch(p.n0 > 1 ? p.n0 : p.n1, p.x.Lg, p.x.eg).U), optin);
     if (p.n0 > 1) {
-      const int uy = col_launch(p.n1, p.L_y, p.e_y).U;
+      const int uy = col_launch(p.n1, p.x.Ly, p.x.ey).U;
       raise_limit(c2c_kernel<false>(uy), optin);
       raise_limit(c2c_kernel<true>(uy), optin);
     }
@@ -1031,21 +1031,21 @@ void fftx_init(const FFTPlan* plan) {
 void fftx_spectrum(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* launches) {
   double2* spec = reinterpret_cast<double2*>(a.spec);
   const long long rows = (long long)p.n0 * p.n1;
-  const FxSched xh = fx_sched(p.sh), x1 = fx_sched(p.s1), x0 = fx_sched(p.s0);
-  const int tiles = (int)((rows + p.L_x - 1) / p.L_x);
+  const FxSched xh = fx_sched(p.x.sh), x1 = fx_sched(p.x.s1), x0 = fx_sched(p.x.s0);
+  const int tiles = (int)((rows + p.x.Lx - 1) / p.x.Lx);
   const dim3 gx = fx_grid(a, tiles, p.nc);
-  const RowLaunch r = row_launch(p.h, p.L_x, p.e_x);
+  const RowLaunch r = row_launch(p.h, p.x.Lx, p.x.ex);
   const auto k = r2c_kernel(r.U);
-  k<<<gx, r.threads, p.smem_xr, st>>>(a.eps, spec, p.h, p.nh, rows, p.N, p.Nk, p.L_x, r.lgp, xh, p.tx_h, p.tx_p, tiles,
+  k<<<gx, r.threads, p.x.smem_x, st>>>(a.eps, spec, p.h, p.nh, rows, p.N, p.Nk, p.x.Lx, r.lgp, xh, p.x.tw_h, p.x.tw_p, tiles,
                                       a.gate);
   GreenFx ga;
   fx_green_constants(p.n0, p.n1, p.n2, a.lambda, a.mu, &ga);
   if (p.n0 > 1) {
     launch_c2c<false>(p, a, x1, st);
-    launch_green(p, p.n0, p.n1 * p.nh, a, x0, p.tx_0, ga, st);
+    launch_green(p, p.n0, p.n1 * p.nh, a, x0, p.x.tw_0, ga, st);
     launch_c2c<true>(p, a, x1, st);
   } else {
-    launch_green(p, p.n1, p.nh, a, x1, p.tx_1, ga, st);
+    launch_green(p, p.n1, p.nh, a, x1, p.x.tw_1, ga, st);
   }
   if (launches) *launches += p.n0 > 1 ? 4 : 2;
 }
@@ -1054,12 +1054,12 @@ double fftx_factor(const FFTPlan& p, double mu) { return (double)(2 * (long doub
 
 void fftx_c2r(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, int64_t* launches) {
   const long long rows = (long long)p.n0 * p.n1;
-  const int tiles = (int)((rows + p.L_x - 1) / p.L_x);
+  const int tiles = (int)((rows + p.x.Lx - 1) / p.x.Lx);
   const dim3 gx = fx_grid(a, tiles, p.nc);
-  const RowLaunch r = row_launch(p.h, p.L_x, p.e_x);
+  const RowLaunch r = row_launch(p.h, p.x.Lx, p.x.ex);
   const auto k = c2r_kernel(r.U);
-  k<<<gx, r.threads, p.smem_xr, st>>>(reinterpret_cast<const double2*>(a.spec), p.nc, p.h, p.nh, rows, p.N, p.Nk, p.L_x,
-                                      r.lgp, fx_sched(p.sh), p.tx_h, p.tx_p, fftx_factor(p, a.mu), a.ebar, a.lambda, a.mu,
+  k<<<gx, r.threads, p.x.smem_x, st>>>(reinterpret_cast<const double2*>(a.spec), p.nc, p.h, p.nh, rows, p.N, p.Nk, p.x.Lx,
+                                      r.lgp, fx_sched(p.x.sh), p.x.tw_h, p.x.tw_p, fftx_factor(p, a.mu), a.ebar, a.lambda, a.mu,
                                       a.sig64, a.msum, tiles, a.gate);
   if (launches) *launches += 1;
 }
