@@ -1051,7 +1051,7 @@ extern "C" void stz_destroy(stz_ctx* c) {
   Fields& f = c->f;
   void* ptrs[] = {f.eps0, f.sig, f.sdev, f.dF, f.dF32, f.Q0, f.Q1, f.deps, f.dnorm, f.rtab64, f.mro, f.prev_deps, f.perm_soft, f.temp_soft,
                   f.tlast, f.amark, f.part, f.gsum, f.gticket, f.lsum, f.lbnd, f.psum, f.spec, f.ktab, f.log,
-                  f.ctl, f.scratch, f.msum, c->err_dev, c->l2buf, c->qbuf, f.lam_site, f.mu_site,
+                  f.ctl, f.scratch, f.msum, c->err_dev, c->l2buf, c->qbuf, c->dispbuf, f.lam_site, f.mu_site,
                   f.inh_tau0, f.inh_eeff, f.inh_last, f.inh_part, c->exptab,
                   c->rx.cq, c->rx.dx, c->rx.dxy, c->rx.ux, c->rx.uxy, c->rx.pn};
   for (void* p : ptrs)
@@ -1278,27 +1278,27 @@ extern "C" int stz_get_field(stz_ctx* c, int32_t which, int32_t comp, double* ho
 // Displacement field of the current eigenstrain (HomogeneousStressSolver with
 // uflag 2, elastic.c:873-900; DispField, io.c:137-240, without the supercell
 // position the caller adds): one FP64 solve whose Green's pass writes
-// u_hat = -i (F - alpha G g)/(mu |k|), into a temporary buffer (print-time only).
+// u_hat = -i (F - alpha G g)/(mu |k|), into a buffer kept from the first call (a
+// driver reads it at every print; an allocation per call took 50 to 290 us more
+// at 256^2 where the allocator had no free chunk to place it in).
 extern "C" int stz_get_displacement(stz_ctx* c, double* host, int64_t count) {
   if (!c || !host) return STZ_ERR_INVALID;
   const long long N = c->kp.N;
   const int dim = c->kp.n0 > 1 ? 3 : 2;
   if (count != (int64_t)dim * N) return STZ_ERR_INVALID;
   cudaSetDevice(c->p.device);
-  double* tmp = nullptr;
-  if (dalloc(&tmp, (size_t)dim * N)) return STZ_ERR_NOMEM;
+  if (!c->dispbuf && dalloc(&c->dispbuf, (size_t)dim * N)) return STZ_ERR_NOMEM;
   SolveArgs a{};
   a.eps = c->f.eps0;
   a.lambda = c->kp.lambda;
   a.mu = c->kp.mu;
   a.out = kOutSig64;
-  a.sig64 = tmp;
+  a.sig64 = c->dispbuf;
   a.spec = c->f.spec;
   a.disp = 1;
   fft_solve(*plan_of(c), a, c->stream, &c->launches);
-  cudaMemcpyAsync(host, tmp, sizeof(double) * dim * N, cudaMemcpyDeviceToHost, c->stream);
+  cudaMemcpyAsync(host, c->dispbuf, sizeof(double) * dim * N, cudaMemcpyDeviceToHost, c->stream);
   const cudaError_t e = cudaStreamSynchronize(c->stream);
-  cudaFree(tmp);
   if (e != cudaSuccess) {
     set_error("displacement solve: %s", cudaGetErrorString(e));
     return STZ_ERR_CUDA;

@@ -1124,6 +1124,19 @@ static bool default_schedule(FFTPlan* p) {
   return plan_set_fx_tiles(p, Lx, Ly, Lg, 224 * 1024);
 }
 
+// Floating-point tiles of a plan that tunes the fixed-point passes and runs the
+// others for its displacement: fewer lines a block (two at least) where the grid
+// would leave SMs without their two blocks. 256^2 with eight lines (17 blocks
+// in Green's pass) took 296 us for a displacement, 123 with two.
+static void spread_tiles(FFTPlan* p) {
+  const long long rows = (long long)p->n0 * p->n1, columns = p->n0 > 1 ? (long long)p->n1 * p->nh : p->nh;
+  int Lx = p->L_x, Ly = p->L_y, Lg = p->L_g;
+  while (Lx > 2 && rows / Lx < 304) Lx /= 2;
+  while (Ly > 2 && (long long)p->nh * p->n0 * p->nc / Ly < 304) Ly /= 2;
+  while (Lg > 2 && columns / Lg < 304) Lg /= 2;
+  plan_set_tiles(p, Lx, Ly, Lg, 224 * 1024, false);
+}
+
 int fft_plan_create(FFTPlan* p, int n0, int n1, int n2, int nc) {
   std::memset((void*)p, 0, sizeof(*p));
   if (n2 < 2 || n2 % 2 != 0 || n1 < 1 || n0 < 1) return STZ_ERR_INVALID;
@@ -1205,6 +1218,7 @@ float time_solve(const FFTPlan& p, const SolveArgs& a, cudaStream_t st, cudaEven
 
 int fft_autotune(FFTPlan* p, cudaStream_t st, int* chosen, PassKind kind) {
   p->kind = kind;
+  if (kind == kPassFx) spread_tiles(p);
   int dev = 0;
   cudaGetDevice(&dev);
   const std::array<int, 6> key = {dev, p->n0, p->n1, p->n2, p->nc, kind};
