@@ -50,18 +50,17 @@ __device__ __forceinline__ double over_2mu(const KParams& kp, double s) {
   return isfinite(q) ? __fma_rn(__fma_rn(-q, 2.0 * kp.mu, s), kp.inv_2mu, q) : s / 2 / kp.mu;
 }
 // isotropicinv (elastic.c:522-531) in DIM dimensions, the trace's coefficient
-// from the host. The mixed form multiplies by 1/(2 mu) on its one-thread commit
-// path; the FP64 forms take the quotient. With divisions the update of a varying
-// medium, two of these per site, took 31 us of a 256^2 iteration's 105 (90 now).
+// from the host. With divisions the update of a varying medium, two of these per
+// site, took 31 us of a 256^2 iteration's 105 (90 now).
 __device__ void iso_inv(const KParams& kp, const double* s, double* e) {
   const int nd = ndiag(kp.nc);
   double tr = 0;
   for (int c = 0; c < nd; c++) tr += s[c];
   const double t = -kp.inv_lam_coef * tr;
-  for (int c = 0; c < kp.nc; c++) e[c] = (c < nd ? t : 0.0) + (kp.fast_inv ? s[c] * kp.inv_2mu : over_2mu(kp, s[c]));
+  for (int c = 0; c < kp.nc; c++) e[c] = (c < nd ? t : 0.0) + over_2mu(kp, s[c]);
 }
 // Component `lane` of the same, its s in every lane of a warp (0 beyond the
-// last).
+// last). The mixed form's steps multiply by 1/(2 mu), as its commits do.
 __device__ double iso_inv_lane(const KParams& kp, double s, int lane) {
   const double s0 = __shfl_sync(FULL, s, 0), s1 = __shfl_sync(FULL, s, 1), s2 = __shfl_sync(FULL, s, 2);
   const double t = -kp.inv_lam_coef * (kp.nc == 3 ? s0 + s1 : s0 + s1 + s2);
@@ -100,42 +99,21 @@ __device__ __forceinline__ int loaded_comp(const KParams& kp) {
   return kp.loading == STZ_LOAD_SHEAR ? shear_comp(kp) : 0;
 }
 
-// eps_avg correction from the mean stress of the solved field
-// (evolution.c:92-97, 263-300)
-__device__ void subtract_error(const KParams& kp, const Ctl* ctl, int athermal, double* tmpStrain) {
-  double ts[6] = {0, 0, 0, 0, 0, 0};
-  if (!kp.no_subtract_error) {
-    for (int c = 0; c < kp.nc; c++) ts[c] = ctl->stress[c];
-    const int zc = (athermal && kp.nc == 3) ? 0 : loaded_comp(kp);
-    ts[zc] = 0.0;
-  }
-  iso_inv(kp, ts, tmpStrain);
-}
-
-// `inv` (optional, here and below): the strain of the stress difference, formed
-// by the caller
-__device__ void hold_stress(const KParams& kp, Ctl* ctl, const double* inv = nullptr) {
-  double d[6] = {0, 0, 0, 0, 0, 0}, de[6];
-  for (int c = 0; c < kp.nc; c++) d[c] = kp.applied[c] - ctl->stress[c];
-  if (inv)
-    for (int c = 0; c < kp.nc; c++) de[c] = inv[c];
-  else iso_inv(kp, d, de);
+// holds the applied stress; inv is the strain of its difference from the mean
+// stress
+__device__ void hold_stress(const KParams& kp, Ctl* ctl, const double* inv) {
   for (int c = 0; c < kp.nc; c++) {
-    ctl->eps_avg[c] += de[c];
-    ctl->u[c] += d[c];
+    ctl->eps_avg[c] += inv[c];
+    ctl->u[c] += kp.applied[c] - ctl->stress[c];
     ctl->stress[c] = kp.applied[c];
   }
 }
 
 // loading after a thermal event (evolution.c:262-317); ctl->stress holds the
-// mean stress of the field solved right after the transformation
-__device__ void load_after_event(const KParams& kp, Ctl* ctl, double t_kmc, const double* inv = nullptr) {
-  double ts[6];
-  if (kp.loading != STZ_LOAD_STRESS) {
-    if (inv)
-      for (int c = 0; c < kp.nc; c++) ts[c] = inv[c];
-    else subtract_error(kp, ctl, 0, ts);
-  }
+// mean stress of the field solved right after the transformation, ts the strain
+// of the error to subtract (evolution.c:92-97, 263-300) or, holding a stress, of
+// the difference from it (both by k_post)
+__device__ void load_after_event(const KParams& kp, Ctl* ctl, double t_kmc, const double* ts) {
   const double rate = kp.strain_rate, nu = kp.poisson, E = kp.young, mu = kp.mu;
   const bool d2 = kp.nc == 3;
   switch (kp.loading) {
@@ -170,7 +148,7 @@ __device__ void load_after_event(const KParams& kp, Ctl* ctl, double t_kmc, cons
       break;
     }
     case STZ_LOAD_STRESS:
-      hold_stress(kp, ctl, inv);
+      hold_stress(kp, ctl, ts);
       break;
   }
 }
@@ -939,7 +917,11 @@ __device__ bool group_reduce(const KParams& kp, const Fields& f, int b, int spli
 }
 
 // ----------------------------------------------------------- selection
-// Rate of (site, mode) exactly as the main pass computed it (raw units).
+// Rate of (site, mode), raw units: in fixed point where the site's values fit, as
+// the main pass computes it with one site per thread. The pass adds the rates of
+// two or four sites before rounding, and sends a whole chunk through the FP64
+// chain for one site out of range, so a search within a chunk meets the chunk's
+// sum to a few roundings (a near tie is counted at 1e-12 of the total).
 template <int MODEL>
 __device__ __forceinline__ double site_rate(const KParams& kp, const Fields& f, const RateFx& rx, const double* u,
                                             double totime, long long s, int m) {
