@@ -963,3 +963,29 @@ def test_fixed_point_rates_under_two_large_stresses(engine_lib):
     assert eng.scalars()["astep"] == 0
     assert abs(eng.events()["total_rate"][-1] / R - 1) < 1e-12
     eng.close()
+
+
+@pytest.mark.parametrize("shape", [(3, 4, 6), (12, 32, 24)])
+@pytest.mark.parametrize("shift", [1e-9, 2e-3])
+def test_octant_update_carries_the_uniform_stress(engine_lib, shape, shift):
+    """test_octant_update_is_the_solve with the field's mean: without the
+    subtracted error and under shear the strain that loading adds after an event
+    is 2 mu of it in the uniform stress, so the whole field, moved by C: of the
+    mean strain's changes between the events, is the solve's (the same bar)."""
+    p = api.default_params(api.MODEL_GLOBAL3D)
+    p.n[0], p.n[1], p.n[2] = shape
+    p.loading, p.solver, p.seed, p.no_subtract_error = api.LOAD_SHEAR, api.SOLVER_KERNEL, 3, 1
+    p.strain_rate, p.end_strain, p.strain_increment = 5e-5, 1.0, 1e9
+    eng = api.Engine(p)
+    for i in range(12):
+        sc = eng.scalars()
+        eng.set_mean_strain([e + shift * (-1) ** i * (c + 1) for c, e in enumerate(sc["eps_avg"])])
+        eng.run(max_events=1)
+    a = [eng.field(api.FIELD_SIGMA, c) for c in range(6)]
+    eng.solve()
+    b = [eng.field(api.FIELD_SIGMA, c) for c in range(6)]
+    size = max(np.abs(v).max() for v in b)
+    assert size > 1e-2
+    for c in range(6):
+        assert np.abs(a[c] - b[c]).max() < 1e-14 * size
+    eng.close()
