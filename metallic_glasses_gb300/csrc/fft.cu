@@ -1085,7 +1085,7 @@ static bool plan_set_fx_tiles(FFTPlan* p, int Lx, int Ly, int Lg, size_t limit =
   const size_t cz = sizeof(double2);
   const int ng = p->n0 > 1 ? p->n0 : p->n1;
   const size_t rx = 2 * (size_t)Lx * fx_ld(p->h + 1) * cz + sizeof(int) * Lx, ry = 2 * (size_t)Ly * fx_ld(p->n1) * cz,
-               rg = 2 * (size_t)p->nc * Lg * fx_ld(ng) * cz + (size_t)ng * Lg;
+               rg = 2 * (size_t)p->nc * Lg * fx_ld(ng) * cz;
   if (Lx < 1 || Ly < 1 || Lg < 1 || (Ly > 1 && Ly * p->n1 > 2048)) return false;
   if (rx > limit || ry > limit || rg > limit) return false;
   FxPasses& x = p->x;
@@ -1120,7 +1120,7 @@ static bool default_schedule(FFTPlan* p) {
   p->x.eg = 2;
   Lx = std::max(1, 1024 / p->h), Ly = 8, Lg = 8;
   while (Ly > 1 && (2 * (size_t)Ly * fx_ld(p->n1) * cz > 100 * 1024 || Ly * p->n1 > 2048)) Ly /= 2;
-  while (Lg > 1 && 2 * (size_t)nc * Lg * fx_ld(ng) * cz + (size_t)ng * Lg > most) Lg /= 2;
+  while (Lg > 1 && 2 * (size_t)nc * Lg * fx_ld(ng) * cz > most) Lg /= 2;
   return plan_set_fx_tiles(p, Lx, Ly, Lg, 224 * 1024);
 }
 

@@ -20,12 +20,14 @@
 // The mean strain's uniform stress C:<eps> is added to the result in FP64
 // instead of entering the k = 0 term, which it would dominate.
 //
-// Measured, solve with host overhead: 422 -> 158 us at 64^3, 2530 -> 784 us at
-// 128^3, 250 -> 91 us at 512^2 (tuned tiles and threads on both sides); the
-// result's error against 113-bit arithmetic 8.6e-16 -> 1.8e-16 at 64^3 and
-// 9.7e-16 -> 6.3e-16 at 512^2 (relative L2, random eigenstrain). The passes are
-// bound by integer issue: about 460, 330, 700, 330 and 650 instructions per
-// complex value, of which a radix-8 stage is 36 to 71.
+// Measured, solve with host overhead: 422 -> 157 us at 64^3, 2530 -> 800 us at
+// 128^3, 250 -> 90 us at 512^2 (tuned tiles and threads on both sides). The
+// result's error against wider arithmetic (relative L2, random eigenstrain, FP64
+// passes before): 8.9e-16 -> 1.6e-16 at 64^3, 1.1e-15 -> 3.4e-16 at 512^2; below
+// FP64 passes' for sparse, smooth, banded and nearly uniform fields too. The
+// passes are bound by integer issue and their phases between barriers: about
+// 500, 300, 640, 300 and 680 instructions per complex value at 64^3, of which a
+// radix-8 stage is 36 to 71.
 #include "fftx.cuh"
 
 #include <algorithm>
@@ -619,7 +621,9 @@ __device__ __forceinline__ void green_tile(int tile, double2* __restrict__ spec,
   // the column's largest wave number: with one shift per column a field of
   // mostly uniform eigenstrain (10% of spread, 512^2) was off by 6.1e-16 of the
   // stress, and FP64 passes by 1.8e-16.
-  signed char* ex = reinterpret_cast<signed char*>(b + NC * L * ld);  // the shifts
+  // the shifts, in the buffer that is free until the inverse transform (a kilobyte
+  // of their own cost the second block per SM at lines of 1024: 288 us for 251)
+  signed char* ex = reinterpret_cast<signed char*>(res == a ? b : a);
   float ns[NC];
 #pragma unroll
   for (int c = 0; c < NC; c++) ns[c] = 0.f;

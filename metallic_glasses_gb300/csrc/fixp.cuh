@@ -4,9 +4,11 @@
 // warp instruction) and a 32 x 32 -> 64 bit integer multiply-add at 32 lanes
 // (one clock). A sum of products and an exponential whose operands are held
 // as 64-bit fixed point therefore cost a fraction of the same sum in FP64, and
-// with the scales chosen below they are more exact: the argument of a rate has
-// an absolute error below 2^-49 where an FP64 argument of size 32 to 64 is
-// rounded by 2^-48 at every operation.
+// with the scales chosen below they are more exact on average. What is cut of a
+// rate's argument (in powers of two) is the products of low halves, 2^-50 at
+// most for each of six in 3D (2^-50.3 together on average, in the mean square)
+// and 2^-47 for each of two in 2D (2^-48), where FP64 rounds an argument of size
+// 32 to 64 by 2^-48 at every operation; a single sum may come out further off.
 //
 // Host and device compile the same functions, so the tests check them on the
 // CPU against higher precision.

@@ -205,7 +205,7 @@ struct ModeSet {
   float mdev_raw[STZ_MODES][5];
 };
 
-// The constants of a 3D FP64 context's fixed-point rates (fixp.cpp).
+// The constants of an FP64 context's fixed-point rates, 3D or 2D (fixp.cpp).
 void rate_fx_constants(const KParams& kp, RateFx* x);
 
 struct BatchDesc {
@@ -226,7 +226,7 @@ struct stz_ctx {
   stz_params p{};
   stz::KParams kp{};
   stz::Fields f{};
-  stz::RateFx rx{};                  // 3D FP64 forms: constants of the fixed-point rates
+  stz::RateFx rx{};                  // FP64 forms: constants of the fixed-point rates (2D: and operands)
   stz::FxExp* exptab = nullptr;      // its exponential table on the device
   int device = 0;
   cudaStream_t stream = nullptr;
