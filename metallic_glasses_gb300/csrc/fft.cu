@@ -1080,13 +1080,17 @@ static bool plan_set_tiles(FFTPlan* p, int Lx, int Ly, int Lg, size_t limit = 20
 }
 
 // The same of the fixed-point passes (padded lines; a thread holds at most eight
-// values of a column).
+// values of a column). Row tiles of more than 9600 values of all components are
+// left out: the descent takes twice the default rows with four values a thread
+// and then misses the better small tiles with eight (128^3 815 us, 797 without
+// them; 64x128x256 785 and 758).
 static bool plan_set_fx_tiles(FFTPlan* p, int Lx, int Ly, int Lg, size_t limit = 200 * 1024) {
   const size_t cz = sizeof(double2);
   const int ng = p->n0 > 1 ? p->n0 : p->n1;
   const size_t rx = 2 * (size_t)Lx * fx_ld(p->h + 1) * cz + sizeof(int) * Lx, ry = 2 * (size_t)Ly * fx_ld(p->n1) * cz,
                rg = 2 * (size_t)p->nc * Lg * fx_ld(ng) * cz;
   if (Lx < 1 || Ly < 1 || Lg < 1 || (Ly > 1 && Ly * p->n1 > 2048)) return false;
+  if (Lx > 1 && Lx * p->h * p->nc > 9600) return false;
   if (rx > limit || ry > limit || rg > limit) return false;
   FxPasses& x = p->x;
   x.Lx = Lx;
